@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 #include <vector>
@@ -117,11 +118,47 @@ void gemm_set_trace(const optional<Tensor>& t) {
   }
 }
 
+// Which kernel runs a product: the tile width (512: the two-CTA kernel) and how many CTAs share the contraction of one tile.
+// The estimate in microseconds is launch + fill + drain of the kernel, plus, per wave of tiles, its K blocks of 64 (or the
+// epilogue of a tile, whichever is longer). The constants are measured over 40 products from 512 x 128 x 128 to
+// 32 x 4096 x 25088 (replayed back to back, B200). A K block is bound by shared-memory bandwidth: TMA writes it and the MMA
+// reads it once, so 64 / 128 / 256 columns cost 48 / 64 / 96 KB at 128 bytes per clock and narrow tiles only pay when they put
+// more SMs to work. Splitting adds the exchange through distributed shared memory; it wins wherever the tiles leave SMs idle:
+// 1024 x 1024 x 4096 29.2 -> 14.3 us (256 wide, 4 CTAs), 768 x 768 x 1792 16.2 -> 9.0, 256 x 256 x 16384 94.7 -> 14.7,
+// 640 x 1024 x 30522 172 -> 39, 32 x 4096 x 25088 179 -> 38 (5.4 TB/s). Splits run one cluster per tile, so they are only
+// considered while every cluster is resident at once.
+struct GemmChoice { int64_t bn, split; };
+GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split) {
+  struct Cost { int bn; double base, kb, epi, exchange; };
+  static const Cost costs[4] = {{64, 2.9, 0.28, 1.0, 2.6}, {128, 4.2, 0.30, 1.5, 2.6}, {256, 4.6, 0.38, 2.3, 3.5}, {512, 6.6, 0.36, 2.5, 0.0}};
+  const int64_t kbs = (K + 63) / 64, sms = num_sms();
+  GemmChoice best{64, 1};
+  double best_us = 1e30;
+  for (const Cost& c : costs) {
+    const bool pair = c.bn == 512;
+    if (pair && (!allow_pair || M < 256 || N < 256)) continue;
+    if (c.bn < 512 && c.bn > 64 && N <= c.bn / 2) continue;              // more than half of the tile would be padding
+    const int64_t tm = pair ? 256 : 128, tn = pair ? 256 : c.bn;
+    const int64_t tiles = ((M + tm - 1) / tm) * ((N + tn - 1) / tn) * batch;
+    const int64_t slots = pair ? sms / 2 : sms;
+    const double waves = (double)((tiles + slots - 1) / slots);
+    const double us = c.base + waves * std::max(c.kb * (double)kbs, c.epi);
+    if (us < best_us) { best_us = us; best = {c.bn, 1}; }
+    if (pair || !allow_split) continue;
+    for (int s = 2; s <= 8 && s <= kbs; ++s) {
+      if (tiles * s > sms || tiles > adb200::gemm_split_max_clusters(s, (int)sms)) continue;
+      const double us_s = c.base + c.kb * (double)((kbs + s - 1) / s) + c.exchange;
+      if (us_s < best_us) { best_us = us_s; best = {c.bn, s}; }
+    }
+  }
+  return best;
+}
+
 // D = alpha * A.B^T (+ epilogue). a: [.., M, K] (K-major) or [.., K, M] (a_mn); b: [.., N, K] or [.., K, N] (b_mn);
 // c: [.., M, N] bf16 or fp32 view with unit inner stride.
 void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_mn, int64_t epilogue, const optional<Tensor>& bias,
                const optional<Tensor>& c2, const optional<Tensor>& aux, double alpha, double beta, Tensor error_flag, int64_t bn,
-               const optional<Tensor>& mask, double drop_p, int64_t drop_seed, const optional<Tensor>& drop_step) {
+               const optional<Tensor>& mask, double drop_p, int64_t drop_seed, const optional<Tensor>& drop_step, int64_t split = 0) {
   const c10::cuda::CUDAGuard guard(a_.device());
   Tensor a = as4d(a_), b = as4d(b_), c = as4d(c_);
   const int M = a_mn ? a.size(3) : a.size(2), K = a_mn ? a.size(2) : a.size(3);
@@ -130,20 +167,16 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
   TORCH_CHECK(a.size(0) == b.size(0) && a.size(1) == b.size(1), "batch dimensions of A and B differ");
   TORCH_CHECK(c.size(0) == a.size(0) && c.size(1) == a.size(1) && c.size(2) == M && c.size(3) == N, "output shape mismatch");
   TORCH_CHECK(c.stride(3) == 1, "output inner stride must be 1");
-  // bn: tile width 64 / 128 / 256 of the one-CTA kernel, or 512 = the 256 x 256 tile of the two-CTA kernel; 0 picks one
-  // (two CTAs when both extents fill a pair's tile and AUTODIST_GEMM_PAIR is not 0)
+  // bn: tile width 64 / 128 / 256 of the one-CTA kernel, or 512 = the 256 x 256 tile of the two-CTA kernel; 0 picks the kernel
+  // (see choose_gemm; two CTAs only when AUTODIST_GEMM_PAIR is not 0)
   const bool softmax_epi = epilogue == adb200::EPI_SOFTMAX || epilogue == adb200::EPI_SOFTMAX_GRAD;
   static bool pair_unavailable = false;        // set when a cluster launch was refused once (see below)
   const bool auto_bn = bn <= 0;
   if (bn <= 0) {
     static const bool pair_default = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR"); return e == nullptr || e[0] != '0'; }();
-    bn = N >= 256 ? 256 : (N > 64 ? 128 : 64);
-    // pairs pay off once their 256 x 256 tiles fill the SM pairs, or when a long contraction makes the shared-memory
-    // fill per FLOP (what the pair halves for B) the limit
-    const int64_t pair_tiles = (int64_t)((M + 255) / 256) * ((N + 255) / 256) * a.size(0) * a.size(1);
-    static const int64_t pair_min_k = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR_MIN_K"); return e != nullptr ? std::atoll(e) : 2048LL; }();
-    if (pair_default && !pair_unavailable && bn == 256 && M >= 256 && !softmax_epi && (pair_tiles >= num_sms() / 2 || K >= pair_min_k))
-      bn = 512;
+    const GemmChoice g = choose_gemm(M, N, K, a.size(0) * a.size(1), pair_default && !pair_unavailable && !softmax_epi, !softmax_epi);
+    bn = g.bn;
+    split = g.split;
   }
   TORCH_CHECK(bn == 64 || bn == 128 || bn == 256 || bn == 512, "bn must be 64, 128, 256 or 512 (two-CTA tile)");
   const bool pair = bn == 512;
@@ -215,6 +248,11 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
     tmC2 = tmC;
     if (epilogue == adb200::EPI_BIAS_GELU && !make_store_map(as4d(*c2), &tmC2)) p.tma_store = 0;
   }
+  if (split > 1) {
+    const cudaError_t e = adb200::launch_gemm_split(tmA, tmB.m[0], p, (int)bn, (int)split, a_mn, b_mn, at::cuda::getCurrentCUDAStream());
+    TORCH_CHECK(e == cudaSuccess, "split GEMM launch failed: ", cudaGetErrorString(e));
+    return;
+  }
   cudaError_t e = pair ? adb200::launch_gemm_pair(tmA, tmB.m[0], p, a_mn, b_mn, num_sms(), at::cuda::getCurrentCUDAStream(),
                                                   p.tma_store ? &tmC : nullptr, p.tma_store ? &tmC2 : nullptr)
                        : adb200::launch_gemm(tmA, tmB, p, (int)bn, a_mn, b_mn, num_sms(), at::cuda::getCurrentCUDAStream(),
@@ -236,6 +274,14 @@ void gemm(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, int6
           const optional<Tensor>& c2, const optional<Tensor>& aux, double alpha, double beta, Tensor error_flag, int64_t bn) {
   TORCH_CHECK(epilogue <= adb200::EPI_BIAS_TANH, "use gemm_softmax for the softmax epilogues");
   gemm_impl(a, b, c, a_mn, b_mn, epilogue, bias, c2, aux, alpha, beta, error_flag, bn, c10::nullopt, 0.0, 0, c10::nullopt);
+}
+
+// gemm with the contraction split over `split` CTAs of a cluster (bn 64 / 128 / 256).
+void gemm_split(const Tensor& a, const Tensor& b, Tensor c, bool a_mn, bool b_mn, int64_t epilogue, const optional<Tensor>& bias,
+                const optional<Tensor>& c2, const optional<Tensor>& aux, double alpha, double beta, Tensor error_flag, int64_t bn, int64_t split) {
+  TORCH_CHECK(epilogue <= adb200::EPI_BIAS_TANH, "no softmax epilogue here");
+  TORCH_CHECK((bn == 64 || bn == 128 || bn == 256) && split >= 2 && split <= 8, "tile width 64, 128 or 256 and a split of 2 to 8 needed");
+  gemm_impl(a, b, c, a_mn, b_mn, epilogue, bias, c2, aux, alpha, beta, error_flag, bn, c10::nullopt, 0.0, 0, c10::nullopt, split);
 }
 
 // Attention products with the row softmax in the epilogue (rows of 128):
@@ -717,6 +763,7 @@ void relaxed_pull(const Tensor& p32_ptrs, Tensor master, Tensor p16, const Tenso
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_set_trace", &gemm_set_trace);
   m.def("gemm", &gemm);
+  m.def("gemm_split", &gemm_split);
   m.def("gemm_softmax", &gemm_softmax);
   m.def("gemm_gathered_b", &gemm_gathered_b);
   m.def("gemm_gathered_bt", &gemm_gathered_bt);

@@ -7,50 +7,56 @@
 namespace adb200 {
 namespace tc {
 
-// The arithmetic of the epilogue on 16 accumulator values of one row, in place: scale, then bias (+ tanh), addend or
-// GELU derivative. `ncols` of the 16 columns starting at `col0` exist (0: nothing is read from memory).
-__device__ __forceinline__ void gemm_epilogue_math16(const GemmParams& p, float* v, int col0, int ncols, long long coff, bool vec_ok) {
+// The arithmetic of the epilogue on NV (16 or 4) accumulator values of one row, in place: scale, then bias (+ tanh), addend
+// or GELU derivative. `ncols` of the NV columns starting at `col0` (a multiple of NV) exist (0: nothing is read from memory).
+template <int NV>
+__device__ __forceinline__ void gemm_epilogue_math(const GemmParams& p, float* v, int col0, int ncols, long long coff, bool vec_ok) {
 #pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
+  for (int j = 0; j < NV; ++j) v[j] *= p.alpha;
   if (p.epilogue == EPI_BIAS || p.epilogue == EPI_BIAS_GELU || p.epilogue == EPI_BIAS_TANH) {
-    if (ncols == 16 && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
+    if (ncols == NV && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
 #pragma unroll
-      for (int j = 0; j < 16; j += 4) {                      // col0 is a multiple of 16: four aligned 16-byte loads
+      for (int j = 0; j < NV; j += 4) {                      // col0 is a multiple of 4: aligned 16-byte loads
         const float4 b4 = __ldg(reinterpret_cast<const float4*>(p.bias + col0 + j));
         v[j] += b4.x; v[j + 1] += b4.y; v[j + 2] += b4.z; v[j + 3] += b4.w;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) if (j < ncols) v[j] += __ldg(p.bias + col0 + j);
+      for (int j = 0; j < NV; ++j) if (j < ncols) v[j] += __ldg(p.bias + col0 + j);
     }
     if (p.epilogue == EPI_BIAS_TANH) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = tanhf(v[j]);
+      for (int j = 0; j < NV; ++j) v[j] = tanhf(v[j]);
     }
   } else if (p.epilogue == EPI_ADD || p.epilogue == EPI_MUL_GELU_GRAD) {
     const __nv_bfloat16* aux = p.aux + coff + col0;
-    float x[16];
-    if (ncols == 16 && vec_ok) {
-      const uint4 u0 = *reinterpret_cast<const uint4*>(aux), u1 = *reinterpret_cast<const uint4*>(aux + 8);
-      const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&u0);
-      const __nv_bfloat162* h1 = reinterpret_cast<const __nv_bfloat162*>(&u1);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f0 = __bfloat1622float2(h0[j]), f1 = __bfloat1622float2(h1[j]);
-        x[2 * j] = f0.x; x[2 * j + 1] = f0.y; x[8 + 2 * j] = f1.x; x[8 + 2 * j + 1] = f1.y;
+    float x[NV];
+    if (ncols == NV && vec_ok) {
+      if constexpr (NV == 16) {
+        const uint4 u0 = *reinterpret_cast<const uint4*>(aux), u1 = *reinterpret_cast<const uint4*>(aux + 8);
+        unpack8_bf16(u0, x);
+        unpack8_bf16(u1, x + 8);
+      } else {
+        const uint2 u = *reinterpret_cast<const uint2*>(aux);
+        const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+        const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+        x[0] = f0.x; x[1] = f0.y; x[2] = f1.x; x[3] = f1.y;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) x[j] = (j < ncols) ? __bfloat162float(aux[j]) : 0.f;
+      for (int j = 0; j < NV; ++j) x[j] = (j < ncols) ? __bfloat162float(aux[j]) : 0.f;
     }
     if (p.epilogue == EPI_ADD) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] += x[j];
+      for (int j = 0; j < NV; ++j) v[j] += x[j];
     } else {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] *= gelu_tanh_grad(x[j]);
+      for (int j = 0; j < NV; ++j) v[j] *= gelu_tanh_grad(x[j]);
     }
   }
+}
+__device__ __forceinline__ void gemm_epilogue_math16(const GemmParams& p, float* v, int col0, int ncols, long long coff, bool vec_ok) {
+  gemm_epilogue_math<16>(p, v, col0, ncols, coff, vec_ok);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------

@@ -53,4 +53,11 @@ cudaError_t launch_gemm(const CUtensorMap& tmA, const TmapArray& tmB, const Gemm
 cudaError_t launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, bool a_mn, bool b_mn, int num_sms,
                              cudaStream_t stream, const CUtensorMap* tmC = nullptr, const CUtensorMap* tmC2 = nullptr);
 
+// The same product with the contraction split over the `split` (2..8) CTAs of a cluster that share one output tile
+// (gemm_split.cu). Maps as for launch_gemm. No fused softmax, no row-sharded B; needs at least `split` K blocks of 64.
+cudaError_t launch_gemm_split(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int bn, int split, bool a_mn, bool b_mn,
+                              cudaStream_t stream);
+// Clusters of `split` such CTAs that the GPU holds at once (0: clusters of that size cannot be scheduled).
+int gemm_split_max_clusters(int split, int num_sms);
+
 }  // namespace adb200

@@ -307,13 +307,13 @@ class BertPretrainer(nn.Module):
         seq = x
         # next-sentence head
         cls = seq.view(B, S, H)[:, 0]                                                   # [B, H] strided view
-        gm(cls, w16["pooler.w"], ws["pooled"], epi=EPI_BIAS_TANH, bias=w32["pooler.b"], bn=128)
-        gm(ws["pooled"], w16["nsp.w"], ws["nsp_logits"][:, :2], epi=EPI_BIAS, bias=w32["nsp.b"], bn=64)
+        gm(cls, w16["pooler.w"], ws["pooled"], epi=EPI_BIAS_TANH, bias=w32["pooler.b"])
+        gm(ws["pooled"], w16["nsp.w"], ws["nsp_logits"][:, :2], epi=EPI_BIAS, bias=w32["nsp.b"])
         E.xent(ws["nsp_logits"], nsp_labels.reshape(-1), None, ws["one"], ws["loss"], 2, 1.0 / B, False, 0.0)
         # masked-LM head
         torch.add(mlm_positions, torch.arange(B, device=ids.device)[:, None] * S, out=ws["flat_pos"].view(B, P))
         E.gather_rows(seq, ws["flat_pos"], ws["xm"])
-        gm(ws["xm"], w16["mlm.dense_w"], ws["hm_u"], epi=EPI_BIAS_GELU, bias=w32["mlm.dense_b"], c2=ws["hm"], bn=128)
+        gm(ws["xm"], w16["mlm.dense_w"], ws["hm_u"], epi=EPI_BIAS_GELU, bias=w32["mlm.dense_b"], c2=ws["hm"])
         E.ln_fwd(ws["hm"], None, w32["mlm.ln_g"], w32["mlm.ln_b"], None, ws["hl"], ws["mm"], ws["mr"], eps, 0.0, 0, None)
         dec = "emb.word" if c.tie_word_embeddings else "mlm.decoder_w"
         gm(ws["hl"], w16[dec], ws["logits"][:, :V], epi=EPI_BIAS, bias=w32["mlm.bias"])
@@ -361,13 +361,13 @@ class BertPretrainer(nn.Module):
         # next-sentence head
         dn = ws["nsp_logits"][:, :2]
         g["nsp.b"].copy_(dn.float().sum(0))
-        gm(dn, ws["pooled"], g["nsp.w"], a_mn=True, b_mn=True, bn=128)
-        gm(dn, w16["nsp.w"], ws["d_pooled"], b_mn=True, bn=128)
+        gm(dn, ws["pooled"], g["nsp.w"], a_mn=True, b_mn=True)
+        gm(dn, w16["nsp.w"], ws["d_pooled"], b_mn=True)
         E.tanh_bwd(ws["d_pooled"], ws["pooled"], ws["d_pre"])
         g["pooler.b"].copy_(ws["d_pre"].float().sum(0))
-        gm(ws["d_pre"], cls, g["pooler.w"], a_mn=True, b_mn=True, bn=128)
+        gm(ws["d_pre"], cls, g["pooler.w"], a_mn=True, b_mn=True)
         d_cls = d_seq.view(B, S, H)[:, 0]
-        gm(ws["d_pre"], w16["pooler.w"], d_cls, b_mn=True, epi=EPI_ADD, aux=d_cls, bn=128)
+        gm(ws["d_pre"], w16["pooler.w"], d_cls, b_mn=True, epi=EPI_ADD, aux=d_cls)
         ready(fl.offsets["pooler.w"], fl.total)
 
         d_out = d_seq
