@@ -601,6 +601,19 @@ void pad_image8(const Tensor& x, Tensor xp, int64_t pad) {
   adb200::pad_image8(x.data_ptr(), x.scalar_type() == at::kFloat ? 1 : 0, x.stride(0), x.stride(1), x.stride(2), x.stride(3), x.size(0),
                      x.size(1), x.size(2), x.size(3), BF(xp), xp.size(1), xp.size(2), (int)pad, STREAM);
 }
+// y = relu?(x * scale + shift (+ res)) over a channels-last matrix [rows, C] with the running statistics (evaluation mode).
+void bn_eval(const Tensor& x, const optional<Tensor>& res, Tensor y, const Tensor& gamma, const Tensor& beta, const Tensor& mean,
+             const Tensor& var, double eps, bool relu) {
+  const int C = x.size(-1), rows = x.numel() / C;
+  TORCH_CHECK(C % 8 == 0 && C <= 4096 && x.is_contiguous() && x.scalar_type() == at::kBFloat16 && y.is_contiguous() && y.numel() == x.numel(),
+              "x and y must be contiguous bf16 [.., C], C % 8 == 0, C <= 4096");
+  if (res.has_value()) TORCH_CHECK(res->is_contiguous() && res->numel() == x.numel() && res->scalar_type() == at::kBFloat16, "residual must match x");
+  for (const Tensor& t : {gamma, beta, mean, var})
+    TORCH_CHECK(t.scalar_type() == at::kFloat && t.numel() == C && t.is_contiguous(), "batch-norm parameters must be fp32 [C]");
+  if (x.numel() == 0) return;
+  adb200::bn_eval(CBF(x), OPT_BF(res), BF(y), gamma.data_ptr<float>(), beta.data_ptr<float>(), mean.data_ptr<float>(), var.data_ptr<float>(),
+                  (float)eps, rows, C, relu ? 1 : 0, STREAM);
+}
 // Bias gradient of a convolution over channels-last dy [.., C]: out (fp32 [C]) = column sums of dy, or of dy masked by y > 0
 // when the convolution had a fused ReLU, in which case the masked gradient is also written to dx. accumulate: out += sums.
 void relu_bwd_colsum(const Tensor& dy, const optional<Tensor>& y, const optional<Tensor>& dx, Tensor out, bool accumulate) {
@@ -820,3 +833,4 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.attr("MAX_COMM_BLOCKS") = adb200::kMaxCommBlocks;
   register_conv(m);
 }
+  m.def("bn_eval", &bn_eval);

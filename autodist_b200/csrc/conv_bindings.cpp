@@ -196,9 +196,33 @@ int split_k(int base_tiles, long long patches) {
   return ks;
 }
 
+// Evaluation-mode batch-norm (and residual) fused behind a forward convolution.
+struct EvalNorm {
+  const Tensor *gamma, *beta, *mean, *var;
+  double eps;
+  const optional<Tensor>* residual;
+};
+
+void set_eval_norm(adb200::ConvParams& p, const EvalNorm* n, const Tensor& y, int Cout) {
+  if (n == nullptr) return;
+  for (const Tensor* t : {n->gamma, n->beta, n->mean, n->var})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->numel() == Cout && t->is_contiguous(), "batch-norm parameters must be fp32 [Cout]");
+  TORCH_CHECK(Cout <= adb200::kMaxStatChannels, "fused batch-norm needs Cout <= 2048");
+  p.mode = adb200::CONV_EVAL;
+  p.bn_gamma = n->gamma->data_ptr<float>(); p.bn_beta = n->beta->data_ptr<float>();
+  p.bn_mean = n->mean->data_ptr<float>(); p.bn_var = n->var->data_ptr<float>();
+  p.bn_eps = (float)n->eps;
+  if (n->residual->has_value()) {
+    const Tensor& r = n->residual->value();
+    check_act(r, "residual");
+    TORCH_CHECK(r.sizes() == y.sizes() && r.data_ptr() != y.data_ptr(), "residual must have the output's shape and its own storage");
+    p.addend = reinterpret_cast<const __nv_bfloat16*>(r.data_ptr());
+  }
+}
+
 // y = conv(x, w) (+ bias) (ReLU); stats (optional, fp32 [2, Cout], zeroed by the caller) receives per-channel sum / sum of squares of y.
-void conv_fprop(const Tensor& x, const Tensor& w, Tensor y, const optional<Tensor>& bias, bool relu, const optional<Tensor>& stats,
-                int64_t stride, int64_t pad, Tensor error_flag) {
+void conv_fprop_impl(const Tensor& x, const Tensor& w, Tensor y, const optional<Tensor>& bias, bool relu, const optional<Tensor>& stats,
+                     int64_t stride, int64_t pad, Tensor error_flag, const EvalNorm* norm) {
   const c10::cuda::CUDAGuard guard(x.device());
   check_act(x, "x"); check_act(y, "y");
   const Geometry g = geometry(x, w, y, stride, pad);
@@ -229,8 +253,22 @@ void conv_fprop(const Tensor& x, const Tensor& w, Tensor y, const optional<Tenso
                 "stats must be fp32 [2, Cout] with Cout <= 2048");
     p.stats = stats->data_ptr<float>();
   }
+  set_eval_norm(p, norm, y, g.Cout);
   p.error_flag = error_flag.data_ptr<int>();
   launch(maps, p, bn);
+}
+
+void conv_fprop(const Tensor& x, const Tensor& w, Tensor y, const optional<Tensor>& bias, bool relu, const optional<Tensor>& stats,
+                int64_t stride, int64_t pad, Tensor error_flag) {
+  conv_fprop_impl(x, w, y, bias, relu, stats, stride, pad, error_flag, nullptr);
+}
+
+// y = relu?(batch_norm(conv(x, w) (+ bias)) (+ residual)) with running statistics (evaluation mode).
+void conv_fprop_bn_eval(const Tensor& x, const Tensor& w, Tensor y, const optional<Tensor>& bias, bool relu, const Tensor& gamma,
+                        const Tensor& beta, const Tensor& mean, const Tensor& var, double eps, const optional<Tensor>& residual, int64_t stride,
+                        int64_t pad, Tensor error_flag) {
+  const EvalNorm n{&gamma, &beta, &mean, &var, eps, &residual};
+  conv_fprop_impl(x, w, y, bias, relu, c10::nullopt, stride, pad, error_flag, &n);
 }
 
 // dx = the input gradient of conv(x, w) given dy. Every element of dx is written.
@@ -388,8 +426,8 @@ void check_rowtap(const Tensor& xp, int64_t KH, int64_t stride, int OH, int OW) 
               "padded image too small for this output size");
 }
 
-void conv_rowtap_fprop(const Tensor& xp, const Tensor& wr, Tensor y, const optional<Tensor>& bias, bool relu, const optional<Tensor>& stats,
-                       int64_t stride, Tensor error_flag) {
+void conv_rowtap_fprop_impl(const Tensor& xp, const Tensor& wr, Tensor y, const optional<Tensor>& bias, bool relu, const optional<Tensor>& stats,
+                            int64_t stride, Tensor error_flag, const EvalNorm* norm) {
   const c10::cuda::CUDAGuard guard(xp.device());
   check_act(y, "y");
   const int N = y.size(0), OH = y.size(1), OW = y.size(2), Cout = y.size(3);
@@ -425,8 +463,21 @@ void conv_rowtap_fprop(const Tensor& xp, const Tensor& wr, Tensor y, const optio
     TORCH_CHECK(stats->scalar_type() == at::kFloat && stats->numel() == 2 * Cout && stats->is_contiguous(), "stats must be fp32 [2, Cout]");
     p.stats = stats->data_ptr<float>();
   }
+  set_eval_norm(p, norm, y, Cout);
   p.error_flag = error_flag.data_ptr<int>();
   launch(maps, p, bn);
+}
+
+void conv_rowtap_fprop(const Tensor& xp, const Tensor& wr, Tensor y, const optional<Tensor>& bias, bool relu, const optional<Tensor>& stats,
+                       int64_t stride, Tensor error_flag) {
+  conv_rowtap_fprop_impl(xp, wr, y, bias, relu, stats, stride, error_flag, nullptr);
+}
+
+void conv_rowtap_fprop_bn_eval(const Tensor& xp, const Tensor& wr, Tensor y, const optional<Tensor>& bias, bool relu, const Tensor& gamma,
+                               const Tensor& beta, const Tensor& mean, const Tensor& var, double eps, const optional<Tensor>& residual,
+                               int64_t stride, Tensor error_flag) {
+  const EvalNorm n{&gamma, &beta, &mean, &var, eps, &residual};
+  conv_rowtap_fprop_impl(xp, wr, y, bias, relu, c10::nullopt, stride, error_flag, &n);
 }
 
 void conv_rowtap_wgrad(const Tensor& dy, const Tensor& xp, Tensor dwr, int64_t stride, Tensor error_flag) {
@@ -468,6 +519,8 @@ void conv_rowtap_wgrad(const Tensor& dy, const Tensor& xp, Tensor dwr, int64_t s
 void register_conv(pybind11::module& m) {
   m.def("conv_set_trace", &conv_set_trace);
   m.def("conv_fprop", &conv_fprop);
+  m.def("conv_fprop_bn_eval", &conv_fprop_bn_eval);
+  m.def("conv_rowtap_fprop_bn_eval", &conv_rowtap_fprop_bn_eval);
   namespace py = pybind11;
   m.def("conv_dgrad", &conv_dgrad, py::arg("dy"), py::arg("w"), py::arg("dx"), py::arg("stride"), py::arg("pad"), py::arg("error_flag"),
         py::arg("addend") = py::none());

@@ -6,8 +6,9 @@
 //                            the image = the padding) and one box of the weight, 128-byte swizzle, ring of stages
 //   warp 1    MMA issuer     tcgen05.mma 128 x BN x 16, bf16 -> fp32 in TMEM, two accumulator buffers
 //   warps 2-5 epilogue       tcgen05.ld, then
-//                              forward:         + bias, ReLU, per-channel sum / sum of squares (batch-norm statistics,
-//                                               reduced in shared memory across the CTA's tiles), bf16 store
+//                              forward:         + bias, evaluation-mode batch-norm, residual, ReLU, per-channel sum / sum of
+//                                               squares (batch-norm statistics, reduced in shared memory across the
+//                                               CTA's tiles), bf16 store
 //                              input gradient:  bf16 store (strided positions for a strided convolution)
 //                              weight gradient: fp32 store or vector atomic add (split-K)
 //
@@ -36,7 +37,7 @@ template <int BN, int MODE> struct ConvCfg {
   static constexpr int EPI_WARPS = 8;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int CHUNKS = BN / 16 / (EPI_WARPS / 4);      // 16-column chunks per epilogue warp
-  static constexpr int STAT_BYTES = (MODE == CONV_FPROP) ? 2 * kMaxStatChannels * 4 : 0;
+  static constexpr int STAT_BYTES = (MODE == CONV_FPROP || MODE == CONV_EVAL) ? 2 * kMaxStatChannels * 4 : 0;
   static constexpr int SMEM = STAGES * (A_BYTES + B_BYTES) + 1024 /*align*/ + 256 /*barriers*/ + STAT_BYTES;
 };
 
@@ -102,7 +103,9 @@ __global__ void __launch_bounds__(ConvCfg<BN, MODE>::THREADS, 1)
 conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvParams p) {
   using C = ConvCfg<BN, MODE>;
   constexpr bool A_MN = MODE == CONV_WGRAD;
-  constexpr bool B_MN = MODE != CONV_FPROP;
+  constexpr bool FWD = MODE == CONV_FPROP || MODE == CONV_EVAL;
+  constexpr bool EVAL = MODE == CONV_EVAL;
+  constexpr bool B_MN = !FWD;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
@@ -173,7 +176,7 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
                 for (int j = 0; j < p.tw; ++j)
                   tma_load_4d(a_dst + j * col_rows * 128, mapA, &full[stage], (tc_.w0 + j) * p.xstep, tc_.h0 + tap.dh, tc_.n0, 0);
               }
-              if (MODE == CONV_FPROP) {
+              if (FWD) {
                 tma_load_4d(b_dst, &maps.w, &full[stage], cb * BK, tap.wtap, tc_.c0, 0);
               } else {
 #pragma unroll
@@ -274,6 +277,27 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
     const int c_lo = ((warp - 2) >> 2) * C::CHUNKS;      // first 16-column chunk of this warp's share of the tile
     int as = 0; uint32_t aphase = 0; bool ok = true;
     const int r = q * 32 + lane;
+    if (EVAL) {
+      // y = conv * scale + shift with the layer's running statistics: the per-channel table is built once per CTA while the
+      // first tile is multiplied (the statistics table's space; the two never occur together)
+      for (int c = threadIdx.x - 64; c < p.Nc; c += C::THREADS - 64) {
+        const float sc = p.bn_gamma[c] * rsqrtf(p.bn_var[c] + p.bn_eps);
+        s_stat[c] = sc;
+        s_stat[p.Nc + c] = fmaf(-p.bn_mean[c], sc, p.bn_beta[c]);
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(C::THREADS - 64) : "memory");
+    }
+    // bias and evaluation-mode batch-norm of 16 forward outputs starting at column col0
+    auto affine16 = [&](float* v, int col0) {
+      if (p.bias != nullptr) {
+#pragma unroll
+        for (int jj = 0; jj < 16; ++jj) if (col0 + jj < p.Nc) v[jj] += __ldg(p.bias + col0 + jj);
+      }
+      if (EVAL) {
+#pragma unroll
+        for (int jj = 0; jj < 16; ++jj) if (col0 + jj < p.Nc) v[jj] = fmaf(v[jj], s_stat[col0 + jj], s_stat[p.Nc + col0 + jj]);
+      }
+    };
     for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
       const TileCoord tc_ = decode_tile<BN, MODE>(p, t);
       if (MODE == CONV_WGRAD && tc_.kend <= tc_.kbeg) continue;
@@ -292,9 +316,10 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
         off = (long long)row * p.ldc + (long long)p.taps[tc_.tap].wtap * p.wtap_stride;
       }
       const long long tw0 = trace != nullptr ? clock64() : 0;
-      if (MODE == CONV_DGRAD) {
+      if (MODE == CONV_DGRAD || EVAL) {
         if (p.addend != nullptr) {
-          // The gradient another consumer of the same tensor produced (a residual fork) is added to this tile. Its whole
+          // The gradient another consumer of the same tensor produced (a residual fork), or the residual of an evaluated
+          // block, is added to this tile. Its whole
           // row segment is requested before the wait for the accumulator, so the loads overlap the tile's MMAs, and
           // the chunk loop below is unrolled so that the prefetched vectors stay in registers.
           uint4 pre[2 * C::CHUNKS];
@@ -317,8 +342,12 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
               tmem_ld16(t_row + (c_lo + c) * 16, v);
               unpack8_bf16(pre[2 * c], a);
               unpack8_bf16(pre[2 * c + 1], a + 8);
+              if (EVAL) affine16(v, col0);
 #pragma unroll
-              for (int jj = 0; jj < 16; ++jj) v[jj] += a[jj];
+              for (int jj = 0; jj < 16; ++jj) {
+                v[jj] += a[jj];
+                if (EVAL && p.relu) v[jj] = v[jj] < 0.f ? 0.f : v[jj];
+              }
               if (valid) {
                 __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + off + col0;
                 store8_bf16(dst, v);                                  // Nc is a multiple of 8: a chunk holds 8 or 16 columns
@@ -366,12 +395,12 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
             }
           }
         } else {
-          if (MODE == CONV_FPROP) {
-            if (p.bias != nullptr) {
+          if (FWD) {
+            affine16(v, col0);
+            if (p.relu && EVAL) {                  // like the library's evaluation path: a NaN stays a NaN
 #pragma unroll
-              for (int jj = 0; jj < 16; ++jj) if (col0 + jj < p.Nc) v[jj] += __ldg(p.bias + col0 + jj);
-            }
-            if (p.relu) {
+              for (int jj = 0; jj < 16; ++jj) v[jj] = v[jj] < 0.f ? 0.f : v[jj];
+            } else if (p.relu) {
 #pragma unroll
               for (int jj = 0; jj < 16; ++jj) v[jj] = fmaxf(v[jj], 0.f);
             }
@@ -461,12 +490,14 @@ cudaError_t launch_one(const ConvMaps& maps, const ConvParams& p, int num_sms, c
 cudaError_t launch_conv(const ConvMaps& maps, const ConvParams& p, int bn, int num_sms, cudaStream_t stream) {
   if (p.tw * p.th * p.tn > BM || p.ntaps < 1 || p.ntaps > kMaxConvTaps) return cudaErrorInvalidValue;
   if (p.mode == CONV_WGRAD && (p.tw * p.th * p.tn != BK || p.ksplit < 1)) return cudaErrorInvalidValue;
-  if (p.mode == CONV_FPROP && p.stats != nullptr && p.Nc > kMaxStatChannels) return cudaErrorInvalidValue;
+  if ((p.mode == CONV_EVAL || (p.mode == CONV_FPROP && p.stats != nullptr)) && p.Nc > kMaxStatChannels) return cudaErrorInvalidValue;
+  if ((p.mode == CONV_EVAL) != (p.bn_mean != nullptr) || (p.mode == CONV_EVAL && p.stats != nullptr)) return cudaErrorInvalidValue;
 #define ADB_CONV_DISPATCH(BN_)                                                                      \
   if (bn == BN_) {                                                                                  \
     if (p.mode == CONV_FPROP) return launch_one<BN_, CONV_FPROP>(maps, p, num_sms, stream);          \
     if (p.mode == CONV_DGRAD) return launch_one<BN_, CONV_DGRAD>(maps, p, num_sms, stream);          \
     if (p.mode == CONV_WGRAD) return launch_one<BN_, CONV_WGRAD>(maps, p, num_sms, stream);          \
+    if (p.mode == CONV_EVAL) return launch_one<BN_, CONV_EVAL>(maps, p, num_sms, stream);            \
   }
   ADB_CONV_DISPATCH(256)
   ADB_CONV_DISPATCH(128)

@@ -6,7 +6,9 @@
 
 namespace adb200 {
 
-enum ConvMode { CONV_FPROP = 0, CONV_DGRAD = 1, CONV_WGRAD = 2 };
+// CONV_EVAL: the forward product with an evaluation-mode batch-norm (and residual) in its epilogue - a mode of its own so that
+// the training kernel keeps its registers
+enum ConvMode { CONV_FPROP = 0, CONV_DGRAD = 1, CONV_WGRAD = 2, CONV_EVAL = 3 };
 
 constexpr int kMaxConvTaps = 49;      // 7 x 7
 constexpr int kMaxStatChannels = 2048;
@@ -46,6 +48,11 @@ struct ConvParams {
   int accumulate;                 // weight gradient: add into `out` (atomics) instead of overwriting it
   const float* bias;              // forward: per output channel, or null
   int relu;                       // forward: clamp at zero after the bias
+  const float* bn_mean;           // CONV_EVAL: running statistics and affine parameters of the batch-norm that follows (after
+  const float* bn_var;            //   the bias, before addend and ReLU); [Nc] each
+  const float* bn_gamma;
+  const float* bn_beta;
+  float bn_eps;
   float* stats;                   // forward: [2, Nc] fp32, per-channel sum and sum of squares are added here, or null
   const __nv_bfloat16* addend;    // pixel modes: tensor of the output's shape added to the result before it is stored, or null
   int* error_flag;

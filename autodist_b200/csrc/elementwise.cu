@@ -1136,6 +1136,37 @@ __global__ void __launch_bounds__(256, 6) bn_apply_kernel(const bf16* __restrict
   }
 }
 
+// Evaluation mode: y = relu?(x * scale + shift) from the running statistics, one pass (the library takes three kernels: the
+// inverse deviation, the normalisation and the ReLU). HBM-bound; the coefficient table costs C rsqrt per block as above.
+// Dynamic shared memory: 2 * C floats.
+__global__ void __launch_bounds__(256, 6) bn_eval_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, bf16* __restrict__ y,
+                                                         long long total8, int C, int relu, const float* __restrict__ gamma,
+                                                         const float* __restrict__ beta, const float* __restrict__ mean,
+                                                         const float* __restrict__ var, float eps) {
+  pdl_sync();
+  extern __shared__ float s_coef[];
+  for (int c = threadIdx.x; c < C; c += blockDim.x) {
+    const float sc = gamma[c] * rsqrtf(var[c] + eps);
+    s_coef[c] = sc;
+    s_coef[C + c] = fmaf(-mean[c], sc, beta[c]);
+  }
+  __syncthreads();
+  const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 2
+  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total8; idx += stride) {
+    const int c = (int)(idx % (C / 8)) * 8;
+    float v[8], rv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    load8(x + idx * 8, v);
+    if (res != nullptr) load8(res + idx * 8, rv);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float o = fmaf(v[j], s_coef[c + j], s_coef[C + c + j]) + rv[j];
+      v[j] = relu && o < 0.f ? 0.f : o;                    // a NaN stays a NaN
+    }
+    store8(y + idx * 8, v);
+  }
+}
+
 // Backward statistics and coefficients in one launch. Each block adds its sums over a chunk of rows into one of kBnSlots
 // shared rows of partials: part[y % kBnSlots][0][c] += sum dy', part[..][1][c] += sum dy' * xhat, dy' = dy masked by the
 // ReLU (y > 0). The last block of a 64-channel group to finish (a ticket counter per group) adds the slots up, clears them
@@ -1694,6 +1725,14 @@ void bn_fwd(const bf16* x, const float* gamma, const float* beta, const bf16* re
   launch_pdl(bn_apply_kernel, dim3((int)(blocks < 1 ? 1 : blocks)), dim3(256), 2 * C * sizeof(float), st, x, res, y, total8, C, relu, sums, gamma, beta, 1.0f / rows,
                                                                                       eps, mean, rstd, run_mean, run_var, batches, momentum, unbias);
   (void)coef;
+}
+void bn_eval(const bf16* x, const bf16* res, bf16* y, const float* gamma, const float* beta, const float* mean, const float* var, float eps,
+             int rows, int C, int relu, cudaStream_t st) {
+  const long long total8 = (long long)rows * (C / 8);
+  long long blocks = (total8 + 256 * 4 - 1) / (256 * 4);
+  if (blocks > 148 * 6) blocks = 148 * 6;
+  launch_pdl(bn_eval_kernel, dim3((int)(blocks < 1 ? 1 : blocks)), dim3(256), 2 * C * sizeof(float), st, x, res, y, total8, C, relu, gamma, beta, mean,
+             var, eps);
 }
 void bn_bwd(const bf16* dy, const bf16* x, const bf16* y, const float* mean, const float* rstd, const float* gamma, bf16* dx, bf16* dres,
             float* part, float* sums, float* coef, int rows, int C, int relu, float* dgamma_acc, float* dbeta_acc, cudaStream_t st) {

@@ -16,7 +16,7 @@ import torch
 from torch import nn
 import torch.nn.functional as F
 
-from autodist_b200.ops.functional import Linear, batch_norm, conv2d, fork, max_pool2d
+from autodist_b200.ops.functional import Linear, batch_norm, batch_norm_eval, conv2d, conv_bn_eval, fork, max_pool2d
 
 CONV_MODE = os.environ.get("AUTODIST_CONV", "own")                      # own | library
 
@@ -54,8 +54,8 @@ def _conv(cin, cout, k, stride=1, padding=0, bias=False, relu=False):
 class BatchNormAct(nn.BatchNorm2d):
     """Batch-norm with an optional fused residual add and ReLU. For bf16 activations on a GPU (the autocast training path)
     the training-mode statistics, the normalisation (+ add + ReLU), the running-statistics update and both backward passes
-    run on the hand-written kernels; fp32 activations, evaluation mode and channel counts that are not a multiple of 8 use
-    the library. ``AUTODIST_NORM_POOL=library`` forces the library everywhere, ``=own`` the kernels for fp32 inputs too."""
+    run on the hand-written kernels, and so does evaluation mode where no gradient is recorded; fp32 activations, evaluation
+    mode with gradients and channel counts that are not a multiple of 8 use the library. ``AUTODIST_NORM_POOL=library`` forces the library everywhere, ``=own`` the kernels for fp32 inputs too."""
 
     def __init__(self, channels, relu=False):
         super().__init__(channels)
@@ -65,6 +65,10 @@ class BatchNormAct(nn.BatchNorm2d):
         if _own_norm_pool(x) and self.training and self.momentum is not None:
             return batch_norm(x, self.weight, self.bias, self.running_mean, self.running_var, True, self.momentum, self.eps, self.relu,
                               residual, sums, self.num_batches_tracked, fork)
+        if not self.training and NORM_POOL_MODE != "library":
+            y = batch_norm_eval(x, self.weight, self.bias, self.running_mean, self.running_var, self.eps, self.relu, residual)
+            if y is not None:
+                return y
         y = super().forward(x)
         if residual is not None:
             y = y + residual
@@ -96,9 +100,16 @@ class _StatsArena:
 _ARENA = _StatsArena()
 
 
+def _hooked(*modules):
+    """Whether a forward hook watches one of ``modules`` (their outputs must then exist on their own)."""
+    m = nn.modules.module
+    return bool(m._global_forward_hooks or m._global_forward_pre_hooks) or any(x._forward_hooks or x._forward_pre_hooks for x in modules)
+
+
 class ConvBN(nn.Module):
     """Convolution followed by batch-norm (+ residual add, + ReLU). On the kernel path the convolution's epilogue already
-    accumulates the per-channel sums the batch-norm needs, so the normalisation reads the activation once."""
+    accumulates the per-channel sums the batch-norm needs, so the normalisation reads the activation once; in evaluation mode
+    without gradients the whole chain is the convolution's epilogue."""
 
     def __init__(self, cin, cout, k, stride=1, padding=0, relu=True):
         super().__init__()
@@ -108,6 +119,13 @@ class ConvBN(nn.Module):
     def forward(self, x, residual=None, in_fork=None, res_fork=None):
         """``in_fork`` / ``res_fork``: the ``GradFork`` of ``x`` / of ``residual`` when that tensor has a second consumer."""
         cout = self.conv.out_channels
+        if not self.bn.training and x.is_cuda and CONV_MODE != "library" and NORM_POOL_MODE != "library" and not _hooked(self.conv, self.bn) \
+                and not self.conv.relu and type(self.bn) is BatchNormAct:
+            bn = self.bn
+            y = conv_bn_eval(x, self.conv.weight, self.conv.bias, self.conv.stride, self.conv.padding, bn.weight, bn.bias, bn.running_mean,
+                             bn.running_var, bn.eps, bn.relu, residual)
+            if y is not None:
+                return y
         fused = x.is_cuda and x.dim() == 4 and CONV_MODE != "library" and NORM_POOL_MODE != "library" and FUSE_BN_STATS and self.training \
             and self.bn.momentum is not None and cout % 8 == 0 and cout <= 2048 and (x.dtype == torch.bfloat16 or torch.is_autocast_enabled())
         if fused:

@@ -353,9 +353,7 @@ def conv2d(x, weight, bias=None, stride=1, padding=0, relu=False, stats=None, fo
     or ``Cin <= 8`` with ``KW <= 8`` (the first layer of an image network, whose input is padded to 8 channels). ``stats``
     (fp32 ``[2, Cout]``, zeroed by the caller) receives the per-channel sum and sum of squares of the output. Other shapes
     and CPU tensors use the library convolution."""
-    cout, kh, kw, cin = weight.shape
-    own = x.is_cuda and cout % 8 == 0 and stride in (1, 2) and kh * kw <= 49 and (cin % 8 == 0 or (cin <= 8 and kw <= 8))
-    if own:
+    if _own_conv(x, weight, stride):
         return _ConvFn.apply(x, weight, bias, int(stride), int(padding), bool(relu), stats, fork)
     y = F.conv2d(x, weight.permute(0, 3, 1, 2).to(x.dtype), None if bias is None else bias.to(x.dtype), stride, padding)
     y = F.relu(y) if relu else y
@@ -365,6 +363,89 @@ def conv2d(x, weight, bias=None, stride=1, padding=0, relu=False, stats=None, fo
             stats[0] += yf.sum((0, 2, 3))
             stats[1] += (yf * yf).sum((0, 2, 3))
     return y
+
+
+def _own_conv(x, weight, stride):
+    """Whether the implicit-GEMM kernels take a convolution of ``x`` with a ``[Cout, KH, KW, Cin]`` weight."""
+    cout, kh, kw, cin = weight.shape
+    return x.is_cuda and cout % 8 == 0 and stride in (1, 2) and kh * kw <= 49 and (cin % 8 == 0 or (cin <= 8 and kw <= 8))
+
+
+def _eval_norm_ready(gamma, beta, mean, var, channels):
+    """fp32 affine parameters and running statistics of ``channels`` entries each, as the evaluation kernels read them."""
+    return all(t is not None and t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() == channels
+               for t in (gamma, beta, mean, var))
+
+
+class _ConvBNEvalFn(torch.autograd.Function):
+    """Evaluation-mode ``relu?(batch_norm(conv(x)) + residual)`` as one kernel. Only called where no gradient is recorded; being
+    an autograd function keeps transforms that it does not support (forward-mode derivatives, vmap) refused."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias, stride, padding, gamma, beta, mean, var, eps, relu, residual):
+        E = ops.ext(required=True)
+        cout, kh, kw, cin = weight.shape
+        err = _error_flag(x.device)
+        b32 = bias.float().contiguous() if bias is not None else None
+        w16 = _bf16_weight(weight)
+        res = _nhwc(residual) if residual is not None else None
+        if cin % 8 != 0:
+            n, _, h, w = x.shape
+            oh, ow, hp, wp = _rowtap_geometry(h, w, kh, kw, stride, padding)
+            xh = torch.empty(n, hp, wp, 8, dtype=torch.bfloat16, device=x.device)
+            E.pad_image8(x, xh, padding)
+            wr = F.pad(F.pad(w16, (0, 8 - cin)).reshape(cout, kh, kw * 8), (0, 64 - kw * 8)).contiguous()
+            y = torch.empty(n, oh, ow, cout, dtype=torch.bfloat16, device=x.device)
+            E.conv_rowtap_fprop_bn_eval(xh, wr, y, b32, relu, gamma, beta, mean, var, eps, res, stride, err)
+        else:
+            xh = _nhwc(x)
+            n, h, w, _ = xh.shape
+            oh, ow = (h + 2 * padding - kh) // stride + 1, (w + 2 * padding - kw) // stride + 1
+            y = torch.empty(n, oh, ow, cout, dtype=torch.bfloat16, device=x.device)
+            E.conv_fprop_bn_eval(xh, w16, y, b32, relu, gamma, beta, mean, var, eps, res, stride, padding, err)
+        return y.permute(0, 3, 1, 2)
+
+    @staticmethod
+    def backward(ctx, dy):
+        raise RuntimeError("the fused evaluation path records no gradient")
+
+
+def conv_bn_eval(x, weight, bias, stride, padding, gamma, beta, running_mean, running_var, eps, relu=False, residual=None):
+    """``relu?(batch_norm(conv2d(x, weight, bias)) + residual)`` with the running statistics, in one kernel, or ``None`` where
+    that kernel does not apply (a gradient is recorded, CPU tensors, shapes or types it does not take)."""
+    cout, kh, kw, _ = weight.shape
+    if torch.is_grad_enabled() or x.dim() != 4 or not _own_conv(x, weight, stride) or cout > 2048 or \
+            not _eval_norm_ready(gamma, beta, running_mean, running_var, cout):
+        return None
+    if residual is not None:
+        oh, ow = (x.shape[2] + 2 * padding - kh) // stride + 1, (x.shape[3] + 2 * padding - kw) // stride + 1
+        if residual.dtype != torch.bfloat16 or tuple(residual.shape) != (x.shape[0], cout, oh, ow) or not residual.is_cuda:
+            return None
+    return _ConvBNEvalFn.apply(x, weight, bias, int(stride), int(padding), gamma, beta, running_mean, running_var, eps, bool(relu), residual)
+
+
+class _BNEvalFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, gamma, beta, mean, var, eps, relu, residual):
+        xh = _nhwc(x)
+        y = torch.empty_like(xh)
+        ops.ext(required=True).bn_eval(xh, _nhwc(residual) if residual is not None else None, y, gamma, beta, mean, var, eps, relu)
+        return y.permute(0, 3, 1, 2)
+
+    @staticmethod
+    def backward(ctx, dy):
+        raise RuntimeError("the fused evaluation path records no gradient")
+
+
+def batch_norm_eval(x, gamma, beta, running_mean, running_var, eps, relu=False, residual=None):
+    """``relu?(batch_norm(x) + residual)`` of a bf16 tensor with the running statistics, in one kernel, or ``None`` where that
+    kernel does not apply."""
+    if torch.is_grad_enabled() or not x.is_cuda or x.dim() != 4 or x.dtype != torch.bfloat16 or x.shape[1] % 8 or x.shape[1] > 4096 or \
+            not _eval_norm_ready(gamma, beta, running_mean, running_var, x.shape[1]):
+        return None
+    if residual is not None and (residual.dtype != torch.bfloat16 or residual.shape != x.shape or not residual.is_cuda):
+        return None
+    return _BNEvalFn.apply(x, gamma, beta, running_mean, running_var, eps, bool(relu), residual)
 
 
 class _BatchNormFn(torch.autograd.Function):
