@@ -517,10 +517,10 @@ void lstm_cell_bwd(const Tensor& gates, const Tensor& c_prev, const Tensor& c, c
 void sumsq(const Tensor& x, Tensor acc, double weight) { adb200::sumsq(x.data_ptr<float>(), x.numel(), acc.data_ptr<float>(), (float)weight, STREAM); }
 void clip_scale(Tensor x, const Tensor& acc, double max_norm) { adb200::clip_scale(x.data_ptr<float>(), x.numel(), acc.data_ptr<float>(), (float)max_norm, STREAM); }
 // Batch-norm over a channels-last matrix x [rows, C] (training mode statistics), optional residual addend and fused ReLU:
-// y = relu?(bn(x) + res). `sums` (optional, fp32 [2, C]) holds sum x and sum x^2 already (from the convolution's epilogue).
+// y = relu?(bn(x) + res). `keep` (uint8, one byte per 8 channels) receives which outputs a fused ReLU let through. `sums` (optional, fp32 [2, C]) holds sum x and sum x^2 already (from the convolution's epilogue).
 void bn_fwd(const Tensor& x, const Tensor& gamma, const Tensor& beta, const optional<Tensor>& res, Tensor y, Tensor mean, Tensor rstd,
             double eps, bool relu, const optional<Tensor>& sums_in, const optional<Tensor>& run_mean, const optional<Tensor>& run_var,
-            const optional<Tensor>& batches, double momentum) {
+            const optional<Tensor>& batches, double momentum, const optional<Tensor>& keep) {
   const int C = x.size(-1), rows = x.numel() / C;
   float* rm = nullptr; float* rv = nullptr; long long* nb = nullptr;
   if (run_mean.has_value()) {
@@ -533,26 +533,46 @@ void bn_fwd(const Tensor& x, const Tensor& gamma, const Tensor& beta, const opti
   TORCH_CHECK(y.is_contiguous() && y.numel() == x.numel() && mean.numel() == C && rstd.numel() == C && gamma.numel() == C && beta.numel() == C,
               "output and per-channel tensors must match x");
   if (res.has_value()) TORCH_CHECK(res->is_contiguous() && res->numel() == x.numel() && res->scalar_type() == at::kBFloat16, "residual must match x");
+  uint8_t* kp = nullptr;
+  if (keep.has_value()) {
+    TORCH_CHECK(keep->scalar_type() == at::kByte && keep->is_contiguous() && keep->numel() * 8 == x.numel(), "keep must hold one byte per 8 elements");
+    kp = keep->data_ptr<uint8_t>();
+  }
   if (sums_in.has_value()) {
     TORCH_CHECK(sums_in->scalar_type() == at::kFloat && sums_in->numel() == 2 * C && sums_in->is_contiguous(), "sums must be fp32 [2, C]");
-    adb200::bn_fwd(CBF(x), gamma.data_ptr<float>(), beta.data_ptr<float>(), OPT_BF(res), BF(y), mean.data_ptr<float>(), rstd.data_ptr<float>(),
-                   nullptr, sums_in->data_ptr<float>(), nullptr, rows, C, (float)eps, relu ? 1 : 0, 1, rm, rv, nb, (float)momentum, STREAM);
+    adb200::bn_fwd(CBF(x), gamma.data_ptr<float>(), beta.data_ptr<float>(), OPT_BF(res), BF(y), kp, mean.data_ptr<float>(),
+                   rstd.data_ptr<float>(), nullptr, sums_in->data_ptr<float>(), rows, C, (float)eps, relu ? 1 : 0, 1, rm, rv, nb, (float)momentum, STREAM);
     return;
   }
   Tensor part = at::empty({(int64_t)adb200::bn_parts(rows, C) * 2 * C}, x.options().dtype(at::kFloat));
   Tensor sums = at::empty({2 * C}, x.options().dtype(at::kFloat));
-  adb200::bn_fwd(CBF(x), gamma.data_ptr<float>(), beta.data_ptr<float>(), OPT_BF(res), BF(y), mean.data_ptr<float>(), rstd.data_ptr<float>(),
-                 part.data_ptr<float>(), sums.data_ptr<float>(), nullptr, rows, C, (float)eps, relu ? 1 : 0, 0, rm, rv, nb, (float)momentum,
+  adb200::bn_fwd(CBF(x), gamma.data_ptr<float>(), beta.data_ptr<float>(), OPT_BF(res), BF(y), kp, mean.data_ptr<float>(), rstd.data_ptr<float>(),
+                 part.data_ptr<float>(), sums.data_ptr<float>(), rows, C, (float)eps, relu ? 1 : 0, 0, rm, rv, nb, (float)momentum,
                  STREAM);
+}
+// y = relu?(x * scale + shift (+ res)) over a channels-last matrix [rows, C] with the running statistics (evaluation mode).
+void bn_eval(const Tensor& x, const optional<Tensor>& res, Tensor y, const Tensor& gamma, const Tensor& beta, const Tensor& mean,
+             const Tensor& var, double eps, bool relu) {
+  const int C = x.size(-1), rows = x.numel() / C;
+  TORCH_CHECK(C % 8 == 0 && C <= 4096 && x.is_contiguous() && x.scalar_type() == at::kBFloat16 && y.is_contiguous() && y.numel() == x.numel(),
+              "x and y must be contiguous bf16 [.., C], C % 8 == 0, C <= 4096");
+  if (res.has_value()) TORCH_CHECK(res->is_contiguous() && res->numel() == x.numel() && res->scalar_type() == at::kBFloat16, "residual must match x");
+  for (const Tensor& t : {gamma, beta, mean, var})
+    TORCH_CHECK(t.scalar_type() == at::kFloat && t.numel() == C && t.is_contiguous(), "batch-norm parameters must be fp32 [C]");
+  if (x.numel() == 0) return;
+  adb200::bn_eval(CBF(x), OPT_BF(res), BF(y), gamma.data_ptr<float>(), beta.data_ptr<float>(), mean.data_ptr<float>(), var.data_ptr<float>(),
+                  (float)eps, rows, C, relu ? 1 : 0, STREAM);
 }
 // Returns [dbeta, dgamma] stacked as a [2, C] fp32 tensor; writes dx and (optional) dres = dy masked by the ReLU.
 // dgamma_acc / dbeta_acc (optional, fp32 [C]): the batch-norm parameters' gradient buffers; the sums are added into them.
-Tensor bn_bwd(const Tensor& dy, const Tensor& x, const Tensor& y, const Tensor& mean, const Tensor& rstd, const Tensor& gamma, Tensor dx,
+Tensor bn_bwd(const Tensor& dy, const Tensor& x, const optional<Tensor>& keep, const Tensor& mean, const Tensor& rstd, const Tensor& gamma, Tensor dx,
               const optional<Tensor>& dres, bool relu, const optional<Tensor>& dgamma_acc, const optional<Tensor>& dbeta_acc) {
   const int C = x.size(-1), rows = x.numel() / C;
   TORCH_CHECK(C % 8 == 0 && C <= 16384 && x.is_contiguous() && dy.is_contiguous() && dx.is_contiguous() && dy.numel() == x.numel() && dx.numel() == x.numel(),
               "dy, x, dx must be contiguous bf16 [.., C] of one shape, C % 8 == 0");
   if (dres.has_value()) TORCH_CHECK(dres->is_contiguous() && dres->numel() == x.numel() && dres->scalar_type() == at::kBFloat16, "dres must match x");
+  TORCH_CHECK(!relu || (keep.has_value() && keep->scalar_type() == at::kByte && keep->is_contiguous() && keep->numel() * 8 == x.numel()),
+              "the forward pass's keep bytes are needed with a fused ReLU");
   // partial sums: a per-device scratch that the kernels keep zero between calls (they add into it and clear what they read);
   // batch-norm backward calls of one device are issued on one stream
   static std::unordered_map<int, Tensor> scratch;
@@ -560,7 +580,7 @@ Tensor bn_bwd(const Tensor& dy, const Tensor& x, const Tensor& y, const Tensor& 
   if (!part.defined() || part.numel() < adb200::bn_bwd_part_floats(C))
     part = at::zeros({(int64_t)adb200::bn_bwd_part_floats(std::max(C, 4096))}, x.options().dtype(at::kFloat));
   Tensor sums = at::empty({5, C}, x.options().dtype(at::kFloat));              // [dbeta, dgamma, A, B, K]
-  adb200::bn_bwd(CBF(dy), CBF(x), CBF(y), mean.data_ptr<float>(), rstd.data_ptr<float>(), gamma.data_ptr<float>(), BF(dx), OPT_BF(dres),
+  adb200::bn_bwd(CBF(dy), CBF(x), relu ? keep->data_ptr<uint8_t>() : nullptr, mean.data_ptr<float>(), rstd.data_ptr<float>(), gamma.data_ptr<float>(), BF(dx), OPT_BF(dres),
                  part.data_ptr<float>(), sums.data_ptr<float>(), sums.data_ptr<float>() + 2 * C, rows, C, relu ? 1 : 0, OPT_F(dgamma_acc),
                  OPT_F(dbeta_acc), STREAM);
   return sums.narrow(0, 0, 2);
@@ -600,19 +620,6 @@ void pad_image8(const Tensor& x, Tensor xp, int64_t pad) {
               xp.size(1) >= x.size(2) + pad && xp.size(2) >= x.size(3) + pad, "xp must be contiguous bf16 [N, Hp, Wp, 8]");
   adb200::pad_image8(x.data_ptr(), x.scalar_type() == at::kFloat ? 1 : 0, x.stride(0), x.stride(1), x.stride(2), x.stride(3), x.size(0),
                      x.size(1), x.size(2), x.size(3), BF(xp), xp.size(1), xp.size(2), (int)pad, STREAM);
-}
-// y = relu?(x * scale + shift (+ res)) over a channels-last matrix [rows, C] with the running statistics (evaluation mode).
-void bn_eval(const Tensor& x, const optional<Tensor>& res, Tensor y, const Tensor& gamma, const Tensor& beta, const Tensor& mean,
-             const Tensor& var, double eps, bool relu) {
-  const int C = x.size(-1), rows = x.numel() / C;
-  TORCH_CHECK(C % 8 == 0 && C <= 4096 && x.is_contiguous() && x.scalar_type() == at::kBFloat16 && y.is_contiguous() && y.numel() == x.numel(),
-              "x and y must be contiguous bf16 [.., C], C % 8 == 0, C <= 4096");
-  if (res.has_value()) TORCH_CHECK(res->is_contiguous() && res->numel() == x.numel() && res->scalar_type() == at::kBFloat16, "residual must match x");
-  for (const Tensor& t : {gamma, beta, mean, var})
-    TORCH_CHECK(t.scalar_type() == at::kFloat && t.numel() == C && t.is_contiguous(), "batch-norm parameters must be fp32 [C]");
-  if (x.numel() == 0) return;
-  adb200::bn_eval(CBF(x), OPT_BF(res), BF(y), gamma.data_ptr<float>(), beta.data_ptr<float>(), mean.data_ptr<float>(), var.data_ptr<float>(),
-                  (float)eps, rows, C, relu ? 1 : 0, STREAM);
 }
 // Bias gradient of a convolution over channels-last dy [.., C]: out (fp32 [C]) = column sums of dy, or of dy masked by y > 0
 // when the convolution had a fused ReLU, in which case the masked gradient is also written to dx. accumulate: out += sums.
@@ -805,6 +812,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("flagged_rows_update", &flagged_rows_update);
   m.def("cast_f32_bf16", &cast_f32_bf16);
   m.def("bn_fwd", &bn_fwd);
+  m.def("bn_eval", &bn_eval);
   m.def("bn_bwd", &bn_bwd);
   m.def("maxpool_fwd", &maxpool_fwd);
   m.def("maxpool_bwd", &maxpool_bwd);
@@ -833,4 +841,3 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.attr("MAX_COMM_BLOCKS") = adb200::kMaxCommBlocks;
   register_conv(m);
 }
-  m.def("bn_eval", &bn_eval);

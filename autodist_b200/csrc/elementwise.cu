@@ -1079,60 +1079,115 @@ __global__ void relu_bwd_colsum_kernel(const bf16* __restrict__ dy, const bf16* 
   }
 }
 
-// y = relu?(x * scale + shift (+ res)) with scale / shift derived from the per-channel sums (sum x, sum x^2): every block
-// first builds the table for all C channels in shared memory (C rsqrt per block instead of one per element), block 0 also
-// records mean / rstd and folds the batch statistics into the running ones - one launch for the whole normalisation.
-// Dynamic shared memory: 2 * C floats.
-__global__ void __launch_bounds__(256, 6) bn_apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, bf16* __restrict__ y, long long total8, int C,
-                                int relu, const float* __restrict__ sums, const float* __restrict__ gamma, const float* __restrict__ beta,
-                                float inv_rows, float eps, float* __restrict__ mean, float* __restrict__ rstd, float* __restrict__ run_mean,
-                                float* __restrict__ run_var, long long* __restrict__ batches, float momentum, float unbias) {
-  pdl_sync();
-  extern __shared__ float s_coef[];                 // [scale (C), shift (C)]
-  // the first elements are requested before the table is built, so that the table's latency hides under them
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  uint4 xq = make_uint4(0, 0, 0, 0), rq = make_uint4(0, 0, 0, 0);
-  if (idx < total8) {
-    xq = *reinterpret_cast<const uint4*>(x + idx * 8);
-    if (res != nullptr) rq = *reinterpret_cast<const uint4*>(res + idx * 8);
+// Row-walking layout of the batch-norm passes: a thread keeps one group of 8 channels (its coefficients stay in registers, so a
+// row costs nothing but its own 16-byte loads and stores) and walks rows, kBnUnroll of them in flight; consecutive threads
+// hold consecutive channel groups, so a block reads whole rows. grid.y covers C > 2048.
+constexpr int kBnThreads = 256;
+constexpr int kBnUnroll = 4;
+
+struct BnWalk {
+  int c;                 // first channel of this thread
+  long long row, step;   // first row, rows between two rows of this thread
+  bool live;
+};
+__device__ __forceinline__ BnWalk bn_walk(int C) {
+  const int c8 = C / 8, tpr = c8 < kBnThreads ? c8 : kBnThreads, rpb = kBnThreads / tpr;
+  const int rl = threadIdx.x / tpr, g = blockIdx.y * kBnThreads + threadIdx.x % tpr;
+  return {g * 8, (long long)blockIdx.x * rpb + rl, (long long)gridDim.x * rpb, rl < rpb && g < c8};
+}
+__device__ __forceinline__ void load_f8(const float* p, float* v) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) {          // parameters may start anywhere in their storage
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = p[j];
+    return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0 && batches != nullptr) *batches += 1;
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    const float mu = sums[c] * inv_rows;
-    const float var = fmaxf(sums[C + c] * inv_rows - mu * mu, 0.f);
-    const float rs = rsqrtf(var + eps);
-    const float sc = gamma[c] * rs;
-    s_coef[c] = sc;
-    s_coef[C + c] = beta[c] - mu * sc;
-    if (blockIdx.x == 0) {
-      mean[c] = mu;
-      rstd[c] = rs;
-      if (run_mean != nullptr) {
-        run_mean[c] = (1.0f - momentum) * run_mean[c] + momentum * mu;
-        run_var[c] = (1.0f - momentum) * run_var[c] + momentum * var * unbias;
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// y = relu?(x * scale + shift (+ res)) with scale / shift derived from the per-channel sums (sum x, sum x^2); the first row's
+// threads also record mean / rstd and fold the batch statistics into the running ones - one launch for the whole
+// normalisation. `keep` (with relu) receives one byte per 8 channels, bit j: y_j > 0, which is all the backward passes need of y:
+// they read 1/16 of the bytes.
+__global__ void __launch_bounds__(kBnThreads, 3) bn_apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, bf16* __restrict__ y,
+                                uint8_t* __restrict__ keep, long long rows, int C, int relu, const float* __restrict__ sums,
+                                const float* __restrict__ gamma, const float* __restrict__ beta, float inv_rows, float eps,
+                                float* __restrict__ mean, float* __restrict__ rstd, float* __restrict__ run_mean, float* __restrict__ run_var,
+                                long long* __restrict__ batches, float momentum, float unbias) {
+  pdl_sync();
+  const BnWalk w = bn_walk(C);
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && batches != nullptr) *batches += 1;
+  if (!w.live) return;
+  const int c = w.c;
+  long long row = w.row;
+  // the first rows are requested before the coefficients, so that their latency hides under them
+  uint4 xq[kBnUnroll], rq[kBnUnroll];
+#pragma unroll
+  for (int u = 0; u < kBnUnroll; ++u) {
+    const long long r = row + u * w.step;
+    xq[u] = rq[u] = make_uint4(0, 0, 0, 0);
+    if (r < rows) {
+      xq[u] = *reinterpret_cast<const uint4*>(x + r * C + c);
+      if (res != nullptr) rq[u] = *reinterpret_cast<const uint4*>(res + r * C + c);
+    }
+  }
+  float sc[8], sh[8];
+  {
+    float s1[8], s2[8], ga[8], be[8];
+    load_f8(sums + c, s1); load_f8(sums + C + c, s2); load_f8(gamma + c, ga); load_f8(beta + c, be);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float mu = s1[j] * inv_rows;
+      const float var = fmaxf(s2[j] * inv_rows - mu * mu, 0.f);
+      const float rs = rsqrtf(var + eps);
+      sc[j] = ga[j] * rs;
+      sh[j] = be[j] - mu * sc[j];
+      if (row == 0) {
+        mean[c + j] = mu;
+        rstd[c + j] = rs;
+        if (run_mean != nullptr) {
+          run_mean[c + j] = (1.0f - momentum) * run_mean[c + j] + momentum * mu;
+          run_var[c + j] = (1.0f - momentum) * run_var[c + j] + momentum * var * unbias;
+        }
       }
     }
   }
-  __syncthreads();
-  while (idx < total8) {
-    const long long next = idx + stride;
-    uint4 xn = make_uint4(0, 0, 0, 0), rn = make_uint4(0, 0, 0, 0);
-    if (next < total8) {
-      xn = *reinterpret_cast<const uint4*>(x + next * 8);
-      if (res != nullptr) rn = *reinterpret_cast<const uint4*>(res + next * 8);
-    }
-    const int c = (int)(idx % (C / 8)) * 8;
-    float v[8], rv[8];
-    unpack8(xq, v);
-    unpack8(rq, rv);
+  while (row < rows) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float o = fmaf(v[j], s_coef[c + j], s_coef[C + c + j]) + rv[j];
-      v[j] = relu ? fmaxf(o, 0.f) : o;
+    for (int u = 0; u < kBnUnroll; ++u) {
+      const long long r = row + u * w.step;
+      if (r >= rows) break;
+      float v[8], rv[8];
+      unpack8(xq[u], v);
+      unpack8(rq[u], rv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float o = fmaf(v[j], sc[j], sh[j]) + rv[j];
+        v[j] = relu ? fmaxf(o, 0.f) : o;
+      }
+      uint4 q;
+      __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+      *reinterpret_cast<uint4*>(y + r * C + c) = q;
+      if (keep != nullptr) {
+        const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
+        uint32_t bits = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)                       // y >= 0 here: positive means any bit below the sign
+          bits |= ((wd[j] & 0x7fffu) != 0 ? 1u : 0u) << (2 * j) | ((wd[j] & 0x7fff0000u) != 0 ? 2u : 0u) << (2 * j);
+        keep[(r * C + c) >> 3] = (uint8_t)bits;
+      }
     }
-    store8(y + idx * 8, v);
-    idx = next; xq = xn; rq = rn;
+    row += kBnUnroll * w.step;
+#pragma unroll
+    for (int u = 0; u < kBnUnroll; ++u) {
+      const long long r = row + u * w.step;
+      if (r < rows) {
+        xq[u] = *reinterpret_cast<const uint4*>(x + r * C + c);
+        if (res != nullptr) rq[u] = *reinterpret_cast<const uint4*>(res + r * C + c);
+      }
+    }
   }
 }
 
@@ -1169,7 +1224,7 @@ __global__ void __launch_bounds__(256, 6) bn_eval_kernel(const bf16* __restrict_
 
 // Backward statistics and coefficients in one launch. Each block adds its sums over a chunk of rows into one of kBnSlots
 // shared rows of partials: part[y % kBnSlots][0][c] += sum dy', part[..][1][c] += sum dy' * xhat, dy' = dy masked by the
-// ReLU (y > 0). The last block of a 64-channel group to finish (a ticket counter per group) adds the slots up, clears them
+// ReLU (the forward pass's `keep` bytes, see bn_apply_kernel). The last block of a 64-channel group to finish (a ticket counter per group) adds the slots up, clears them
 // and its counter, and writes what the second pass needs:
 //   dx = gamma * rstd * (dy' - dbeta / M - xhat * dgamma / M) = A * dy' + B * x + K per channel; coef = [A (C), B (C), K (C)]
 // together with sums = [dbeta (C), dgamma (C)], which are also added into dbeta_acc / dgamma_acc (the parameters'
@@ -1178,7 +1233,7 @@ __global__ void __launch_bounds__(256, 6) bn_eval_kernel(const bf16* __restrict_
 constexpr int kBnSlots = 16;
 constexpr int kBnCounterFloats = 256;          // ticket counters in front of the slots: one per 64 channels, C <= 16384
 
-__global__ void __launch_bounds__(256, 4) bn_bwd_stats_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ y,
+__global__ void __launch_bounds__(256, 4) bn_bwd_stats_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const uint8_t* __restrict__ keep,
                                     const float* __restrict__ mean, const float* __restrict__ rstd, const float* __restrict__ gamma,
                                     unsigned int* __restrict__ counters, float* __restrict__ part, float* __restrict__ sums,
                                     float* __restrict__ coef, float* __restrict__ dgamma_acc, float* __restrict__ dbeta_acc,
@@ -1192,28 +1247,28 @@ __global__ void __launch_bounds__(256, 4) bn_bwd_stats_kernel(const bf16* __rest
   // a = sum dy', b = sum dy' * x; sum dy' * xhat = rstd * (b - mean * a) is formed once per block from the totals
   float a[8] = {0, 0, 0, 0, 0, 0, 0, 0}, b[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (c < C) {
-    for (int r = r0 + rl; r < r1; r += 64) {
-      uint4 dq[2], xq[2], yq[2];
+    for (int r = r0 + rl; r < r1; r += 128) {
+      uint4 dq[4], xq[4];
+      uint32_t kq[4];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
+      for (int u = 0; u < 4; ++u) {
         const int rr = r + 32 * u;
         dq[u] = xq[u] = make_uint4(0, 0, 0, 0);
-        yq[u] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);      // bf16 ones: keeps the gradient
+        kq[u] = 0xffu;
         if (rr < r1) {
           dq[u] = *reinterpret_cast<const uint4*>(dy + (long long)rr * C + c);
           xq[u] = *reinterpret_cast<const uint4*>(x + (long long)rr * C + c);
-          if (relu) yq[u] = *reinterpret_cast<const uint4*>(y + (long long)rr * C + c);
+          if (relu) kq[u] = keep[((long long)rr * C + c) >> 3];
         }
       }
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        float d[8], xv[8], yv[8];
+      for (int u = 0; u < 4; ++u) {
+        float d[8], xv[8];
         unpack8(dq[u], d);
         unpack8(xq[u], xv);
-        unpack8(yq[u], yv);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const float g = yv[i] <= 0.f ? 0.f : d[i];
+          const float g = (kq[u] >> i) & 1u ? d[i] : 0.f;
           a[i] += g;
           b[i] = fmaf(g, xv[i], b[i]);
         }
@@ -1263,36 +1318,45 @@ __global__ void __launch_bounds__(256, 4) bn_bwd_stats_kernel(const bf16* __rest
   if (threadIdx.x == 0) counters[blockIdx.x] = 0u;
 }
 
-__global__ void bn_bwd_apply_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ y,
-                                    const float* __restrict__ coef, bf16* __restrict__ dx, bf16* __restrict__ dres, long long total8, int C,
-                                    int relu) {
+__global__ void __launch_bounds__(kBnThreads, 3) bn_bwd_apply_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
+                                    const uint8_t* __restrict__ keep, const float* __restrict__ coef, bf16* __restrict__ dx,
+                                    bf16* __restrict__ dres, long long rows, int C, int relu) {
   pdl_sync();
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= total8) return;
-  const int c = (int)(idx % (C / 8)) * 8;
-  float d[8], xv[8], yv[8];
-  load8(dy + idx * 8, d);
-  load8(x + idx * 8, xv);
-  if (relu) load8(y + idx * 8, yv);
-  float ca[8], cb[8], ck[8];                          // per-channel coefficients, six 16-byte loads
+  const BnWalk w = bn_walk(C);
+  if (!w.live) return;
+  const int c = w.c;
+  float ca[8], cb[8], ck[8];
+  load_f8(coef + c, ca); load_f8(coef + C + c, cb); load_f8(coef + 2 * C + c, ck);
+  for (long long row = w.row; row < rows; row += kBnUnroll * w.step) {
+    uint4 dq[kBnUnroll], xq[kBnUnroll];
+    uint32_t kq[kBnUnroll];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const float4 a4 = *reinterpret_cast<const float4*>(coef + c + 4 * h);
-    const float4 b4 = *reinterpret_cast<const float4*>(coef + C + c + 4 * h);
-    const float4 k4 = *reinterpret_cast<const float4*>(coef + 2 * C + c + 4 * h);
-    ca[4 * h] = a4.x; ca[4 * h + 1] = a4.y; ca[4 * h + 2] = a4.z; ca[4 * h + 3] = a4.w;
-    cb[4 * h] = b4.x; cb[4 * h + 1] = b4.y; cb[4 * h + 2] = b4.z; cb[4 * h + 3] = b4.w;
-    ck[4 * h] = k4.x; ck[4 * h + 1] = k4.y; ck[4 * h + 2] = k4.z; ck[4 * h + 3] = k4.w;
-  }
-  float gm[8];
+    for (int u = 0; u < kBnUnroll; ++u) {
+      const long long r = row + u * w.step;
+      kq[u] = 0xffu;
+      if (r < rows) {
+        dq[u] = *reinterpret_cast<const uint4*>(dy + r * C + c);
+        xq[u] = *reinterpret_cast<const uint4*>(x + r * C + c);
+        if (relu) kq[u] = keep[(r * C + c) >> 3];
+      }
+    }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float g = (relu && yv[j] <= 0.f) ? 0.f : d[j];
-    gm[j] = g;
-    d[j] = fmaf(ca[j], g, fmaf(cb[j], xv[j], ck[j]));
+    for (int u = 0; u < kBnUnroll; ++u) {
+      const long long r = row + u * w.step;
+      if (r >= rows) break;
+      float d[8], xv[8], gm[8];
+      unpack8(dq[u], d);
+      unpack8(xq[u], xv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float g = (kq[u] >> j) & 1u ? d[j] : 0.f;
+        gm[j] = g;
+        d[j] = fmaf(ca[j], g, fmaf(cb[j], xv[j], ck[j]));
+      }
+      store8(dx + r * C + c, d);
+      if (dres != nullptr) store8(dres + r * C + c, gm);    // gradient of the residual branch: dy masked by the ReLU
+    }
   }
-  store8(dx + idx * 8, d);
-  if (dres != nullptr) store8(dres + idx * 8, gm);      // gradient of the residual branch: dy masked by the ReLU
 }
 
 // Max pooling over [N, H, W, C] windows (k x k, stride, pad). The forward pass records, per output element, which
@@ -1706,25 +1770,29 @@ int bn_parts(int rows, int C) {
   if (parts > 512) parts = 512;
   return parts < 1 ? 1 : parts;
 }
-// part: [bn_parts, 2, C]; sums: [2, C]; coef: [2, C] (forward) or [3, C] (backward)
+// part: [bn_parts, 2, C]; sums: [2, C]; coef (backward): [3, C]
 // sums_given: `sums` already holds the per-channel sum and sum of squares (the convolution's epilogue produced them); the
 // whole normalisation is then one launch.
-void bn_fwd(const bf16* x, const float* gamma, const float* beta, const bf16* res, bf16* y, float* mean, float* rstd, float* part, float* sums,
-            float* coef, int rows, int C, float eps, int relu, int sums_given, float* run_mean, float* run_var, long long* batches,
+// One wave of resident blocks (three per SM) unless that leaves a thread fewer than kBnUnroll rows.
+dim3 bn_grid(long long rows, int C) {
+  const int c8 = C / 8, tpr = c8 < kBnThreads ? c8 : kBnThreads, rpb = kBnThreads / tpr, gy = (c8 + kBnThreads - 1) / kBnThreads;
+  long long blocks = (rows + (long long)rpb * kBnUnroll - 1) / ((long long)rpb * kBnUnroll);
+  const long long cap = (148 * 3 + gy - 1) / gy;
+  if (blocks > cap) blocks = cap;
+  return dim3((unsigned)(blocks < 1 ? 1 : blocks), (unsigned)gy);
+}
+// keep (optional, [rows, C / 8] bytes): which outputs are positive, for the backward pass of a fused ReLU
+void bn_fwd(const bf16* x, const float* gamma, const float* beta, const bf16* res, bf16* y, uint8_t* keep, float* mean, float* rstd, float* part,
+            float* sums, int rows, int C, float eps, int relu, int sums_given, float* run_mean, float* run_var, long long* batches,
             float momentum, cudaStream_t st) {
-  const long long total8 = (long long)rows * (C / 8);
   const float unbias = rows > 1 ? (float)rows / (float)(rows - 1) : 1.0f;
   if (!sums_given) {
     const int parts = bn_parts(rows, C), rpb = (rows + parts - 1) / parts;
     launch_pdl(bn_stats_kernel, dim3(dim3(blocks_for(C, 64), parts)), dim3(256), 0, st, x, part, rows, C, rpb);
     launch_pdl(colsum_f32_kernel, dim3(blocks_for(2 * C, 32)), dim3(256), 0, st, part, sums, parts, 2 * C, 0);
   }
-  // a few elements per thread: the per-block table of 2 * C coefficients is amortised over at least 4 x 2048 elements
-  long long blocks = (total8 + 256 * 4 - 1) / (256 * 4);
-  if (blocks > 148 * 6) blocks = 148 * 6;          // one resident wave (6 blocks of 256 threads per SM)
-  launch_pdl(bn_apply_kernel, dim3((int)(blocks < 1 ? 1 : blocks)), dim3(256), 2 * C * sizeof(float), st, x, res, y, total8, C, relu, sums, gamma, beta, 1.0f / rows,
-                                                                                      eps, mean, rstd, run_mean, run_var, batches, momentum, unbias);
-  (void)coef;
+  launch_pdl(bn_apply_kernel, bn_grid(rows, C), dim3(kBnThreads), 0, st, x, res, y, relu ? keep : nullptr, (long long)rows, C, relu, sums, gamma, beta,
+             1.0f / rows, eps, mean, rstd, run_mean, run_var, batches, momentum, unbias);
 }
 void bn_eval(const bf16* x, const bf16* res, bf16* y, const float* gamma, const float* beta, const float* mean, const float* var, float eps,
              int rows, int C, int relu, cudaStream_t st) {
@@ -1734,14 +1802,13 @@ void bn_eval(const bf16* x, const bf16* res, bf16* y, const float* gamma, const 
   launch_pdl(bn_eval_kernel, dim3((int)(blocks < 1 ? 1 : blocks)), dim3(256), 2 * C * sizeof(float), st, x, res, y, total8, C, relu, gamma, beta, mean,
              var, eps);
 }
-void bn_bwd(const bf16* dy, const bf16* x, const bf16* y, const float* mean, const float* rstd, const float* gamma, bf16* dx, bf16* dres,
+void bn_bwd(const bf16* dy, const bf16* x, const uint8_t* keep, const float* mean, const float* rstd, const float* gamma, bf16* dx, bf16* dres,
             float* part, float* sums, float* coef, int rows, int C, int relu, float* dgamma_acc, float* dbeta_acc, cudaStream_t st) {
   const int parts = bn_parts(rows, C), rpb = (rows + parts - 1) / parts;
-  launch_pdl(bn_bwd_stats_kernel, dim3(dim3(blocks_for(C, 64), parts)), dim3(256), 0, st, dy, x, y, mean, rstd, gamma, reinterpret_cast<unsigned int*>(part),
+  launch_pdl(bn_bwd_stats_kernel, dim3(dim3(blocks_for(C, 64), parts)), dim3(256), 0, st, dy, x, keep, mean, rstd, gamma, reinterpret_cast<unsigned int*>(part),
                                                                       part + kBnCounterFloats, sums, coef, dgamma_acc, dbeta_acc, rows, C, rpb,
                                                                       relu, 1.0f / rows);
-  const long long total8 = (long long)rows * (C / 8);
-  launch_pdl(bn_bwd_apply_kernel, dim3(blocks_for(total8, 256)), dim3(256), 0, st, dy, x, y, coef, dx, dres, total8, C, relu);
+  launch_pdl(bn_bwd_apply_kernel, bn_grid(rows, C), dim3(kBnThreads), 0, st, dy, x, keep, coef, dx, dres, (long long)rows, C, relu);
 }
 // dx = relu'(y) * dy (skipped when y is null) and out[c] (+)= column sums of dx. part: [bn_parts(rows, C), C] floats.
 void relu_bwd_colsum(const bf16* dy, const bf16* y, bf16* dx, float* part, float* out, int rows, int C, int accumulate, cudaStream_t st) {

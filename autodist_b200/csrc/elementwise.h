@@ -51,12 +51,12 @@ void sumsq(const float* x, long long n, float* acc, float weight, cudaStream_t s
 void clip_scale(float* x, long long n, const float* acc, float max_norm, cudaStream_t st);
 int bn_parts(int rows, int C);
 int bn_bwd_part_floats(int C);
-void bn_fwd(const bf16_t* x, const float* gamma, const float* beta, const bf16_t* res, bf16_t* y, float* mean, float* rstd, float* part,
-            float* sums, float* coef, int rows, int C, float eps, int relu, int sums_given, float* run_mean, float* run_var,
+void bn_fwd(const bf16_t* x, const float* gamma, const float* beta, const bf16_t* res, bf16_t* y, uint8_t* keep, float* mean, float* rstd,
+            float* part, float* sums, int rows, int C, float eps, int relu, int sums_given, float* run_mean, float* run_var,
             long long* batches, float momentum, cudaStream_t st);
 void bn_eval(const __nv_bfloat16* x, const __nv_bfloat16* res, __nv_bfloat16* y, const float* gamma, const float* beta, const float* mean,
              const float* var, float eps, int rows, int C, int relu, cudaStream_t st);
-void bn_bwd(const bf16_t* dy, const bf16_t* x, const bf16_t* y, const float* mean, const float* rstd, const float* gamma, bf16_t* dx,
+void bn_bwd(const bf16_t* dy, const bf16_t* x, const uint8_t* keep, const float* mean, const float* rstd, const float* gamma, bf16_t* dx,
             bf16_t* dres, float* part, float* sums, float* coef, int rows, int C, int relu, float* dgamma_acc, float* dbeta_acc, cudaStream_t st);
 void maxpool_fwd(const bf16_t* x, bf16_t* y, uint8_t* code, int N, int H, int W, int C, int k, int stride, int pad, int Ho, int Wo,
                  cudaStream_t st);

@@ -465,8 +465,9 @@ class _BatchNormFn(torch.autograd.Function):
         rstd = torch.empty_like(mean)
         g32, b32 = gamma.detach().float().contiguous(), beta.detach().float().contiguous()
         res = _nhwc(residual) if residual is not None else None
-        E.bn_fwd(xh, g32, b32, res, y, mean, rstd, eps, relu, sums, run_mean, run_var, batches, momentum)
-        ctx.save_for_backward(xh, y, mean, rstd, g32)
+        keep = torch.empty(xh.numel() // 8, dtype=torch.uint8, device=x.device) if relu else None       # which outputs the ReLU let through
+        E.bn_fwd(xh, g32, b32, res, y, mean, rstd, eps, relu, sums, run_mean, run_var, batches, momentum, keep)
+        ctx.save_for_backward(xh, keep, mean, rstd, g32)
         ctx.params = (gamma, beta)
         ctx.set_materialize_grads(False)                     # mean / rstd carry no gradient: no zero tensors for them
         _count_use(ctx, gamma, 1)
@@ -480,7 +481,7 @@ class _BatchNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, _dm, _dr):
         E = ops.ext(required=True)
-        xh, y, mean, rstd, g32 = ctx.saved_tensors
+        xh, keep, mean, rstd, g32 = ctx.saved_tensors
         if dy is None:
             return (None,) * 9
         dyh = _nhwc(dy)
@@ -491,7 +492,7 @@ class _BatchNormFn(torch.autograd.Function):
         gamma, beta = ctx.params
         acc_g, acc_b = _direct_grad(gamma), _direct_grad(beta)
         direct = acc_g is not None and acc_b is not None
-        sums = E.bn_bwd(dyh, xh, y, mean, rstd, g32, dx, dres if ctx.relu else None, ctx.relu, acc_g if direct else None,
+        sums = E.bn_bwd(dyh, xh, keep, mean, rstd, g32, dx, dres if ctx.relu else None, ctx.relu, acc_g if direct else None,
                         acc_b if direct else None)
         dr = dres.permute(0, 3, 1, 2).to(ctx.dtypes[2]) if dres is not None else None
         if ctx.fork is not None and dr is not None:
