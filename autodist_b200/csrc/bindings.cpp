@@ -120,17 +120,20 @@ void gemm_set_trace(const optional<Tensor>& t) {
 
 // Which kernel runs a product: the tile width (512: the two-CTA kernel) and how many CTAs share the contraction of one tile.
 // The estimate in microseconds is launch + fill + drain of the kernel, plus, per wave of tiles, its K blocks of 64 (or the
-// epilogue of a tile, whichever is longer). The constants are measured over 40 products from 512 x 128 x 128 to
-// 32 x 4096 x 25088 (replayed back to back, B200). A K block is bound by shared-memory bandwidth: TMA writes it and the MMA
-// reads it once, so 64 / 128 / 256 columns cost 48 / 64 / 96 KB at 128 bytes per clock and narrow tiles only pay when they put
-// more SMs to work. Splitting adds the exchange through distributed shared memory; it wins wherever the tiles leave SMs idle:
-// 1024 x 1024 x 4096 29.2 -> 14.3 us (256 wide, 4 CTAs), 768 x 768 x 1792 16.2 -> 9.0, 256 x 256 x 16384 94.7 -> 14.7,
-// 640 x 1024 x 30522 172 -> 39, 32 x 4096 x 25088 179 -> 38 (5.4 TB/s). Splits run one cluster per tile, so they are only
-// considered while every cluster is resident at once.
+// epilogue of a tile, whichever is longer). The constants are measured over 60 products from 512 x 128 x 128 to
+// 32 x 4096 x 25088 (B200, replayed back to back on one set of operands and on rotating sets that do not fit the L2). A K
+// block is bound by shared-memory bandwidth: TMA writes it and the MMA reads it once, so 64 / 128 / 256 columns cost 48 / 64 /
+// 96 KB at 128 bytes per clock and narrow tiles only pay when they put more SMs to work. The two-CTA kernel moves the fewest
+// bytes per product and suffers least from operands that come from memory (4096 x 1024 x 3072 cold: 27.7 us against 31.5 of
+// the 256-wide one-CTA kernel; hot: 26.7 against 23.8), so it has the larger base and the smaller slope. Splitting adds the
+// exchange through distributed shared memory; it wins wherever the tiles leave SMs idle: 1024 x 1024 x 4096 29.2 -> 14.3 us
+// (256 wide, 4 CTAs), 768 x 768 x 1792 16.2 -> 9.0, 256 x 256 x 16384 94.7 -> 14.7, 640 x 1024 x 30522 172 -> 39,
+// 32 x 4096 x 25088 179 -> 38 (5.4 TB/s). Splits run one cluster per tile, so they are only considered while every cluster is
+// resident at once. Narrow tiles store directly: 8192 x 1024 x 128 fp32 takes 14.0 us with 64 columns, 9.2 with 256.
 struct GemmChoice { int64_t bn, split; };
 GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split) {
   struct Cost { int bn; double base, kb, epi, exchange; };
-  static const Cost costs[4] = {{64, 2.9, 0.28, 1.0, 2.6}, {128, 4.2, 0.30, 1.5, 2.6}, {256, 4.6, 0.38, 2.3, 3.5}, {512, 6.6, 0.36, 2.5, 0.0}};
+  static const Cost costs[4] = {{64, 2.9, 0.30, 1.6, 2.6}, {128, 4.2, 0.33, 2.7, 2.6}, {256, 4.6, 0.48, 2.5, 3.5}, {512, 7.0, 0.41, 2.5, 0.0}};
   const int64_t kbs = (K + 63) / 64, sms = num_sms();
   GemmChoice best{64, 1};
   double best_us = 1e30;
@@ -247,6 +250,7 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
     p.tma_store = 1;
     tmC2 = tmC;
     if (epilogue == adb200::EPI_BIAS_GELU && !make_store_map(as4d(*c2), &tmC2)) p.tma_store = 0;
+    if ((epilogue == adb200::EPI_ADD || epilogue == adb200::EPI_MUL_GELU_GRAD) && !make_store_map(as4d(*aux), &tmC2)) p.tma_store = 0;
   }
   if (split > 1) {
     const cudaError_t e = adb200::launch_gemm_split(tmA, tmB.m[0], p, (int)bn, (int)split, a_mn, b_mn, at::cuda::getCurrentCUDAStream());

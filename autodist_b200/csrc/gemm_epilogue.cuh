@@ -7,6 +7,18 @@
 namespace adb200 {
 namespace tc {
 
+// The auxiliary operand's part: addend, or GELU derivative at a pre-activation.
+template <int NV>
+__device__ __forceinline__ void gemm_epilogue_aux(const GemmParams& p, float* v, const float* x) {
+  if (p.epilogue == EPI_ADD) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) v[j] += x[j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) v[j] *= gelu_tanh_grad(x[j]);
+  }
+}
+
 // The arithmetic of the epilogue on NV (16 or 4) accumulator values of one row, in place: scale, then bias (+ tanh), addend
 // or GELU derivative. `ncols` of the NV columns starting at `col0` (a multiple of NV) exist (0: nothing is read from memory).
 template <int NV>
@@ -46,13 +58,7 @@ __device__ __forceinline__ void gemm_epilogue_math(const GemmParams& p, float* v
 #pragma unroll
       for (int j = 0; j < NV; ++j) x[j] = (j < ncols) ? __bfloat162float(aux[j]) : 0.f;
     }
-    if (p.epilogue == EPI_ADD) {
-#pragma unroll
-      for (int j = 0; j < NV; ++j) v[j] += x[j];
-    } else {
-#pragma unroll
-      for (int j = 0; j < NV; ++j) v[j] *= gelu_tanh_grad(x[j]);
-    }
+    gemm_epilogue_aux<NV>(p, v, x);
   }
 }
 __device__ __forceinline__ void gemm_epilogue_math16(const GemmParams& p, float* v, int col0, int ncols, long long coff, bool vec_ok) {
@@ -65,12 +71,22 @@ __device__ __forceinline__ void gemm_epilogue_math16(const GemmParams& p, float*
 // epilogue warp stages 32 rows x 128 bytes (64 bf16 or 32 fp32 columns) in the 128-byte-swizzled layout and one lane hands
 // the box to the TMA unit, which writes whole lines (or adds them into an fp32 output: beta = 1). Rows and columns
 // past the matrix are clipped by the copy itself. Two 4 KB buffers per warp alternate, so staging overlaps the copy.
+//
+// With two warps per scheduler nothing hides a global load behind other work, so what the epilogue reads is requested while
+// the tile is still being multiplied: the auxiliary operand (addend or pre-activation) comes by TMA into the two staging
+// buffers and is replaced there by the result, each lane keeps four columns of the bias and hands them around by shuffles.
+// A tile's drain is exposed once per launch and, with a short contraction, once per tile: 4096 x 4096 x 1024 on SM pairs,
+// time of a 128 x 256 drain / whole product back to back: bias 5.5 -> 3.7 us / 35.6 -> 35, bias + GELU 8.5 -> 6.9 / 45 -> 39-43,
+// GELU derivative 47.9 -> 41, addend (4096 x 1024 x 4096) 35.3 -> 30.7.
 struct EpiStage {
   const CUtensorMap* tmC;      // output map, box (128 bytes of columns, 32 rows, 1, 1), 128-byte swizzle
-  const CUtensorMap* tmC2;     // second output of EPI_BIAS_GELU
-  uint32_t smem;               // shared address of this warp's 4 KB staging buffers (1024-byte aligned)
+  const CUtensorMap* tmC2;     // EPI_BIAS_GELU: second output; EPI_ADD / EPI_MUL_GELU_GRAD: the auxiliary operand (same box)
+  uint32_t smem;               // shared address of this warp's two 4 KB staging buffers (1024-byte aligned)
+  uint64_t* aux_bar;           // two barriers of this warp: auxiliary box g has landed in buffer g
   int units;                   // copies issued so far by this warp (picks the buffer)
-  int bufs;                    // 2: staging of one box overlaps the copy of the one before; 1: they alternate
+  uint32_t aux_phase;          // bit g: parity the next wait on aux_bar[g] expects
+  uint32_t aux_pending;        // bit g: a load into buffer g has been requested and not yet waited for
+  float4 bias;                 // this lane's four of the 128 columns' biases (0 past the matrix or without a bias)
 };
 
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
@@ -87,71 +103,169 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// box_row: first output row of this warp's 32 rows; lane = row inside the box. Other arguments as gemm_epilogue_row.
-// BNW: columns this warp drains (the tile's width, or half of it when two warps share a TMEM lane quarter).
+// Requests what the epilogue of the next tile reads (see EpiStage). BNW <= 128 columns starting at n0.
 template <int BNW>
-__device__ __forceinline__ void gemm_epilogue_row_tma(const GemmParams& p, EpiStage& st, uint32_t t_row, int row, int box_row, int n0, int b_lo,
-                                                      int b_hi, long long coff, bool vec_ok, int lane) {
-  const bool f32 = p.c_is_fp32 != 0;
-  const int gcols = f32 ? 32 : 64;                   // columns in one 128-byte staging row
-  const bool two = p.epilogue == EPI_BIAS_GELU;      // two outputs (bf16): the pre-activation, then its GELU
-  const uint32_t swz = (uint32_t)(lane & 7);
-#pragma unroll 1
-  for (int g = 0; g * gcols < BNW; ++g) {
-    const int gcol0 = n0 + g * gcols;
-    if (gcol0 >= p.N) break;                          // uniform over the CTA
-    if (lane == 0) {                                  // the buffer about to be written is no longer being read
-      if (st.bufs < 2) bulk_wait_read<0>(); else bulk_wait_read<1>();
+__device__ __forceinline__ void gemm_epilogue_prefetch(const GemmParams& p, EpiStage& st, int box_row, int n0, int b_lo, int b_hi, int lane) {
+  if (box_row >= p.M) return;
+  if (p.epilogue == EPI_BIAS || p.epilogue == EPI_BIAS_GELU || p.epilogue == EPI_BIAS_TANH) {
+    static_assert(BNW == 128, "one float4 of bias per lane");
+    const int col = n0 + lane * 4;
+    st.bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (col < p.N) st.bias.x = __ldg(p.bias + col);
+    if (col + 1 < p.N) st.bias.y = __ldg(p.bias + col + 1);
+    if (col + 2 < p.N) st.bias.z = __ldg(p.bias + col + 2);
+    if (col + 3 < p.N) st.bias.w = __ldg(p.bias + col + 3);
+  } else if (p.epilogue == EPI_ADD || p.epilogue == EPI_MUL_GELU_GRAD) {
+    if (lane == 0) bulk_wait_read<0>();               // the previous tile's copies have left both buffers
+#pragma unroll
+    for (int g = 0; g < BNW / 64; ++g) {
+      if (n0 + g * 64 >= p.N) break;
+      if (lane == 0) {
+        mbar_expect_tx(&st.aux_bar[g], 4096);
+        asm volatile(
+            "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+            ::"r"(st.smem + (uint32_t)g * 4096u), "l"(st.tmC2), "r"(smem_u32(&st.aux_bar[g])), "r"(n0 + g * 64), "r"(box_row), "r"(b_lo), "r"(b_hi)
+            : "memory");
+      }
+      st.aux_pending |= 1u << g;
     }
-    __syncwarp();
-    const uint32_t base = st.smem + (st.bufs < 2 ? 0u : (uint32_t)(st.units & 1)) * 4096u;
+  }
+}
+
+// Scale, bias and tanh of NV values starting `col` columns into the 128 that `st.bias` covers.
+template <int NV>
+__device__ __forceinline__ void gemm_epilogue_bias(const GemmParams& p, const EpiStage& st, float* v, int col) {
+#pragma unroll
+  for (int j = 0; j < NV; ++j) v[j] *= p.alpha;
+  if (p.epilogue == EPI_BIAS || p.epilogue == EPI_BIAS_GELU || p.epilogue == EPI_BIAS_TANH) {
+#pragma unroll
+    for (int j = 0; j < NV; j += 4) {
+      const int src = (col + j) >> 2;
+      v[j] += __shfl_sync(0xffffffffu, st.bias.x, src);
+      v[j + 1] += __shfl_sync(0xffffffffu, st.bias.y, src);
+      v[j + 2] += __shfl_sync(0xffffffffu, st.bias.z, src);
+      v[j + 3] += __shfl_sync(0xffffffffu, st.bias.w, src);
+    }
+    if (p.epilogue == EPI_BIAS_TANH) {
+#pragma unroll
+      for (int j = 0; j < NV; ++j) v[j] = tanhf(v[j]);
+    }
+  }
+}
+
+// Before the warp leaves: auxiliary boxes that nobody waited for (another role gave up) land first.
+__device__ __forceinline__ void gemm_epilogue_drain(EpiStage& st) {
+  for (int g = 0; g < 2; ++g)
+    if (st.aux_pending & (1u << g)) {
+      const long long t0 = clock64();
+      while (!mbar_try(&st.aux_bar[g], (st.aux_phase >> g) & 1u) && clock64() - t0 < 20000000LL) {}
+    }
+}
+
+// box_row: first output row of this warp's 32 rows; lane = row inside the box. Other arguments as gemm_epilogue_row.
+// BNW: columns this warp drains (the tile's width, or half of it when two warps share a TMEM lane quarter). Returns false when
+// an auxiliary box did not arrive in time.
+template <int BNW>
+__device__ __forceinline__ bool gemm_epilogue_row_tma(const GemmParams& p, EpiStage& st, uint32_t t_row, int row, int box_row, int n0, int b_lo,
+                                                      int b_hi, int lane, volatile int* abort_flag) {
+  if (box_row >= p.M) return true;                    // none of this warp's rows exist
+  const bool f32 = p.c_is_fp32 != 0;
+  const bool two = p.epilogue == EPI_BIAS_GELU;      // two outputs (bf16): the pre-activation, then its GELU
+  const bool aux = p.epilogue == EPI_ADD || p.epilogue == EPI_MUL_GELU_GRAD;
+  const uint32_t swz = (uint32_t)(lane & 7);
+  if (f32) {
+    // fp32: boxes of 32 columns; bias is the only epilogue such outputs take
+#pragma unroll 1
+    for (int g = 0; g < BNW / 32; ++g) {
+      const int gcol0 = n0 + g * 32;
+      if (gcol0 >= p.N) break;                        // uniform over the CTA
+      if (lane == 0) bulk_wait_read<1>();             // the buffer about to be written is no longer being read
+      const uint32_t base = st.smem + (uint32_t)(st.units & 1) * 4096u;
+      const uint32_t buf = base + (uint32_t)lane * 128u;
+      float v[32];
+      __syncwarp();                                   // tcgen05.ld is warp-collective
+      tmem_ld32(t_row + g * 32, v);
+      gemm_epilogue_bias<32>(p, st, v, g * 32);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        st_shared_v4(buf + (((uint32_t)i ^ swz) << 4), __float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]), __float_as_uint(v[4 * i + 2]),
+                     __float_as_uint(v[4 * i + 3]));
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // the staged rows are visible to the TMA unit
+      __syncwarp();
+      if (lane == 0) {
+        if (p.beta != 0.0f) tma_reduce_add_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
+        else tma_store_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
+        bulk_commit();
+      }
+      st.units += 1;
+    }
+    return true;
+  }
+#pragma unroll 1
+  for (int g = 0; g < BNW / 64; ++g) {
+    const int gcol0 = n0 + g * 64;
+    if (gcol0 >= p.N) break;                          // uniform over the CTA
+    uint32_t base;
+    if (aux) {
+      base = st.smem + (uint32_t)g * 4096u;           // the auxiliary box is already there
+      if (!mbar_wait(&st.aux_bar[g], (st.aux_phase >> g) & 1u, abort_flag)) return false;
+      st.aux_phase ^= 1u << g;
+      st.aux_pending &= ~(1u << g);
+    } else {
+      if (lane == 0) bulk_wait_read<1>();             // the buffer about to be written is no longer being read
+      base = st.smem + (uint32_t)(st.units & 1) * 4096u;
+    }
     const uint32_t buf = base + (uint32_t)lane * 128u;
     uint32_t act[32];                                 // packed GELU values of the group (two outputs only)
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc) {
-      if (f32 && cc >= 2) break;
-      float v[16];
+    for (int h = 0; h < 2; ++h) {
+      float v[32];
       __syncwarp();                                   // tcgen05.ld is warp-collective
-      tmem_ld16(t_row + g * gcols + cc * 16, v);
-      const int col0 = gcol0 + cc * 16;
-      const int ncols = (row < p.M) ? max(0, min(16, p.N - col0)) : 0;
-      gemm_epilogue_math16(p, v, col0, ncols, coff, vec_ok);
-      if (f32) {
+      tmem_ld32(t_row + g * 64 + h * 32, v);
+      if (aux) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          st_shared_v4(buf + (((uint32_t)(cc * 4 + i) ^ swz) << 4), __float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]),
-                       __float_as_uint(v[4 * i + 2]), __float_as_uint(v[4 * i + 3]));
+        for (int i = 0; i < 4; ++i) {
+          float x[8];
+          unpack8_bf16(ld_shared_v4(buf + (((uint32_t)(h * 4 + i) ^ swz) << 4)), x);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[8 * i + j] *= p.alpha;
+          gemm_epilogue_aux<8>(p, v + 8 * i, x);
+        }
       } else {
+        gemm_epilogue_bias<32>(p, st, v, g * 64 + h * 32);
+      }
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-          st_shared_v4(buf + (((uint32_t)(cc * 2 + h) ^ swz) << 4), pack_bf16x2(v[8 * h], v[8 * h + 1]), pack_bf16x2(v[8 * h + 2], v[8 * h + 3]),
-                       pack_bf16x2(v[8 * h + 4], v[8 * h + 5]), pack_bf16x2(v[8 * h + 6], v[8 * h + 7]));
+      for (int i = 0; i < 4; ++i) {
+        st_shared_v4(buf + (((uint32_t)(h * 4 + i) ^ swz) << 4), pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
+                     pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
         if (two) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) act[cc * 8 + j] = pack_bf16x2(gelu_tanh(v[2 * j]), gelu_tanh(v[2 * j + 1]));
+          for (int j = 0; j < 4; ++j) act[h * 16 + i * 4 + j] = pack_bf16x2(gelu_tanh(v[8 * i + 2 * j]), gelu_tanh(v[8 * i + 2 * j + 1]));
         }
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the staged rows are visible to the TMA unit
     __syncwarp();
     if (lane == 0) {
-      if (f32 && p.beta != 0.0f) tma_reduce_add_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
-      else tma_store_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
+      tma_store_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
       bulk_commit();
     }
     st.units += 1;
     if (two) {
-      // second output from the values kept in registers, through the other buffer (or the same one once it has been read)
-      if (lane == 0) {
-        if (st.bufs < 2) bulk_wait_read<0>(); else bulk_wait_read<1>();
-      }
+      // second output from the values kept in registers, through the other buffer
+      if (lane == 0) bulk_wait_read<1>();
       __syncwarp();
-      const uint32_t base2 = st.smem + (st.bufs < 2 ? 0u : (uint32_t)(st.units & 1)) * 4096u;
+      const uint32_t base2 = st.smem + (uint32_t)(st.units & 1) * 4096u;
       const uint32_t buf2 = base2 + (uint32_t)lane * 128u;
 #pragma unroll
       for (int j = 0; j < 8; ++j)
@@ -165,6 +279,7 @@ __device__ __forceinline__ void gemm_epilogue_row_tma(const GemmParams& p, EpiSt
       st.units += 1;
     }
   }
+  return true;
 }
 
 // t_row: TMEM address of this thread's lane at the first column of the accumulator; row: output row (may be >= M);

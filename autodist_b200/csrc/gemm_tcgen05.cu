@@ -39,9 +39,9 @@ template <int BN> struct Cfg {
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int CW = BN / (EPI_WARPS / 4);          // columns per epilogue warp
   static constexpr int TMEM_COLS = 2 * BN;              // double-buffered fp32 accumulator
-  // TMA-store staging (widest tile only): one 4 KB buffer per epilogue warp. The whole CTA stays near 208 KB so that the
+  // TMA-store staging (widest tile only): two 4 KB buffers per epilogue warp. The whole CTA stays near 210 KB so that the
   // blocks of a small kernel launched behind it (programmatic dependent launch) still fit beside it on the SM.
-  static constexpr int STAGING = (BN == 256) ? EPI_WARPS * 4096 : 0;
+  static constexpr int STAGING = (BN == 256) ? EPI_WARPS * 8192 : 0;
   static constexpr int SMEM = STAGES * (A_BYTES + B_BYTES) + STAGING + 1024 /*align*/ + 256 /*barriers*/;
 };
 
@@ -62,6 +62,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* aux_bars = tempty + 3;                      // widest tile: two per epilogue warp (behind the slot and the flag)
+  constexpr int AUX_BARS = BN == 256 ? 2 * C::EPI_WARPS : 0;
+  static_assert((2 * C::STAGES + 4 + 1 + AUX_BARS) * 8 <= 256, "barrier area");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -69,6 +72,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 32 * C::EPI_WARPS); }
+    for (int s = 0; s < AUX_BARS; ++s) mbar_init(&aux_bars[s], 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -179,13 +183,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
     const int half = (warp - 2) >> 2;                  // 0, or 1 for the second warp of a lane quarter
     int as = 0; uint32_t aphase = 0; bool ok = true;
     const bool vec_ok = (p.ldc % 8 == 0);
-    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 4096u, 0, 1};
+    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, make_float4(0.f, 0.f, 0.f, 0.f)};
     for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
       const int b = (int)(t / per_batch), rem = (int)(t % per_batch);
       const int tn = rem / tiles_m, tm = rem % tiles_m;
       const int b_lo = b % p.batch_lo, b_hi = b / p.batch_lo;
       const int row = tm * BM + q * 32 + lane;
-      const int n0 = tn * BN;
+      const int n_w = tn * BN + half * C::CW;
+      const int box_row = tm * BM + q * 32;
+      if constexpr (BN == 256) {
+        if (p.tma_store) gemm_epilogue_prefetch<C::CW>(p, est, box_row, n_w, b_lo, b_hi, lane);
+      }
       if (!mbar_wait(&tfull[as], aphase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const long long coff = (long long)b_hi * p.strideC_hi + (long long)b_lo * p.strideC_lo + (long long)row * p.ldc;
@@ -259,16 +267,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
       }
       if (!handled) {
         const uint32_t t_w = t_row + (uint32_t)(half * C::CW);
-        const int n_w = n0 + half * C::CW;
-        if (BN == 256 && p.tma_store) gemm_epilogue_row_tma<C::CW>(p, est, t_w, row, tm * BM + q * 32, n_w, b_lo, b_hi, coff, vec_ok, lane);
-        else gemm_epilogue_row<C::CW>(p, t_w, row, n_w, coff, vec_ok);
+        bool staged = false;
+        if constexpr (BN == 256) {
+          staged = p.tma_store != 0;
+          if (staged) ok = gemm_epilogue_row_tma<C::CW>(p, est, t_w, row, box_row, n_w, b_lo, b_hi, lane, abort_flag);
+        }
+        if (!staged) gemm_epilogue_row<C::CW>(p, t_w, row, n_w, coff, vec_ok);
       }
+      if (!ok) break;
       __syncwarp();
       tc_fence_before();
       mbar_arrive(&tempty[as]);
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
     if (BN == 256 && p.tma_store && lane == 0) bulk_wait_all();       // this warp's output copies have landed
+    if (BN == 256) gemm_epilogue_drain(est);
     if (!ok && lane == 0) {
       *abort_flag = 1;
       if (p.error_flag) atomicExch(p.error_flag, 3);

@@ -43,8 +43,8 @@ struct TmapArray {
 // `bn` is the N extent of the tile (64, 128 or 256). The tensor maps must be 4-D bf16 maps with 128-byte swizzle:
 //   K-major operand : dims (K, rows, batch_lo, batch_hi), box (64, 128 for A / bn for B, 1, 1)
 //   MN-major operand: dims (rows, K, batch_lo, batch_hi), box (64, 64, 1, 1)
-// With p.tma_store, `tmC` (and `tmC2` for EPI_BIAS_GELU) map the output: same element type as C, box (128 bytes of columns,
-// 32 rows, 1, 1), 128-byte swizzle; fp32 outputs need beta 0 or 1. Otherwise both may be null.
+// With p.tma_store, `tmC` (and `tmC2`: the second output of EPI_BIAS_GELU, the auxiliary operand of EPI_ADD and
+// EPI_MUL_GELU_GRAD) map the output: same element type as C, box (128 bytes of columns, 32 rows, 1, 1), 128-byte swizzle; fp32 outputs need beta 0 or 1. Otherwise both may be null.
 cudaError_t launch_gemm(const CUtensorMap& tmA, const TmapArray& tmB, const GemmParams& p, int bn, bool a_mn,
                         bool b_mn, int num_sms, cudaStream_t stream, const CUtensorMap* tmC = nullptr, const CUtensorMap* tmC2 = nullptr);
 

@@ -35,11 +35,11 @@ using namespace tc;
 
 constexpr int BN2 = 256;                 // tile width; each CTA stages BN2 / 2 rows of B
 constexpr int B2_BYTES = (BN2 / 2) * BK * 2;
-constexpr int STAGES2 = 5;              // 5 x 32 KB + 32 KB of output staging: the CTA stays at 193 KB (room for a dependent kernel's blocks)
+constexpr int STAGES2 = 5;              // 5 x 32 KB of operands + 64 KB of output staging: 226 of the SM's 227 KB
 constexpr int TMEM_COLS2 = 2 * BN2;
 constexpr int EPI_WARPS2 = 8;            // two per TMEM lane quarter, half of the tile's columns each
 constexpr int kThreads2 = 64 + 32 * EPI_WARPS2;
-constexpr int STAGING2 = EPI_WARPS2 * 4096;   // TMA-store staging: one 4 KB buffer per epilogue warp
+constexpr int STAGING2 = EPI_WARPS2 * 8192;   // TMA-store staging: two 4 KB buffers per epilogue warp
 constexpr int SMEM2 = STAGES2 * (A_BYTES + B2_BYTES) + STAGING2 + 1024 /*align*/ + 256 /*barriers*/;
 
 __device__ __forceinline__ long long now_ns() {
@@ -65,6 +65,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* aux_bars = tempty + 3;                      // two per epilogue warp (behind the slot and the flag)
+  static_assert((2 * STAGES2 + 4 + 1 + 2 * EPI_WARPS2) * 8 <= 256, "barrier area");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -78,6 +80,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES2; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 2 * EPI_WARPS2); }
+    for (int s = 0; s < 2 * EPI_WARPS2; ++s) mbar_init(&aux_bars[s], 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -185,22 +188,24 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     const int half = (warp - 2) >> 2;                  // which half of the tile's columns this warp drains
     int as = 0; uint32_t aphase = 0; bool ok = true;
     const bool vec_ok = (p.ldc % 8 == 0);
-    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 4096u, 0, 1};
+    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, make_float4(0.f, 0.f, 0.f, 0.f)};
     for (long long t = pair; t < total && ok; t += pairs) {
       const int b = (int)(t / per_batch), rem = (int)(t % per_batch);
       const int tn = rem / tiles_m, tm = rem % tiles_m;
       const int b_lo = b % p.batch_lo, b_hi = b / p.batch_lo;
       const int row = tm * 256 + (int)rank * 128 + q * 32 + lane;
-      const int n0 = tn * BN2;
+      const int n_w = tn * BN2 + half * (BN2 / 2);
+      const int box_row = tm * 256 + (int)rank * 128 + q * 32;
+      if (p.tma_store) gemm_epilogue_prefetch<BN2 / 2>(p, est, box_row, n_w, b_lo, b_hi, lane);
       if (!mbar_wait(&tfull[as], aphase, abort_flag)) { ok = false; break; }
       const long long e0 = trace != nullptr ? now_ns() : 0;
       tc_fence_after();
       const long long coff = (long long)b_hi * p.strideC_hi + (long long)b_lo * p.strideC_lo + (long long)row * p.ldc;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN2);
       const uint32_t t_w = t_row + (uint32_t)(half * (BN2 / 2));
-      const int n_w = n0 + half * (BN2 / 2);
-      if (p.tma_store) gemm_epilogue_row_tma<BN2 / 2>(p, est, t_w, row, tm * 256 + (int)rank * 128 + q * 32, n_w, b_lo, b_hi, coff, vec_ok, lane);
+      if (p.tma_store) ok = gemm_epilogue_row_tma<BN2 / 2>(p, est, t_w, row, box_row, n_w, b_lo, b_hi, lane, abort_flag);
       else gemm_epilogue_row<BN2 / 2>(p, t_w, row, n_w, coff, vec_ok);
+      if (!ok) break;
       __syncwarp();
       tc_fence_before();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty[as]), 0));
@@ -208,6 +213,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
     if (p.tma_store && lane == 0) bulk_wait_all();       // this warp's output copies have landed
+    gemm_epilogue_drain(est);
     if (!ok && lane == 0) {
       *abort_flag = 1;
       if (p.error_flag) atomicExch(p.error_flag, 43);
