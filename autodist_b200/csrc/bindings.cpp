@@ -11,6 +11,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "attention.h"
 #include "comm.h"
 #include "elementwise.h"
 #include "gemm_tcgen05.h"
@@ -452,6 +453,63 @@ void softmax_bwd(Tensor dp, const Tensor& p, double scale, double pd, int64_t se
   const int S = p.size(-1);
   adb200::softmax_bwd(BF(dp), CBF(p), p.numel() / S, S, (float)scale, (float)pd, (uint64_t)seed, OPT_LL(step), STREAM);
 }
+// Fused self-attention over the projection qkv [B * S, 3 * heads * 64] (bf16; q, k, v side by side): writes ctx [B * S, heads * 64]
+// and lse [B, heads, S], with dropout also the decisions (keep). mask: additive fp32 [B, S] over the keys.
+adb200::AttnParams attn_params(const Tensor& qkv, const optional<Tensor>& mask, const Tensor& ctx, const Tensor& lse, int64_t B, int64_t S,
+                               int64_t heads, double scale, double pd, int64_t seed, const optional<Tensor>& step, Tensor error_flag,
+                               const optional<Tensor>& keep) {
+  const int64_t H = heads * 64;
+  TORCH_CHECK(B > 0 && heads > 0 && S > 0 && S <= 1024, "attention takes 1 to 1024 tokens");
+  TORCH_CHECK(qkv.is_cuda() && qkv.scalar_type() == at::kBFloat16 && qkv.is_contiguous() && qkv.numel() == B * S * 3 * H, "qkv must be contiguous bf16 [B * S, 3 * heads * 64]");
+  TORCH_CHECK(ctx.scalar_type() == at::kBFloat16 && ctx.is_contiguous() && ctx.numel() == B * S * H, "ctx must be contiguous bf16 [B * S, heads * 64]");
+  TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.numel() == B * heads * S, "lse must be fp32 [B, heads, S]");
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(ctx.data_ptr()) % 16 == 0, "ctx must be 16-byte aligned");
+  if (mask.has_value()) TORCH_CHECK(mask->scalar_type() == at::kFloat && mask->is_contiguous() && mask->numel() == B * S, "mask must be fp32 [B, S]");
+  adb200::AttnParams p{};
+  p.B = (int)B; p.S = (int)S; p.heads = (int)heads;
+  p.scale = (float)scale;
+  p.mask = OPT_F(mask);
+  p.lse = lse.data_ptr<float>();
+  p.drop_p = (float)pd; p.seed = (unsigned long long)seed; p.step = OPT_LL(step);
+  if (pd > 0) {
+    TORCH_CHECK(keep.has_value() && keep->scalar_type() == at::kInt && keep->is_contiguous() && keep->numel() >= B * heads * S * adb200::attn_keep_words((int)S),
+                "dropout needs int32 [B, heads, S, 4 * ceil(S / 128)] for its decisions");
+    p.keep = reinterpret_cast<uint32_t*>(keep->data_ptr<int>());
+  }
+  p.ctx = reinterpret_cast<__nv_bfloat16*>(ctx.data_ptr());
+  p.error_flag = error_flag.data_ptr<int>();
+  return p;
+}
+// [B, heads, S, 64] view of 64 columns per head starting at column `off` of a [B * S, ld] matrix
+CUtensorMap head_map(const Tensor& t, int64_t B, int64_t S, int64_t heads, int64_t ld, int64_t off, int rows = 128) {
+  return make_map(t.view({B, S, ld}).narrow(2, off, heads * 64).view({B, S, heads, 64}).permute({0, 2, 1, 3}), rows);
+}
+void attn_fwd(const Tensor& qkv, const optional<Tensor>& mask, Tensor ctx, Tensor lse, int64_t B, int64_t S, int64_t heads, double scale,
+              double pd, int64_t seed, const optional<Tensor>& step, Tensor error_flag, const optional<Tensor>& keep) {
+  const c10::cuda::CUDAGuard guard(qkv.device());
+  const adb200::AttnParams p = attn_params(qkv, mask, ctx, lse, B, S, heads, scale, pd, seed, step, error_flag, keep);
+  const int64_t H = heads * 64;
+  cudaError_t e = adb200::launch_attn_fwd(head_map(qkv, B, S, heads, 3 * H, 0), head_map(qkv, B, S, heads, 3 * H, H),
+                                          head_map(qkv, B, S, heads, 3 * H, 2 * H), p, STREAM);
+  TORCH_CHECK(e == cudaSuccess, "attention launch failed: ", cudaGetErrorString(e));
+}
+// dqkv = gradient of qkv given dctx, with ctx, lse and keep as the forward pass left them. delta: scratch of lse's shape.
+void attn_bwd(const Tensor& qkv, const optional<Tensor>& mask, const Tensor& ctx, const Tensor& dctx, const Tensor& lse, Tensor delta, Tensor dqkv,
+              int64_t B, int64_t S, int64_t heads, double scale, double pd, Tensor error_flag, const optional<Tensor>& keep) {
+  const c10::cuda::CUDAGuard guard(qkv.device());
+  adb200::AttnParams p = attn_params(qkv, mask, ctx, lse, B, S, heads, scale, pd, 0, c10::nullopt, error_flag, keep);
+  TORCH_CHECK(delta.scalar_type() == at::kFloat && delta.is_contiguous() && delta.numel() == lse.numel(), "delta must match lse");
+  p.delta = delta.data_ptr<float>();
+  const int64_t H = heads * 64;
+  TORCH_CHECK(dctx.scalar_type() == at::kBFloat16 && dctx.is_contiguous() && dctx.numel() == B * S * H, "dctx must match ctx");
+  TORCH_CHECK(dqkv.scalar_type() == at::kBFloat16 && dqkv.is_contiguous() && dqkv.numel() == qkv.numel(), "dqkv must match qkv");
+  p.dctx = CBF(dctx);
+  adb200::AttnGradMaps grads;
+  for (int i = 0; i < 3; ++i) grads.m[i] = head_map(dqkv, B, S, heads, 3 * H, i * H, 32);
+  cudaError_t e = adb200::launch_attn_bwd(head_map(qkv, B, S, heads, 3 * H, 0), head_map(qkv, B, S, heads, 3 * H, H),
+                                          head_map(qkv, B, S, heads, 3 * H, 2 * H), head_map(dctx, B, S, heads, H, 0), grads, p, num_sms(), STREAM);
+  TORCH_CHECK(e == cudaSuccess, "attention launch failed: ", cudaGetErrorString(e));
+}
 void xent(Tensor logits, const Tensor& labels, const optional<Tensor>& weights, Tensor denom, Tensor loss_sum, int64_t V, double loss_scale,
           bool compute_denom, double eps) {
   const int ld = logits.size(-1), rows = logits.numel() / ld;
@@ -788,6 +846,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_set_trace", &gemm_set_trace);
   m.def("gemm", &gemm);
   m.def("gemm_split", &gemm_split);
+  m.def("attn_fwd", &attn_fwd);
+  m.def("attn_bwd", &attn_bwd);
   m.def("gemm_softmax", &gemm_softmax);
   m.def("gemm_gathered_b", &gemm_gathered_b);
   m.def("gemm_gathered_bt", &gemm_gathered_bt);

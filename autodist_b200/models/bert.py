@@ -13,9 +13,9 @@ Two execution paths over the same parameters:
 * the fused path (CUDA, after ``materialize``) - forward **and** backward are
   explicit sequences of the hand-written sm_100a kernels: tcgen05 GEMMs (the
   backward products read the forward tensors as MN-major operands, so nothing is
-  transposed), attention as batched tcgen05 GEMMs over strided views of the
-  fused QKV projection, fused bias/GELU/residual epilogues, layernorm /
-  softmax / cross-entropy kernels. Gradients are written straight into the flat
+  transposed), fused attention kernels over strided views of the
+  QKV projection, fused bias/GELU/residual epilogues, layernorm /
+  cross-entropy kernels. Gradients are written straight into the flat
   fp32 gradient buffer; ``grad_ready`` is called as parameter ranges complete so
   that the engine can start their all-reduce while the rest of the backward
   pass still runs.
@@ -125,9 +125,9 @@ class BertPretrainer(nn.Module):
         self._ws = None
         self._seed = 0x5EED
         self.training_dropout = True
-        # S == 128: softmax inside the QK^T / dP GEMM epilogues. Measured slower than the stand-alone softmax kernels
-        # (20.9 vs 20.1 ms per BERT-large step: a 64-deep contraction cannot hide a 128-exponential epilogue), so off.
-        self.fused_attention_softmax = False
+        # Heads of 64 columns run on the fused attention kernels (csrc/attention.cu); other head sizes, and ``False`` here, on
+        # batched GEMMs with the stand-alone softmax kernels.
+        self.fused_attention = True
         # Bias gradients (column sums) on a side stream next to the weight-gradient GEMMs instead of between them.
         self.side_stream_bias_grads = os.environ.get("AUTODIST_BERT_SIDE_STREAM", "1") == "1"
 
@@ -186,8 +186,12 @@ class BertPretrainer(nn.Module):
         self._ws = None
         return self.flat
 
+    def _fused_attention(self, S):
+        c = self.config
+        return self.fused_attention and c.hidden_size == 64 * c.num_attention_heads and S in (64, 128, 256, 512, 1024)
+
     def _workspace(self, B, S, P):
-        key = (B, S, P)
+        key = (B, S, P, self._fused_attention(S))
         if self._ws is not None and self._ws["key"] == key:
             return self._ws
         from autodist_b200 import ops
@@ -204,11 +208,18 @@ class BertPretrainer(nn.Module):
         def f32(*shape):
             return torch.empty(*shape, dtype=torch.float32, device=dev)
 
-        drop_a = c.attention_probs_dropout_prob > 0 and self.training_dropout
+        fused = self._fused_attention(S)
+        drop_p = c.attention_probs_dropout_prob > 0 and self.training_dropout
+        drop_a = drop_p and not fused
+
+        def scores():
+            return None if fused else bf(B, nh, S, S)
+
         layers = []
         for _ in range(c.num_hidden_layers):
             layers.append({
-                "qkv": bf(T, 3 * H), "p": bf(B, nh, S, S), "pd": bf(B, nh, S, S) if drop_a else None,
+                "qkv": bf(T, 3 * H), "p": scores(), "pd": scores() if drop_a else None, "lse": f32(B, nh, S) if fused else None,
+                "keep": torch.empty(B, nh, S, (S + 127) // 128 * 4, dtype=torch.int32, device=dev) if fused and drop_p else None,
                 "ctx": bf(T, H), "z1": bf(T, H), "m1": f32(T), "r1": f32(T), "x1": bf(T, H),
                 "u": bf(T, Fd), "g": bf(T, Fd), "z2": bf(T, H), "m2": f32(T), "r2": f32(T), "out": bf(T, H)})
         n_part = max( E.colsum_parts(T) * max(4 * H, Fd, 3 * H, 2 * H),
@@ -216,10 +227,10 @@ class BertPretrainer(nn.Module):
         ws = {
             "key": key, "E": E, "layers": layers, "Vp": Vp,
             "z0": bf(T, H), "m0": f32(T), "r0": f32(T), "x0": bf(T, H), "mask": f32(B, S),
-            "tmp": bf(T, H), "scores": bf(B, nh, S, S),
+            "tmp": bf(T, H), "scores": scores(),
             # backward scratch
             "d_a": bf(T, H), "d_b": bf(T, H), "d_c": bf(T, H), "d_big": bf(T, Fd), "d_qkv": bf(T, 3 * H),
-            "d_p": bf(B, nh, S, S), "part": f32(n_part),
+            "d_p": scores(), "delta": f32(B, nh, S) if fused else None, "part": f32(n_part),
             "ln_part": torch.zeros(E.ln_bwd_part_floats(H), dtype=torch.float32, device=dev),     # zero between calls by contract
             # bias gradients are column sums that nothing in the layer waits for: they run on a side stream next to the
             # GEMMs, each with its own partial-sum scratch (joined before the layer's gradients are reported ready)
@@ -264,7 +275,7 @@ class BertPretrainer(nn.Module):
         gm = lambda *a, **k: self._gemm(ws, *a, **k)   # noqa: E731
         seed = lambda l, site: self._seed + 64 * l + site   # noqa: E731
         scale = 1.0 / math.sqrt(D)
-        fused_sm = S == 128 and self.fused_attention_softmax
+        fused = self._fused_attention(S)
 
         ids = input_ids.reshape(-1)
         tts = segment_ids.reshape(-1)
@@ -291,13 +302,13 @@ class BertPretrainer(nn.Module):
         for l, A in enumerate(ws["layers"]):
             n = f"layers.{l}."
             gm(x, w16[n + "qkv_w"], A["qkv"], epi=EPI_BIAS, bias=w32[n + "qkv_b"])
-            q, k, v = (heads_view(A["qkv"], i) for i in range(3))
-            if fused_sm:      # scores never leave the SM: scale, mask, softmax and dropout run in the GEMM epilogue
-                E.gemm_softmax(q, k, A["p"], A["pd"] if pa > 0 else None, ws["mask"], None, False, scale, pa, seed(l, 1), step, ws["err"])
+            if fused:         # scores and probabilities never leave the SM
+                E.attn_fwd(A["qkv"], ws["mask"], A["ctx"], A["lse"], B, S, nh, scale, pa, seed(l, 1), step, ws["err"], A["keep"])
             else:
+                q, k, v = (heads_view(A["qkv"], i) for i in range(3))
                 gm(q, k, ws["scores"], bn=128)
                 E.softmax_fwd(ws["scores"], ws["mask"], A["p"], A["pd"] if pa > 0 else None, scale, pa, seed(l, 1), step)
-            gm(A["pd"] if pa > 0 else A["p"], v, ctx_view(A["ctx"]), b_mn=True, bn=64)
+                gm(A["pd"] if pa > 0 else A["p"], v, ctx_view(A["ctx"]), b_mn=True, bn=64)
             gm(A["ctx"], w16[n + "out_w"], ws["tmp"], epi=EPI_BIAS, bias=w32[n + "out_b"])
             E.ln_fwd(ws["tmp"], x, w32[n + "ln1_g"], w32[n + "ln1_b"], A["z1"], A["x1"], A["m1"], A["r1"], eps, ph, seed(l, 2), step)
             gm(A["x1"], w16[n + "w1"], A["u"], epi=EPI_BIAS_GELU, bias=w32[n + "b1"], c2=A["g"])
@@ -392,17 +403,17 @@ class BertPretrainer(nn.Module):
             gm(dao, A["ctx"], g[n + "out_w"], a_mn=True, b_mn=True)                     # dWo
             dctx = dx1                                                                  # reuse again
             gm(dao, w16[n + "out_w"], dctx, b_mn=True)                                  # dctx = dao . Wo
-            q, k, v = (heads_view(A["qkv"], i) for i in range(3))
-            dq, dk, dv = (heads_view(ws["d_qkv"], i) for i in range(3))
-            pdrop = A["pd"] if pa > 0 else A["p"]
-            gm(pdrop, ctx_view(dctx), dv, a_mn=True, b_mn=True, bn=64)                  # dV = P^T . dctx
-            if fused_sm:      # dS = scale * P * (dP - sum(dP * P)) in the epilogue of dP = dctx . V^T
-                E.gemm_softmax(ctx_view(dctx), v, ws["d_p"], None, None, A["p"], True, scale, pa, seed(l, 1), step, ws["err"])
+            if fused:
+                E.attn_bwd(A["qkv"], ws["mask"], A["ctx"], dctx, A["lse"], ws["delta"], ws["d_qkv"], B, S, nh, scale, pa, ws["err"], A["keep"])
             else:
+                q, k, v = (heads_view(A["qkv"], i) for i in range(3))
+                dq, dk, dv = (heads_view(ws["d_qkv"], i) for i in range(3))
+                pdrop = A["pd"] if pa > 0 else A["p"]
+                gm(pdrop, ctx_view(dctx), dv, a_mn=True, b_mn=True, bn=64)              # dV = P^T . dctx
                 gm(ctx_view(dctx), v, ws["d_p"], bn=128)                                # dP = dctx . V^T
                 E.softmax_bwd(ws["d_p"], A["p"], scale, pa, seed(l, 1), step)           # dS (in place)
-            gm(ws["d_p"], k, dq, b_mn=True, bn=64)                                      # dQ = dS . K
-            gm(ws["d_p"], q, dk, a_mn=True, b_mn=True, bn=64)                           # dK = dS^T . Q
+                gm(ws["d_p"], k, dq, b_mn=True, bn=64)                                  # dQ = dS . K
+                gm(ws["d_p"], q, dk, a_mn=True, b_mn=True, bn=64)                       # dK = dS^T . Q
             bias_grad(ws["d_qkv"], g[n + "qkv_b"], 3)
             gm(ws["d_qkv"], x_in, g[n + "qkv_w"], a_mn=True, b_mn=True)                 # dWqkv
             d_prev = dctx

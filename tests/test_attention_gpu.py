@@ -1,0 +1,73 @@
+"""Fused attention kernels against fp64, with the dropout decisions of the stand-alone softmax kernel."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(B, S, nh, pd, seed=5, masked=True):
+    from autodist_b200 import ops
+    E = ops.ext(required=True)
+    torch.manual_seed(B * S + nh)
+    dev, H = "cuda", nh * 64
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    step = torch.tensor([3], dtype=torch.int64, device=dev)
+    qkv = (torch.randn(B * S, 3 * H, device=dev) * 1.5).bfloat16()
+    mask = None
+    if masked:
+        mask = torch.zeros(B, S, device=dev)
+        for b in range(B):
+            mask[b, S - (b * 7) % (S // 4 + 1):] = -10000.0
+    scale = 1 / math.sqrt(64)
+    ctx, dqkv = torch.empty(B * S, H, device=dev, dtype=torch.bfloat16), torch.full_like(qkv, float("nan"))
+    lse = torch.empty(B, nh, S, device=dev)
+    keep_bits = torch.full((B, nh, S, (S + 127) // 128 * 4), -1, dtype=torch.int32, device=dev) if pd > 0 else None
+    E.attn_fwd(qkv, mask, ctx, lse, B, S, nh, scale, pd, seed, step, err, keep_bits)
+    dctx = torch.randn(B * S, H, device=dev).bfloat16()
+    E.attn_bwd(qkv, mask, ctx, dctx, lse, torch.empty_like(lse), dqkv, B, S, nh, scale, pd, err, keep_bits)
+    torch.cuda.synchronize()
+    assert err.item() == 0
+    keep = torch.ones(B, nh, S, S, device=dev, dtype=torch.float64)
+    if pd > 0:
+        zero, u, d = torch.zeros(B, nh, S, S, device=dev, dtype=torch.bfloat16), *(torch.empty(B, nh, S, S, device=dev, dtype=torch.bfloat16) for _ in range(2))
+        E.softmax_fwd(zero, None, u, d, 1.0, pd, seed, step)
+        keep = (d != 0).double() / (1 - pd)
+        assert 0.5 * pd < (d == 0).float().mean().item() < 2 * pd
+    q, k, v = (t.double() for t in qkv.view(B, S, 3, nh, 64).permute(2, 0, 3, 1, 4))
+    g = dctx.double().view(B, S, nh, 64).permute(0, 2, 1, 3)
+    s = q @ k.transpose(-1, -2) * scale + (0 if mask is None else mask.double()[:, None, None])
+    P = torch.softmax(s, -1)
+    Pk = P * keep
+    o = Pk @ v
+    dP = (g @ v.transpose(-1, -2)) * keep
+    D = (P * dP).sum(-1, keepdim=True)
+    dS = P * (dP - D) * scale
+    grads = (dS @ k, dS.transpose(-1, -2) @ q, Pk.transpose(-1, -2) @ g)
+    # bounds: P and dS are rounded to bf16 (2^-9) before their products; the row sums come from the rounded context (2^-9 of sum |dO| |O|);
+    # fp32 scores and exponentials err by about 2^-18 of P; the results are rounded to bf16 (2^-9); doubled
+    ep, u = 2.0 ** -9 + 2.0 ** -17, 2.0 ** -8
+    dD = 2.0 ** -9 * (g.abs() * o.abs()).sum(-1, keepdim=True)
+    eS = ep * dS.abs() + scale * P * (dD + 2.0 ** -17 * (dP.abs() + D.abs()))
+    bounds = (2 * eS @ k.abs(), 2 * eS.transpose(-1, -2) @ q.abs(), 2 * ep * Pk.transpose(-1, -2) @ g.abs())
+    got = [t.double() for t in dqkv.view(B, S, 3, nh, 64).permute(2, 0, 3, 1, 4)]
+    out = ctx.double().view(B, S, nh, 64).permute(0, 2, 1, 3)
+    assert ((out - o).abs() <= 2 * ep * Pk @ v.abs() + u * o.abs() + 1e-6).all()
+    assert ((lse.double() - torch.logsumexp(s, -1)).abs() <= 1e-4).all()
+    for name, a, r, e in zip("qkv", got, grads, bounds):
+        worst = ((a - r).abs() / (e + u * r.abs() + 1e-6)).max().item()
+        assert worst <= 1.0, f"d{name}: {worst} times the bound"
+    return out, got
+
+
+@pytest.mark.parametrize("pd", [0.0, 0.1])
+@pytest.mark.parametrize("B,S,nh", [(1, 64, 1), (3, 128, 2), (2, 256, 3), (1, 512, 2), (1, 1024, 1), (20, 128, 16), (5, 64, 7), (9, 256, 12)])
+def test_attention_matches_fp64(B, S, nh, pd):
+    _run(B, S, nh, pd)
+
+
+def test_attention_without_mask_and_repeatable():
+    a, ga = _run(2, 256, 2, 0.1, masked=False)
+    b, gb = _run(2, 256, 2, 0.1, masked=False)
+    assert torch.equal(a, b) and all(torch.equal(x, y) for x, y in zip(ga, gb))
