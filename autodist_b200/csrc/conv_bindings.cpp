@@ -170,6 +170,11 @@ void set_grid(adb200::ConvParams& p, int GW, int GH, int GN, Patch pt) {
   p.tiles_w = ceil_div(GW, pt.tw); p.tiles_h = ceil_div(GH, pt.th); p.tiles_n = ceil_div(GN, pt.tn);
 }
 
+// Map of the written pixel grid (GW x GH x GN, first pixel at element `off`, strides in elements) for the staged epilogue.
+CUtensorMap grid_map(const void* base, int64_t off, int64_t C, const adb200::ConvParams& p, int64_t sw, int64_t sh, int64_t sn) {
+  return map4(reinterpret_cast<const char*>(base) + off * 2, C, p.GW, p.GH, p.GN, sw, sh, sn, 64, p.tw, p.th, p.tn);
+}
+
 // Tuning aid: when set (int64 CUDA tensor of at least 8 x SM-count words, zeroed by the caller), the next launches record
 // clock64 marks per CTA into it.
 long long* g_trace = nullptr;
@@ -254,6 +259,9 @@ void conv_fprop_impl(const Tensor& x, const Tensor& w, Tensor y, const optional<
     p.stats = stats->data_ptr<float>();
   }
   set_eval_norm(p, norm, y, g.Cout);
+  p.staged = 1;
+  maps.out = grid_map(p.out, 0, g.Cout, p, g.Cout, (int64_t)GW * g.Cout, (int64_t)GH * GW * g.Cout);
+  maps.add = p.addend != nullptr ? grid_map(p.addend, 0, g.Cout, p, g.Cout, (int64_t)GW * g.Cout, (int64_t)GH * GW * g.Cout) : maps.out;
   p.error_flag = error_flag.data_ptr<int>();
   launch(maps, p, bn);
 }
@@ -336,6 +344,11 @@ void conv_dgrad(const Tensor& dy, const Tensor& w, Tensor dx, int64_t stride, in
       p.out = dx.data_ptr(); p.ldc = g.Cin;
       p.addend = addend.has_value() ? reinterpret_cast<const __nv_bfloat16*>(addend->data_ptr()) : nullptr;
       p.os = classes; p.oh0 = ph; p.ow0 = pw;
+      p.staged = 1;
+      const int64_t off = ((int64_t)ph * p.OW + pw) * g.Cin, sw = (int64_t)classes * g.Cin, sh = (int64_t)classes * p.OW * g.Cin,
+                    sn = (int64_t)p.OH * p.OW * g.Cin;
+      maps.out = grid_map(p.out, off, g.Cin, p, sw, sh, sn);
+      maps.add = p.addend != nullptr ? grid_map(p.addend, off, g.Cin, p, sw, sh, sn) : maps.out;
       p.error_flag = error_flag.data_ptr<int>();
       launch(maps, p, bn);
     }
@@ -464,6 +477,12 @@ void conv_rowtap_fprop_impl(const Tensor& xp, const Tensor& wr, Tensor y, const 
     p.stats = stats->data_ptr<float>();
   }
   set_eval_norm(p, norm, y, Cout);
+  maps.out = maps.w;
+  if (!p.wsplit) {            // boxes per patch column hold the pixels in another order: that fallback stores directly
+    p.staged = 1;
+    maps.out = grid_map(p.out, 0, Cout, p, Cout, (int64_t)OW * Cout, (int64_t)OH * OW * Cout);
+  }
+  maps.add = p.staged && p.addend != nullptr ? grid_map(p.addend, 0, Cout, p, Cout, (int64_t)OW * Cout, (int64_t)OH * OW * Cout) : maps.out;
   p.error_flag = error_flag.data_ptr<int>();
   launch(maps, p, bn);
 }

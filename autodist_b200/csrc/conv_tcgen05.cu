@@ -30,7 +30,9 @@ using namespace tc;
 
 template <int BN, int MODE> struct ConvCfg {
   static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int STAGES = (BN == 256) ? 4 : (BN == 128 ? 6 : 8);
+  // Pixel modes keep two output boxes (128 pixels x 64 channels, 16 KB) per half of the epilogue warps; 64-wide tiles share them.
+  static constexpr int STAGING = (MODE == CONV_WGRAD) ? 0 : (BN == 64 ? 2 : 4) * A_BYTES;
+  static constexpr int STAGES = (MODE == CONV_WGRAD) ? (BN == 256 ? 4 : (BN == 128 ? 6 : 8)) : (BN == 256 ? 3 : (BN == 128 ? 4 : 7));
   static constexpr int TMEM_COLS = 2 * BN;
   // Eight epilogue warps: two per TMEM lane quarter, half of the tile's columns each. Layers with a short contraction
   // (1 x 1 convolutions) spend longer draining a tile than multiplying it, and four warps could not keep up.
@@ -38,7 +40,7 @@ template <int BN, int MODE> struct ConvCfg {
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int CHUNKS = BN / 16 / (EPI_WARPS / 4);      // 16-column chunks per epilogue warp
   static constexpr int STAT_BYTES = (MODE == CONV_FPROP || MODE == CONV_EVAL) ? 2 * kMaxStatChannels * 4 : 0;
-  static constexpr int SMEM = STAGES * (A_BYTES + B_BYTES) + 1024 /*align*/ + 256 /*barriers*/ + STAT_BYTES;
+  static constexpr int SMEM = STAGES * (A_BYTES + B_BYTES) + STAGING + 1024 /*align*/ + 256 /*barriers*/ + STAT_BYTES;
 };
 
 struct TileCoord {
@@ -98,6 +100,235 @@ __device__ __forceinline__ float warp_column_sums16(float* v, int lane) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+__device__ __forceinline__ void store_box(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+               ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void sts4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ uint4 lds4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t lds1(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+
+// Epilogue of the pixel modes through shared memory. A 1 x 1 convolution multiplies a tile in a few microseconds, so the drain is
+// what bounds it: direct stores wrote 32 rows in 16-byte pieces per instruction, and the batch-norm sums took 34 shuffles per
+// 16 columns. Here the warps stage boxes of 128 pixels x 64 channels in the 128-byte-swizzled layout (row = pixel of the patch, the
+// order of the input boxes), one thread per half hands a box to the TMA unit, and the sums are taken from the staged
+// bf16 values: lane l adds channels 2l, 2l + 1 over its warp's 32 rows, 32 conflict-free reads per 64 channels. The addend (residual or
+// fork gradient) comes by TMA into the box ahead of the accumulator and is replaced by the result.
+// 64 images, 1 x 1, with sums (without the staging -> now, us): 64 -> 256 channels at 56 x 56 91 -> 34, 128 -> 512 at 28 x 28
+// 52 -> 21.5, 256 -> 1024 at 14 x 14 29 -> 16; input gradient with addend: to 256 channels at 56 x 56 66 -> 44, to 512 at
+// 28 x 28 39 -> 28, to 1024 at 14 x 14 21 -> 13. The staging takes one to two of the operand stages; the 3 x 3 layers, which those
+// feed, did not slow down (256 -> 256 at 14 x 14: 19.5 -> 18.4).
+// Warps: TMEM lane quarter q = warp % 4, half hf: columns [hf * BN / 2, (hf + 1) * BN / 2). BN 256: two boxes per half; 128: one;
+// 64: both halves share a box. Box buffers alternate; they are free again once the issuing thread has seen its copies read.
+template <int BN, int MODE>
+__device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvMaps& maps, long long total, uint32_t tmem_base, uint64_t* tfull,
+                                                uint64_t* tempty, uint64_t* add_bars, uint32_t staging, float* s_stat, bool do_stats,
+                                                volatile int* abort_flag, long long* trace) {
+  constexpr bool EVAL = MODE == CONV_EVAL, FWD = MODE != CONV_DGRAD;
+  constexpr int CW = BN / 2;                           // columns of this warp
+  constexpr int BOXES = BN == 256 ? 2 : 1;             // boxes it takes part in per tile
+  constexpr int PARTY = BN == 64 ? 256 : 128;          // threads that fill a box together
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q = warp & 3, hf = (warp - 2) >> 2;
+  const int r = q * 32 + lane;
+  const int rows = p.tw * p.th * p.tn;
+  const bool issuer = lane == 0 && (BN == 64 ? warp == 2 : (warp - 2) % 4 == 0);
+  const int bar_id = BN == 64 ? 2 : 2 + hf;
+  const uint32_t boxes = staging + (BN == 64 ? 0u : (uint32_t)hf * 2u * A_BYTES);       // two buffers
+  uint64_t* abar = add_bars + (BN == 64 ? 0 : 2 * hf);
+  const uint32_t swz = (uint32_t)(r & 7);
+  const bool add = (MODE == CONV_DGRAD || EVAL) && p.addend != nullptr;
+  const bool bias = FWD && p.bias != nullptr;
+  auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(PARTY) : "memory"); };
+  if constexpr (EVAL) {
+    // y = conv * scale + shift with the layer's running statistics: the per-channel table is built once per CTA while the
+    // first tile is multiplied (in the statistics table's space; the two never occur together)
+    for (int c = threadIdx.x - 64; c < p.Nc; c += 256) {
+      const float sc = p.bn_gamma[c] * rsqrtf(p.bn_var[c] + p.bn_eps);
+      s_stat[c] = sc;
+      s_stat[p.Nc + c] = fmaf(-p.bn_mean[c], sc, p.bn_beta[c]);
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+  }
+  bool ok = true;
+  auto wait = [&](uint64_t* bar, uint32_t parity) {    // a warp that gives up walks on, so that nobody is left behind at a barrier
+    if (ok && !mbar_wait(bar, parity, abort_flag)) { ok = false; *abort_flag = 1; }
+  };
+  int as = 0; uint32_t aphase = 0;
+  uint32_t use[2] = {0, 0};                            // how often each buffer received an addend
+  // Batch-norm sums of this lane's two channels per box (sum, sum, squares, squares), kept in registers while the tiles of this
+  // CTA cover the same channels: atomics on shared memory per tile cost as much as the drain.
+  float acc[BOXES][4];
+  int acc_c0 = -1;
+  auto flush = [&]() {
+    if (acc_c0 < 0) return;
+#pragma unroll
+    for (int g = 0; g < BOXES; ++g) {
+      const int c = (BN == 64 ? acc_c0 : acc_c0 + hf * CW) + 64 * g + 2 * lane;
+      if (c < p.Nc) {
+        atomicAdd(&s_stat[c], acc[g][0]);
+        atomicAdd(&s_stat[c + 1], acc[g][1]);
+        atomicAdd(&s_stat[p.Nc + c], acc[g][2]);
+        atomicAdd(&s_stat[p.Nc + c + 1], acc[g][3]);
+      }
+    }
+  };
+  int buf = 0;
+  for (long long t = blockIdx.x; t < total; t += gridDim.x) {
+    const TileCoord tc_ = decode_tile<BN, MODE>(p, t);
+    const int c_w = tc_.c0 + hf * CW;                  // first column of this warp
+    const int c_box = BN == 64 ? tc_.c0 : c_w;         // first column of its first box
+    const long long tw0 = trace != nullptr ? clock64() : 0;
+    if (issuer) {
+      store_wait_read();                               // the copies of the tile before have left the buffers
+      if (add) {
+#pragma unroll
+        for (int g = 0; g < BOXES; ++g) {
+          const int bb = BOXES == 2 ? g : buf;
+          if (c_box + 64 * g >= p.Nc) continue;
+          mbar_expect_tx(&abar[bb], (uint32_t)rows * 128u);
+          asm volatile(
+              "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+              ::"r"(boxes + (uint32_t)bb * A_BYTES), "l"(&maps.add), "r"(smem_u32(&abar[bb])), "r"(c_box + 64 * g), "r"(tc_.w0), "r"(tc_.h0), "r"(tc_.n0)
+              : "memory");
+        }
+      }
+    }
+    float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);       // four columns of the bias per lane, handed around by shuffles
+    if (bias && lane * 4 < CW) {
+      const int c = c_w + lane * 4;                    // Nc is a multiple of 8: four columns exist together
+      if (c < p.Nc) b4 = make_float4(__ldg(p.bias + c), __ldg(p.bias + c + 1), __ldg(p.bias + c + 2), __ldg(p.bias + c + 3));
+    }
+    bool valid = true;
+    if (do_stats) {
+      const int gw = tc_.w0 + r % p.tw, gh = tc_.h0 + (r / p.tw) % p.th, gn = tc_.n0 + r / (p.tw * p.th);
+      valid = r < rows && gw < p.GW && gh < p.GH && gn < p.GN;
+    }
+    if (!add) meet();                                  // with an addend its arrival says that the buffer may be written
+    wait(&tfull[as], aphase);
+    const long long tw1 = trace != nullptr ? clock64() : 0;
+    tc_fence_after();
+    const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN + hf * CW);
+    if (MODE == CONV_FPROP && do_stats && tc_.c0 != acc_c0) {
+      flush();
+      acc_c0 = tc_.c0;
+#pragma unroll
+      for (int g = 0; g < BOXES; ++g) acc[g][0] = acc[g][1] = acc[g][2] = acc[g][3] = 0.f;
+    }
+    bool released = false;
+#pragma unroll
+    for (int g = 0; g < BOXES; ++g) {
+      const int bb = BOXES == 2 ? g : buf;
+      const int col0 = c_w + 64 * g;                   // first column of this warp in the box
+      if (c_box + 64 * g >= p.Nc) break;               // uniform over the party
+      const uint32_t box = boxes + (uint32_t)bb * A_BYTES;
+      const uint32_t line = box + (uint32_t)r * 128u;
+      if (add) wait(&abar[bb], use[bb] & 1u);
+      if (add) ++use[bb];
+#pragma unroll
+      for (int h = 0; h < CW / 32 / BOXES; ++h) {
+        const int ch = (BN == 64 ? hf * 4 : h * 4);    // first 16-byte chunk of the 32 columns inside the box line
+        const int col = col0 + h * 32;
+        float v[32];
+        __syncwarp();
+        tmem_ld32(t_row + g * 64 + h * 32, v);
+        if (bias) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4) {
+            const int src = (g * 64 + h * 32 + j) >> 2;
+            v[j] += __shfl_sync(0xffffffffu, b4.x, src);
+            v[j + 1] += __shfl_sync(0xffffffffu, b4.y, src);
+            v[j + 2] += __shfl_sync(0xffffffffu, b4.z, src);
+            v[j + 3] += __shfl_sync(0xffffffffu, b4.w, src);
+          }
+        }
+        if constexpr (EVAL) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 8)
+            if (col + j < p.Nc) {                      // Nc is a multiple of 8
+#pragma unroll
+              for (int x = 0; x < 8; ++x) v[j + x] = fmaf(v[j + x], s_stat[col + j + x], s_stat[p.Nc + col + j + x]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t at = line + (((uint32_t)(ch + j) ^ swz) << 4);
+          float* w = v + 8 * j;
+          if (add) {
+            float a[8];
+            unpack8_bf16(lds4(at), a);
+#pragma unroll
+            for (int x = 0; x < 8; ++x) w[x] += a[x];
+          }
+          if (FWD && p.relu) {
+#pragma unroll
+            for (int x = 0; x < 8; ++x) w[x] = EVAL ? (w[x] < 0.f ? 0.f : w[x]) : fmaxf(w[x], 0.f);      // evaluation keeps a NaN
+          }
+          if (do_stats && !valid) {                    // pixels that do not exist count for nothing
+#pragma unroll
+            for (int x = 0; x < 8; ++x) w[x] = 0.f;
+          }
+          sts4(at, pack2(w[0], w[1]), pack2(w[2], w[3]), pack2(w[4], w[5]), pack2(w[6], w[7]));
+        }
+      }
+      if (g == BOXES - 1) {                            // the accumulator has been read
+        tc_fence_before();
+        mbar_arrive(&tempty[as]);
+        released = true;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      meet();
+      if (issuer && ok) store_box(&maps.out, box, c_box + 64 * g, tc_.w0, tc_.h0, tc_.n0);
+      if constexpr (MODE == CONV_FPROP) {
+        if (do_stats) {
+          // statistics of what the next layer reads: the staged bf16 values. 64-wide tiles: each half takes 16 of the quarter's rows.
+          constexpr int NR = BN == 64 ? 16 : 32;
+          const uint32_t base = box + (uint32_t)(q * 32 + (BN == 64 ? hf * 16 : 0)) * 128u;
+#pragma unroll
+          for (int i = 0; i < NR; ++i) {
+            const uint32_t u = lds1(base + (uint32_t)i * 128u + ((((uint32_t)(lane >> 2)) ^ (uint32_t)(i & 7)) << 4) + (uint32_t)(lane & 3) * 4u);
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u));
+            acc[g][0] += f.x; acc[g][1] += f.y;
+            acc[g][2] = fmaf(f.x, f.x, acc[g][2]); acc[g][3] = fmaf(f.y, f.y, acc[g][3]);
+          }
+        }
+      }
+    }
+    if (!released) {                                   // this warp's last columns lie past the matrix
+      tc_fence_before();
+      mbar_arrive(&tempty[as]);
+    }
+    if (trace != nullptr && threadIdx.x == 64) { trace[5] += clock64() - tw1; trace[6] += tw1 - tw0; }
+    if (BOXES == 1) buf ^= 1;
+    if (++as == 2) { as = 0; aphase ^= 1; }
+  }
+  if (MODE == CONV_FPROP && do_stats) flush();
+  if (issuer) {
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");                            // this thread's copies have landed
+    for (int b = 0; add && !ok && b < 2; ++b) {        // addends nobody waited for land before the CTA leaves
+      const long long w0 = clock64();
+      while (!mbar_try(&abar[b], use[b] & 1u) && clock64() - w0 < 2000000LL) {}
+    }
+  }
+  return ok;
+}
+
 template <int BN, int MODE>
 __global__ void __launch_bounds__(ConvCfg<BN, MODE>::THREADS, 1)
 conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvParams p) {
@@ -110,14 +341,16 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
   uint8_t* sB = smem + C::STAGES * A_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::STAGES * (A_BYTES + C::B_BYTES));
+  uint8_t* staging = smem + C::STAGES * (A_BYTES + C::B_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + C::STAGING);
   uint64_t* full = bars;
   uint64_t* empty = bars + C::STAGES;
   uint64_t* tfull = bars + 2 * C::STAGES;
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  float* s_stat = reinterpret_cast<float*>(smem + C::STAGES * (A_BYTES + C::B_BYTES) + 256);
+  uint64_t* add_bars = tempty + 3;                 // pixel modes: two per half of the epilogue warps (behind the slot and the flag)
+  float* s_stat = reinterpret_cast<float*>(staging + C::STAGING + 256);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -126,6 +359,7 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(&tfull[s], 1); mbar_init(&tempty[s], 32 * C::EPI_WARPS); }
+    for (int s = 0; s < 4; ++s) mbar_init(&add_bars[s], 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -277,7 +511,7 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
     const int c_lo = ((warp - 2) >> 2) * C::CHUNKS;      // first 16-column chunk of this warp's share of the tile
     int as = 0; uint32_t aphase = 0; bool ok = true;
     const int r = q * 32 + lane;
-    if (EVAL) {
+    if (EVAL && p.staged == 0) {
       // y = conv * scale + shift with the layer's running statistics: the per-channel table is built once per CTA while the
       // first tile is multiplied (the statistics table's space; the two never occur together)
       for (int c = threadIdx.x - 64; c < p.Nc; c += C::THREADS - 64) {
@@ -298,7 +532,12 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
         for (int jj = 0; jj < 16; ++jj) if (col0 + jj < p.Nc) v[jj] = fmaf(v[jj], s_stat[col0 + jj], s_stat[p.Nc + col0 + jj]);
       }
     };
-    for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
+    bool staged = false;
+    if constexpr (MODE != CONV_WGRAD) {
+      staged = p.staged != 0;
+      if (staged) ok = staged_epilogue<BN, MODE>(p, maps, total, tmem_base, tfull, tempty, add_bars, smem_u32(staging), s_stat, do_stats, abort_flag, trace);
+    }
+    for (long long t = blockIdx.x; t < total && ok && !staged; t += gridDim.x) {
       const TileCoord tc_ = decode_tile<BN, MODE>(p, t);
       if (MODE == CONV_WGRAD && tc_.kend <= tc_.kbeg) continue;
       bool valid;
@@ -316,52 +555,6 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
         off = (long long)row * p.ldc + (long long)p.taps[tc_.tap].wtap * p.wtap_stride;
       }
       const long long tw0 = trace != nullptr ? clock64() : 0;
-      if (MODE == CONV_DGRAD || EVAL) {
-        if (p.addend != nullptr) {
-          // The gradient another consumer of the same tensor produced (a residual fork), or the residual of an evaluated
-          // block, is added to this tile. Its whole
-          // row segment is requested before the wait for the accumulator, so the loads overlap the tile's MMAs, and
-          // the chunk loop below is unrolled so that the prefetched vectors stay in registers.
-          uint4 pre[2 * C::CHUNKS];
-          const int cw0 = tc_.c0 + c_lo * 16;
-          const __nv_bfloat16* src = p.addend + off + cw0;
-#pragma unroll
-          for (int h = 0; h < 2 * C::CHUNKS; ++h) {
-            pre[h] = make_uint4(0, 0, 0, 0);
-            if (valid && cw0 + h * 8 < p.Nc) pre[h] = *reinterpret_cast<const uint4*>(src + h * 8);
-          }
-          if (!mbar_wait(&tfull[as], aphase, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN);
-#pragma unroll
-          for (int c = 0; c < C::CHUNKS; ++c) {
-            const int col0 = cw0 + c * 16;
-            if (col0 < p.Nc) {                     // uniform over the warp
-              float v[16], a[16];
-              __syncwarp();
-              tmem_ld16(t_row + (c_lo + c) * 16, v);
-              unpack8_bf16(pre[2 * c], a);
-              unpack8_bf16(pre[2 * c + 1], a + 8);
-              if (EVAL) affine16(v, col0);
-#pragma unroll
-              for (int jj = 0; jj < 16; ++jj) {
-                v[jj] += a[jj];
-                if (EVAL && p.relu) v[jj] = v[jj] < 0.f ? 0.f : v[jj];
-              }
-              if (valid) {
-                __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + off + col0;
-                store8_bf16(dst, v);                                  // Nc is a multiple of 8: a chunk holds 8 or 16 columns
-                if (col0 + 8 < p.Nc) store8_bf16(dst + 8, v + 8);
-              }
-            }
-          }
-          __syncwarp();
-          tc_fence_before();
-          mbar_arrive(&tempty[as]);
-          if (++as == 2) { as = 0; aphase ^= 1; }
-          continue;
-        }
-      }
       if (!mbar_wait(&tfull[as], aphase, abort_flag)) { ok = false; break; }
       const long long tw1 = trace != nullptr ? clock64() : 0;
       tc_fence_after();
@@ -397,6 +590,10 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
         } else {
           if (FWD) {
             affine16(v, col0);
+            if (EVAL && p.addend != nullptr) {
+#pragma unroll
+              for (int jj = 0; jj < 16; ++jj) if (jj < ncols) v[jj] += __bfloat162float(p.addend[off + col0 + jj]);
+            }
             if (p.relu && EVAL) {                  // like the library's evaluation path: a NaN stays a NaN
 #pragma unroll
               for (int jj = 0; jj < 16; ++jj) v[jj] = v[jj] < 0.f ? 0.f : v[jj];

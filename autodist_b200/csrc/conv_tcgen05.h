@@ -48,6 +48,7 @@ struct ConvParams {
   int accumulate;                 // weight gradient: add into `out` (atomics) instead of overwriting it
   const float* bias;              // forward: per output channel, or null
   int relu;                       // forward: clamp at zero after the bias
+  int staged;                     // pixel modes: the output goes through shared memory and TMA (maps.out, and maps.add with an addend)
   const float* bn_mean;           // CONV_EVAL: running statistics and affine parameters of the batch-norm that follows (after
   const float* bn_var;            //   the bias, before addend and ReLU); [Nc] each
   const float* bn_gamma;
@@ -64,6 +65,8 @@ struct ConvMaps {
   CUtensorMap act[4];             // input (forward / weight gradient) or dY (input gradient), per parity class
   CUtensorMap w;                  // weight
   CUtensorMap dy;                 // weight gradient: dY
+  CUtensorMap out;                // pixel modes with staged output: the written pixel grid, box (64, tw, th, tn)
+  CUtensorMap add;                // the addend over the same grid, same box
 };
 
 cudaError_t launch_conv(const ConvMaps& maps, const ConvParams& p, int bn, int num_sms, cudaStream_t stream);
