@@ -438,6 +438,13 @@ void gather_rows_f32(const Tensor& src, const Tensor& idx, Tensor out) {
   TORCH_CHECK(src.scalar_type() == at::kFloat && src.is_contiguous() && src.size(-1) % 8 == 0, "fp32 contiguous table, width a multiple of 8");
   adb200::gather_rows_f32(src.data_ptr<float>(), idx.data_ptr<int64_t>(), BF(out), idx.numel(), src.size(-1), STREAM);
 }
+// dst[idx[r]] += src[r] (fp32 both); every index must be a row of dst.
+void scatter_add_rows_f32(Tensor dst, const Tensor& idx, const Tensor& src) {
+  TORCH_CHECK(dst.is_cuda() && dst.dim() == 2 && dst.is_contiguous() && dst.scalar_type() == at::kFloat && src.is_contiguous() &&
+              src.scalar_type() == at::kFloat && idx.is_contiguous() && idx.scalar_type() == at::kLong && src.numel() == idx.numel() * dst.size(1),
+              "dst [V, H] and src [n, H] must be contiguous fp32, idx int64 [n]");
+  adb200::scatter_add_rows_f32(dst.data_ptr<float>(), idx.data_ptr<int64_t>(), src.data_ptr<float>(), idx.numel(), dst.size(1), STREAM);
+}
 void scatter_add_rows_bf16(Tensor dst, const Tensor& idx, const Tensor& src) {
   adb200::scatter_add_rows_bf16(BF(dst), idx.data_ptr<int64_t>(), CBF(src), idx.numel(), src.size(-1), STREAM);
 }
@@ -858,6 +865,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("colsum_parts", &adb200::colsum_parts);
   m.def("embed_sum", &embed_sum);
   m.def("scatter_add_rows", &scatter_add_rows);
+  m.def("scatter_add_rows_f32", &scatter_add_rows_f32);
   m.def("strided_rowsum", &strided_rowsum);
   m.def("keyed_colsum", &keyed_colsum);
   m.def("gather_rows", &gather_rows);

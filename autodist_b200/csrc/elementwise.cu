@@ -375,6 +375,24 @@ __global__ void scatter_add_rows_kernel(float* __restrict__ dst, const int64_t* 
 }
 
 // out[k][c] = sum over rows r = k + j*stride (j < count) of x[r][c]: position-embedding gradient (k = position).
+// The same with fp32 source rows: one thread per four columns (vector atomics when the rows are 16-byte aligned). Replaces the
+// sort-based embedding gradient of the library: 16384 rows of 192 took 16 radix-sort passes and a dozen helpers, 0.3 ms.
+__global__ void scatter_add_rows_f32_kernel(float* __restrict__ dst, const int64_t* __restrict__ idx, const float* __restrict__ src,
+                                            long long total, int h4, int H, int vec) {
+  pdl_sync();
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  const long long row = t / h4;
+  const int c = (int)(t % h4) * 4;
+  const float* a = src + row * H + c;
+  float* d = dst + idx[row] * (long long)H + c;
+  if (vec) {
+    atomicAdd(reinterpret_cast<float4*>(d), *reinterpret_cast<const float4*>(a));
+  } else {
+    for (int j = 0; j < 4 && c + j < H; ++j) atomicAdd(d + j, a[j]);
+  }
+}
+
 __global__ void strided_rowsum_kernel(const bf16* __restrict__ x, float* __restrict__ out, int keys, int stride, int count, int H) {
   pdl_sync();
   const int k = blockIdx.y;
@@ -1655,6 +1673,11 @@ void embed_sum(const bf16* word, const bf16* pos, const bf16* type, const int64_
 }
 void scatter_add_rows(float* dst, const int64_t* idx, const bf16* src, int rows, int H, float scale, cudaStream_t st) {
   launch_pdl(scatter_add_rows_kernel, dim3(blocks_for(rows, 4)), dim3(128), 0, st, dst, idx, src, rows, H, scale);
+}
+void scatter_add_rows_f32(float* dst, const int64_t* idx, const float* src, long long rows, int H, cudaStream_t st) {
+  const int h4 = (H + 3) / 4;
+  const int vec = H % 4 == 0 && ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0;
+  if (rows > 0) launch_pdl(scatter_add_rows_f32_kernel, dim3(blocks_for(rows * h4, 256)), dim3(256), 0, st, dst, idx, src, rows * h4, h4, H, vec);
 }
 void strided_rowsum(const bf16* x, float* out, int keys, int stride, int count, int H, cudaStream_t st) {
   dim3 grid(blocks_for(H / 8, 128), keys);

@@ -16,6 +16,7 @@ void ln_bwd(const bf16_t* dy, const bf16_t* z, const float* mean, const float* r
 void embed_sum(const bf16_t* word, const bf16_t* pos, const bf16_t* type, const int64_t* ids, const int64_t* tt, bf16_t* z, int rows, int S,
                int H, long long V, long long types, int* error, cudaStream_t st);
 void scatter_add_rows(float* dst, const int64_t* idx, const bf16_t* src, int rows, int H, float scale, cudaStream_t st);
+void scatter_add_rows_f32(float* dst, const int64_t* idx, const float* src, long long rows, int H, cudaStream_t st);
 void strided_rowsum(const bf16_t* x, float* out, int keys, int stride, int count, int H, cudaStream_t st);
 int colsum_parts(int rows);
 void keyed_colsum(const bf16_t* x, const int64_t* key, float* part, float* out, int rows, int H, int keys, int accumulate, cudaStream_t st);

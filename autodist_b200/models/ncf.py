@@ -13,7 +13,7 @@ import torch
 from torch import nn
 import torch.nn.functional as F
 
-from autodist_b200.ops.functional import Linear
+from autodist_b200.ops.functional import Linear, dense_lookup
 
 
 @dataclass
@@ -50,11 +50,14 @@ class NeuMF(nn.Module):
 
     def logits(self, users, items):
         c = self.config
-        sparse = not c.dense_gradient
-        u = F.embedding(users, self.user_emb, sparse=sparse)
-        i = F.embedding(items, self.item_emb, sparse=sparse)
-        gmf = u[:, :c.mf_dim] * i[:, :c.mf_dim]
-        x = torch.cat([u[:, c.mf_dim:], i[:, c.mf_dim:]], 1)
+        if c.dense_gradient:
+            u, i = dense_lookup(self.user_emb, users), dense_lookup(self.item_emb, items)
+        else:
+            u, i = F.embedding(users, self.user_emb, sparse=True), F.embedding(items, self.item_emb, sparse=True)
+        parts = [c.mf_dim, c.layers[0] // 2]
+        (um, ul), (im, il) = u.split(parts, 1), i.split(parts, 1)
+        gmf = um * im
+        x = torch.cat([ul, il], 1)
         for layer in self.mlp:
             x = F.relu(layer(x)).to(gmf.dtype)
         return self.head(torch.cat([gmf, x], 1)).squeeze(1)

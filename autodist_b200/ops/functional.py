@@ -4,6 +4,7 @@
 produced in fp32). On CPU tensors the same functions fall back to the plain PyTorch expression, which is also the
 numerics reference of the tests.
 """
+import os
 import warnings
 
 import torch
@@ -586,6 +587,42 @@ class _SparseLookupFn(torch.autograd.Function):
         with warnings.catch_warnings():
             warnings.simplefilter("ignore")                                   # the library's notice that invariants are unchecked
             return torch.sparse_coo_tensor(flat[None], vals, ctx.shape, check_invariants=False), None
+
+
+class _DenseLookupFn(torch.autograd.Function):
+    """Rows ``ids`` of an fp32 table whose gradient lives in an engine's flat buffer: the backward pass adds the gradient rows
+    straight into it (no sort, no table-sized temporary, no accumulation pass)."""
+
+    @staticmethod
+    def forward(ctx, table, ids):
+        ctx.save_for_backward(ids)
+        ctx.table = table
+        _count_use(ctx, table, 0)
+        return F.embedding(ids, table)
+
+    @staticmethod
+    def backward(ctx, dy):
+        (ids,) = ctx.saved_tensors
+        acc = _direct_grad(ctx.table)
+        rows = dy.reshape(-1, dy.shape[-1]).float().contiguous()
+        flat = ids.reshape(-1).contiguous()
+        if acc is None:
+            acc = torch.zeros(ctx.table.shape, dtype=torch.float32, device=dy.device)
+            ops.ext(required=True).scatter_add_rows_f32(acc, flat, rows)
+            return acc.to(ctx.table.dtype), None
+        ops.ext(required=True).scatter_add_rows_f32(acc, flat, rows)
+        _grad_written(ctx.table)
+        return None, None
+
+
+def dense_lookup(table, ids):
+    """``F.embedding(ids, table)``. Where an engine keeps the table's gradient in a flat buffer, the gradient rows are added
+    into it by atomics (the order of addition varies); deterministic runs and all other tables use the library."""
+    direct = table.is_cuda and table.dtype == torch.float32 and table.dim() == 2 and ids.dtype == torch.int64 and _direct_grad(table) is not None
+    if direct and torch.is_grad_enabled() and os.environ.get("AUTODIST_DETERMINISTIC") != "1" and \
+            not torch.are_deterministic_algorithms_enabled():
+        return _DenseLookupFn.apply(table, ids)
+    return F.embedding(ids, table)
 
 
 class _ShardedLookupFn(torch.autograd.Function):
