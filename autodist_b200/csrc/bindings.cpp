@@ -445,6 +445,26 @@ void scatter_add_rows_f32(Tensor dst, const Tensor& idx, const Tensor& src) {
               "dst [V, H] and src [n, H] must be contiguous fp32, idx int64 [n]");
   adb200::scatter_add_rows_f32(dst.data_ptr<float>(), idx.data_ptr<int64_t>(), src.data_ptr<float>(), idx.numel(), dst.size(1), STREAM);
 }
+// One step of a whole-sequence LSTM layer: gates bf16 [B, 4S] (i, j, f, o), c fp32 [B, S], h / dh / dgates bf16; S a multiple of 4.
+void check_lstm_seq(const Tensor& gates, const Tensor& c_prev, const Tensor& c, const Tensor& h) {
+  const int64_t n = c_prev.numel();
+  for (const Tensor& t : {gates, c_prev, c, h})
+    TORCH_CHECK(t.is_cuda() && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, "contiguous 16-byte aligned CUDA tensors needed");
+  TORCH_CHECK(c_prev.dim() == 2 && c_prev.size(1) % 4 == 0 && gates.numel() == 4 * n && c.numel() == n && h.numel() == n &&
+              gates.scalar_type() == at::kBFloat16 && h.scalar_type() == at::kBFloat16 && c_prev.scalar_type() == at::kFloat && c.scalar_type() == at::kFloat,
+              "gates bf16 [B, 4S], c fp32 [B, S], h bf16 [B, S], S a multiple of 4");
+}
+void lstm_seq_fwd(const Tensor& gates, const Tensor& c_prev, Tensor c, Tensor h, double forget_bias) {
+  check_lstm_seq(gates, c_prev, c, h);
+  adb200::lstm_seq_fwd(CBF(gates), c_prev.data_ptr<float>(), c.data_ptr<float>(), BF(h), c_prev.size(0), c_prev.size(1), (float)forget_bias, STREAM);
+}
+void lstm_seq_bwd(const Tensor& gates, const Tensor& c_prev, const Tensor& c, const Tensor& dh, const optional<Tensor>& dc_next, Tensor dgates,
+                  Tensor dc_prev, double forget_bias) {
+  check_lstm_seq(gates, c_prev, c, dh);
+  check_lstm_seq(dgates, dc_prev, c, dh);
+  adb200::lstm_seq_bwd(CBF(gates), c_prev.data_ptr<float>(), c.data_ptr<float>(), CBF(dh), OPT_F(dc_next), BF(dgates), dc_prev.data_ptr<float>(),
+                       c_prev.size(0), c_prev.size(1), (float)forget_bias, STREAM);
+}
 void scatter_add_rows_bf16(Tensor dst, const Tensor& idx, const Tensor& src) {
   adb200::scatter_add_rows_bf16(BF(dst), idx.data_ptr<int64_t>(), CBF(src), idx.numel(), src.size(-1), STREAM);
 }
@@ -866,6 +886,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embed_sum", &embed_sum);
   m.def("scatter_add_rows", &scatter_add_rows);
   m.def("scatter_add_rows_f32", &scatter_add_rows_f32);
+  m.def("lstm_seq_fwd", &lstm_seq_fwd);
+  m.def("lstm_seq_bwd", &lstm_seq_bwd);
   m.def("strided_rowsum", &strided_rowsum);
   m.def("keyed_colsum", &keyed_colsum);
   m.def("gather_rows", &gather_rows);

@@ -934,6 +934,71 @@ __global__ void lstm_cell_bwd_kernel(const float* __restrict__ gates, const floa
   dc_prev[idx] = dct * sf;
 }
 
+// The cell of a whole-sequence layer: gates, dh and dgates are bf16 (what the products around it write and read), four columns per
+// thread with 8- and 16-byte accesses, S a multiple of 4. dc_next may be null (the last step); it may alias dc_prev.
+__device__ __forceinline__ void load4b(const bf16* p, float* v) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void store4b(bf16* p, const float* v) {
+  __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+}
+__global__ void lstm_seq_fwd_kernel(const bf16* __restrict__ gates, const float* __restrict__ c_prev, float* __restrict__ c, bf16* __restrict__ h,
+                                    int B, int S, float forget_bias) {
+  pdl_sync();
+  const int s4 = S / 4;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)B * s4) return;
+  const long long b = t / s4;
+  const int s = (int)(t % s4) * 4;
+  const bf16* g = gates + b * 4 * S + s;
+  const long long at = b * S + s;
+  float i[4], j[4], f[4], o[4], hv[4];
+  load4b(g, i); load4b(g + S, j); load4b(g + 2 * S, f); load4b(g + 3 * S, o);
+  const float4 cp = *reinterpret_cast<const float4*>(c_prev + at);
+  float cn[4] = {cp.x, cp.y, cp.z, cp.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    cn[e] = sigmoidf_(f[e] + forget_bias) * cn[e] + sigmoidf_(i[e]) * tanhf(j[e]);
+    hv[e] = sigmoidf_(o[e]) * tanhf(cn[e]);
+  }
+  *reinterpret_cast<float4*>(c + at) = make_float4(cn[0], cn[1], cn[2], cn[3]);
+  store4b(h + at, hv);
+}
+__global__ void lstm_seq_bwd_kernel(const bf16* __restrict__ gates, const float* __restrict__ c_prev, const float* __restrict__ c,
+                                    const bf16* __restrict__ dh, const float* dc_next, bf16* __restrict__ dgates, float* dc_prev, int B, int S,
+                                    float forget_bias) {
+  pdl_sync();
+  const int s4 = S / 4;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)B * s4) return;
+  const long long b = t / s4;
+  const int s = (int)(t % s4) * 4;
+  const bf16* g = gates + b * 4 * S + s;
+  bf16* dg = dgates + b * 4 * S + s;
+  const long long at = b * S + s;
+  float i[4], j[4], f[4], o[4], d[4], dc[4] = {0, 0, 0, 0};
+  load4b(g, i); load4b(g + S, j); load4b(g + 2 * S, f); load4b(g + 3 * S, o); load4b(dh + at, d);
+  const float4 cp4 = *reinterpret_cast<const float4*>(c_prev + at), c4 = *reinterpret_cast<const float4*>(c + at);
+  if (dc_next != nullptr) { const float4 n4 = *reinterpret_cast<const float4*>(dc_next + at); dc[0] = n4.x; dc[1] = n4.y; dc[2] = n4.z; dc[3] = n4.w; }
+  const float cp[4] = {cp4.x, cp4.y, cp4.z, cp4.w}, cc[4] = {c4.x, c4.y, c4.z, c4.w};
+  float di[4], dj[4], df[4], dv[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float si = sigmoidf_(i[e]), tj = tanhf(j[e]), sf = sigmoidf_(f[e] + forget_bias), so = sigmoidf_(o[e]), tc = tanhf(cc[e]);
+    const float dct = dc[e] + d[e] * so * (1.0f - tc * tc);
+    di[e] = dct * tj * si * (1.0f - si);
+    dj[e] = dct * si * (1.0f - tj * tj);
+    df[e] = dct * cp[e] * sf * (1.0f - sf);
+    dv[e] = d[e] * tc * so * (1.0f - so);
+    dc[e] = dct * sf;
+  }
+  store4b(dg, di); store4b(dg + S, dj); store4b(dg + 2 * S, df); store4b(dg + 3 * S, dv);
+  *reinterpret_cast<float4*>(dc_prev + at) = make_float4(dc[0], dc[1], dc[2], dc[3]);
+}
+
 // ------------------------------------------------------------------------------------------------ global-norm clip (K19)
 // acc += weight * sum(x^2); later x *= min(1, max_norm / (sqrt(acc) + 1e-6)). The norm never visits the host.
 __global__ void sumsq_kernel(const float* __restrict__ x, long long n, float* __restrict__ acc, float weight) {
@@ -1775,6 +1840,13 @@ void lstm_cell_fwd(const float* gates, const float* c_prev, float* c, bf16* h, i
 void lstm_cell_bwd(const float* gates, const float* c_prev, const float* c, const float* dh, const float* dc_next, float* dgates,
                    float* dc_prev, int B, int S, float fb, cudaStream_t st) {
   launch_pdl(lstm_cell_bwd_kernel, dim3(blocks_for((long long)B * S, 256)), dim3(256), 0, st, gates, c_prev, c, dh, dc_next, dgates, dc_prev, B, S, fb);
+}
+void lstm_seq_fwd(const bf16* gates, const float* c_prev, float* c, bf16* h, int B, int S, float fb, cudaStream_t st) {
+  launch_pdl(lstm_seq_fwd_kernel, dim3(blocks_for((long long)B * (S / 4), 128)), dim3(128), 0, st, gates, c_prev, c, h, B, S, fb);
+}
+void lstm_seq_bwd(const bf16* gates, const float* c_prev, const float* c, const bf16* dh, const float* dc_next, bf16* dgates, float* dc_prev, int B,
+                  int S, float fb, cudaStream_t st) {
+  launch_pdl(lstm_seq_bwd_kernel, dim3(blocks_for((long long)B * (S / 4), 128)), dim3(128), 0, st, gates, c_prev, c, dh, dc_next, dgates, dc_prev, B, S, fb);
 }
 void sumsq(const float* x, long long n, float* acc, float weight, cudaStream_t st) {
   const int blocks = (int)(n / 1024 + 1 < 592 ? n / 1024 + 1 : 592);

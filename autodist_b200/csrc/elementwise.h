@@ -17,6 +17,9 @@ void embed_sum(const bf16_t* word, const bf16_t* pos, const bf16_t* type, const 
                int H, long long V, long long types, int* error, cudaStream_t st);
 void scatter_add_rows(float* dst, const int64_t* idx, const bf16_t* src, int rows, int H, float scale, cudaStream_t st);
 void scatter_add_rows_f32(float* dst, const int64_t* idx, const float* src, long long rows, int H, cudaStream_t st);
+void lstm_seq_fwd(const bf16_t* gates, const float* c_prev, float* c, bf16_t* h, int B, int S, float fb, cudaStream_t st);
+void lstm_seq_bwd(const bf16_t* gates, const float* c_prev, const float* c, const bf16_t* dh, const float* dc_next, bf16_t* dgates, float* dc_prev,
+                  int B, int S, float fb, cudaStream_t st);
 void strided_rowsum(const bf16_t* x, float* out, int keys, int stride, int count, int H, cudaStream_t st);
 int colsum_parts(int rows);
 void keyed_colsum(const bf16_t* x, const int64_t* key, float* part, float* out, int rows, int H, int keys, int accumulate, cudaStream_t st);

@@ -12,7 +12,7 @@ import torch
 from torch import nn
 import torch.nn.functional as F
 
-from autodist_b200.ops.functional import linear, lstm_cell, sparse_lookup
+from autodist_b200.ops.functional import linear, lstm_layer, sparse_lookup
 
 
 @dataclass
@@ -75,15 +75,7 @@ class LM1B(nn.Module):
         inputs = sparse_lookup(self.emb, x).to(dt)               # row-sparse gradient: only the looked-up rows travel
         if self.training and c.keep_prob < 1.0:
             inputs = F.dropout(inputs, 1.0 - c.keep_prob)
-        h = torch.zeros(Bsz, c.projected_size, dtype=dt, device=x.device)
-        cell = torch.zeros(Bsz, c.state_size, dtype=torch.float32, device=x.device)
-        outs = []
-        for t in range(T):
-            gates = linear(torch.cat([inputs[:, t], h], 1), self.W, self.B)
-            cell, hidden = lstm_cell(gates, cell, 1.0)
-            h = linear(hidden.to(dt), self.W_P)
-            outs.append(h)
-        out = torch.stack(outs, 1).reshape(Bsz * T, c.projected_size)
+        out = lstm_layer(inputs, self.W, self.B, self.W_P, 1.0).reshape(Bsz * T, c.projected_size)
         if self.training and c.keep_prob < 1.0:
             out = F.dropout(out, 1.0 - c.keep_prob)
         # sampled softmax: true class + shared log-uniform negatives, logits corrected by -log(expected count)

@@ -144,6 +144,95 @@ def lstm_cell(gates, c_prev, forget_bias=1.0):
     return c, torch.sigmoid(o) * torch.tanh(c)
 
 
+class _LSTMLayerFn(torch.autograd.Function):
+    """A projected LSTM layer over a whole sequence. Per step: one product for the gates, the cell, one product for the
+    projection, which lands in the next step's operand; backward likewise, the gradient of the carried state being added in the
+    product's epilogue. The weight gradients are one product each over all steps instead of one read-modify-write of the
+    gradient buffer per step."""
+
+    @staticmethod
+    def forward(ctx, inputs, weight, bias, proj, forget_bias):
+        E = ops.ext(required=True)
+        dev, err = inputs.device, _error_flag(inputs.device)
+        B, T, D = inputs.shape
+        P, S = proj.shape
+        w16, p16, b32 = _bf16_weight(weight), _bf16_weight(proj), bias.detach().float().contiguous()
+        xh = torch.empty(T + 1, B, D + P, dtype=torch.bfloat16, device=dev)           # [x_t, h_{t-1}]; the last slot only holds h
+        xh[:T, :, :D].copy_(inputs.transpose(0, 1))
+        xh[0, :, D:].zero_()
+        gates = torch.empty(T, B, 4 * S, dtype=torch.bfloat16, device=dev)
+        c = torch.empty(T + 1, B, S, dtype=torch.float32, device=dev)
+        c[0].zero_()
+        hid = torch.empty(T, B, S, dtype=torch.bfloat16, device=dev)
+        for t in range(T):
+            E.gemm(xh[t], w16, gates[t], False, False, 1, b32, None, None, 1.0, 0.0, err, 0)
+            E.lstm_seq_fwd(gates[t], c[t], c[t + 1], hid[t], forget_bias)
+            E.gemm(hid[t], p16, xh[t + 1, :, D:], False, False, 0, None, None, None, 1.0, 0.0, err, 0)
+        ctx.save_for_backward(xh, gates, c, hid, w16, p16)
+        ctx.params, ctx.fb, ctx.dims, ctx.x_dtype = (weight, bias, proj), forget_bias, (B, T, D, P, S), inputs.dtype
+        for k, p in ((1, weight), (2, bias), (3, proj)):
+            _count_use(ctx, p, k)
+        return xh[1:, :, D:].transpose(0, 1).contiguous()                             # [B, T, P]
+
+    @staticmethod
+    def backward(ctx, dout):
+        E = ops.ext(required=True)
+        xh, gates, c, hid, w16, p16 = ctx.saved_tensors
+        weight, bias, proj = ctx.params
+        B, T, D, P, S = ctx.dims
+        dev, err = dout.device, _error_flag(dout.device)
+        # slot t: gradient of [x_t, h_{t-1}]; h_{t-1} starts with what the layer's output brings
+        dxh = torch.empty(T + 1, B, D + P, dtype=torch.bfloat16, device=dev)
+        dxh[:T, :, :D].zero_()
+        dxh[0, :, D:].zero_()
+        dxh[1:, :, D:].copy_(dout.transpose(0, 1))
+        dgates = torch.empty_like(gates)
+        dhid = torch.empty(B, S, dtype=torch.bfloat16, device=dev)
+        dc = torch.empty(B, S, dtype=torch.float32, device=dev)
+        for t in range(T - 1, -1, -1):
+            E.gemm(dxh[t + 1, :, D:], p16, dhid, False, True, 0, None, None, None, 1.0, 0.0, err, 0)
+            E.lstm_seq_bwd(gates[t], c[t], c[t + 1], dhid, dc if t + 1 < T else None, dgates[t], dc, ctx.fb)
+            E.gemm(dgates[t], w16, dxh[t], False, True, 4, None, None, dxh[t], 1.0, 0.0, err, 0)
+        rows = T * B
+        dg2, x2, h2 = dgates.view(rows, 4 * S), xh[:T].view(rows, D + P), hid.view(rows, S)
+        dh2 = dxh[1:].view(rows, D + P)[:, D:]
+        grads = []
+        for p, a, b in ((weight, dg2, x2), (proj, dh2, h2)):
+            acc = _direct_grad(p)
+            g = acc if acc is not None else torch.empty(p.shape, dtype=torch.float32, device=dev)
+            E.gemm(a, b, g, True, True, 0, None, None, None, 1.0, 1.0 if acc is not None else 0.0, err, 0)
+            if acc is not None:
+                _grad_written(p)
+            grads.append(None if acc is not None else g.to(p.dtype))
+        acc = _direct_grad(bias)
+        db = acc if acc is not None else torch.empty(4 * S, dtype=torch.float32, device=dev)
+        E.keyed_colsum(dg2, None, torch.empty(E.colsum_parts(rows) * 4 * S, dtype=torch.float32, device=dev), db, 1, acc is not None)
+        if acc is not None:
+            _grad_written(bias)
+        dx = dxh[:T, :, :D].transpose(0, 1).to(ctx.x_dtype) if ctx.needs_input_grad[0] else None
+        return dx, grads[0], None if acc is not None else db.to(bias.dtype), grads[1], None
+
+
+def lstm_layer(inputs, weight, bias, proj, forget_bias=1.0):
+    """Outputs ``[B, T, P]`` of a projected LSTM over ``inputs`` [B, T, D] from a zero state: ``gates = [x_t, h] @ weight.T + bias``
+    (order i, j, f, o), ``h = (o * tanh(c)) @ proj.T``."""
+    B, T, D = inputs.shape
+    P, S = proj.shape
+    fused = inputs.is_cuda and B > 0 and T > 0 and D % 8 == 0 and P % 8 == 0 and S % 8 == 0 and \
+        tuple(weight.shape) == (4 * S, D + P) and bias is not None and bias.numel() == 4 * S and \
+        getattr(weight, "_gathered", None) is None and getattr(proj, "_gathered", None) is None
+    if fused:
+        return _LSTMLayerFn.apply(inputs, weight, bias, proj, float(forget_bias))
+    h = torch.zeros(B, P, dtype=inputs.dtype, device=inputs.device)
+    cell = torch.zeros(B, S, dtype=torch.float32, device=inputs.device)
+    outs = []
+    for t in range(T):
+        cell, hidden = lstm_cell(linear(torch.cat([inputs[:, t], h], 1), weight, bias), cell, forget_bias)
+        h = linear(hidden.to(inputs.dtype), proj)
+        outs.append(h)
+    return torch.stack(outs, 1)
+
+
 def clip_by_global_norm_(grads, max_norm, weights=None, all_reduce=None):
     """Scale fp32 CUDA gradients in place so that their joint L2 norm is at most ``max_norm``; the norm stays on the
     device. ``weights`` weighs each tensor's squared sum (replicated tensors count once across ranks);
