@@ -1,10 +1,14 @@
 // Python bindings of the implicit-GEMM convolution: geometry -> patch shape, filter-tap table and tensor maps.
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <torch/extension.h>
 
+#include <algorithm>
+#include <array>
+#include <map>
 #include <mutex>
 
 #include "conv_tcgen05.h"
@@ -66,7 +70,7 @@ struct Patch { int tw, th, tn; };
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Patch of at most `limit` pixels (exactly `limit` when `exact`) that wastes the fewest rows over the grid.
-Patch choose_patch(int GW, int GH, int GN, int limit, bool exact, bool wsplit) {
+Patch search_patch(int GW, int GH, int GN, int limit, bool exact, bool wsplit) {
   Patch best{1, 1, 1};
   double best_eff = -1.0;
   long long best_area = 0;
@@ -93,6 +97,19 @@ Patch choose_patch(int GW, int GH, int GN, int limit, bool exact, bool wsplit) {
   }
   TORCH_CHECK(best_eff > 0, "no patch shape fits this convolution");
   return best;
+}
+
+// The search walks some 700 shapes (7 us of host time, a third of an eager layer's launch), so its answers are kept per thread,
+// by sizes alone; a program has a few dozen geometries, a sweep over many more starts over.
+Patch choose_patch(int GW, int GH, int GN, int limit, bool exact, bool wsplit) {
+  thread_local std::map<std::array<int, 6>, Patch> known;
+  const std::array<int, 6> key{GW, GH, GN, limit, exact ? 1 : 0, wsplit ? 1 : 0};
+  const auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  const Patch p = search_patch(GW, GH, GN, limit, exact, wsplit);
+  if (known.size() >= 1024) known.clear();
+  known.emplace(key, p);
+  return p;
 }
 
 int pick_bn(int n) { return n >= 256 ? 256 : (n > 64 ? 128 : 64); }
@@ -277,6 +294,39 @@ void conv_fprop_bn_eval(const Tensor& x, const Tensor& w, Tensor y, const option
                         int64_t pad, Tensor error_flag) {
   const EvalNorm n{&gamma, &beta, &mean, &var, eps, &residual};
   conv_fprop_impl(x, w, y, bias, relu, c10::nullopt, stride, pad, error_flag, &n);
+}
+
+// The same from and to logical [N, C, H, W] tensors (channels-last in memory, any float type in), with every check and allocation
+// made here: an eager evaluation pass is bounded by host time, and the Python steps around the call cost as much as the launch.
+// Returns nothing where the kernel does not apply or where a transform (vmap, forward-mode derivatives, subclasses) watches the
+// tensors; the caller then takes its general route.
+optional<Tensor> conv_bn_eval_nchw(const Tensor& x, const Tensor& w, const optional<Tensor>& bias, int64_t stride, int64_t pad, const Tensor& gamma,
+                                   const Tensor& beta, const Tensor& mean, const Tensor& var, double eps, bool relu,
+                                   const optional<Tensor>& residual, Tensor error_flag) {
+  if (at::GradMode::is_enabled() || !x.is_cuda() || x.dim() != 4 || w.dim() != 4 || (stride != 1 && stride != 2) || x.numel() == 0) return c10::nullopt;
+  const int64_t cout = w.size(0), kh = w.size(1), kw = w.size(2), cin = w.size(3);
+  if (cin % 8 || cout % 8 || cout > adb200::kMaxStatChannels || kh * kw > adb200::kMaxConvTaps || x.size(1) != cin ||
+      w.scalar_type() != at::kBFloat16 || !w.is_contiguous() || w.device() != x.device()) return c10::nullopt;
+  auto watched = [](const Tensor& t) { return at::isTensorSubclassLike(t) || t._fw_grad(0).defined(); };
+  if (watched(x) || watched(w)) return c10::nullopt;
+  for (const Tensor* t : {&gamma, &beta, &mean, &var})
+    if (t->device() != x.device() || t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() != cout || watched(*t)) return c10::nullopt;
+  if (bias.has_value() && (bias->scalar_type() != at::kFloat || !bias->is_contiguous() || bias->numel() != cout || bias->device() != x.device() ||
+                           watched(*bias))) return c10::nullopt;
+  const int64_t oh = (x.size(2) + 2 * pad - kh) / stride + 1, ow = (x.size(3) + 2 * pad - kw) / stride + 1;
+  if (oh < 1 || ow < 1 || (stride == 2 && (x.size(2) < 2 || x.size(3) < 2))) return c10::nullopt;
+  optional<Tensor> res;
+  if (residual.has_value()) {
+    if (residual->scalar_type() != at::kBFloat16 || residual->device() != x.device() || watched(*residual) ||
+        residual->sizes() != at::IntArrayRef({x.size(0), cout, oh, ow})) return c10::nullopt;
+    res = residual->permute({0, 2, 3, 1}).contiguous();
+  }
+  const c10::cuda::CUDAGuard guard(x.device());
+  const Tensor xh = x.permute({0, 2, 3, 1}).to(at::kBFloat16).contiguous();
+  Tensor y = at::empty({x.size(0), oh, ow, cout}, xh.options());
+  const EvalNorm n{&gamma, &beta, &mean, &var, eps, &res};
+  conv_fprop_impl(xh, w, y, bias, relu, c10::nullopt, stride, pad, error_flag, &n);
+  return y.permute({0, 3, 1, 2});
 }
 
 // dx = the input gradient of conv(x, w) given dy. Every element of dx is written.
@@ -539,6 +589,7 @@ void register_conv(pybind11::module& m) {
   m.def("conv_set_trace", &conv_set_trace);
   m.def("conv_fprop", &conv_fprop);
   m.def("conv_fprop_bn_eval", &conv_fprop_bn_eval);
+  m.def("conv_bn_eval_nchw", &conv_bn_eval_nchw);
   m.def("conv_rowtap_fprop_bn_eval", &conv_rowtap_fprop_bn_eval);
   namespace py = pybind11;
   m.def("conv_dgrad", &conv_dgrad, py::arg("dy"), py::arg("w"), py::arg("dx"), py::arg("stride"), py::arg("pad"), py::arg("error_flag"),

@@ -103,7 +103,12 @@ _ARENA = _StatsArena()
 def _hooked(*modules):
     """Whether a forward hook watches one of ``modules`` (their outputs must then exist on their own)."""
     m = nn.modules.module
-    return bool(m._global_forward_hooks or m._global_forward_pre_hooks) or any(x._forward_hooks or x._forward_pre_hooks for x in modules)
+    if m._global_forward_hooks or m._global_forward_pre_hooks:
+        return True
+    for x in modules:
+        if x._forward_hooks or x._forward_pre_hooks:
+            return True
+    return False
 
 
 class ConvBN(nn.Module):
@@ -118,12 +123,12 @@ class ConvBN(nn.Module):
 
     def forward(self, x, residual=None, in_fork=None, res_fork=None):
         """``in_fork`` / ``res_fork``: the ``GradFork`` of ``x`` / of ``residual`` when that tensor has a second consumer."""
-        cout = self.conv.out_channels
-        if not self.bn.training and x.is_cuda and CONV_MODE != "library" and NORM_POOL_MODE != "library" and not _hooked(self.conv, self.bn) \
-                and not self.conv.relu and type(self.bn) is BatchNormAct:
-            bn = self.bn
-            y = conv_bn_eval(x, self.conv.weight, self.conv.bias, self.conv.stride, self.conv.padding, bn.weight, bn.bias, bn.running_mean,
-                             bn.running_var, bn.eps, bn.relu, residual)
+        conv, bn = self.conv, self.bn
+        cout = conv.out_channels
+        if not bn.training and x.is_cuda and CONV_MODE != "library" and NORM_POOL_MODE != "library" and not conv.relu \
+                and type(bn) is BatchNormAct and not torch.is_grad_enabled() and not _hooked(conv, bn):
+            y = conv_bn_eval(x, conv.weight, conv.bias, conv.stride, conv.padding, bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.eps,
+                             bn.relu, residual)
             if y is not None:
                 return y
         fused = x.is_cuda and x.dim() == 4 and CONV_MODE != "library" and NORM_POOL_MODE != "library" and FUSE_BN_STATS and self.training \

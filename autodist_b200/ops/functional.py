@@ -503,8 +503,15 @@ class _ConvBNEvalFn(torch.autograd.Function):
 def conv_bn_eval(x, weight, bias, stride, padding, gamma, beta, running_mean, running_var, eps, relu=False, residual=None):
     """``relu?(batch_norm(conv2d(x, weight, bias)) + residual)`` with the running statistics, in one kernel, or ``None`` where
     that kernel does not apply (a gradient is recorded, CPU tensors, shapes or types it does not take)."""
+    if torch.is_grad_enabled() or not x.is_cuda:
+        return None
+    if weight.shape[3] % 8 == 0 and running_mean is not None and running_var is not None and gamma is not None and beta is not None:
+        y = ops.ext(required=True).conv_bn_eval_nchw(x, _bf16_weight(weight), bias, stride, padding, gamma, beta, running_mean, running_var, eps,
+                                                     relu, residual, _error_flag(x.device))
+        if y is not None:
+            return y
     cout, kh, kw, _ = weight.shape
-    if torch.is_grad_enabled() or x.dim() != 4 or not _own_conv(x, weight, stride) or cout > 2048 or \
+    if x.dim() != 4 or not _own_conv(x, weight, stride) or cout > 2048 or \
             not _eval_norm_ready(gamma, beta, running_mean, running_var, cout):
         return None
     if residual is not None:
