@@ -1401,7 +1401,9 @@ __global__ void __launch_bounds__(256, 4) bn_bwd_stats_kernel(const bf16* __rest
   if (threadIdx.x == 0) counters[blockIdx.x] = 0u;
 }
 
-__global__ void __launch_bounds__(kBnThreads, 3) bn_bwd_apply_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
+// Two blocks per SM: 24 coefficients and four rows of two tensors per thread take 104 registers; at three blocks per SM the
+// compiler spilled 224 bytes.
+__global__ void __launch_bounds__(kBnThreads, 2) bn_bwd_apply_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
                                     const uint8_t* __restrict__ keep, const float* __restrict__ coef, bf16* __restrict__ dx,
                                     bf16* __restrict__ dres, long long rows, int C, int relu) {
   pdl_sync();
@@ -1868,11 +1870,11 @@ int bn_parts(int rows, int C) {
 // part: [bn_parts, 2, C]; sums: [2, C]; coef (backward): [3, C]
 // sums_given: `sums` already holds the per-channel sum and sum of squares (the convolution's epilogue produced them); the
 // whole normalisation is then one launch.
-// One wave of resident blocks (three per SM) unless that leaves a thread fewer than kBnUnroll rows.
-dim3 bn_grid(long long rows, int C) {
+// One wave of resident blocks (`per_sm` per SM) unless that leaves a thread fewer than kBnUnroll rows.
+dim3 bn_grid(long long rows, int C, int per_sm) {
   const int c8 = C / 8, tpr = c8 < kBnThreads ? c8 : kBnThreads, rpb = kBnThreads / tpr, gy = (c8 + kBnThreads - 1) / kBnThreads;
   long long blocks = (rows + (long long)rpb * kBnUnroll - 1) / ((long long)rpb * kBnUnroll);
-  const long long cap = (148 * 3 + gy - 1) / gy;
+  const long long cap = (148 * per_sm + gy - 1) / gy;
   if (blocks > cap) blocks = cap;
   return dim3((unsigned)(blocks < 1 ? 1 : blocks), (unsigned)gy);
 }
@@ -1886,7 +1888,7 @@ void bn_fwd(const bf16* x, const float* gamma, const float* beta, const bf16* re
     launch_pdl(bn_stats_kernel, dim3(dim3(blocks_for(C, 64), parts)), dim3(256), 0, st, x, part, rows, C, rpb);
     launch_pdl(colsum_f32_kernel, dim3(blocks_for(2 * C, 32)), dim3(256), 0, st, part, sums, parts, 2 * C, 0);
   }
-  launch_pdl(bn_apply_kernel, bn_grid(rows, C), dim3(kBnThreads), 0, st, x, res, y, relu ? keep : nullptr, (long long)rows, C, relu, sums, gamma, beta,
+  launch_pdl(bn_apply_kernel, bn_grid(rows, C, 3), dim3(kBnThreads), 0, st, x, res, y, relu ? keep : nullptr, (long long)rows, C, relu, sums, gamma, beta,
              1.0f / rows, eps, mean, rstd, run_mean, run_var, batches, momentum, unbias);
 }
 void bn_eval(const bf16* x, const bf16* res, bf16* y, const float* gamma, const float* beta, const float* mean, const float* var, float eps,
@@ -1903,7 +1905,7 @@ void bn_bwd(const bf16* dy, const bf16* x, const uint8_t* keep, const float* mea
   launch_pdl(bn_bwd_stats_kernel, dim3(dim3(blocks_for(C, 64), parts)), dim3(256), 0, st, dy, x, keep, mean, rstd, gamma, reinterpret_cast<unsigned int*>(part),
                                                                       part + kBnCounterFloats, sums, coef, dgamma_acc, dbeta_acc, rows, C, rpb,
                                                                       relu, 1.0f / rows);
-  launch_pdl(bn_bwd_apply_kernel, bn_grid(rows, C), dim3(kBnThreads), 0, st, dy, x, keep, coef, dx, dres, (long long)rows, C, relu);
+  launch_pdl(bn_bwd_apply_kernel, bn_grid(rows, C, 2), dim3(kBnThreads), 0, st, dy, x, keep, coef, dx, dres, (long long)rows, C, relu);
 }
 // dx = relu'(y) * dy (skipped when y is null) and out[c] (+)= column sums of dx. part: [bn_parts(rows, C), C] floats.
 void relu_bwd_colsum(const bf16* dy, const bf16* y, bf16* dx, float* part, float* out, int rows, int C, int accumulate, cudaStream_t st) {
