@@ -652,14 +652,29 @@ void bn_eval(const Tensor& x, const optional<Tensor>& res, Tensor y, const Tenso
   adb200::bn_eval(CBF(x), OPT_BF(res), BF(y), gamma.data_ptr<float>(), beta.data_ptr<float>(), mean.data_ptr<float>(), var.data_ptr<float>(),
                   (float)eps, rows, C, relu ? 1 : 0, STREAM);
 }
+// Per-channel sum and sum of squares [2, C] of a channels-last matrix, as a convolution's epilogue leaves them.
+Tensor bn_sums(const Tensor& x) {
+  const int C = x.size(-1), rows = x.numel() / std::max(C, 1);
+  TORCH_CHECK(C > 0 && C % 8 == 0 && rows > 0 && x.is_contiguous() && x.scalar_type() == at::kBFloat16, "x must be contiguous bf16 [.., C], C % 8 == 0");
+  Tensor part = at::empty({(int64_t)adb200::bn_parts(rows, C) * 2 * C}, x.options().dtype(at::kFloat));
+  Tensor sums = at::empty({2, C}, x.options().dtype(at::kFloat));
+  adb200::bn_sums(CBF(x), part.data_ptr<float>(), sums.data_ptr<float>(), rows, C, STREAM);
+  return sums;
+}
 // Returns [dbeta, dgamma] stacked as a [2, C] fp32 tensor; writes dx and (optional) dres = dy masked by the ReLU.
 // dgamma_acc / dbeta_acc (optional, fp32 [C]): the batch-norm parameters' gradient buffers; the sums are added into them.
 Tensor bn_bwd(const Tensor& dy, const Tensor& x, const optional<Tensor>& keep, const Tensor& mean, const Tensor& rstd, const Tensor& gamma, Tensor dx,
-              const optional<Tensor>& dres, bool relu, const optional<Tensor>& dgamma_acc, const optional<Tensor>& dbeta_acc) {
+              const optional<Tensor>& dres, bool relu, const optional<Tensor>& dgamma_acc, const optional<Tensor>& dbeta_acc,
+              const optional<Tensor>& add) {
   const int C = x.size(-1), rows = x.numel() / C;
   TORCH_CHECK(C % 8 == 0 && C <= 16384 && x.is_contiguous() && dy.is_contiguous() && dx.is_contiguous() && dy.numel() == x.numel() && dx.numel() == x.numel(),
               "dy, x, dx must be contiguous bf16 [.., C] of one shape, C % 8 == 0");
   if (dres.has_value()) TORCH_CHECK(dres->is_contiguous() && dres->numel() == x.numel() && dres->scalar_type() == at::kBFloat16, "dres must match x");
+  if (add.has_value()) {            // [rows, C] view whose rows may lie further apart than C
+    TORCH_CHECK(add->dim() == 2 && add->size(0) == rows && add->size(1) == C && add->scalar_type() == at::kBFloat16 && (C == 1 || add->stride(1) == 1) &&
+                add->stride(0) >= C && add->stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(add->data_ptr()) % 16 == 0,
+                "the addend must be a bf16 [rows, C] view with aligned rows");
+  }
   TORCH_CHECK(!relu || (keep.has_value() && keep->scalar_type() == at::kByte && keep->is_contiguous() && keep->numel() * 8 == x.numel()),
               "the forward pass's keep bytes are needed with a fused ReLU");
   // partial sums: a per-device scratch that the kernels keep zero between calls (they add into it and clear what they read);
@@ -671,7 +686,7 @@ Tensor bn_bwd(const Tensor& dy, const Tensor& x, const optional<Tensor>& keep, c
   Tensor sums = at::empty({5, C}, x.options().dtype(at::kFloat));              // [dbeta, dgamma, A, B, K]
   adb200::bn_bwd(CBF(dy), CBF(x), relu ? keep->data_ptr<uint8_t>() : nullptr, mean.data_ptr<float>(), rstd.data_ptr<float>(), gamma.data_ptr<float>(), BF(dx), OPT_BF(dres),
                  part.data_ptr<float>(), sums.data_ptr<float>(), sums.data_ptr<float>() + 2 * C, rows, C, relu ? 1 : 0, OPT_F(dgamma_acc),
-                 OPT_F(dbeta_acc), STREAM);
+                 OPT_F(dbeta_acc), add.has_value() ? CBF(*add) : nullptr, add.has_value() ? add->stride(0) : 0, STREAM);
   return sums.narrow(0, 0, 2);
 }
 // code: uint8 [N, Ho, Wo, C], the window position of each output's first maximum
@@ -906,6 +921,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("flagged_rows_update", &flagged_rows_update);
   m.def("cast_f32_bf16", &cast_f32_bf16);
   m.def("bn_fwd", &bn_fwd);
+  m.def("bn_sums", &bn_sums);
   m.def("bn_eval", &bn_eval);
   m.def("bn_bwd", &bn_bwd);
   m.def("maxpool_fwd", &maxpool_fwd);

@@ -1401,32 +1401,35 @@ __global__ void __launch_bounds__(256, 4) bn_bwd_stats_kernel(const bf16* __rest
   if (threadIdx.x == 0) counters[blockIdx.x] = 0u;
 }
 
-// Two blocks per SM: 24 coefficients and four rows of two tensors per thread take 104 registers; at three blocks per SM the
-// compiler spilled 224 bytes.
+// ADD: another gradient of x, read from rows `add_ld` apart, is added. Two blocks per SM: 24 coefficients and four rows of two or
+// three tensors per thread take 104 to 121 registers; at three blocks per SM the compiler spilled 224 bytes.
+template <bool ADD>
 __global__ void __launch_bounds__(kBnThreads, 2) bn_bwd_apply_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
-                                    const uint8_t* __restrict__ keep, const float* __restrict__ coef, bf16* __restrict__ dx,
-                                    bf16* __restrict__ dres, long long rows, int C, int relu) {
+                                    const uint8_t* __restrict__ keep, const float* __restrict__ coef, const bf16* __restrict__ add,
+                                    long long add_ld, bf16* __restrict__ dx, bf16* __restrict__ dres, long long rows, int C, int relu) {
+  constexpr int U = kBnUnroll;
   pdl_sync();
   const BnWalk w = bn_walk(C);
   if (!w.live) return;
   const int c = w.c;
   float ca[8], cb[8], ck[8];
   load_f8(coef + c, ca); load_f8(coef + C + c, cb); load_f8(coef + 2 * C + c, ck);
-  for (long long row = w.row; row < rows; row += kBnUnroll * w.step) {
-    uint4 dq[kBnUnroll], xq[kBnUnroll];
-    uint32_t kq[kBnUnroll];
+  for (long long row = w.row; row < rows; row += U * w.step) {
+    uint4 dq[U], xq[U], aq[ADD ? U : 1];
+    uint32_t kq[U];
 #pragma unroll
-    for (int u = 0; u < kBnUnroll; ++u) {
+    for (int u = 0; u < U; ++u) {
       const long long r = row + u * w.step;
       kq[u] = 0xffu;
       if (r < rows) {
         dq[u] = *reinterpret_cast<const uint4*>(dy + r * C + c);
         xq[u] = *reinterpret_cast<const uint4*>(x + r * C + c);
         if (relu) kq[u] = keep[(r * C + c) >> 3];
+        if (ADD) aq[u] = *reinterpret_cast<const uint4*>(add + r * add_ld + c);
       }
     }
 #pragma unroll
-    for (int u = 0; u < kBnUnroll; ++u) {
+    for (int u = 0; u < U; ++u) {
       const long long r = row + u * w.step;
       if (r >= rows) break;
       float d[8], xv[8], gm[8];
@@ -1437,6 +1440,11 @@ __global__ void __launch_bounds__(kBnThreads, 2) bn_bwd_apply_kernel(const bf16*
         const float g = (kq[u] >> j) & 1u ? d[j] : 0.f;
         gm[j] = g;
         d[j] = fmaf(ca[j], g, fmaf(cb[j], xv[j], ck[j]));
+      }
+      if (ADD) {                                            // the gradient x received from its other consumer
+        unpack8(aq[u], xv);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) d[j] += xv[j];
       }
       store8(dx + r * C + c, d);
       if (dres != nullptr) store8(dres + r * C + c, gm);    // gradient of the residual branch: dy masked by the ReLU
@@ -1878,16 +1886,18 @@ dim3 bn_grid(long long rows, int C, int per_sm) {
   if (blocks > cap) blocks = cap;
   return dim3((unsigned)(blocks < 1 ? 1 : blocks), (unsigned)gy);
 }
+// sums [2, C] = per-channel sum and sum of squares of x. part: [bn_parts, 2, C]
+void bn_sums(const bf16* x, float* part, float* sums, int rows, int C, cudaStream_t st) {
+  const int parts = bn_parts(rows, C), rpb = (rows + parts - 1) / parts;
+  launch_pdl(bn_stats_kernel, dim3(dim3(blocks_for(C, 64), parts)), dim3(256), 0, st, x, part, rows, C, rpb);
+  launch_pdl(colsum_f32_kernel, dim3(blocks_for(2 * C, 32)), dim3(256), 0, st, part, sums, parts, 2 * C, 0);
+}
 // keep (optional, [rows, C / 8] bytes): which outputs are positive, for the backward pass of a fused ReLU
 void bn_fwd(const bf16* x, const float* gamma, const float* beta, const bf16* res, bf16* y, uint8_t* keep, float* mean, float* rstd, float* part,
             float* sums, int rows, int C, float eps, int relu, int sums_given, float* run_mean, float* run_var, long long* batches,
             float momentum, cudaStream_t st) {
   const float unbias = rows > 1 ? (float)rows / (float)(rows - 1) : 1.0f;
-  if (!sums_given) {
-    const int parts = bn_parts(rows, C), rpb = (rows + parts - 1) / parts;
-    launch_pdl(bn_stats_kernel, dim3(dim3(blocks_for(C, 64), parts)), dim3(256), 0, st, x, part, rows, C, rpb);
-    launch_pdl(colsum_f32_kernel, dim3(blocks_for(2 * C, 32)), dim3(256), 0, st, part, sums, parts, 2 * C, 0);
-  }
+  if (!sums_given) bn_sums(x, part, sums, rows, C, st);
   launch_pdl(bn_apply_kernel, bn_grid(rows, C, 3), dim3(kBnThreads), 0, st, x, res, y, relu ? keep : nullptr, (long long)rows, C, relu, sums, gamma, beta,
              1.0f / rows, eps, mean, rstd, run_mean, run_var, batches, momentum, unbias);
 }
@@ -1900,12 +1910,13 @@ void bn_eval(const bf16* x, const bf16* res, bf16* y, const float* gamma, const 
              var, eps);
 }
 void bn_bwd(const bf16* dy, const bf16* x, const uint8_t* keep, const float* mean, const float* rstd, const float* gamma, bf16* dx, bf16* dres,
-            float* part, float* sums, float* coef, int rows, int C, int relu, float* dgamma_acc, float* dbeta_acc, cudaStream_t st) {
+            float* part, float* sums, float* coef, int rows, int C, int relu, float* dgamma_acc, float* dbeta_acc, const bf16* add, long long add_ld,
+            cudaStream_t st) {
   const int parts = bn_parts(rows, C), rpb = (rows + parts - 1) / parts;
   launch_pdl(bn_bwd_stats_kernel, dim3(dim3(blocks_for(C, 64), parts)), dim3(256), 0, st, dy, x, keep, mean, rstd, gamma, reinterpret_cast<unsigned int*>(part),
                                                                       part + kBnCounterFloats, sums, coef, dgamma_acc, dbeta_acc, rows, C, rpb,
                                                                       relu, 1.0f / rows);
-  launch_pdl(bn_bwd_apply_kernel, bn_grid(rows, C, 2), dim3(kBnThreads), 0, st, dy, x, keep, coef, dx, dres, (long long)rows, C, relu);
+  launch_pdl(add != nullptr ? bn_bwd_apply_kernel<true> : bn_bwd_apply_kernel<false>, bn_grid(rows, C, 2), dim3(kBnThreads), 0, st, dy, x, keep, coef, add, add_ld, dx, dres, (long long)rows, C, relu);
 }
 // dx = relu'(y) * dy (skipped when y is null) and out[c] (+)= column sums of dx. part: [bn_parts(rows, C), C] floats.
 void relu_bwd_colsum(const bf16* dy, const bf16* y, bf16* dx, float* part, float* out, int rows, int C, int accumulate, cudaStream_t st) {

@@ -61,7 +61,9 @@ void bn_fwd(const bf16_t* x, const float* gamma, const float* beta, const bf16_t
 void bn_eval(const __nv_bfloat16* x, const __nv_bfloat16* res, __nv_bfloat16* y, const float* gamma, const float* beta, const float* mean,
              const float* var, float eps, int rows, int C, int relu, cudaStream_t st);
 void bn_bwd(const bf16_t* dy, const bf16_t* x, const uint8_t* keep, const float* mean, const float* rstd, const float* gamma, bf16_t* dx,
-            bf16_t* dres, float* part, float* sums, float* coef, int rows, int C, int relu, float* dgamma_acc, float* dbeta_acc, cudaStream_t st);
+            bf16_t* dres, float* part, float* sums, float* coef, int rows, int C, int relu, float* dgamma_acc, float* dbeta_acc, const bf16_t* add,
+            long long add_ld, cudaStream_t st);
+void bn_sums(const bf16_t* x, float* part, float* sums, int rows, int C, cudaStream_t st);
 void maxpool_fwd(const bf16_t* x, bf16_t* y, uint8_t* code, int N, int H, int W, int C, int k, int stride, int pad, int Ho, int Wo,
                  cudaStream_t st);
 void maxpool_bwd(const uint8_t* code, const bf16_t* dy, bf16_t* dx, int N, int H, int W, int C, int k, int stride, int pad, int Ho,

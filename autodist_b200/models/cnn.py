@@ -16,7 +16,8 @@ import torch
 from torch import nn
 import torch.nn.functional as F
 
-from autodist_b200.ops.functional import Linear, batch_norm, batch_norm_eval, conv2d, conv_bn_eval, fork, max_pool2d
+from autodist_b200.ops.functional import (Linear, batch_norm, batch_norm_eval, cat_channels, channel_sums, conv2d, conv_bn_eval, fork,
+                                          max_pool2d)
 
 CONV_MODE = os.environ.get("AUTODIST_CONV", "own")                      # own | library
 
@@ -61,10 +62,10 @@ class BatchNormAct(nn.BatchNorm2d):
         super().__init__(channels)
         self.relu = relu
 
-    def forward(self, x, residual=None, sums=None, fork=None):
+    def forward(self, x, residual=None, sums=None, fork=None, in_fork=None):
         if _own_norm_pool(x) and self.training and self.momentum is not None:
             return batch_norm(x, self.weight, self.bias, self.running_mean, self.running_var, True, self.momentum, self.eps, self.relu,
-                              residual, sums, self.num_batches_tracked, fork)
+                              residual, sums, self.num_batches_tracked, fork, in_fork)
         if not self.training and NORM_POOL_MODE != "library":
             y = batch_norm_eval(x, self.weight, self.bias, self.running_mean, self.running_var, self.eps, self.relu, residual)
             if y is not None:
@@ -244,6 +245,18 @@ class _DenseLayer(nn.Module):
     def forward(self, x):
         return torch.cat([x, self.f(x)], 1)
 
+    def step(self, x, sums):
+        """Training step on the kernel path: ``sums`` are the per-channel sums of ``x``; returns the concatenation and its sums. Every
+        batch-norm gets its statistics from the convolution that produced the channels (the ones of earlier layers are the
+        same numbers again), and the gradient that reaches ``x`` through the concatenation is added inside the first
+        batch-norm's backward pass."""
+        bn1, conv1, bn2, conv2 = self.f
+        xa, xc, box = fork(x) if FORK_FUSION else (x, x, None)
+        s1, s2 = _ARENA.take(conv1.out_channels, x.device), _ARENA.take(conv2.out_channels, x.device)
+        h = conv1(bn1(xa, sums=sums, in_fork=box), s1)
+        new = conv2(bn2(h, sums=s1), s2)
+        return cat_channels(xc, new, box), torch.cat([sums, s2], 1)
+
 
 class DenseNet121(nn.Module):
     def __init__(self, num_classes=1000, growth=32, blocks=(6, 12, 24, 16)):
@@ -261,8 +274,25 @@ class DenseNet121(nn.Module):
         self.features = nn.Sequential(*mods)
         self.fc = Linear(c, num_classes)
 
+    def _fused(self, x):
+        mods = list(self.features.modules())
+        return x.is_cuda and self.training and torch.is_autocast_enabled() and CONV_MODE != "library" and NORM_POOL_MODE != "library" and \
+            FUSE_BN_STATS and not _hooked(*mods) and \
+            all(m.training and m.momentum is not None and m.num_features % 8 == 0 for m in mods if isinstance(m, BatchNormAct))
+
     def forward(self, x):
-        return self.fc(torch.flatten(F.adaptive_avg_pool2d(self.features(x), 1), 1))
+        if self._fused(x):
+            sums = None
+            for m in self.features:
+                if isinstance(m, _DenseLayer):
+                    x, sums = m.step(x, channel_sums(x) if sums is None else sums)
+                elif isinstance(m, BatchNormAct) and sums is not None:      # the transition's, or the last one
+                    x, sums = m(x, sums=sums), None
+                else:
+                    x, sums = m(x), None
+        else:
+            x = self.features(x)
+        return self.fc(torch.flatten(F.adaptive_avg_pool2d(x, 1), 1))
 
 
 class _InceptionBlock(nn.Module):
@@ -321,7 +351,8 @@ class ImageClassifier(nn.Module):
         if images.is_cuda:
             images = images.contiguous(memory_format=torch.channels_last)
             if self._stat_floats is None:
-                self._stat_floats = sum(2 * m.conv.out_channels for m in self.net.modules() if isinstance(m, ConvBN))
+                self._stat_floats = sum(2 * m.conv.out_channels for m in self.net.modules() if isinstance(m, ConvBN)) + \
+                    sum(2 * (m.f[1].out_channels + m.f[3].out_channels) for m in self.net.modules() if isinstance(m, _DenseLayer))
             _ARENA.begin(self._stat_floats, images.device)
             try:
                 with torch.autocast("cuda", dtype=self.compute_dtype):

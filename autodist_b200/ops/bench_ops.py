@@ -48,7 +48,7 @@ def _cnn_rows(E, dev, flush, hbm):
     rows.append({"kernel": "bn_fwd+relu 64x56x56x256", "ms": round(ms, 4), "gbs": round(3 * nbytes / ms / 1e6, 1),
                  "library_ms": round(ms_lib, 4), "frac_of_measured_peak": round(3 * nbytes / ms / 1e6 / hbm, 3)})
     dy, dx = torch.randn_like(xh), torch.empty_like(xh)
-    ms = _time(lambda: E.bn_bwd(dy, xh, keep, mean, rstd, gamma, dx, None, True, None, None), flush=flush)
+    ms = _time(lambda: E.bn_bwd(dy, xh, keep, mean, rstd, gamma, dx, None, True, None, None, None), flush=flush)
     rows.append({"kernel": "bn_bwd+relu 64x56x56x256", "ms": round(ms, 4), "gbs": round(5 * nbytes / ms / 1e6, 1),
                  "frac_of_measured_peak": round(5 * nbytes / ms / 1e6 / hbm, 3)})
     N, C, Hh, W = 64, 64, 112, 112                                   # the ResNet stem pool

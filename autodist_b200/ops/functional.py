@@ -545,15 +545,56 @@ def batch_norm_eval(x, gamma, beta, running_mean, running_var, eps, relu=False, 
     return _BNEvalFn.apply(x, gamma, beta, running_mean, running_var, eps, bool(relu), residual)
 
 
+def _row_view(t, xh):
+    """``t`` (logical [N, C, H, W]) as a bf16 [N * H * W, C] view whose rows lie a constant, 16-byte aligned distance apart - a channel
+    slice of a channels-last tensor is one - or ``None``. ``xh`` is the channels-last tensor it is added to."""
+    n, h, w, c = xh.shape
+    if t.dtype != torch.bfloat16 or tuple(t.shape) != (n, c, h, w) or not t.is_cuda:
+        return None
+    p = t.permute(0, 2, 3, 1)
+    ld = next((p.stride(d) // k for d, k in ((2, 1), (1, w), (0, h * w)) if p.shape[d] > 1), c)
+    regular = all(p.shape[d] == 1 or p.stride(d) == ld * k for d, k in ((2, 1), (1, w), (0, h * w)))
+    if not regular or (c > 1 and p.stride(3) != 1) or ld < c or ld % 8 or t.data_ptr() % 16:
+        return None
+    return p.as_strided((n * h * w, c), (ld, 1))
+
+
+class _CatChannelsFn(torch.autograd.Function):
+    """``torch.cat([x, new], 1)`` whose gradient for ``x`` is left, as a view, for the kernel of ``x``'s other consumer."""
+
+    @staticmethod
+    def forward(ctx, x, new, fork):
+        ctx.fork, ctx.c = fork, x.shape[1]
+        return torch.cat([x, new], 1)
+
+    @staticmethod
+    def backward(ctx, dy):
+        dx, dn = dy[:, :ctx.c], dy[:, ctx.c:]
+        if ctx.needs_input_grad[0] and ctx.fork.grad is None:
+            ctx.fork.grad, dx = dx, None
+        return dx, dn, None
+
+
+def cat_channels(x, new, fork=None):
+    """Channel concatenation; ``fork`` is the ``GradFork`` of ``x`` when a ``batch_norm(in_fork=...)`` reads it too."""
+    return torch.cat([x, new], 1) if fork is None else _CatChannelsFn.apply(x, new, fork)
+
+
+def channel_sums(x):
+    """Per-channel sum and sum of squares (fp32 ``[2, C]``) of a CUDA tensor, as ``conv2d(stats=...)`` leaves them."""
+    with torch.no_grad():
+        return ops.ext(required=True).bn_sums(_nhwc(x.detach()))
+
+
 class _BatchNormFn(torch.autograd.Function):
     """Training-mode batch-norm over channels-last activations on the hand-written kernels, with the tail of a residual
     block fused in: ``y = relu?(bn(x) + residual)``. ``sums`` (fp32 ``[2, C]``: sum and sum of squares per channel, as the
     convolution's epilogue leaves them) skips the statistics pass."""
 
     @staticmethod
-    def forward(ctx, x, gamma, beta, residual, eps, relu, sums, running, fork=None):
+    def forward(ctx, x, gamma, beta, residual, eps, relu, sums, running, fork=None, in_fork=None):
         E = ops.ext(required=True)
-        ctx.fork = fork
+        ctx.fork, ctx.in_fork = fork, in_fork
         run_mean, run_var, batches, momentum = running if running is not None else (None, None, None, 0.0)
         xh = _nhwc(x)                                                            # [N, H, W, C]
         c = xh.shape[-1]
@@ -580,7 +621,7 @@ class _BatchNormFn(torch.autograd.Function):
         E = ops.ext(required=True)
         xh, keep, mean, rstd, g32 = ctx.saved_tensors
         if dy is None:
-            return (None,) * 9
+            return (None,) * 10
         dyh = _nhwc(dy)
         dx = torch.empty_like(xh)
         dres = None
@@ -589,8 +630,13 @@ class _BatchNormFn(torch.autograd.Function):
         gamma, beta = ctx.params
         acc_g, acc_b = _direct_grad(gamma), _direct_grad(beta)
         direct = acc_g is not None and acc_b is not None
+        other = ctx.in_fork.take() if ctx.in_fork is not None else None         # what x's other consumer left: added in the same pass
+        add = _row_view(other, xh) if other is not None else None
         sums = E.bn_bwd(dyh, xh, keep, mean, rstd, g32, dx, dres if ctx.relu else None, ctx.relu, acc_g if direct else None,
-                        acc_b if direct else None)
+                        acc_b if direct else None, add)
+        gx = dx.permute(0, 3, 1, 2).to(ctx.dtypes[0])
+        if other is not None and add is None:
+            gx = gx + other
         dr = dres.permute(0, 3, 1, 2).to(ctx.dtypes[2]) if dres is not None else None
         if ctx.fork is not None and dr is not None:
             other = ctx.fork.take()
@@ -601,14 +647,15 @@ class _BatchNormFn(torch.autograd.Function):
         if direct:
             _grad_written(gamma)
             _grad_written(beta)
-            return dx.permute(0, 3, 1, 2).to(ctx.dtypes[0]), None, None, dr, None, None, None, None, None
-        return dx.permute(0, 3, 1, 2).to(ctx.dtypes[0]), sums[1].to(ctx.dtypes[1]), sums[0].to(ctx.dtypes[1]), dr, None, None, None, None, None
+            return gx, None, None, dr, None, None, None, None, None, None
+        return gx, sums[1].to(ctx.dtypes[1]), sums[0].to(ctx.dtypes[1]), dr, None, None, None, None, None, None
 
 
 def batch_norm(x, gamma, beta, running_mean=None, running_var=None, training=True, momentum=0.1, eps=1e-5, relu=False,
-               residual=None, sums=None, num_batches_tracked=None, fork=None):
+               residual=None, sums=None, num_batches_tracked=None, fork=None, in_fork=None):
     """``relu?(batch_norm(x) + residual)`` of an NCHW / channels-last tensor; updates the running statistics like
-    ``F.batch_norm``. ``sums``: per-channel sum / sum of squares of ``x`` when a preceding kernel already produced them."""
+    ``F.batch_norm``. ``sums``: per-channel sum / sum of squares of ``x`` when a preceding kernel already produced them;
+    ``fork`` / ``in_fork``: the ``GradFork`` of ``residual`` / of ``x`` when that tensor has a second consumer."""
     if not (x.is_cuda and training and x.shape[1] % 8 == 0):
         y = F.batch_norm(x, running_mean, running_var, gamma.to(x.dtype) if x.dtype != gamma.dtype and not x.is_cuda else gamma,
                          beta, training, momentum, eps)
@@ -618,7 +665,7 @@ def batch_norm(x, gamma, beta, running_mean=None, running_var=None, training=Tru
     running = None
     if running_mean is not None and running_mean.dtype == torch.float32 and running_var.dtype == torch.float32:
         running = (running_mean, running_var, num_batches_tracked, float(momentum))     # folded into the statistics kernel
-    y, mean, rstd = _BatchNormFn.apply(x, gamma, beta, residual, eps, relu, sums, running, fork)
+    y, mean, rstd = _BatchNormFn.apply(x, gamma, beta, residual, eps, relu, sums, running, fork, in_fork)
     if running is None and running_mean is not None:
         with torch.no_grad():
             n = x.numel() // x.shape[1]

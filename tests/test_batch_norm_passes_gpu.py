@@ -39,3 +39,46 @@ def test_training_batch_norm(n, c, h, relu, with_res):
         assert ((res.grad.double() - rd.grad).abs() <= tol * rd.grad.abs()).all()
     if rows > 1:
         assert ((rm.double() - mean).abs() <= 1e-5 + 1e-5 * mean.abs()).all() and ((rv.double() - var).abs() <= 1e-4 * var.abs() + 1e-5).all()
+
+
+@pytest.mark.parametrize("n,c,extra,h,w", [(2, 24, 8, 5, 3), (1, 64, 32, 1, 1), (3, 96, 4, 2, 7), (1, 8, 8, 1, 9)])
+def test_concatenation_gradient_is_added_inside_batch_norm(n, c, extra, h, w):
+    """Sliced rows that the kernel can read in place, and (4 extra channels) ones it cannot."""
+    from autodist_b200.ops import functional as Fn
+    torch.manual_seed(c)
+    x0 = torch.randn(n, c, h, w, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    new = torch.randn(n, extra, h, w, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    gamma, beta = torch.rand(c, device="cuda") + 0.5, torch.randn(c, device="cuda")
+    dcat, dy = (torch.randn(n, k, h, w, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last) for k in (c + extra, c))
+    assert torch.allclose(Fn.channel_sums(x0)[1], x0.double().pow(2).sum((0, 2, 3)).float(), rtol=1e-5)
+    grads = []
+    for fused in (True, False):
+        x = x0.clone().requires_grad_(True)
+        g, b = gamma.clone().requires_grad_(True), beta.clone().requires_grad_(True)
+        xa, xc, box = Fn.fork(x * 1) if fused else (x, x, None)
+        y = Fn.batch_norm(xa, g, b, relu=True, sums=Fn.channel_sums(x0), in_fork=box)
+        out = Fn.cat_channels(xc, new, box)
+        torch.autograd.backward([out, y], [dcat, dy])
+        grads.append(x.grad)
+    # one rounding to bf16 instead of three
+    assert ((grads[0].float() - grads[1].float()).abs() <= 2.0 ** -7 * grads[1].float().abs() + 2.0 ** -7 * dcat[:, :c].float().abs() + 1e-3).all()
+
+
+def test_dense_network_step_matches_the_plain_route(monkeypatch):
+    from autodist_b200.models import cnn
+    torch.manual_seed(0)
+    net = cnn.DenseNet121(growth=8, blocks=(2, 2, 2, 2), num_classes=16).cuda()
+    x = torch.randn(4, 3, 64, 64, device="cuda").contiguous(memory_format=torch.channels_last)
+    state = {k: v.clone() for k, v in net.state_dict().items()}
+    outs = []
+    for plain in (False, True):
+        net.load_state_dict(state)
+        net.zero_grad()
+        monkeypatch.setattr(cnn, "FUSE_BN_STATS", not plain)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = net(x)
+        y.float().pow(2).sum().backward()
+        outs.append((y.detach().float(), net.features[0].bn.running_var.clone(), net.fc.weight.grad.clone(),
+                     net.features[-1].running_mean.clone()))
+    for a, b in zip(*outs):                    # the same values in another order of summation and with fewer roundings
+        assert (a - b).norm() <= 0.05 * b.norm()
