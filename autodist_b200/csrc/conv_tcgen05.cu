@@ -2,10 +2,10 @@
 // weight gradient over channels-last bf16 activations, no im2col matrix in memory.
 //
 // Same persistent, warp-specialised shape as the GEMM (gemm_tcgen05.cu):
-//   warp 0    TMA producer   per K block one box of the activation patch shifted by the filter tap (zero fill outside
+//   warps 0, 10 TMA producers per K block one box of the activation patch shifted by the filter tap (zero fill outside
 //                            the image = the padding) and one box of the weight, 128-byte swizzle, ring of stages
 //   warp 1    MMA issuer     tcgen05.mma 128 x BN x 16, bf16 -> fp32 in TMEM, two accumulator buffers
-//   warps 2-5 epilogue       tcgen05.ld, then
+//   warps 2-9 epilogue       tcgen05.ld, then
 //                              forward:         + bias, evaluation-mode batch-norm, residual, ReLU, per-channel sum / sum of
 //                                               squares (batch-norm statistics, reduced in shared memory across the
 //                                               CTA's tiles), bf16 store
@@ -19,6 +19,8 @@
 // TMEM and returns.
 //
 // The reference's convolutions are tf.keras layers running in cuDNN (examples/benchmark/imagenet.py:232-249).
+#include <type_traits>
+
 #include "conv_tcgen05.h"
 #include "pdl.cuh"
 #include "tcgen05_common.cuh"
@@ -37,7 +39,7 @@ template <int BN, int MODE> struct ConvCfg {
   // Eight epilogue warps: two per TMEM lane quarter, half of the tile's columns each. Layers with a short contraction
   // (1 x 1 convolutions) spend longer draining a tile than multiplying it, and four warps could not keep up.
   static constexpr int EPI_WARPS = 8;
-  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  static constexpr int THREADS = 96 + 32 * EPI_WARPS;           // two producer warps, the MMA issuer, the epilogue
   static constexpr int CHUNKS = BN / 16 / (EPI_WARPS / 4);      // 16-column chunks per epilogue warp
   static constexpr int STAT_BYTES = (MODE == CONV_FPROP || MODE == CONV_EVAL) ? 2 * kMaxStatChannels * 4 : 0;
   static constexpr int SMEM = STAGES * (A_BYTES + B_BYTES) + STAGING + 1024 /*align*/ + 256 /*barriers*/ + STAT_BYTES;
@@ -387,11 +389,15 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
   const int rows = p.tw * p.th * p.tn;
   const int col_rows = p.th * p.tn;                 // rows of one patch column (wsplit boxes)
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+  // One operand per producer warp (A and the byte count: the first warp, B: the last). A K block takes one to six copies, and a
+  // single thread that issued all of them bounded every narrow or MN-major tile. Weight gradients of 3 x 3 layers, 32 images (one
+  // producer that divided per patch / without the divisions / two producers, us): 64 -> 64 at 224 x 224 602 / 462 / 467,
+  // 128 -> 128 at 112 x 112 200 / 157 / 127, 256 -> 256 at 56 x 56 125 / 103 / 90.
+  auto produce = [&](auto operand) {
+    constexpr bool LOAD_A = decltype(operand)::value == 0, LOAD_B = !LOAD_A;
+    {
       int stage = 0; uint32_t phase = 0; bool ok = true;
-      if (trace != nullptr) trace[1] = clock64();
+      if (LOAD_A && trace != nullptr) trace[1] = clock64();
       for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
         const TileCoord tc_ = decode_tile<BN, MODE>(p, t);
         if (MODE != CONV_WGRAD) {
@@ -401,16 +407,18 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
             const CUtensorMap* mapA = &maps.act[tap.amap];
             for (int cb = 0; cb < kcb; ++cb) {
               if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
-              mbar_expect_tx(&full[stage], a_bytes + C::B_BYTES);
+              if (LOAD_A) mbar_expect_tx(&full[stage], a_bytes + C::B_BYTES);
               uint8_t* a_dst = sA + stage * A_BYTES;
               uint8_t* b_dst = sB + stage * C::B_BYTES;
-              if (!p.wsplit) {
+              if (LOAD_B) {
+              } else if (!p.wsplit) {
                 tma_load_4d(a_dst, mapA, &full[stage], cb * BK, tc_.w0 + tap.dw, tc_.h0 + tap.dh, tc_.n0);
               } else {
                 for (int j = 0; j < p.tw; ++j)
                   tma_load_4d(a_dst + j * col_rows * 128, mapA, &full[stage], (tc_.w0 + j) * p.xstep, tc_.h0 + tap.dh, tc_.n0, 0);
               }
-              if (FWD) {
+              if (LOAD_A) {
+              } else if (FWD) {
                 tma_load_4d(b_dst, &maps.w, &full[stage], cb * BK, tap.wtap, tc_.c0, 0);
               } else {
 #pragma unroll
@@ -423,33 +431,39 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
         } else {
           const ConvTap tap = p.taps[tc_.tap];
           const CUtensorMap* mapX = &maps.act[tap.amap];
-          for (int pi = tc_.kbeg; pi < tc_.kend; ++pi) {
-            const int w0 = (pi % p.tiles_w) * p.tw;
-            const int h0 = ((pi / p.tiles_w) % p.tiles_h) * p.th;
-            const int n0 = (pi / (p.tiles_w * p.tiles_h)) * p.tn;
+          // the patch walks on by additions: divisions per patch made this one thread the bound of narrow tiles
+          int w0 = (tc_.kbeg % p.tiles_w) * p.tw;
+          int h0 = ((tc_.kbeg / p.tiles_w) % p.tiles_h) * p.th;
+          int n0 = (tc_.kbeg / (p.tiles_w * p.tiles_h)) * p.tn;
+          const int w_end = p.tiles_w * p.tw, h_end = p.tiles_h * p.th;
+          auto next_patch = [&]() {
+            w0 += p.tw;
+            if (w0 >= w_end) { w0 = 0; h0 += p.th; if (h0 >= h_end) { h0 = 0; n0 += p.tn; } }
+          };
+          for (int pi = tc_.kbeg; pi < tc_.kend; ++pi, next_patch()) {
             if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
             // output channels beyond Cout need no load: those accumulator rows are never stored
             const int a_chunks = (tc_.m0 + 64 < p.Mc) ? 2 : 1;
-            mbar_expect_tx(&full[stage], a_chunks * (BK * 128) + C::B_BYTES);
+            if (LOAD_A) mbar_expect_tx(&full[stage], a_chunks * (BK * 128) + C::B_BYTES);
             uint8_t* a_dst = sA + stage * A_BYTES;
             uint8_t* b_dst = sB + stage * C::B_BYTES;
             if (!p.wsplit) {
-              for (int j = 0; j < a_chunks; ++j) tma_load_4d(a_dst + j * (BK * 128), &maps.dy, &full[stage], tc_.m0 + 64 * j, w0, h0, n0);
+              for (int j = 0; LOAD_A && j < a_chunks; ++j) tma_load_4d(a_dst + j * (BK * 128), &maps.dy, &full[stage], tc_.m0 + 64 * j, w0, h0, n0);
 #pragma unroll
-              for (int j = 0; j < BN / 64; ++j)
+              for (int j = 0; LOAD_B && j < BN / 64; ++j)
                 tma_load_4d(b_dst + j * (BK * 128), mapX, &full[stage], tc_.c0 + 64 * j, w0 + tap.dw, h0 + tap.dh, n0);
             } else {
               for (int jw = 0; jw < p.tw; ++jw) {
-                for (int j = 0; j < a_chunks; ++j)
+                for (int j = 0; LOAD_A && j < a_chunks; ++j)
                   tma_load_4d(a_dst + j * (BK * 128) + jw * col_rows * 128, &maps.dy, &full[stage], tc_.m0 + 64 * j, w0 + jw, h0, n0);
-                tma_load_4d(b_dst + jw * col_rows * 128, mapX, &full[stage], (w0 + jw) * p.xstep, h0 + tap.dh, n0, 0);
+                if (LOAD_B) tma_load_4d(b_dst + jw * col_rows * 128, mapX, &full[stage], (w0 + jw) * p.xstep, h0 + tap.dh, n0, 0);
               }
             }
             if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
           }
         }
       }
-      if (trace != nullptr) trace[2] = clock64();
+      if (LOAD_A && trace != nullptr) trace[2] = clock64();
       if (!ok) {
         *abort_flag = 1;
         if (p.error_flag) atomicExch(p.error_flag, 11);
@@ -461,6 +475,11 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
         }
       }
     }
+  };
+  if (warp == 0) {
+    if (lane == 0) produce(std::integral_constant<int, 0>{});
+  } else if (warp == 2 + C::EPI_WARPS) {
+    if (lane == 0) produce(std::integral_constant<int, 1>{});
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
@@ -514,12 +533,12 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
     if (EVAL && p.staged == 0) {
       // y = conv * scale + shift with the layer's running statistics: the per-channel table is built once per CTA while the
       // first tile is multiplied (the statistics table's space; the two never occur together)
-      for (int c = threadIdx.x - 64; c < p.Nc; c += C::THREADS - 64) {
+      for (int c = threadIdx.x - 64; c < p.Nc; c += 256) {
         const float sc = p.bn_gamma[c] * rsqrtf(p.bn_var[c] + p.bn_eps);
         s_stat[c] = sc;
         s_stat[p.Nc + c] = fmaf(-p.bn_mean[c], sc, p.bn_beta[c]);
       }
-      asm volatile("bar.sync 1, %0;" ::"n"(C::THREADS - 64) : "memory");
+      asm volatile("bar.sync 1, 256;" ::: "memory");
     }
     // bias and evaluation-mode batch-norm of 16 forward outputs starting at column col0
     auto affine16 = [&](float* v, int col0) {
