@@ -130,11 +130,17 @@ void gemm_set_trace(const optional<Tensor>& t) {
 // exchange through distributed shared memory; it wins wherever the tiles leave SMs idle: 1024 x 1024 x 4096 29.2 -> 14.3 us
 // (256 wide, 4 CTAs), 768 x 768 x 1792 16.2 -> 9.0, 256 x 256 x 16384 94.7 -> 14.7, 640 x 1024 x 30522 172 -> 39,
 // 32 x 4096 x 25088 179 -> 38 (5.4 TB/s). Splits run one cluster per tile, so they are only considered while every cluster is
-// resident at once. Narrow tiles store directly: 8192 x 1024 x 128 fp32 takes 14.0 us with 64 columns, 9.2 with 256.
+// resident at once. The epilogue of a tile counts by kind (plain, bias, activation or auxiliary operand): narrow tiles store
+// directly and read what they need when they need it (8192 x 1024 x 128 fp32: 14.0 us with 64 columns, 9.2 with 256;
+// 1792 x 3072 x 768 with bias + GELU: 26.9 us with 128 columns, 18.2 with 256), and the last wave's is exposed.
 struct GemmChoice { int64_t bn, split; };
-GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split) {
-  struct Cost { int bn; double base, kb, epi, exchange; };
-  static const Cost costs[4] = {{64, 2.9, 0.30, 1.6, 2.6}, {128, 4.2, 0.33, 2.7, 2.6}, {256, 4.6, 0.48, 2.5, 3.5}, {512, 7.0, 0.41, 2.5, 0.0}};
+GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split, int64_t epilogue, bool both_mn) {
+  struct Cost { int bn; double base, kb, epi[3], exchange; };
+  static const Cost costs[4] = {{64, 2.9, 0.30, {1.6, 2.0, 3.6}, 2.6},
+                                {128, 4.2, 0.33, {2.7, 3.4, 7.5}, 2.6},
+                                {256, 4.6, 0.48, {2.5, 3.7, 6.5}, 3.5},
+                                {512, 7.0, 0.41, {2.5, 3.7, 6.5}, 0.0}};
+  const int kind = epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2);
   const int64_t kbs = (K + 63) / 64, sms = num_sms();
   GemmChoice best{64, 1};
   double best_us = 1e30;
@@ -146,12 +152,14 @@ GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allo
     const int64_t tiles = ((M + tm - 1) / tm) * ((N + tn - 1) / tn) * batch;
     const int64_t slots = pair ? sms / 2 : sms;
     const double waves = (double)((tiles + slots - 1) / slots);
-    const double us = c.base + waves * std::max(c.kb * (double)kbs, c.epi);
+    const double kb = c.bn == 128 && both_mn ? 0.42 : c.kb;          // four copies per K block for one producer thread
+    const double extra = c.epi[kind] - c.epi[0];                       // the last wave's drain (the plain one is part of the base)
+    const double us = c.base + (waves - 1) * std::max(kb * (double)kbs, c.epi[kind]) + kb * (double)kbs + extra;
     if (us < best_us) { best_us = us; best = {c.bn, 1}; }
     if (pair || !allow_split) continue;
     for (int s = 2; s <= 8 && s <= kbs; ++s) {
       if (tiles * s > sms || tiles > adb200::gemm_split_max_clusters(s, (int)sms)) continue;
-      const double us_s = c.base + c.kb * (double)((kbs + s - 1) / s) + c.exchange;
+      const double us_s = c.base + kb * (double)((kbs + s - 1) / s) + c.exchange + extra / s;
       if (us_s < best_us) { best_us = us_s; best = {c.bn, s}; }
     }
   }
@@ -178,7 +186,8 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
   const bool auto_bn = bn <= 0;
   if (bn <= 0) {
     static const bool pair_default = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR"); return e == nullptr || e[0] != '0'; }();
-    const GemmChoice g = choose_gemm(M, N, K, a.size(0) * a.size(1), pair_default && !pair_unavailable && !softmax_epi, !softmax_epi);
+    const GemmChoice g = choose_gemm(M, N, K, a.size(0) * a.size(1), pair_default && !pair_unavailable && !softmax_epi, !softmax_epi, epilogue,
+                                      a_mn && b_mn);
     bn = g.bn;
     split = g.split;
   }
