@@ -18,6 +18,10 @@
 // softmax kernels (elementwise.cu): same counter-based function of (seed, step, offset in [B, heads, S, S]). Hashing costs as
 // much as the rest of a pass, so the forward pass keeps the decisions as bits (1/16 of the scores' bf16 bytes).
 //
+// Per layer, 16 heads, dropout 0.1 (separate products and softmax kernels -> here): 32 x 128 tokens forward 37 -> 17 us, backward
+// 52 -> 21; 6 x 512 tokens forward about 85 -> 37, backward about 140 -> 64. The backward pass took 124 us while it hashed the
+// decisions again, read its row sums when it needed them and stored 32-byte pieces of the gradients directly.
+//
 // Every mbarrier wait is bounded: a role that gives up raises `abort`, which ends the waits of the others, and records a code.
 #include "attention.h"
 #include "gemm_epilogue.cuh"
