@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "conv_tcgen05.h"
+#include "eval_norm.cuh"
 #include "pdl.cuh"
 #include "tcgen05_common.cuh"
 
@@ -116,6 +117,7 @@ __device__ __forceinline__ uint4 lds4(uint32_t addr) {
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ void sts1(uint32_t addr, uint32_t a) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(a) : "memory"); }
 __device__ __forceinline__ uint32_t lds1(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
@@ -124,6 +126,71 @@ __device__ __forceinline__ uint32_t lds1(uint32_t addr) {
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
+}
+
+// Evaluation mode, 32 rows x 32 columns of one warp: bias, batch-norm, residual, ReLU, rounded to bf16 wherever layers of their own would
+// round (see eval_norm.cuh). A thread that owns a row needs the four coefficients of every column, 128 floats per 32 outputs, and the
+// shared-memory reads of those bounded the drain; so the accumulator is read in the fragment layout: lane l holds columns
+// 8 k + 2 (l % 4), + 1 of the rows l / 4 + 8 i, and a column's coefficients serve four rows (one ResNet-50 evaluation pass of 32 images:
+// a row per thread 1285 us, this 1133).
+// `tab`: the columns' coefficients, BN floats between two of them; `rows`: shared address of the warp's 32 staged lines.
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint32_t round2(uint64_t v) {
+  const float2 f = unpack_f32x2(v);
+  return pack2(f.x, f.y);
+}
+__device__ __forceinline__ uint64_t widen2(uint32_t u) { return pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+
+template <int BN>
+__device__ __forceinline__ void eval_piece(uint32_t taddr, int cols, const float* tab, bool bias, bool add, bool relu, uint32_t rows, int chunk, int lane) {
+  uint32_t r[32];                              // [rows 0-15, 16-31][k][row l / 4 or + 8][column]
+  __syncwarp();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr), "r"(taddr + (16u << 16)) : "memory");
+  const uint32_t swz = (uint32_t)(lane >> 2);  // line % 8 of every row of this lane
+  const uint32_t mine = rows + (uint32_t)(lane >> 2) * 128u + (uint32_t)(lane & 3) * 4u;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (8 * k >= cols) break;                  // columns come in groups of 8
+    const float* t = tab + 8 * k + 2 * (lane & 3);
+    const uint64_t neg_mean = *reinterpret_cast<const uint64_t*>(t), inv = *reinterpret_cast<const uint64_t*>(t + BN);
+    const uint64_t gamma = *reinterpret_cast<const uint64_t*>(t + 2 * BN), beta = *reinterpret_cast<const uint64_t*>(t + 3 * BN);
+    const uint64_t b = bias ? *reinterpret_cast<const uint64_t*>(t + 4 * BN) : 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t* a = r + (i >> 1) * 16 + k * 4 + (i & 1) * 2;
+      const uint32_t at = mine + (uint32_t)i * 1024u + (((uint32_t)(chunk + k) ^ swz) << 4);
+      uint64_t v = pack_f32x2(__uint_as_float(a[0]), __uint_as_float(a[1]));
+      if (bias) v = add2(v, b);
+      v = widen2(round2(v));                                                    // the convolution's result
+      uint32_t w = round2(fma2(mul2(gamma, add2(v, neg_mean)), inv, beta));     // normalised (eval_norm)
+      if (add) w = round2(add2(widen2(w), widen2(lds1(at))));
+      if (relu) asm("max.NaN.bf16x2 %0, %1, %2;" : "=r"(w) : "r"(w), "r"(0u));  // a NaN stays a NaN
+      sts1(at, w);
+    }
+  }
 }
 
 // Epilogue of the pixel modes through shared memory. A 1 x 1 convolution multiplies a tile in a few microseconds, so the drain is
@@ -158,16 +225,10 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
   const bool add = (MODE == CONV_DGRAD || EVAL) && p.addend != nullptr;
   const bool bias = FWD && p.bias != nullptr;
   auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "n"(PARTY) : "memory"); };
-  if constexpr (EVAL) {
-    // y = conv * scale + shift with the layer's running statistics: the per-channel table is built once per CTA while the
-    // first tile is multiplied (in the statistics table's space; the two never occur together)
-    for (int c = threadIdx.x - 64; c < p.Nc; c += 256) {
-      const float sc = p.bn_gamma[c] * rsqrtf(p.bn_var[c] + p.bn_eps);
-      s_stat[c] = sc;
-      s_stat[p.Nc + c] = fmaf(-p.bn_mean[c], sc, p.bn_beta[c]);
-    }
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-  }
+  // Evaluation-mode batch-norm: the coefficients of the tile's columns (-mean, 1 / deviation, gamma, beta and the convolution's bias,
+  // BN floats each, in the statistics table's space - the two never occur together) are rebuilt when the columns change, while the
+  // tile is multiplied.
+  int norm_c0 = -1;
   bool ok = true;
   auto wait = [&](uint64_t* bar, uint32_t parity) {    // a warp that gives up walks on, so that nobody is left behind at a barrier
     if (ok && !mbar_wait(bar, parity, abort_flag)) { ok = false; *abort_flag = 1; }
@@ -213,7 +274,7 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
       }
     }
     float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);       // four columns of the bias per lane, handed around by shuffles
-    if (bias && lane * 4 < CW) {
+    if (!EVAL && bias && lane * 4 < CW) {
       const int c = c_w + lane * 4;                    // Nc is a multiple of 8: four columns exist together
       if (c < p.Nc) b4 = make_float4(__ldg(p.bias + c), __ldg(p.bias + c + 1), __ldg(p.bias + c + 2), __ldg(p.bias + c + 3));
     }
@@ -222,7 +283,25 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
       const int gw = tc_.w0 + r % p.tw, gh = tc_.h0 + (r / p.tw) % p.th, gn = tc_.n0 + r / (p.tw * p.th);
       valid = r < rows && gw < p.GW && gh < p.GH && gn < p.GN;
     }
-    if (!add) meet();                                  // with an addend its arrival says that the buffer may be written
+    bool table = false;
+    if constexpr (EVAL) {
+      // nobody reads the old table any more: the party met after its last box
+      table = tc_.c0 != norm_c0;
+      norm_c0 = tc_.c0;
+      if (table) {
+        constexpr int COLS = BN == 64 ? BN : CW;       // columns of this party
+        const int t0 = BN == 64 ? 0 : hf * CW;
+        for (int c = (int)threadIdx.x - 64 - (BN == 64 ? 0 : hf * 128); c < COLS; c += PARTY)
+          if (tc_.c0 + t0 + c < p.Nc) {
+            const int ch = tc_.c0 + t0 + c;
+            const float4 n = eval_norm_of(p.bn_mean, p.bn_var, p.bn_gamma, p.bn_beta, p.bn_eps, ch);
+            float* at = s_stat + t0 + c;
+            at[0] = -n.x; at[BN] = n.y; at[2 * BN] = n.z; at[3 * BN] = n.w;
+            at[4 * BN] = bias ? p.bias[ch] : 0.f;
+          }
+      }
+    }
+    if (!add || table) meet();                         // with an addend its arrival says that the buffer may be written
     wait(&tfull[as], aphase);
     const long long tw1 = trace != nullptr ? clock64() : 0;
     tc_fence_after();
@@ -246,7 +325,11 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
 #pragma unroll
       for (int h = 0; h < CW / 32 / BOXES; ++h) {
         const int ch = (BN == 64 ? hf * 4 : h * 4);    // first 16-byte chunk of the 32 columns inside the box line
-        const int col = col0 + h * 32;
+        if constexpr (EVAL) {
+          eval_piece<BN>(t_row + g * 64 + h * 32, p.Nc - (col0 + h * 32), s_stat + hf * CW + g * 64 + h * 32, bias, add, p.relu != 0,
+                         box + (uint32_t)(q * 32) * 128u, ch, lane);
+          continue;
+        }
         float v[32];
         __syncwarp();
         tmem_ld32(t_row + g * 64 + h * 32, v);
@@ -260,14 +343,6 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
             v[j + 3] += __shfl_sync(0xffffffffu, b4.w, src);
           }
         }
-        if constexpr (EVAL) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 8)
-            if (col + j < p.Nc) {                      // Nc is a multiple of 8
-#pragma unroll
-              for (int x = 0; x < 8; ++x) v[j + x] = fmaf(v[j + x], s_stat[col + j + x], s_stat[p.Nc + col + j + x]);
-            }
-        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const uint32_t at = line + (((uint32_t)(ch + j) ^ swz) << 4);
@@ -280,7 +355,7 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
           }
           if (FWD && p.relu) {
 #pragma unroll
-            for (int x = 0; x < 8; ++x) w[x] = EVAL ? (w[x] < 0.f ? 0.f : w[x]) : fmaxf(w[x], 0.f);      // evaluation keeps a NaN
+            for (int x = 0; x < 8; ++x) w[x] = fmaxf(w[x], 0.f);
           }
           if (do_stats && !valid) {                    // pixels that do not exist count for nothing
 #pragma unroll
@@ -530,16 +605,6 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
     const int c_lo = ((warp - 2) >> 2) * C::CHUNKS;      // first 16-column chunk of this warp's share of the tile
     int as = 0; uint32_t aphase = 0; bool ok = true;
     const int r = q * 32 + lane;
-    if (EVAL && p.staged == 0) {
-      // y = conv * scale + shift with the layer's running statistics: the per-channel table is built once per CTA while the
-      // first tile is multiplied (the statistics table's space; the two never occur together)
-      for (int c = threadIdx.x - 64; c < p.Nc; c += 256) {
-        const float sc = p.bn_gamma[c] * rsqrtf(p.bn_var[c] + p.bn_eps);
-        s_stat[c] = sc;
-        s_stat[p.Nc + c] = fmaf(-p.bn_mean[c], sc, p.bn_beta[c]);
-      }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-    }
     // bias and evaluation-mode batch-norm of 16 forward outputs starting at column col0
     auto affine16 = [&](float* v, int col0) {
       if (p.bias != nullptr) {
@@ -548,7 +613,9 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
       }
       if (EVAL) {
 #pragma unroll
-        for (int jj = 0; jj < 16; ++jj) if (col0 + jj < p.Nc) v[jj] = fmaf(v[jj], s_stat[col0 + jj], s_stat[p.Nc + col0 + jj]);
+        for (int jj = 0; jj < 16; ++jj)
+          if (col0 + jj < p.Nc)
+            v[jj] = round_bf16(eval_norm(round_bf16(v[jj]), eval_norm_of(p.bn_mean, p.bn_var, p.bn_gamma, p.bn_beta, p.bn_eps, col0 + jj)));
       }
     };
     bool staged = false;

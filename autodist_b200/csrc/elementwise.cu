@@ -13,6 +13,7 @@
 #include <stdint.h>
 
 #include "elementwise.h"
+#include "eval_norm.cuh"
 #include "pdl.cuh"
 
 namespace adb200 {
@@ -1274,34 +1275,44 @@ __global__ void __launch_bounds__(kBnThreads, 3) bn_apply_kernel(const bf16* __r
   }
 }
 
-// Evaluation mode: y = relu?(x * scale + shift) from the running statistics, one pass (the library takes three kernels: the
-// inverse deviation, the normalisation and the ReLU). HBM-bound; the coefficient table costs C rsqrt per block as above.
-// Dynamic shared memory: 2 * C floats.
-__global__ void __launch_bounds__(256, 6) bn_eval_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, bf16* __restrict__ y,
-                                                         long long total8, int C, int relu, const float* __restrict__ gamma,
-                                                         const float* __restrict__ beta, const float* __restrict__ mean,
-                                                         const float* __restrict__ var, float eps) {
+// Evaluation mode: y = relu?(batch_norm(x) + res) from the running statistics, one pass (the library takes three kernels: the
+// inverse deviation, the normalisation and the ReLU), rounding where those round. HBM-bound, in the row-walking layout.
+__global__ void __launch_bounds__(kBnThreads, 2) bn_eval_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, bf16* __restrict__ y,
+                                                                long long rows, int C, int relu, const float* __restrict__ gamma,
+                                                                const float* __restrict__ beta, const float* __restrict__ mean,
+                                                                const float* __restrict__ var, float eps) {
   pdl_sync();
-  extern __shared__ float s_coef[];
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    const float sc = gamma[c] * rsqrtf(var[c] + eps);
-    s_coef[c] = sc;
-    s_coef[C + c] = fmaf(-mean[c], sc, beta[c]);
-  }
-  __syncthreads();
-  const long long stride = (long long)gridDim.x * blockDim.x;
-#pragma unroll 2
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total8; idx += stride) {
-    const int c = (int)(idx % (C / 8)) * 8;
-    float v[8], rv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    load8(x + idx * 8, v);
-    if (res != nullptr) load8(res + idx * 8, rv);
+  const BnWalk w = bn_walk(C);
+  if (!w.live) return;
+  float4 n[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float o = fmaf(v[j], s_coef[c + j], s_coef[C + c + j]) + rv[j];
-      v[j] = relu && o < 0.f ? 0.f : o;                    // a NaN stays a NaN
+  for (int j = 0; j < 8; ++j) n[j] = eval_norm_of(mean, var, gamma, beta, eps, w.c + j);
+  for (long long row = w.row; row < rows; row += kBnUnroll * w.step) {
+    uint4 xq[kBnUnroll], rq[kBnUnroll];
+#pragma unroll
+    for (int u = 0; u < kBnUnroll; ++u) {
+      const long long r = row + u * w.step;
+      rq[u] = make_uint4(0, 0, 0, 0);
+      if (r < rows) {
+        xq[u] = *reinterpret_cast<const uint4*>(x + r * C + w.c);
+        if (res != nullptr) rq[u] = *reinterpret_cast<const uint4*>(res + r * C + w.c);
+      }
     }
-    store8(y + idx * 8, v);
+#pragma unroll
+    for (int u = 0; u < kBnUnroll; ++u) {
+      const long long r = row + u * w.step;
+      if (r >= rows) break;
+      float v[8], rv[8];
+      unpack8(xq[u], v);
+      unpack8(rq[u], rv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[j] = eval_norm(v[j], n[j]);
+        if (res != nullptr) v[j] = round_bf16(v[j]) + rv[j];
+        v[j] = relu && v[j] < 0.f ? 0.f : v[j];              // a NaN stays a NaN
+      }
+      store8(y + r * C + w.c, v);
+    }
   }
 }
 
@@ -1903,11 +1914,7 @@ void bn_fwd(const bf16* x, const float* gamma, const float* beta, const bf16* re
 }
 void bn_eval(const bf16* x, const bf16* res, bf16* y, const float* gamma, const float* beta, const float* mean, const float* var, float eps,
              int rows, int C, int relu, cudaStream_t st) {
-  const long long total8 = (long long)rows * (C / 8);
-  long long blocks = (total8 + 256 * 4 - 1) / (256 * 4);
-  if (blocks > 148 * 6) blocks = 148 * 6;
-  launch_pdl(bn_eval_kernel, dim3((int)(blocks < 1 ? 1 : blocks)), dim3(256), 2 * C * sizeof(float), st, x, res, y, total8, C, relu, gamma, beta, mean,
-             var, eps);
+  launch_pdl(bn_eval_kernel, bn_grid(rows, C, 2), dim3(kBnThreads), 0, st, x, res, y, (long long)rows, C, relu, gamma, beta, mean, var, eps);
 }
 void bn_bwd(const bf16* dy, const bf16* x, const uint8_t* keep, const float* mean, const float* rstd, const float* gamma, bf16* dx, bf16* dres,
             float* part, float* sums, float* coef, int rows, int C, int relu, float* dgamma_acc, float* dbeta_acc, const bf16* add, long long add_ld,
