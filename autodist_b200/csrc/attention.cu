@@ -67,6 +67,7 @@ __device__ __forceinline__ float ex2(float x) {
 // Decision bits of 32 consecutive scores whose first has offset `base` (a multiple of 32): mix64 of one counter decides four, and
 // the counters' products with the odd constant are formed by additions.
 __device__ __forceinline__ uint32_t keep_bits32(uint64_t seed, uint64_t base, uint32_t thresh16) {
+  if (thresh16 > 0xffffu) return 0u;                       // probability 1: no 16-bit field reaches the threshold, nothing is kept
   constexpr uint64_t kStep = 0x9E3779B97F4A7C15ull;
   const uint64_t x0 = seed + (base >> 2) * kStep;
   const uint32_t limit = thresh16 << 16;
@@ -86,6 +87,9 @@ __device__ __forceinline__ uint32_t keep_bits32(uint64_t seed, uint64_t base, ui
   }
   return bits;
 }
+
+// 1 / keep probability. With probability 1 no score is kept: context and gradients are zero, and any finite factor will do.
+__device__ __forceinline__ float inverse_keep(float drop_p) { return drop_p > 0.f && drop_p < 1.f ? 1.0f / (1.0f - drop_p) : 1.0f; }
 
 // A wait of the elementwise warps, which meet in named barriers: a warp whose wait fails raises the abort flag and walks on
 // without waiting, so that nobody is left behind at a barrier.
@@ -219,7 +223,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
     const float scale2 = p.scale * kLog2e;                 // scores, maxima and exponents are kept in base 2
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
     const uint32_t thresh = (uint32_t)(p.drop_p * 65536.0f);
-    const float inv_keep = p.drop_p > 0.f ? 1.0f / (1.0f - p.drop_p) : 1.0f;
+    const float inv_keep = inverse_keep(p.drop_p);
     const uint64_t sd = p.seed + (p.step ? (uint64_t)(*p.step) * 0x100000001B3ull : 0ull);
     const uint64_t row_off = (((uint64_t)b * p.heads + h) * p.S + row) * p.S;
     const long long keep_row = (((long long)b * p.heads + h) * p.S + row) * attn_keep_words(p.S);
@@ -490,7 +494,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
     const int q = warp & 3, cb = warp >> 2;                // TMEM lane quarter, block of 32 keys
     const int r = q * 32 + lane;
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-    const float inv_keep = p.drop_p > 0.f ? 1.0f / (1.0f - p.drop_p) : 1.0f;
+    const float inv_keep = inverse_keep(p.drop_p);
     const float scale2 = p.scale * kLog2e, log2_keep = __log2f(inv_keep), delta_scale = p.scale / inv_keep;
     const int words = attn_keep_words(p.S);
     const uint32_t row_smem = (uint32_t)(cb >> 1) * TILE + (uint32_t)r * 128u;

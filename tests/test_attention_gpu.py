@@ -71,3 +71,21 @@ def test_attention_without_mask_and_repeatable():
     a, ga = _run(2, 256, 2, 0.1, masked=False)
     b, gb = _run(2, 256, 2, 0.1, masked=False)
     assert torch.equal(a, b) and all(torch.equal(x, y) for x, y in zip(ga, gb))
+
+
+@pytest.mark.parametrize("B,S,nh", [(2, 64, 1), (3, 128, 2), (1, 512, 2)])
+def test_dropout_of_probability_one_leaves_zeros(B, S, nh):
+    """Nothing is kept: a context and gradients of zeros, as the softmax kernels and the library's dropout give."""
+    from autodist_b200 import ops
+    E = ops.ext(required=True)
+    H = nh * 64
+    err, step = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.tensor([3], device="cuda")
+    qkv, dctx = torch.randn(B * S, 3 * H, device="cuda").bfloat16(), torch.randn(B * S, H, device="cuda").bfloat16()
+    ctx, dqkv = torch.full_like(dctx, float("nan")), torch.full_like(qkv, float("nan"))
+    lse = torch.empty(B, nh, S, device="cuda")
+    keep = torch.full((B, nh, S, (S + 127) // 128 * 4), -1, dtype=torch.int32, device="cuda")
+    E.attn_fwd(qkv, None, ctx, lse, B, S, nh, 0.125, 1.0, 5, step, err, keep)
+    E.attn_bwd(qkv, None, ctx, dctx, lse, torch.empty_like(lse), dqkv, B, S, nh, 0.125, 1.0, err, keep)
+    probs, dropped = (torch.empty(B, nh, S, S, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    E.softmax_fwd(torch.zeros_like(probs), None, probs, dropped, 1.0, 1.0, 5, step)
+    assert (dropped == 0).all() and (ctx == 0).all() and (dqkv == 0).all() and err.item() == 0
