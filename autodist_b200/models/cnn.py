@@ -102,12 +102,13 @@ _ARENA = _StatsArena()
 
 
 def _hooked(*modules):
-    """Whether a forward hook watches one of ``modules`` (their outputs must then exist on their own)."""
+    """Whether a hook watches one of ``modules``: their outputs must then exist on their own, and (backward hooks) the modules must
+    be called as such."""
     m = nn.modules.module
-    if m._global_forward_hooks or m._global_forward_pre_hooks:
+    if m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks:
         return True
     for x in modules:
-        if x._forward_hooks or x._forward_pre_hooks:
+        if x._forward_hooks or x._forward_pre_hooks or x._backward_hooks or x._backward_pre_hooks:
             return True
     return False
 
