@@ -64,6 +64,11 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// The additive mask in base 2. Finite masks end at -65536: a key that far below another one has a weight of zero either way, and the
+// lowest float, which would overflow here, keeps its place above minus infinity (a key that does not exist). Scores of a row
+// whose keys all lie there are told apart to 2^-7.
+__device__ __forceinline__ float mask_base2(float mask) { return mask > -INFINITY ? fmaxf(mask * kLog2e, -65536.f) : mask; }
+
 // Decision bits of 32 consecutive scores whose first has offset `base` (a multiple of 32): mix64 of one counter decides four, and
 // the counters' products with the odd constant are formed by additions.
 __device__ __forceinline__ uint32_t keep_bits32(uint64_t seed, uint64_t base, uint32_t thresh16) {
@@ -219,7 +224,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
     const int r = q * 32 + lane;                           // row of the tile
     const int row = qt * 128 + r;                          // query
     for (int c = threadIdx.x; c < tiles * 128; c += FWD_SOFT)
-      s_mask[c] = c < p.S ? (p.mask != nullptr ? p.mask[(long long)b * p.S + c] * kLog2e : 0.f) : -INFINITY;
+      s_mask[c] = c < p.S ? (p.mask != nullptr ? mask_base2(p.mask[(long long)b * p.S + c]) : 0.f) : -INFINITY;
     const float scale2 = p.scale * kLog2e;                 // scores, maxima and exponents are kept in base 2
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
     const uint32_t thresh = (uint32_t)(p.drop_p * 65536.0f);
@@ -261,7 +266,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
       red[hf * 128 + r] = mx;
       named_sync(1, FWD_SOFT);
       const float m_new = fmaxf(m, fmaxf(mx, red[(hf ^ 1) * 128 + r]));
-      const float corr_new = ex2(m - m_new);
+      // Keys masked with minus infinity up to here: nothing to rescale, and the exponents are taken against 0 instead of the maximum
+      // (a row without any key ends as 0 / 0).
+      const float base = m_new > -INFINITY ? m_new : 0.f;
+      const float corr_new = ex2(m - base);
       m = m_new;
       l *= corr_new;
       if (j > 0) {                                         // the context of the tiles before, in terms of their maximum
@@ -287,10 +295,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
           tmem_ld16(tS + lane_base + hf * 64 + c * 32 + e * 16, v);
           if (plain) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = ex2(fmaf(v[i], scale2, m0 - m));
+            for (int i = 0; i < 16; ++i) v[i] = ex2(fmaf(v[i], scale2, m0 - base));
           } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = ex2(fmaf(v[i], scale2, mk[c * 32 + e * 16 + i] - m));
+            for (int i = 0; i < 16; ++i) v[i] = ex2(fmaf(v[i], scale2, mk[c * 32 + e * 16 + i] - base));
           }
 #pragma unroll
           for (int i = 0; i < 16; i += 4) l += (v[i] + v[i + 1]) + (v[i + 2] + v[i + 3]);
@@ -514,7 +522,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
         f.delta = p.delta[at];
         if (p.drop_p > 0.f) f.keep = p.keep[at * words + kt * 4 + cb];
       }
-      if (key < p.S) f.mask = p.mask != nullptr ? p.mask[(long long)b * p.S + key] : 0.f;
+      if (key < p.S) f.mask = p.mask != nullptr ? mask_base2(p.mask[(long long)b * p.S + key]) : 0.f;
       return f;
     };
     bool ok = true, stored = false;
@@ -532,7 +540,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
         const float mask0 = __shfl_sync(0xffffffffu, now.mask, 0);
         const bool plain = __all_sync(0xffffffffu, now.mask == mask0);
         const float row_off = log2_keep - now.lse * kLog2e, nd = -now.delta * delta_scale;
-        const float off0 = fmaf(mask0, kLog2e, row_off);
+        const float off0 = mask0 + row_off;
         soft_wait(s_full, (uint32_t)t & 1u, abort_flag, ok);
         tc_fence_after();
 #pragma unroll
@@ -546,7 +554,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
             for (int e = 0; e < 16; ++e) s[e] = ex2(fmaf(s[e], scale2, off0));
           } else {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) s[e] = ex2(fmaf(s[e], scale2, fmaf(__shfl_sync(0xffffffffu, now.mask, c * 16 + e), kLog2e, row_off)));
+            for (int e = 0; e < 16; ++e) s[e] = ex2(fmaf(s[e], scale2, __shfl_sync(0xffffffffu, now.mask, c * 16 + e) + row_off));
           }
           uint32_t pw[8], dw[8];
 #pragma unroll

@@ -7,7 +7,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _run(B, S, nh, pd, seed=5, masked=True):
+def _run(B, S, nh, pd, seed=5, masked=True, mask=None):
     from autodist_b200 import ops
     E = ops.ext(required=True)
     torch.manual_seed(B * S + nh)
@@ -15,8 +15,7 @@ def _run(B, S, nh, pd, seed=5, masked=True):
     err = torch.zeros(1, dtype=torch.int32, device=dev)
     step = torch.tensor([3], dtype=torch.int64, device=dev)
     qkv = (torch.randn(B * S, 3 * H, device=dev) * 1.5).bfloat16()
-    mask = None
-    if masked:
+    if mask is None and masked:
         mask = torch.zeros(B, S, device=dev)
         for b in range(B):
             mask[b, S - (b * 7) % (S // 4 + 1):] = -10000.0
@@ -65,6 +64,28 @@ def _run(B, S, nh, pd, seed=5, masked=True):
 @pytest.mark.parametrize("B,S,nh", [(1, 64, 1), (3, 128, 2), (2, 256, 3), (1, 512, 2), (1, 1024, 1), (20, 128, 16), (5, 64, 7), (9, 256, 12)])
 def test_attention_matches_fp64(B, S, nh, pd):
     _run(B, S, nh, pd)
+
+
+@pytest.mark.parametrize("low", [-math.inf, torch.finfo(torch.float32).min])
+@pytest.mark.parametrize("B,S,nh", [(2, 64, 2), (3, 256, 2), (2, 512, 1)])
+def test_keys_out_of_reach(B, S, nh, low):
+    """Masks of minus infinity and of the lowest float, among them whole leading tiles, with at least one key left per row."""
+    mask = torch.zeros(B, S, device="cuda")
+    mask[0, :S // 2 + 9] = low
+    mask[1, 3:] = low
+    mask[1, S - 1] = 0.0
+    if B > 2:
+        mask[2, ::3] = low
+    _run(B, S, nh, 0.1, mask=mask)
+
+
+def test_a_row_without_any_key_is_not_a_number():
+    from autodist_b200 import ops
+    E = ops.ext(required=True)
+    qkv, ctx = torch.randn(256, 192, device="cuda").bfloat16(), torch.zeros(256, 64, device="cuda", dtype=torch.bfloat16)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    E.attn_fwd(qkv, torch.full((1, 256), -math.inf, device="cuda"), ctx, torch.empty(1, 1, 256, device="cuda"), 1, 256, 1, 0.125, 0.0, 0, None, err, None)
+    assert torch.isnan(ctx).all() and err.item() == 0
 
 
 def test_attention_without_mask_and_repeatable():
