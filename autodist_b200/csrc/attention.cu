@@ -69,8 +69,9 @@ __device__ __forceinline__ float ex2(float x) {
 // whose keys all lie there are told apart to 2^-7.
 __device__ __forceinline__ float mask_base2(float mask) { return mask > -INFINITY ? fmaxf(mask * kLog2e, -65536.f) : mask; }
 
-// Decision bits of 32 consecutive scores whose first has offset `base` (a multiple of 32): mix64 of one counter decides four, and
-// the counters' products with the odd constant are formed by additions.
+// Decision bits of 32 consecutive scores whose first has offset `base` (a multiple of 4: one counter decides four neighbours, so with
+// dropout the rows must be multiples of four long; the launchers check it). mix64 of consecutive counters, their products with the
+// odd constant formed by additions.
 __device__ __forceinline__ uint32_t keep_bits32(uint64_t seed, uint64_t base, uint32_t thresh16) {
   if (thresh16 > 0xffffu) return 0u;                       // probability 1: no 16-bit field reaches the threshold, nothing is kept
   constexpr uint64_t kStep = 0x9E3779B97F4A7C15ull;
@@ -644,7 +645,7 @@ cudaError_t launch_bwd(const CUtensorMap& q, const CUtensorMap& k, const CUtenso
 }  // namespace
 
 cudaError_t launch_attn_fwd(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const AttnParams& p, cudaStream_t stream) {
-  if (p.S < 1 || p.S > FWD_MAX_S || p.B < 1 || p.heads < 1 || (p.drop_p > 0.f && p.keep == nullptr) || !(p.scale > 0.f)) return cudaErrorInvalidValue;
+  if (p.S < 1 || p.S > FWD_MAX_S || p.B < 1 || p.heads < 1 || (p.drop_p > 0.f && (p.keep == nullptr || p.S % 4 != 0)) || !(p.scale > 0.f)) return cudaErrorInvalidValue;
   static const cudaError_t configured = cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM);
   if (configured != cudaSuccess) return configured;
   const long long grid = (long long)p.B * p.heads * ((p.S + 127) / 128);
@@ -656,7 +657,7 @@ cudaError_t launch_attn_bwd(const CUtensorMap& q, const CUtensorMap& k, const CU
                             const AttnParams& p, int num_sms, cudaStream_t stream) {
   if (p.S < 1 || p.S > FWD_MAX_S || p.B < 1 || p.heads < 1) return cudaErrorInvalidValue;
   if ((long long)p.B * p.heads * ((p.S + 127) / 128) > 0x3fffffffLL) return cudaErrorInvalidValue;
-  if (p.delta == nullptr || (p.drop_p > 0.f && p.keep == nullptr)) return cudaErrorInvalidValue;
+  if (p.delta == nullptr || (p.drop_p > 0.f && (p.keep == nullptr || p.S % 4 != 0))) return cudaErrorInvalidValue;
   const long long groups = (long long)p.B * p.S * p.heads, blocks = (groups * 8 + 255) / 256;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
   const cudaError_t d = launch_pdl(attn_delta_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, p, groups);

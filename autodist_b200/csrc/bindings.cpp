@@ -496,6 +496,7 @@ adb200::AttnParams attn_params(const Tensor& qkv, const optional<Tensor>& mask, 
                                const optional<Tensor>& keep) {
   const int64_t H = heads * 64;
   TORCH_CHECK(B > 0 && heads > 0 && S > 0 && S <= 1024, "attention takes 1 to 1024 tokens");
+  TORCH_CHECK(!(pd > 0) || S % 4 == 0, "attention with dropout takes a multiple of 4 tokens (one random number decides four neighbouring scores)");
   TORCH_CHECK(qkv.is_cuda() && qkv.scalar_type() == at::kBFloat16 && qkv.is_contiguous() && qkv.numel() == B * S * 3 * H, "qkv must be contiguous bf16 [B * S, 3 * heads * 64]");
   TORCH_CHECK(ctx.scalar_type() == at::kBFloat16 && ctx.is_contiguous() && ctx.numel() == B * S * H, "ctx must be contiguous bf16 [B * S, heads * 64]");
   TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.numel() == B * heads * S, "lse must be fp32 [B, heads, S]");

@@ -7,6 +7,21 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+def _decisions(count, pd, seed):
+    """Which of ``count`` scores dropout keeps: 16 bits of a counter-based 64-bit hash each, four per counter."""
+    def wrap(v):
+        return v - (1 << 64) if v >= 1 << 63 else v
+
+    def shift(x, n):                                            # logical, on signed words
+        return (x >> n) & ((1 << (64 - n)) - 1)
+    x = torch.arange((count + 3) // 4, dtype=torch.int64, device="cuda") * wrap(0x9E3779B97F4A7C15) + wrap(seed & ((1 << 64) - 1))
+    x = (x ^ shift(x, 30)) * wrap(0xBF58476D1CE4E5B9)
+    x = (x ^ shift(x, 27)) * wrap(0x94D049BB133111EB)
+    x = x ^ shift(x, 31)
+    fields = torch.stack([shift(x, 16 * j) & 0xFFFF if j else x & 0xFFFF for j in range(4)], 1).reshape(-1)[:count]
+    return fields >= int(pd * 65536)
+
+
 def _run(B, S, nh, pd, seed=5, masked=True, mask=None):
     from autodist_b200 import ops
     E = ops.ext(required=True)
@@ -29,7 +44,9 @@ def _run(B, S, nh, pd, seed=5, masked=True, mask=None):
     torch.cuda.synchronize()
     assert err.item() == 0
     keep = torch.ones(B, nh, S, S, device=dev, dtype=torch.float64)
-    if pd > 0:
+    if pd > 0 and S not in (64, 128, 256, 512, 1024):          # the softmax kernels take no such rows: the same decisions row by row
+        keep = _decisions(B * nh * S * S, pd, seed + int(step) * 0x100000001B3).view(B, nh, S, S).double() / (1 - pd)
+    elif pd > 0:
         zero, u, d = torch.zeros(B, nh, S, S, device=dev, dtype=torch.bfloat16), *(torch.empty(B, nh, S, S, device=dev, dtype=torch.bfloat16) for _ in range(2))
         E.softmax_fwd(zero, None, u, d, 1.0, pd, seed, step)
         keep = (d != 0).double() / (1 - pd)
@@ -110,3 +127,28 @@ def test_dropout_of_probability_one_leaves_zeros(B, S, nh):
     probs, dropped = (torch.empty(B, nh, S, S, device="cuda", dtype=torch.bfloat16) for _ in range(2))
     E.softmax_fwd(torch.zeros_like(probs), None, probs, dropped, 1.0, 1.0, 5, step)
     assert (dropped == 0).all() and (ctx == 0).all() and (dqkv == 0).all() and err.item() == 0
+
+
+@pytest.mark.parametrize("pd", [0.0, 0.1])
+@pytest.mark.parametrize("B,S,nh", [(3, 4, 2), (2, 100, 3), (2, 192, 2), (40, 200, 4), (1, 1000, 2)])
+def test_lengths_that_end_inside_a_tile(B, S, nh, pd):
+    _run(B, S, nh, pd)
+
+
+@pytest.mark.parametrize("B,S,nh", [(2, 1, 1), (1, 131, 2)])
+def test_odd_lengths_without_dropout(B, S, nh):
+    _run(B, S, nh, 0.0)
+
+
+def test_dropout_takes_multiples_of_four_tokens():
+    """One counter decides four neighbouring scores: rows of another length would share their decisions."""
+    from autodist_b200 import ops
+    E = ops.ext(required=True)
+    B, S, nh = 2, 130, 1
+    qkv, ctx = torch.randn(B * S, 192, device="cuda").bfloat16(), torch.empty(B * S, 64, device="cuda", dtype=torch.bfloat16)
+    lse, keep = torch.empty(B, nh, S, device="cuda"), torch.empty(B, nh, S, 8, dtype=torch.int32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    with pytest.raises(RuntimeError, match="multiple of 4"):
+        E.attn_fwd(qkv, None, ctx, lse, B, S, nh, 0.125, 0.1, 5, None, err, keep)
+    with pytest.raises(RuntimeError, match="multiple of 4"):
+        E.attn_bwd(qkv, None, ctx, ctx, lse, torch.empty_like(lse), torch.empty_like(qkv), B, S, nh, 0.125, 0.1, err, keep)
