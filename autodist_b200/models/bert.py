@@ -192,7 +192,10 @@ class BertPretrainer(nn.Module):
 
     def _workspace(self, B, S, P):
         key = (B, S, P, self._fused_attention(S))
+        drop_p = self.config.attention_probs_dropout_prob > 0 and self.training_dropout
         if self._ws is not None and self._ws["key"] == key:
+            if drop_p:
+                self._dropout_buffers(self._ws, B, S)
             return self._ws
         from autodist_b200 import ops
         E = ops.ext(required=True)
@@ -209,8 +212,6 @@ class BertPretrainer(nn.Module):
             return torch.empty(*shape, dtype=torch.float32, device=dev)
 
         fused = self._fused_attention(S)
-        drop_p = c.attention_probs_dropout_prob > 0 and self.training_dropout
-        drop_a = drop_p and not fused
 
         def scores():
             return None if fused else bf(B, nh, S, S)
@@ -218,8 +219,7 @@ class BertPretrainer(nn.Module):
         layers = []
         for _ in range(c.num_hidden_layers):
             layers.append({
-                "qkv": bf(T, 3 * H), "p": scores(), "pd": scores() if drop_a else None, "lse": f32(B, nh, S) if fused else None,
-                "keep": torch.empty(B, nh, S, (S + 127) // 128 * 4, dtype=torch.int32, device=dev) if fused and drop_p else None,
+                "qkv": bf(T, 3 * H), "p": scores(), "pd": None, "lse": f32(B, nh, S) if fused else None, "keep": None,
                 "ctx": bf(T, H), "z1": bf(T, H), "m1": f32(T), "r1": f32(T), "x1": bf(T, H),
                 "u": bf(T, Fd), "g": bf(T, Fd), "z2": bf(T, H), "m2": f32(T), "r2": f32(T), "out": bf(T, H)})
         n_part = max( E.colsum_parts(T) * max(4 * H, Fd, 3 * H, 2 * H),
@@ -247,8 +247,19 @@ class BertPretrainer(nn.Module):
             "err": torch.zeros(1, dtype=torch.int32, device=dev),
             "step": torch.zeros(1, dtype=torch.int64, device=dev),
         }
+        if drop_p:
+            self._dropout_buffers(ws, B, S)
         self._ws = ws
         return ws
+
+    def _dropout_buffers(self, ws, B, S):
+        """What a layer keeps of its attention dropout (decision bits, or dropped probabilities): made when dropout is first used
+        with a workspace, which may have been built without it."""
+        nh, dev, fused = self.config.num_attention_heads, self.flat.device, ws["key"][3]
+        name, shape, dtype = ("keep", (B, nh, S, (S + 127) // 128 * 4), torch.int32) if fused else ("pd", (B, nh, S, S), torch.bfloat16)
+        for A in ws["layers"]:
+            if A[name] is None:
+                A[name] = torch.empty(*shape, dtype=dtype, device=dev)
 
     def _gemm(self, ws, a, b, c, a_mn=False, b_mn=False, epi=EPI_NONE, bias=None, c2=None, aux=None, alpha=1.0, beta=0.0, bn=0):
         ws["E"].gemm(a, b, c, a_mn, b_mn, epi, bias, c2, aux, alpha, beta, ws["err"], bn)

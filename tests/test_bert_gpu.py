@@ -65,3 +65,26 @@ def test_dropout_path_runs_and_is_reproducible():
     assert abs(l3 - l1) > 1e-4 * abs(l1)                           # next step -> new masks
     assert torch.isfinite(model.flat.grad).all()
     model.check_error()
+
+
+@pytest.mark.parametrize("fused", [True, False])
+def test_dropout_switched_on_after_a_step_without_it(fused):
+    """The workspace of a shape is built by its first step; what dropout needs is added when a later step uses it."""
+    from autodist_b200.models.bert import BertConfig, BertPretrainer, synthetic_batch
+    torch.manual_seed(0)
+    cfg = BertConfig.tiny()
+    model = BertPretrainer(cfg)
+    model.fused_attention = fused
+    model.materialize("cuda")
+    batch = {k: v.cuda() for k, v in synthetic_batch(cfg, 2, 128, 8).items()}
+    model.training_dropout = False
+    plain = model.fused_forward_backward(**batch).item()
+    grad = model.flat.grad.clone()
+    held = model._ws["x0"].data_ptr()
+    model.training_dropout = True
+    model.fused_forward_backward(**batch)
+    assert model._ws["x0"].data_ptr() == held                      # the buffers that a captured step may hold stay where they are
+    assert torch.isfinite(model.flat.grad).all() and (model.flat.grad - grad).norm() > 0.01 * grad.norm()
+    model.training_dropout = False
+    assert abs(model.fused_forward_backward(**batch).item() - plain) < 1e-5 * abs(plain)
+    model.check_error()
