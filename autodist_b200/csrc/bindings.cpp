@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <tuple>
 #include <unordered_map>
 #include <vector>
 
@@ -166,6 +167,28 @@ GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allo
   return best;
 }
 
+// The kernel that bn = 0 asks for. AUTODIST_GEMM_PAIR=0 rules the two-CTA kernel out. AUTODIST_GEMM_PAIR_MIN_K sets a fixed rule
+// for it in place of the estimate: products with a pair's tile in both extents whose tiles fill the SM pairs, or whose contraction
+// is at least that long.
+bool g_pair_unavailable = false;               // set when a cluster launch was refused once (see gemm_impl)
+GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn) {
+  static const bool pair_default = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR"); return e == nullptr || e[0] != '0'; }();
+  static const int64_t pair_min_k = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR_MIN_K"); return e != nullptr ? std::atoll(e) : -1LL; }();
+  const bool softmax_epi = epilogue == adb200::EPI_SOFTMAX || epilogue == adb200::EPI_SOFTMAX_GRAD;
+  bool pair = pair_default && !g_pair_unavailable && !softmax_epi;
+  if (pair && pair_min_k >= 0) {
+    const int64_t pair_tiles = ((M + 255) / 256) * ((N + 255) / 256) * batch;
+    if (M >= 256 && N >= 256 && (pair_tiles >= num_sms() / 2 || K >= pair_min_k)) return {512, 1};
+    pair = false;
+  }
+  return choose_gemm(M, N, K, batch, pair, !softmax_epi, epilogue, both_mn);
+}
+// (tile width, contraction split) of gemm(..., bn = 0) for a product of these extents: 512 is the two-CTA kernel.
+std::tuple<int64_t, int64_t> gemm_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn) {
+  const GemmChoice g = auto_choice(M, N, K, batch, epilogue, both_mn);
+  return {g.bn, g.split};
+}
+
 // D = alpha * A.B^T (+ epilogue). a: [.., M, K] (K-major) or [.., K, M] (a_mn); b: [.., N, K] or [.., K, N] (b_mn);
 // c: [.., M, N] bf16 or fp32 view with unit inner stride.
 void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_mn, int64_t epilogue, const optional<Tensor>& bias,
@@ -180,14 +203,11 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
   TORCH_CHECK(c.size(0) == a.size(0) && c.size(1) == a.size(1) && c.size(2) == M && c.size(3) == N, "output shape mismatch");
   TORCH_CHECK(c.stride(3) == 1, "output inner stride must be 1");
   // bn: tile width 64 / 128 / 256 of the one-CTA kernel, or 512 = the 256 x 256 tile of the two-CTA kernel; 0 picks the kernel
-  // (see choose_gemm; two CTAs only when AUTODIST_GEMM_PAIR is not 0)
+  // (see choose_gemm and auto_choice)
   const bool softmax_epi = epilogue == adb200::EPI_SOFTMAX || epilogue == adb200::EPI_SOFTMAX_GRAD;
-  static bool pair_unavailable = false;        // set when a cluster launch was refused once (see below)
   const bool auto_bn = bn <= 0;
-  if (bn <= 0) {
-    static const bool pair_default = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR"); return e == nullptr || e[0] != '0'; }();
-    const GemmChoice g = choose_gemm(M, N, K, a.size(0) * a.size(1), pair_default && !pair_unavailable && !softmax_epi, !softmax_epi, epilogue,
-                                      a_mn && b_mn);
+  if (auto_bn) {
+    const GemmChoice g = auto_choice(M, N, K, a.size(0) * a.size(1), epilogue, a_mn && b_mn);
     bn = g.bn;
     split = g.split;
   }
@@ -275,7 +295,7 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
     // A device (or partition of one) that cannot schedule clusters of two refuses the launch: remember it and run this and
     // every later product on the one-CTA kernel.
     (void)cudaGetLastError();
-    pair_unavailable = true;
+    g_pair_unavailable = true;
     tmB.m[0] = make_map(b, b_mn ? 64 : 256);
     for (int i = 1; i < 8; ++i) tmB.m[i] = tmB.m[0];
     e = adb200::launch_gemm(tmA, tmB, p, 256, a_mn, b_mn, num_sms(), at::cuda::getCurrentCUDAStream(), p.tma_store ? &tmC : nullptr,
@@ -898,6 +918,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_set_trace", &gemm_set_trace);
   m.def("gemm", &gemm);
   m.def("gemm_split", &gemm_split);
+  m.def("gemm_choice", &gemm_choice);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("gemm_softmax", &gemm_softmax);

@@ -1,4 +1,8 @@
 """The GEMM that splits the contraction over a thread-block cluster, at the edges of its tiles, splits and layouts."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -62,7 +66,22 @@ def test_the_chooser_splits_products_with_few_tiles(M, N, K, batch):
     torch.manual_seed(K)
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
     a, b, ref, mag = _operands(M, N, K, True, True, batch)
+    bn, split = E.gemm_choice(M, N, K, batch, 0, True)
+    assert bn < 512 and split >= 2
     c = torch.empty(batch, M, N, device="cuda")
     E.gemm(a, b, c, True, True, 0, None, None, None, 1.0, 0.0, err, 0)
     assert err.item() == 0
     _close(c, ref, mag, K, 2.0 ** -23)
+
+
+@pytest.mark.parametrize("env,chosen", [({"AUTODIST_GEMM_PAIR_MIN_K": "512"}, (True, True, True, False)),
+                                        ({"AUTODIST_GEMM_PAIR_MIN_K": "1000000"}, (False, False, True, False)),
+                                        ({"AUTODIST_GEMM_PAIR_MIN_K": "0", "AUTODIST_GEMM_PAIR": "0"}, (False, False, False, False))])
+def test_a_fixed_rule_for_the_pair_kernel(env, chosen):
+    """AUTODIST_GEMM_PAIR_MIN_K: products of at least one pair tile whose tiles fill the SM pairs or whose contraction is that long."""
+    code = ("from autodist_b200 import ops; E = ops.ext(required=True); print([E.gemm_choice(*s, 1, 0, False)[0] == 512 for s in "
+            "((512, 512, 600), (1024, 4096, 4096), (2560, 2304, 64), (200, 4096, 4096))])")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, **env), capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    assert out.stdout.strip().splitlines()[-1] == str(list(chosen))

@@ -95,10 +95,11 @@ def test_gemm_on_sm_pairs(E, err, a_mn, b_mn, M, N, K, batch):
 
 def test_gemm_picks_the_pair_kernel_for_large_products_and_matches_the_one_cta_kernel(E, err):
     torch.manual_seed(7)
-    M, N, K = 2560, 2304, 512
+    M, N, K = 2560, 2304, 2048
     a, b = _rand(M, K), _rand(N, K)
     c0, c1 = (torch.empty(M, N, dtype=torch.bfloat16, device="cuda") for _ in range(2))
-    E.gemm(a, b, c0, False, False, 0, None, None, None, 1.0, 0.0, err, 0)        # chooser: 90 pair tiles >= 74 pairs
+    assert E.gemm_choice(M, N, K, 1, 0, False) == (512, 1)                       # two waves of pairs, long enough to pay for them
+    E.gemm(a, b, c0, False, False, 0, None, None, None, 1.0, 0.0, err, 0)
     E.gemm(a, b, c1, False, False, 0, None, None, None, 1.0, 0.0, err, 256)
     torch.cuda.synchronize()
     assert err.item() == 0
