@@ -128,6 +128,9 @@ class BertPretrainer(nn.Module):
         # Heads of 64 columns run on the fused attention kernels (csrc/attention.cu); other head sizes, and ``False`` here, on
         # batched GEMMs with the stand-alone softmax kernels.
         self.fused_attention = True
+        # S == 128: softmax inside the QK^T / dP GEMM epilogues in place of both. Slower than the stand-alone softmax kernels (20.9 vs
+        # 20.1 ms per BERT-large step: a 64-deep contraction cannot hide a 128-exponential epilogue), so off.
+        self.fused_attention_softmax = False
         # Bias gradients (column sums) on a side stream next to the weight-gradient GEMMs instead of between them.
         self.side_stream_bias_grads = os.environ.get("AUTODIST_BERT_SIDE_STREAM", "1") == "1"
 
@@ -186,9 +189,12 @@ class BertPretrainer(nn.Module):
         self._ws = None
         return self.flat
 
+    def _softmax_in_gemm(self, S):
+        return S == 128 and self.fused_attention_softmax
+
     def _fused_attention(self, S):
         c = self.config
-        return self.fused_attention and c.hidden_size == 64 * c.num_attention_heads and S in (64, 128, 256, 512, 1024)
+        return self.fused_attention and not self._softmax_in_gemm(S) and c.hidden_size == 64 * c.num_attention_heads and S in (64, 128, 256, 512, 1024)
 
     def _workspace(self, B, S, P):
         key = (B, S, P, self._fused_attention(S))
@@ -286,7 +292,7 @@ class BertPretrainer(nn.Module):
         gm = lambda *a, **k: self._gemm(ws, *a, **k)   # noqa: E731
         seed = lambda l, site: self._seed + 64 * l + site   # noqa: E731
         scale = 1.0 / math.sqrt(D)
-        fused = self._fused_attention(S)
+        fused, fused_sm = self._fused_attention(S), self._softmax_in_gemm(S)
 
         ids = input_ids.reshape(-1)
         tts = segment_ids.reshape(-1)
@@ -317,8 +323,11 @@ class BertPretrainer(nn.Module):
                 E.attn_fwd(A["qkv"], ws["mask"], A["ctx"], A["lse"], B, S, nh, scale, pa, seed(l, 1), step, ws["err"], A["keep"])
             else:
                 q, k, v = (heads_view(A["qkv"], i) for i in range(3))
-                gm(q, k, ws["scores"], bn=128)
-                E.softmax_fwd(ws["scores"], ws["mask"], A["p"], A["pd"] if pa > 0 else None, scale, pa, seed(l, 1), step)
+                if fused_sm:  # scale, mask, softmax and dropout run in the GEMM epilogue
+                    E.gemm_softmax(q, k, A["p"], A["pd"] if pa > 0 else None, ws["mask"], None, False, scale, pa, seed(l, 1), step, ws["err"])
+                else:
+                    gm(q, k, ws["scores"], bn=128)
+                    E.softmax_fwd(ws["scores"], ws["mask"], A["p"], A["pd"] if pa > 0 else None, scale, pa, seed(l, 1), step)
                 gm(A["pd"] if pa > 0 else A["p"], v, ctx_view(A["ctx"]), b_mn=True, bn=64)
             gm(A["ctx"], w16[n + "out_w"], ws["tmp"], epi=EPI_BIAS, bias=w32[n + "out_b"])
             E.ln_fwd(ws["tmp"], x, w32[n + "ln1_g"], w32[n + "ln1_b"], A["z1"], A["x1"], A["m1"], A["r1"], eps, ph, seed(l, 2), step)
@@ -421,8 +430,11 @@ class BertPretrainer(nn.Module):
                 dq, dk, dv = (heads_view(ws["d_qkv"], i) for i in range(3))
                 pdrop = A["pd"] if pa > 0 else A["p"]
                 gm(pdrop, ctx_view(dctx), dv, a_mn=True, b_mn=True, bn=64)              # dV = P^T . dctx
-                gm(ctx_view(dctx), v, ws["d_p"], bn=128)                                # dP = dctx . V^T
-                E.softmax_bwd(ws["d_p"], A["p"], scale, pa, seed(l, 1), step)           # dS (in place)
+                if fused_sm:  # dS = scale * P * (dP - sum(dP * P)) in the epilogue of dP = dctx . V^T
+                    E.gemm_softmax(ctx_view(dctx), v, ws["d_p"], None, None, A["p"], True, scale, pa, seed(l, 1), step, ws["err"])
+                else:
+                    gm(ctx_view(dctx), v, ws["d_p"], bn=128)                            # dP = dctx . V^T
+                    E.softmax_bwd(ws["d_p"], A["p"], scale, pa, seed(l, 1), step)       # dS (in place)
                 gm(ws["d_p"], k, dq, b_mn=True, bn=64)                                  # dQ = dS . K
                 gm(ws["d_p"], q, dk, a_mn=True, b_mn=True, bn=64)                       # dK = dS^T . Q
             bias_grad(ws["d_qkv"], g[n + "qkv_b"], 3)

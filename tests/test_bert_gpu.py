@@ -23,9 +23,10 @@ def _setup(tie):
     return cfg, model, ref, batch
 
 
-@pytest.mark.parametrize("tie", [False, True])
-def test_fused_bert_matches_reference(tie):
+def _matches_reference(tie, **options):
     cfg, model, ref, batch = _setup(tie)
+    for name, value in options.items():
+        setattr(model, name, value)
     ref = ref.cuda()
     cuda_batch = {k: v.cuda() for k, v in batch.items()}
     loss_ref = ref.reference_loss(**cuda_batch)
@@ -44,6 +45,21 @@ def test_fused_bert_matches_reference(tie):
         if err > 0.08:
             bad.append((n, round(err, 3), denom))
     assert not bad, bad
+
+
+@pytest.mark.parametrize("tie", [False, True])
+def test_fused_bert_matches_reference(tie):
+    _matches_reference(tie)
+
+
+@pytest.mark.parametrize("options,kernel", [({}, "attn_fwd"), ({"fused_attention": False}, "softmax_fwd"), ({"fused_attention_softmax": True}, "gemm_softmax")])
+def test_each_attention_route_matches_reference(options, kernel, monkeypatch):
+    from autodist_b200 import ops
+    E, calls = ops.ext(required=True), set()
+    for name in ("attn_fwd", "softmax_fwd", "gemm_softmax"):
+        monkeypatch.setattr(E, name, lambda *a, _f=getattr(E, name), _n=name: (calls.add(_n), _f(*a))[1])
+    _matches_reference(False, **options)
+    assert calls == {kernel}
 
 
 def test_dropout_path_runs_and_is_reproducible():
