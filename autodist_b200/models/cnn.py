@@ -16,8 +16,7 @@ import torch
 from torch import nn
 import torch.nn.functional as F
 
-from autodist_b200.ops.functional import (Linear, batch_norm, batch_norm_eval, cat_channels, channel_sums, conv2d, conv_bn_eval, fork,
-                                          max_pool2d)
+from autodist_b200.ops.functional import (Linear, batch_norm, batch_norm_eval, channel_sums, conv2d, conv_bn_eval, fork, max_pool2d)
 
 CONV_MODE = os.environ.get("AUTODIST_CONV", "own")                      # own | library
 
@@ -62,10 +61,15 @@ class BatchNormAct(nn.BatchNorm2d):
         super().__init__(channels)
         self.relu = relu
 
-    def forward(self, x, residual=None, sums=None, fork=None, in_fork=None):
+    def forward(self, x, residual=None, sums=None, fork=None, alias=False):
+        """``alias``: returns ``(y, x)`` with an ``x`` for its second consumer (``ops.functional.batch_norm``)."""
         if _own_norm_pool(x) and self.training and self.momentum is not None:
             return batch_norm(x, self.weight, self.bias, self.running_mean, self.running_var, True, self.momentum, self.eps, self.relu,
-                              residual, sums, self.num_batches_tracked, fork, in_fork)
+                              residual, sums, self.num_batches_tracked, fork, alias)
+        y = self._library(x, residual)
+        return (y, x) if alias else y
+
+    def _library(self, x, residual):
         if not self.training and NORM_POOL_MODE != "library":
             y = batch_norm_eval(x, self.weight, self.bias, self.running_mean, self.running_var, self.eps, self.relu, residual)
             if y is not None:
@@ -74,6 +78,10 @@ class BatchNormAct(nn.BatchNorm2d):
         if residual is not None:
             y = y + residual
         return F.relu(y, inplace=True) if self.relu else y
+
+    def takes_sums(self):
+        """Whether a training pass on the kernel path normalises with sums that a convolution left."""
+        return self.training and self.momentum is not None and self.num_features % 8 == 0
 
 
 class _StatsArena:
@@ -246,17 +254,28 @@ class _DenseLayer(nn.Module):
     def forward(self, x):
         return torch.cat([x, self.f(x)], 1)
 
-    def step(self, x, sums):
+    def steps(self):
+        """The four modules where they can be run one by one - as built, no hook anywhere, batch statistics - or ``None``."""
+        f = self.f
+        if type(self) is not _DenseLayer or type(f) is not nn.Sequential or len(f) != 4 or "forward" in self.__dict__ or "forward" in f.__dict__:
+            return None
+        mods = bn1, conv1, bn2, conv2 = tuple(f._modules.values())
+        if type(bn1) is BatchNormAct and type(bn2) is BatchNormAct and type(conv1) is Conv2d and type(conv2) is Conv2d and \
+                not _hooked(self, f, *mods) and bn1.takes_sums() and bn2.takes_sums():
+            return mods
+        return None
+
+    @staticmethod
+    def step(mods, x, sums):
         """Training step on the kernel path: ``sums`` are the per-channel sums of ``x``; returns the concatenation and its sums. Every
         batch-norm gets its statistics from the convolution that produced the channels (the ones of earlier layers are the
         same numbers again), and the gradient that reaches ``x`` through the concatenation is added inside the first
         batch-norm's backward pass."""
-        bn1, conv1, bn2, conv2 = self.f
-        xa, xc, box = fork(x) if FORK_FUSION else (x, x, None)
+        bn1, conv1, bn2, conv2 = mods
         s1, s2 = _ARENA.take(conv1.out_channels, x.device), _ARENA.take(conv2.out_channels, x.device)
-        h = conv1(bn1(xa, sums=sums, in_fork=box), s1)
-        new = conv2(bn2(h, sums=s1), s2)
-        return cat_channels(xc, new, box), torch.cat([sums, s2], 1)
+        h, x = bn1(x, sums=sums, alias=True) if FORK_FUSION else (bn1(x, sums=sums), x)
+        new = conv2(bn2(conv1(h, s1), sums=s1), s2)
+        return torch.cat([x, new], 1), torch.cat([sums, s2], 1)
 
 
 class DenseNet121(nn.Module):
@@ -275,24 +294,39 @@ class DenseNet121(nn.Module):
         self.features = nn.Sequential(*mods)
         self.fc = Linear(c, num_classes)
 
-    def _fused(self, x):
-        mods = list(self.features.modules())
-        return x.is_cuda and self.training and torch.is_autocast_enabled() and CONV_MODE != "library" and NORM_POOL_MODE != "library" and \
-            FUSE_BN_STATS and not _hooked(*mods) and \
-            all(m.training and m.momentum is not None and m.num_features % 8 == 0 for m in mods if isinstance(m, BatchNormAct))
+    def _plan(self, x):
+        """``[(module, its steps or None)]`` where the features can be run module by module with the sums handed along, else ``None``.
+        The containers are then not called: no hook may watch them. (Looked up per forward pass, with as few steps of the host as
+        possible: an eager step is bound by them.)"""
+        f = self.features
+        if not (x.is_cuda and self.training and torch.is_autocast_enabled() and CONV_MODE != "library" and NORM_POOL_MODE != "library" and
+                FUSE_BN_STATS) or type(f) is not nn.Sequential or "forward" in f.__dict__ or _hooked(f):
+            return None
+        plan = []
+        for m in f._modules.values():
+            steps = None
+            if isinstance(m, _DenseLayer):
+                steps = m.steps()
+                if steps is None:
+                    return None
+            elif _hooked(*m.modules()) or (isinstance(m, BatchNormAct) and not m.takes_sums()):
+                return None
+            plan.append((m, steps))
+        return plan
 
     def forward(self, x):
-        if self._fused(x):
+        plan = self._plan(x)
+        if plan is None:
+            x = self.features(x)
+        else:
             sums = None
-            for m in self.features:
-                if isinstance(m, _DenseLayer):
-                    x, sums = m.step(x, channel_sums(x) if sums is None else sums)
-                elif isinstance(m, BatchNormAct) and sums is not None:      # the transition's, or the last one
+            for m, steps in plan:
+                if steps is not None:
+                    x, sums = _DenseLayer.step(steps, x, channel_sums(x) if sums is None else sums)
+                elif sums is not None and isinstance(m, BatchNormAct):      # the transition's, or the last one
                     x, sums = m(x, sums=sums), None
                 else:
                     x, sums = m(x), None
-        else:
-            x = self.features(x)
         return self.fc(torch.flatten(F.adaptive_avg_pool2d(x, 1), 1))
 
 

@@ -559,27 +559,6 @@ def _row_view(t, xh):
     return p.as_strided((n * h * w, c), (ld, 1))
 
 
-class _CatChannelsFn(torch.autograd.Function):
-    """``torch.cat([x, new], 1)`` whose gradient for ``x`` is left, as a view, for the kernel of ``x``'s other consumer."""
-
-    @staticmethod
-    def forward(ctx, x, new, fork):
-        ctx.fork, ctx.c = fork, x.shape[1]
-        return torch.cat([x, new], 1)
-
-    @staticmethod
-    def backward(ctx, dy):
-        dx, dn = dy[:, :ctx.c], dy[:, ctx.c:]
-        if ctx.needs_input_grad[0] and ctx.fork.grad is None:
-            ctx.fork.grad, dx = dx, None
-        return dx, dn, None
-
-
-def cat_channels(x, new, fork=None):
-    """Channel concatenation; ``fork`` is the ``GradFork`` of ``x`` when a ``batch_norm(in_fork=...)`` reads it too."""
-    return torch.cat([x, new], 1) if fork is None else _CatChannelsFn.apply(x, new, fork)
-
-
 def channel_sums(x):
     """Per-channel sum and sum of squares (fp32 ``[2, C]``) of a CUDA tensor, as ``conv2d(stats=...)`` leaves them."""
     with torch.no_grad():
@@ -592,9 +571,9 @@ class _BatchNormFn(torch.autograd.Function):
     convolution's epilogue leaves them) skips the statistics pass."""
 
     @staticmethod
-    def forward(ctx, x, gamma, beta, residual, eps, relu, sums, running, fork=None, in_fork=None):
+    def forward(ctx, x, gamma, beta, residual, eps, relu, sums, running, fork=None, alias=False):
         E = ops.ext(required=True)
-        ctx.fork, ctx.in_fork = fork, in_fork
+        ctx.fork = fork
         run_mean, run_var, batches, momentum = running if running is not None else (None, None, None, 0.0)
         xh = _nhwc(x)                                                            # [N, H, W, C]
         c = xh.shape[-1]
@@ -614,14 +593,14 @@ class _BatchNormFn(torch.autograd.Function):
         ctx.has_res = residual is not None
         ctx.dtypes = (x.dtype, gamma.dtype, residual.dtype if residual is not None else None)
         ctx.mark_non_differentiable(mean, rstd)
-        return y.permute(0, 3, 1, 2), mean, rstd
+        return y.permute(0, 3, 1, 2), mean, rstd, x.view_as(x) if alias else None
 
     @staticmethod
-    def backward(ctx, dy, _dm, _dr):
+    def backward(ctx, dy, _dm, _dr, other):
         E = ops.ext(required=True)
         xh, keep, mean, rstd, g32 = ctx.saved_tensors
         if dy is None:
-            return (None,) * 10
+            return (other,) + (None,) * 9
         dyh = _nhwc(dy)
         dx = torch.empty_like(xh)
         dres = None
@@ -630,8 +609,7 @@ class _BatchNormFn(torch.autograd.Function):
         gamma, beta = ctx.params
         acc_g, acc_b = _direct_grad(gamma), _direct_grad(beta)
         direct = acc_g is not None and acc_b is not None
-        other = ctx.in_fork.take() if ctx.in_fork is not None else None         # what x's other consumer left: added in the same pass
-        add = _row_view(other, xh) if other is not None else None
+        add = _row_view(other, xh) if other is not None else None               # what x's alias received: added in the same pass
         sums = E.bn_bwd(dyh, xh, keep, mean, rstd, g32, dx, dres if ctx.relu else None, ctx.relu, acc_g if direct else None,
                         acc_b if direct else None, add)
         gx = dx.permute(0, 3, 1, 2).to(ctx.dtypes[0])
@@ -652,20 +630,22 @@ class _BatchNormFn(torch.autograd.Function):
 
 
 def batch_norm(x, gamma, beta, running_mean=None, running_var=None, training=True, momentum=0.1, eps=1e-5, relu=False,
-               residual=None, sums=None, num_batches_tracked=None, fork=None, in_fork=None):
+               residual=None, sums=None, num_batches_tracked=None, fork=None, alias=False):
     """``relu?(batch_norm(x) + residual)`` of an NCHW / channels-last tensor; updates the running statistics like
     ``F.batch_norm``. ``sums``: per-channel sum / sum of squares of ``x`` when a preceding kernel already produced them;
-    ``fork`` / ``in_fork``: the ``GradFork`` of ``residual`` / of ``x`` when that tensor has a second consumer."""
+    ``fork``: the ``GradFork`` of ``residual`` when that tensor has a second consumer. ``alias``: returns ``(y, x)`` with an ``x``
+    for its second consumer, whose gradient is added inside the backward pass (a channel slice is read in place)."""
     if not (x.is_cuda and training and x.shape[1] % 8 == 0):
         y = F.batch_norm(x, running_mean, running_var, gamma.to(x.dtype) if x.dtype != gamma.dtype and not x.is_cuda else gamma,
                          beta, training, momentum, eps)
         if residual is not None:
             y = y + residual
-        return F.relu(y) if relu else y
+        y = F.relu(y) if relu else y
+        return (y, x) if alias else y
     running = None
     if running_mean is not None and running_mean.dtype == torch.float32 and running_var.dtype == torch.float32:
         running = (running_mean, running_var, num_batches_tracked, float(momentum))     # folded into the statistics kernel
-    y, mean, rstd = _BatchNormFn.apply(x, gamma, beta, residual, eps, relu, sums, running, fork, in_fork)
+    y, mean, rstd, x_alias = _BatchNormFn.apply(x, gamma, beta, residual, eps, relu, sums, running, fork, alias)
     if running is None and running_mean is not None:
         with torch.no_grad():
             n = x.numel() // x.shape[1]
@@ -674,7 +654,7 @@ def batch_norm(x, gamma, beta, running_mean=None, running_var=None, training=Tru
             running_var.mul_(1 - momentum).add_(var.to(running_var.dtype), alpha=momentum)
         if num_batches_tracked is not None:
             num_batches_tracked.add_(1)
-    return y
+    return (y, x_alias) if alias else y
 
 
 class _MaxPoolFn(torch.autograd.Function):

@@ -55,9 +55,9 @@ def test_concatenation_gradient_is_added_inside_batch_norm(n, c, extra, h, w):
     for fused in (True, False):
         x = x0.clone().requires_grad_(True)
         g, b = gamma.clone().requires_grad_(True), beta.clone().requires_grad_(True)
-        xa, xc, box = Fn.fork(x * 1) if fused else (x, x, None)
-        y = Fn.batch_norm(xa, g, b, relu=True, sums=Fn.channel_sums(x0), in_fork=box)
-        out = Fn.cat_channels(xc, new, box)
+        y = Fn.batch_norm(x * 1, g, b, relu=True, sums=Fn.channel_sums(x0), alias=True) if fused else Fn.batch_norm(x, g, b, relu=True, sums=Fn.channel_sums(x0))
+        y, xc = y if fused else (y, x)
+        out = torch.cat([xc, new], 1)
         torch.autograd.backward([out, y], [dcat, dy])
         grads.append(x.grad)
     # one rounding to bf16 instead of three
@@ -82,3 +82,35 @@ def test_dense_network_step_matches_the_plain_route(monkeypatch):
                      net.features[-1].running_mean.clone()))
     for a, b in zip(*outs):                    # the same values in another order of summation and with fewer roundings
         assert (a - b).norm() <= 0.05 * b.norm()
+
+
+def test_dense_network_step_records_no_more_functions_than_the_plain_route(monkeypatch):
+    """An eager step is bound by the host, where every autograd function written in Python costs as much as a launch."""
+    from autodist_b200.models import cnn
+    torch.manual_seed(0)
+    net = cnn.DenseNet121(growth=8, blocks=(2, 2, 2, 2), num_classes=16).cuda()
+    x = torch.randn(4, 3, 64, 64, device="cuda").contiguous(memory_format=torch.channels_last)
+    counts = []
+    for fused in (True, False):
+        monkeypatch.setattr(cnn, "FUSE_BN_STATS", fused)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            stack, seen = [net(x).sum().grad_fn], set()
+        while stack:
+            node = stack.pop()
+            if node is not None and node not in seen:
+                seen.add(node)
+                stack += [n for n, _ in node.next_functions]
+        counts.append(sum("FnBackward" in n.name() for n in seen))
+    assert 0 < counts[0] <= counts[1]
+
+
+def test_a_changed_layer_keeps_to_the_plain_route():
+    from autodist_b200.models import cnn
+    net = cnn.DenseNet121(growth=8, blocks=(2, 2, 2, 2), num_classes=16).cuda()
+    x = torch.randn(2, 3, 64, 64, device="cuda").contiguous(memory_format=torch.channels_last)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert net._plan(x) is not None
+        net.features[3].f.append(torch.nn.Dropout(0.5))                # five modules where the kernel path expects four
+        assert net._plan(x) is None
+        net(x).float().sum().backward()
+    assert torch.isfinite(net.fc.weight.grad).all()
