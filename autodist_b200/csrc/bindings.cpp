@@ -108,6 +108,15 @@ bool make_store_map(const Tensor& v, CUtensorMap* out) {
   return r == CUDA_SUCCESS;
 }
 
+// Whether every row of a 4-D output view starts on a 16-byte boundary.
+bool rows_aligned(const Tensor& v) {
+  const int64_t n = 16 / v.element_size();
+  if (reinterpret_cast<uintptr_t>(v.data_ptr()) % 16 != 0) return false;
+  for (int d = 0; d < 3; ++d)
+    if (v.size(d) > 1 && v.stride(d) % n != 0) return false;
+  return true;
+}
+
 // Tuning aid: when set (int64 CUDA tensor of at least 8 x SM-count words, zeroed by the caller), launches of the two-CTA
 // GEMM record nanosecond marks per CTA into it (see gemm_tcgen05_2cta.cu).
 long long* g_gemm_trace = nullptr;
@@ -270,6 +279,8 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
       p.aux = reinterpret_cast<const __nv_bfloat16*>(av.data_ptr());
     }
   }
+  p.vec_ok = rows_aligned(c) && (p.C2 == nullptr || rows_aligned(as4d(*c2))) && (p.aux == nullptr || rows_aligned(as4d(*aux)));
+  TORCH_CHECK(!softmax_epi || p.vec_ok, "the softmax epilogues need outputs that start on 16-byte boundaries");
   p.error_flag = error_flag.data_ptr<int>();
   // Output through shared memory and TMA (whole lines instead of 16-byte pieces of 32 rows per store instruction) for
   // products large enough to care; AUTODIST_GEMM_TMA_STORE=0 keeps direct stores everywhere.
@@ -360,6 +371,7 @@ void gemm_gathered_b(const Tensor& a_, const std::vector<int64_t>& shard_ptrs, i
   adb200::GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.batch_lo = 1; p.batch_hi = 1;
   p.C = c.data_ptr(); p.ldc = c.stride(2); p.strideC_lo = 0; p.strideC_hi = 0;
+  p.vec_ok = rows_aligned(c);
   p.c_is_fp32 = c.scalar_type() == at::kFloat;
   p.epilogue = (int)epilogue; p.alpha = 1.0f; p.beta = 0.0f;
   p.bias = nullptr; p.C2 = nullptr; p.aux = nullptr;
@@ -404,6 +416,7 @@ void gemm_gathered_bt(const Tensor& a_, const std::vector<int64_t>& shard_ptrs, 
   adb200::GemmParams p{};
   p.M = M; p.N = (int)cols; p.K = K; p.batch_lo = 1; p.batch_hi = 1;
   p.C = c.data_ptr(); p.ldc = c.stride(2); p.strideC_lo = 0; p.strideC_hi = 0;
+  p.vec_ok = rows_aligned(c);
   p.c_is_fp32 = c.scalar_type() == at::kFloat;
   p.epilogue = adb200::EPI_NONE; p.alpha = 1.0f; p.beta = 0.0f;
   p.error_flag = error_flag.data_ptr<int>();

@@ -298,7 +298,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     if (p.c_is_fp32) {
       float* dst = reinterpret_cast<float*>(p.C) + coff + col0;
       if (p.beta != 0.0f) {
-        if (ncols == 16 && (p.ldc % 4 == 0)) {
+        if (ncols == 16 && vec_ok) {
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
             float4 o = *reinterpret_cast<float4*>(dst + j);
@@ -309,7 +309,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
 #pragma unroll
           for (int j = 0; j < 16; ++j) if (j < ncols) dst[j] += v[j];
         }
-      } else if (ncols == 16 && (p.ldc % 4 == 0)) {
+      } else if (ncols == 16 && vec_ok) {
 #pragma unroll
         for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
       } else {

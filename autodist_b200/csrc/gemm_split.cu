@@ -52,7 +52,6 @@ __device__ __forceinline__ void reduce_and_store(const GemmParams& p, uint32_t t
   const int rows = min(BM, p.M - m0);                        // rows of the tile that exist
   const int r0 = (int)rank * rows / S, r1 = ((int)rank + 1) * rows / S;
   constexpr int CH = BN / 4;                                 // 16-byte chunks per row
-  const bool vec_ok = (p.ldc % 8 == 0);
   uint32_t peer[S];
 #pragma unroll
   for (int s = 0; s < S; ++s) peer[s] = map_to_cta(tile, (uint32_t)s);
@@ -69,11 +68,12 @@ __device__ __forceinline__ void reduce_and_store(const GemmParams& p, uint32_t t
     const int row = m0 + r, col0 = n0 + 4 * c;
     const int ncols = min(4, p.N - col0);
     if (ncols <= 0) continue;
+    const bool wide = ncols == 4 && p.vec_ok != 0;
     const long long coff = batch_off + (long long)row * p.ldc;
-    gemm_epilogue_math<4>(p, v, col0, ncols, coff, vec_ok);
+    gemm_epilogue_math<4>(p, v, col0, ncols, coff, p.vec_ok != 0);
     if (p.c_is_fp32) {
       float* dst = reinterpret_cast<float*>(p.C) + coff + col0;
-      if (ncols == 4 && p.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+      if (wide) {
         float4 o = make_float4(v[0], v[1], v[2], v[3]);
         if (p.beta != 0.0f) {
           const float4 old = *reinterpret_cast<const float4*>(dst);
@@ -86,8 +86,7 @@ __device__ __forceinline__ void reduce_and_store(const GemmParams& p, uint32_t t
       }
     } else {
       __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + coff + col0;
-      const bool wide = ncols == 4 && vec_ok;
-      if (wide && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+      if (wide) {
         *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
       } else {
 #pragma unroll
@@ -95,7 +94,7 @@ __device__ __forceinline__ void reduce_and_store(const GemmParams& p, uint32_t t
       }
       if (p.epilogue == EPI_BIAS_GELU) {
         __nv_bfloat16* dst2 = p.C2 + coff + col0;
-        if (wide && (reinterpret_cast<uintptr_t>(dst2) & 7) == 0) {
+        if (wide) {
           *reinterpret_cast<uint2*>(dst2) = make_uint2(pack_bf16x2(gelu_tanh(v[0]), gelu_tanh(v[1])), pack_bf16x2(gelu_tanh(v[2]), gelu_tanh(v[3])));
         } else {
 #pragma unroll

@@ -182,7 +182,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;                  // 0, or 1 for the second warp of a lane quarter
     int as = 0; uint32_t aphase = 0; bool ok = true;
-    const bool vec_ok = (p.ldc % 8 == 0);
+    const bool vec_ok = p.vec_ok != 0;
     EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, make_float4(0.f, 0.f, 0.f, 0.f)};
     for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
       const int b = (int)(t / per_batch), rem = (int)(t % per_batch);

@@ -14,6 +14,7 @@ struct GemmParams {
   int batch_lo, batch_hi;      // two batch dimensions (1 when unused)
   void* C;                     // output, bf16 or fp32, row-major with leading dimension ldc (elements)
   long long ldc, strideC_lo, strideC_hi;
+  int vec_ok;                  // rows of C (C2, aux) start on 16-byte boundaries: vector loads and stores are possible
   int c_is_fp32;
   __nv_bfloat16* C2;           // EPI_BIAS_GELU: gelu(C) goes here (same strides as C)
   const float* bias;           // EPI_BIAS*: one value per output column

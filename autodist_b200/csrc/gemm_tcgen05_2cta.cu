@@ -187,7 +187,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;                  // which half of the tile's columns this warp drains
     int as = 0; uint32_t aphase = 0; bool ok = true;
-    const bool vec_ok = (p.ldc % 8 == 0);
+    const bool vec_ok = p.vec_ok != 0;
     EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, make_float4(0.f, 0.f, 0.f, 0.f)};
     for (long long t = pair; t < total && ok; t += pairs) {
       const int b = (int)(t / per_batch), rem = (int)(t % per_batch);

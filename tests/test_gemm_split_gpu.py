@@ -85,3 +85,38 @@ def test_a_fixed_rule_for_the_pair_kernel(env, chosen):
     out = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, **env), capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stderr
     assert out.stdout.strip().splitlines()[-1] == str(list(chosen))
+
+
+@pytest.mark.parametrize("bn,split", [(64, 1), (128, 1), (256, 1), (512, 1), (64, 2), (256, 3)])
+@pytest.mark.parametrize("offset", [1, 4])
+def test_outputs_that_start_anywhere_in_their_storage(bn, split, offset):
+    """Rows off the 16-byte boundaries of the vector stores: output, second output and auxiliary operand."""
+    from autodist_b200 import ops
+    E = ops.ext(required=True)
+    torch.manual_seed(bn + split)
+    M, N, K, ld = 300, 272, 264, 280
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a, b, ref, mag = _operands(M, N, K, False, False)
+    ref, mag = ref[0], mag[0]
+
+    def view(dtype, at):
+        return torch.zeros(at + M * ld, dtype=dtype, device="cuda")[at:].view(M, ld)[:, :N]
+
+    def run(c, epilogue, bias, c2, aux, beta):
+        args = (a[0], b[0], c, False, False, epilogue, bias, c2, aux, 1.0, beta, err, bn)
+        E.gemm(*args) if split == 1 else E.gemm_split(*args, split)
+
+    c32 = view(torch.float32, offset)
+    for times in (1, 2):
+        run(c32, 0, None, None, None, 1.0)
+        _close(c32, times * ref, times * mag, K, 2.0 ** -22)
+    bias = torch.randn(offset + N, device="cuda")[offset:]
+    pre, act = view(torch.bfloat16, offset), view(torch.bfloat16, offset)
+    run(pre, 2, bias, act, None, 0.0)
+    _close(pre, ref + bias.double(), mag + bias.double().abs(), K, 2.0 ** -8)
+    for where in (0, offset):                                       # the output, then the addend alone off the boundary
+        out, add = view(torch.bfloat16, offset - where), view(torch.bfloat16, where)
+        add.copy_(pre)
+        run(out, 4, None, None, add, 0.0)
+        _close(out, ref + pre.double(), mag + pre.double().abs(), K, 2.0 ** -8)
+    assert err.item() == 0
