@@ -682,6 +682,26 @@ void bn_fwd(const Tensor& x, const Tensor& gamma, const Tensor& beta, const opti
                  part.data_ptr<float>(), sums.data_ptr<float>(), rows, C, (float)eps, relu ? 1 : 0, 0, rm, rv, nb, (float)momentum,
                  STREAM);
 }
+// The same from a logical [N, C, H, W] tensor with every view and allocation made here: an eager step is bounded by host time, and the
+// Python steps around a call cost more than its launches. Returns x as it was read (bf16 [N, H, W, C]), y (logical [N, C, H, W]), the
+// keep bytes (with relu), mean, rstd and gamma in fp32.
+std::tuple<Tensor, Tensor, optional<Tensor>, Tensor, Tensor, Tensor> bn_fwd_nchw(const Tensor& x, const Tensor& gamma, const Tensor& beta,
+                                                                                 const optional<Tensor>& res, double eps, bool relu,
+                                                                                 const optional<Tensor>& sums, const optional<Tensor>& run_mean,
+                                                                                 const optional<Tensor>& run_var, const optional<Tensor>& batches,
+                                                                                 double momentum) {
+  TORCH_CHECK(x.is_cuda() && x.dim() == 4, "x must be a CUDA [N, C, H, W] tensor");
+  auto nhwc = [](const Tensor& t) { return t.permute({0, 2, 3, 1}).to(at::kBFloat16).contiguous(); };
+  const Tensor xh = nhwc(x);
+  const Tensor g32 = gamma.detach().to(at::kFloat).contiguous(), b32 = beta.detach().to(at::kFloat).contiguous();
+  Tensor y = at::empty_like(xh);
+  Tensor mean = at::empty({xh.size(3)}, xh.options().dtype(at::kFloat)), rstd = at::empty_like(mean);
+  optional<Tensor> r, keep;
+  if (res.has_value()) r = nhwc(*res);
+  if (relu) keep = at::empty({xh.numel() / 8}, xh.options().dtype(at::kByte));
+  bn_fwd(xh, g32, b32, r, y, mean, rstd, eps, relu, sums, run_mean, run_var, batches, momentum, keep);
+  return {xh, y.permute({0, 3, 1, 2}), keep, mean, rstd, g32};
+}
 // y = relu?(x * scale + shift (+ res)) over a channels-last matrix [rows, C] with the running statistics (evaluation mode).
 void bn_eval(const Tensor& x, const optional<Tensor>& res, Tensor y, const Tensor& gamma, const Tensor& beta, const Tensor& mean,
              const Tensor& var, double eps, bool relu) {
@@ -706,6 +726,8 @@ Tensor bn_sums(const Tensor& x) {
 }
 // Returns [dbeta, dgamma] stacked as a [2, C] fp32 tensor; writes dx and (optional) dres = dy masked by the ReLU.
 // dgamma_acc / dbeta_acc (optional, fp32 [C]): the batch-norm parameters' gradient buffers; the sums are added into them.
+// add (optional, bf16, logical [N, C, H, W] with x [N, H, W, C]): another gradient of x, added to dx. A channel slice of a
+// channels-last tensor, whose rows lie a constant distance apart, is read in place.
 Tensor bn_bwd(const Tensor& dy, const Tensor& x, const optional<Tensor>& keep, const Tensor& mean, const Tensor& rstd, const Tensor& gamma, Tensor dx,
               const optional<Tensor>& dres, bool relu, const optional<Tensor>& dgamma_acc, const optional<Tensor>& dbeta_acc,
               const optional<Tensor>& add) {
@@ -713,10 +735,19 @@ Tensor bn_bwd(const Tensor& dy, const Tensor& x, const optional<Tensor>& keep, c
   TORCH_CHECK(C % 8 == 0 && C <= 16384 && x.is_contiguous() && dy.is_contiguous() && dx.is_contiguous() && dy.numel() == x.numel() && dx.numel() == x.numel(),
               "dy, x, dx must be contiguous bf16 [.., C] of one shape, C % 8 == 0");
   if (dres.has_value()) TORCH_CHECK(dres->is_contiguous() && dres->numel() == x.numel() && dres->scalar_type() == at::kBFloat16, "dres must match x");
-  if (add.has_value()) {            // [rows, C] view whose rows may lie further apart than C
-    TORCH_CHECK(add->dim() == 2 && add->size(0) == rows && add->size(1) == C && add->scalar_type() == at::kBFloat16 && (C == 1 || add->stride(1) == 1) &&
-                add->stride(0) >= C && add->stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(add->data_ptr()) % 16 == 0,
-                "the addend must be a bf16 [rows, C] view with aligned rows");
+  Tensor other;
+  int64_t other_ld = 0;
+  if (add.has_value()) {
+    TORCH_CHECK(x.dim() == 4 && add->is_cuda() && add->scalar_type() == at::kBFloat16 && add->dim() == 4 && add->size(0) == x.size(0) &&
+                add->size(1) == C && add->size(2) == x.size(1) && add->size(3) == x.size(2), "the addend must be bf16 [N, C, H, W]");
+    other = add->permute({0, 2, 3, 1});
+    other_ld = C;
+    const int64_t pixels[3] = {(int64_t)x.size(1) * x.size(2), x.size(2), 1};      // pixels between two neighbours of a dimension
+    for (int d = 2; d >= 0; --d)
+      if (x.size(d) > 1) { other_ld = other.stride(d) / pixels[d]; break; }
+    bool regular = other.stride(3) == 1 && other_ld >= C && other_ld % 8 == 0 && reinterpret_cast<uintptr_t>(other.data_ptr()) % 16 == 0;
+    for (int d = 0; d < 3; ++d) regular &= x.size(d) <= 1 || other.stride(d) == other_ld * pixels[d];
+    if (!regular) { other = other.clone(at::MemoryFormat::Contiguous); other_ld = C; }
   }
   TORCH_CHECK(!relu || (keep.has_value() && keep->scalar_type() == at::kByte && keep->is_contiguous() && keep->numel() * 8 == x.numel()),
               "the forward pass's keep bytes are needed with a fused ReLU");
@@ -729,7 +760,7 @@ Tensor bn_bwd(const Tensor& dy, const Tensor& x, const optional<Tensor>& keep, c
   Tensor sums = at::empty({5, C}, x.options().dtype(at::kFloat));              // [dbeta, dgamma, A, B, K]
   adb200::bn_bwd(CBF(dy), CBF(x), relu ? keep->data_ptr<uint8_t>() : nullptr, mean.data_ptr<float>(), rstd.data_ptr<float>(), gamma.data_ptr<float>(), BF(dx), OPT_BF(dres),
                  part.data_ptr<float>(), sums.data_ptr<float>(), sums.data_ptr<float>() + 2 * C, rows, C, relu ? 1 : 0, OPT_F(dgamma_acc),
-                 OPT_F(dbeta_acc), add.has_value() ? CBF(*add) : nullptr, add.has_value() ? add->stride(0) : 0, STREAM);
+                 OPT_F(dbeta_acc), other.defined() ? CBF(other) : nullptr, other_ld, STREAM);
   return sums.narrow(0, 0, 2);
 }
 // code: uint8 [N, Ho, Wo, C], the window position of each output's first maximum
@@ -965,6 +996,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("flagged_rows_update", &flagged_rows_update);
   m.def("cast_f32_bf16", &cast_f32_bf16);
   m.def("bn_fwd", &bn_fwd);
+  m.def("bn_fwd_nchw", &bn_fwd_nchw);
   m.def("bn_sums", &bn_sums);
   m.def("bn_eval", &bn_eval);
   m.def("bn_bwd", &bn_bwd);

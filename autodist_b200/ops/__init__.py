@@ -20,7 +20,7 @@ launch_count = 0      # kernels launched through the extension by this process (
 class _Counting:
     """Thin proxy over the extension module that counts kernel-launching calls."""
     _NO_LAUNCH = {"ln_bwd_blocks", "ln_bwd_part_floats", "colsum_parts", "gemm_choice", "MAX_COMM_BLOCKS"}
-    _MULTI = {"ln_bwd": 2, "keyed_colsum": 2, "bn_fwd": 3, "bn_bwd": 3, "attn_bwd": 2}
+    _MULTI = {"ln_bwd": 2, "keyed_colsum": 2, "bn_fwd": 3, "bn_fwd_nchw": 3, "bn_bwd": 3, "attn_bwd": 2}
 
     def __init__(self, mod):
         self._mod = mod

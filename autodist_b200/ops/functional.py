@@ -545,20 +545,6 @@ def batch_norm_eval(x, gamma, beta, running_mean, running_var, eps, relu=False, 
     return _BNEvalFn.apply(x, gamma, beta, running_mean, running_var, eps, bool(relu), residual)
 
 
-def _row_view(t, xh):
-    """``t`` (logical [N, C, H, W]) as a bf16 [N * H * W, C] view whose rows lie a constant, 16-byte aligned distance apart - a channel
-    slice of a channels-last tensor is one - or ``None``. ``xh`` is the channels-last tensor it is added to."""
-    n, h, w, c = xh.shape
-    if t.dtype != torch.bfloat16 or tuple(t.shape) != (n, c, h, w) or not t.is_cuda:
-        return None
-    p = t.permute(0, 2, 3, 1)
-    ld = next((p.stride(d) // k for d, k in ((2, 1), (1, w), (0, h * w)) if p.shape[d] > 1), c)
-    regular = all(p.shape[d] == 1 or p.stride(d) == ld * k for d, k in ((2, 1), (1, w), (0, h * w)))
-    if not regular or (c > 1 and p.stride(3) != 1) or ld < c or ld % 8 or t.data_ptr() % 16:
-        return None
-    return p.as_strided((n * h * w, c), (ld, 1))
-
-
 def channel_sums(x):
     """Per-channel sum and sum of squares (fp32 ``[2, C]``) of a CUDA tensor, as ``conv2d(stats=...)`` leaves them."""
     with torch.no_grad():
@@ -575,15 +561,8 @@ class _BatchNormFn(torch.autograd.Function):
         E = ops.ext(required=True)
         ctx.fork = fork
         run_mean, run_var, batches, momentum = running if running is not None else (None, None, None, 0.0)
-        xh = _nhwc(x)                                                            # [N, H, W, C]
-        c = xh.shape[-1]
-        y = torch.empty_like(xh)
-        mean = torch.empty(c, dtype=torch.float32, device=x.device)
-        rstd = torch.empty_like(mean)
-        g32, b32 = gamma.detach().float().contiguous(), beta.detach().float().contiguous()
-        res = _nhwc(residual) if residual is not None else None
-        keep = torch.empty(xh.numel() // 8, dtype=torch.uint8, device=x.device) if relu else None       # which outputs the ReLU let through
-        E.bn_fwd(xh, g32, b32, res, y, mean, rstd, eps, relu, sums, run_mean, run_var, batches, momentum, keep)
+        # keep: which outputs the ReLU let through
+        xh, y, keep, mean, rstd, g32 = E.bn_fwd_nchw(x, gamma, beta, residual, eps, relu, sums, run_mean, run_var, batches, momentum)
         ctx.save_for_backward(xh, keep, mean, rstd, g32)
         ctx.params = (gamma, beta)
         ctx.set_materialize_grads(False)                     # mean / rstd carry no gradient: no zero tensors for them
@@ -593,7 +572,7 @@ class _BatchNormFn(torch.autograd.Function):
         ctx.has_res = residual is not None
         ctx.dtypes = (x.dtype, gamma.dtype, residual.dtype if residual is not None else None)
         ctx.mark_non_differentiable(mean, rstd)
-        return y.permute(0, 3, 1, 2), mean, rstd, x.view_as(x) if alias else None
+        return y, mean, rstd, x.view_as(x) if alias else None
 
     @staticmethod
     def backward(ctx, dy, _dm, _dr, other):
@@ -609,7 +588,7 @@ class _BatchNormFn(torch.autograd.Function):
         gamma, beta = ctx.params
         acc_g, acc_b = _direct_grad(gamma), _direct_grad(beta)
         direct = acc_g is not None and acc_b is not None
-        add = _row_view(other, xh) if other is not None else None               # what x's alias received: added in the same pass
+        add = other if other is not None and other.dtype == torch.bfloat16 else None       # what x's alias received: added in the same pass
         sums = E.bn_bwd(dyh, xh, keep, mean, rstd, g32, dx, dres if ctx.relu else None, ctx.relu, acc_g if direct else None,
                         acc_b if direct else None, add)
         gx = dx.permute(0, 3, 1, 2).to(ctx.dtypes[0])

@@ -41,15 +41,16 @@ def test_training_batch_norm(n, c, h, relu, with_res):
         assert ((rm.double() - mean).abs() <= 1e-5 + 1e-5 * mean.abs()).all() and ((rv.double() - var).abs() <= 1e-4 * var.abs() + 1e-5).all()
 
 
-@pytest.mark.parametrize("n,c,extra,h,w", [(2, 24, 8, 5, 3), (1, 64, 32, 1, 1), (3, 96, 4, 2, 7), (1, 8, 8, 1, 9)])
-def test_concatenation_gradient_is_added_inside_batch_norm(n, c, extra, h, w):
-    """Sliced rows that the kernel can read in place, and (4 extra channels) ones it cannot."""
+@pytest.mark.parametrize("layout", [torch.channels_last, torch.contiguous_format])
+@pytest.mark.parametrize("n,c,extra,h,w", [(2, 24, 8, 5, 3), (1, 64, 32, 1, 1), (3, 96, 4, 2, 7), (1, 8, 8, 1, 9), (4, 16, 16, 1, 1)])
+def test_concatenation_gradient_is_added_inside_batch_norm(n, c, extra, h, w, layout):
+    """Sliced rows that the kernel can read in place, and (4 extra channels, channels apart) ones it cannot."""
     from autodist_b200.ops import functional as Fn
     torch.manual_seed(c)
     x0 = torch.randn(n, c, h, w, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
     new = torch.randn(n, extra, h, w, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
     gamma, beta = torch.rand(c, device="cuda") + 0.5, torch.randn(c, device="cuda")
-    dcat, dy = (torch.randn(n, k, h, w, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last) for k in (c + extra, c))
+    dcat, dy = (torch.randn(n, k, h, w, device="cuda").bfloat16().contiguous(memory_format=layout) for k in (c + extra, c))
     assert torch.allclose(Fn.channel_sums(x0)[1], x0.double().pow(2).sum((0, 2, 3)).float(), rtol=1e-5)
     grads = []
     for fused in (True, False):
