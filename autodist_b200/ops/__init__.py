@@ -17,10 +17,22 @@ _TRIED = False
 launch_count = 0      # kernels launched through the extension by this process (a graph replay re-launches its capture)
 
 
+def _dgrad_launches(dy, w, dx, stride, pad, *_):
+    """One launch per parity class of the input pixels that a filter tap reaches."""
+    kh, kw = w.shape[1:3]
+    return sum(1 for ph in range(min(stride, dx.shape[1])) for pw in range(min(stride, dx.shape[2]))
+               if any((ph + pad - r) % stride == 0 for r in range(kh)) and any((pw + pad - s) % stride == 0 for s in range(kw)))
+
+
 class _Counting:
     """Thin proxy over the extension module that counts kernel-launching calls."""
-    _NO_LAUNCH = {"ln_bwd_blocks", "ln_bwd_part_floats", "colsum_parts", "gemm_choice", "MAX_COMM_BLOCKS"}
-    _MULTI = {"ln_bwd": 2, "keyed_colsum": 2, "bn_fwd": 3, "bn_fwd_nchw": 3, "bn_bwd": 3, "attn_bwd": 2}
+    _NO_LAUNCH = {"ln_bwd_blocks", "ln_bwd_part_floats", "colsum_parts", "gemm_choice", "gemm_set_trace", "conv_set_trace", "MAX_COMM_BLOCKS"}
+    #: kernels per call where that is not one: a number, or a function of the call's arguments
+    _MULTI = {"ln_bwd": 2, "keyed_colsum": 2, "relu_bwd_colsum": 2, "bn_sums": 2, "bn_bwd": 2,
+              "bn_fwd": lambda *a: 1 if a[9] is not None else 3, "bn_fwd_nchw": lambda *a: 1 if a[6] is not None else 3,       # sums given or not
+              "attn_bwd": lambda *a: 2 if a[8] <= 128 else 3,                                                                # tokens
+              "xent": lambda *a: 2 if a[7] else 1,                                                                           # sums the weights
+              "conv_dgrad": _dgrad_launches}
 
     def __init__(self, mod):
         self._mod = mod
@@ -35,10 +47,16 @@ class _Counting:
 
     @staticmethod
     def _wrap(fn, n):
-        def call(*args):
-            global launch_count
-            launch_count += n
-            return fn(*args)
+        if callable(n):
+            def call(*args):
+                global launch_count
+                launch_count += n(*args)
+                return fn(*args)
+        else:
+            def call(*args):
+                global launch_count
+                launch_count += n
+                return fn(*args)
         return call
 
 

@@ -715,3 +715,47 @@ def test_sparse_row_updates_match_the_torch_sparse_optimizers(kind):
     Fn.sparse_rows_update_("sgd", p, (torch.tensor([V + 3, -1], device="cuda"), torch.ones(2, H, device="cuda")), 0.1)
     torch.cuda.synchronize()
     assert torch.equal(p, before) and untouched.all()
+
+
+def test_the_launch_count_is_what_the_device_ran(E, err):
+    """Calls that launch a number of kernels that depends on their arguments, against the profiler's list of kernels."""
+    from autodist_b200 import ops
+    from torch.profiler import ProfilerActivity, profile
+
+    def bf(*shape):
+        return torch.randn(*shape, device="cuda").bfloat16()
+
+    def f32(*shape):
+        return torch.zeros(*shape, device="cuda")
+
+    def attn_bwd(B, S):
+        qkv, ctx, lse = bf(B * S, 192), bf(B * S, 64), f32(B, 1, S)
+        return lambda: E.attn_bwd(qkv, None, ctx, ctx, lse, torch.empty_like(lse), torch.empty_like(qkv), B, S, 1, 0.125, 0.0, err, None)
+
+    def bn(sums):
+        x, p = bf(2, 16, 5, 5), f32(16)
+        return lambda: E.bn_fwd_nchw(x, p, p, None, 1e-5, True, sums, None, None, None, 0.1)
+
+    def dgrad(k, stride, pad, h):
+        oh = (h + 2 * pad - k) // stride + 1
+        dy, w, dx = bf(1, oh, oh, 8), bf(8, k, k, 8), bf(1, h, h, 8)
+        return lambda: E.conv_dgrad(dy, w, dx, stride, pad, err)
+
+    def xent(own):
+        logits, labels, one = bf(4, 16), torch.zeros(4, dtype=torch.int64, device="cuda"), torch.ones(4, device="cuda")
+        return lambda: E.xent(logits, labels, one, torch.ones(1, device="cuda"), f32(1), 16, 1.0, own, 1e-5)
+
+    x, img = bf(64, 16), bf(2, 5, 5, 16)
+    calls = [attn_bwd(2, 128), attn_bwd(2, 256), bn(None), bn(f32(2, 16)), dgrad(3, 1, 1, 6), dgrad(3, 2, 1, 6), dgrad(1, 2, 0, 6), dgrad(2, 2, 0, 6),
+             xent(True), xent(False), lambda: E.bn_sums(img), lambda: E.relu_bwd_colsum(img, img, torch.empty_like(img), f32(16), False),
+             lambda: E.keyed_colsum(x, None, f32(E.colsum_parts(64) * 16), f32(16), 1, False)]
+    for call in calls:
+        call()
+    torch.cuda.synchronize()
+    for i, call in enumerate(calls):
+        before = ops.launch_count
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            call()
+            torch.cuda.synchronize()
+        ran = sum(e.count for e in prof.key_averages() if "adb200" in e.key)
+        assert ran == ops.launch_count - before, f"call {i}: {ran} kernels, counted {ops.launch_count - before}"
