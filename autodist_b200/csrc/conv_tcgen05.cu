@@ -623,6 +623,7 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
       staged = p.staged != 0;
       if (staged) ok = staged_epilogue<BN, MODE>(p, maps, total, tmem_base, tfull, tempty, add_bars, smem_u32(staging), s_stat, do_stats, abort_flag, trace);
     }
+    if constexpr (MODE != CONV_DGRAD)                    // the input gradient is always staged (see launch_conv)
     for (long long t = blockIdx.x; t < total && ok && !staged; t += gridDim.x) {
       const TileCoord tc_ = decode_tile<BN, MODE>(p, t);
       if (MODE == CONV_WGRAD && tc_.kend <= tc_.kbeg) continue;
@@ -774,6 +775,7 @@ cudaError_t launch_conv(const ConvMaps& maps, const ConvParams& p, int bn, int n
   if (p.tw * p.th * p.tn > BM || p.ntaps < 1 || p.ntaps > kMaxConvTaps) return cudaErrorInvalidValue;
   if (p.mode == CONV_WGRAD && (p.tw * p.th * p.tn != BK || p.ksplit < 1)) return cudaErrorInvalidValue;
   if ((p.mode == CONV_EVAL || (p.mode == CONV_FPROP && p.stats != nullptr)) && p.Nc > kMaxStatChannels) return cudaErrorInvalidValue;
+  if (p.mode == CONV_DGRAD && p.staged == 0) return cudaErrorInvalidValue;
   if ((p.mode == CONV_EVAL) != (p.bn_mean != nullptr) || (p.mode == CONV_EVAL && p.stats != nullptr)) return cudaErrorInvalidValue;
 #define ADB_CONV_DISPATCH(BN_)                                                                      \
   if (bn == BN_) {                                                                                  \
