@@ -73,7 +73,6 @@ __device__ __forceinline__ float mask_base2(float mask) { return mask > -INFINIT
 // dropout the rows must be multiples of four long; the launchers check it). mix64 of consecutive counters, their products with the
 // odd constant formed by additions.
 __device__ __forceinline__ uint32_t keep_bits32(uint64_t seed, uint64_t base, uint32_t thresh16) {
-  if (thresh16 > 0xffffu) return 0u;                       // probability 1: no 16-bit field reaches the threshold, nothing is kept
   constexpr uint64_t kStep = 0x9E3779B97F4A7C15ull;
   const uint64_t x0 = seed + (base >> 2) * kStep;
   const uint32_t limit = thresh16 << 16;
@@ -229,6 +228,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
     const float scale2 = p.scale * kLog2e;                 // scores, maxima and exponents are kept in base 2
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
     const uint32_t thresh = (uint32_t)(p.drop_p * 65536.0f);
+    const uint32_t some = thresh > 0xffffu ? 0u : 0xffffffffu;      // probability 1: no 16-bit field reaches the threshold
     const float inv_keep = inverse_keep(p.drop_p);
     const uint64_t sd = p.seed + (p.step ? (uint64_t)(*p.step) * 0x100000001B3ull : 0ull);
     const uint64_t row_off = (((uint64_t)b * p.heads + h) * p.S + row) * p.S;
@@ -287,7 +287,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
         const int key = j * 128 + hf * 64 + c * 32;
         uint32_t bits = 0xffffffffu;
         if (p.drop_p > 0.f) {
-          bits = keep_bits32(sd, row_off + (uint64_t)key, thresh);
+          bits = keep_bits32(sd, row_off + (uint64_t)key, thresh) & some;
           if (row < p.S) p.keep[keep_row + (key >> 5)] = bits;
         }
 #pragma unroll
@@ -523,7 +523,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
         f.delta = p.delta[at];
         if (p.drop_p > 0.f) f.keep = p.keep[at * words + kt * 4 + cb];
       }
-      if (key < p.S) f.mask = p.mask != nullptr ? mask_base2(p.mask[(long long)b * p.S + key]) : 0.f;
+      if (key < p.S) f.mask = p.mask != nullptr ? p.mask[(long long)b * p.S + key] : 0.f;
       return f;
     };
     bool ok = true, stored = false;
@@ -538,8 +538,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
         else if (item + (int)gridDim.x < items) next = fetch(item + gridDim.x, 0);
         // With ps = P / keep probability: P keep = ps where kept, dS = ps * (scale * dP where kept - delta * scale * keep probability).
         // Most blocks of 32 keys carry one mask value; the exponent's argument is then one fused multiply-add.
-        const float mask0 = __shfl_sync(0xffffffffu, now.mask, 0);
-        const bool plain = __all_sync(0xffffffffu, now.mask == mask0);
+        const float mask2 = mask_base2(now.mask), mask0 = __shfl_sync(0xffffffffu, mask2, 0);
+        const bool plain = __all_sync(0xffffffffu, mask2 == mask0);
         const float row_off = log2_keep - now.lse * kLog2e, nd = -now.delta * delta_scale;
         const float off0 = mask0 + row_off;
         soft_wait(s_full, (uint32_t)t & 1u, abort_flag, ok);
@@ -555,7 +555,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
             for (int e = 0; e < 16; ++e) s[e] = ex2(fmaf(s[e], scale2, off0));
           } else {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) s[e] = ex2(fmaf(s[e], scale2, __shfl_sync(0xffffffffu, now.mask, c * 16 + e) + row_off));
+            for (int e = 0; e < 16; ++e) s[e] = ex2(fmaf(s[e], scale2, __shfl_sync(0xffffffffu, mask2, c * 16 + e) + row_off));
           }
           uint32_t pw[8], dw[8];
 #pragma unroll
