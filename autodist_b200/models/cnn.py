@@ -121,6 +121,11 @@ def _hooked(*modules):
     return False
 
 
+def _as_built(module, cls):
+    """Whether calling ``module`` runs ``cls.forward`` (no subclass, no forward of its own)."""
+    return type(module) is cls and "forward" not in module.__dict__
+
+
 class ConvBN(nn.Module):
     """Convolution followed by batch-norm (+ residual add, + ReLU). On the kernel path the convolution's epilogue already
     accumulates the per-channel sums the batch-norm needs, so the normalisation reads the activation once; in evaluation mode
@@ -135,8 +140,8 @@ class ConvBN(nn.Module):
         """``in_fork`` / ``res_fork``: the ``GradFork`` of ``x`` / of ``residual`` when that tensor has a second consumer."""
         conv, bn = self.conv, self.bn
         cout = conv.out_channels
-        if not bn.training and x.is_cuda and CONV_MODE != "library" and NORM_POOL_MODE != "library" and not conv.relu \
-                and type(bn) is BatchNormAct and not torch.is_grad_enabled() and not _hooked(conv, bn):
+        if not bn.training and x.is_cuda and CONV_MODE != "library" and NORM_POOL_MODE != "library" and not torch.is_grad_enabled() \
+                and _as_built(conv, Conv2d) and _as_built(bn, BatchNormAct) and not conv.relu and not _hooked(conv, bn):
             y = conv_bn_eval(x, conv.weight, conv.bias, conv.stride, conv.padding, bn.weight, bn.bias, bn.running_mean, bn.running_var, bn.eps,
                              bn.relu, residual)
             if y is not None:
@@ -257,10 +262,10 @@ class _DenseLayer(nn.Module):
     def steps(self):
         """The four modules where they can be run one by one - as built, no hook anywhere, batch statistics - or ``None``."""
         f = self.f
-        if type(self) is not _DenseLayer or type(f) is not nn.Sequential or len(f) != 4 or "forward" in self.__dict__ or "forward" in f.__dict__:
+        if not _as_built(self, _DenseLayer) or not _as_built(f, nn.Sequential) or len(f) != 4:
             return None
         mods = bn1, conv1, bn2, conv2 = tuple(f._modules.values())
-        if type(bn1) is BatchNormAct and type(bn2) is BatchNormAct and type(conv1) is Conv2d and type(conv2) is Conv2d and \
+        if _as_built(bn1, BatchNormAct) and _as_built(bn2, BatchNormAct) and _as_built(conv1, Conv2d) and _as_built(conv2, Conv2d) and \
                 not _hooked(self, f, *mods) and bn1.takes_sums() and bn2.takes_sums():
             return mods
         return None
@@ -300,7 +305,7 @@ class DenseNet121(nn.Module):
         possible: an eager step is bound by them.)"""
         f = self.features
         if not (x.is_cuda and self.training and torch.is_autocast_enabled() and CONV_MODE != "library" and NORM_POOL_MODE != "library" and
-                FUSE_BN_STATS) or type(f) is not nn.Sequential or "forward" in f.__dict__ or _hooked(f):
+                FUSE_BN_STATS) or not _as_built(f, nn.Sequential) or _hooked(f):
             return None
         plan = []
         for m in f._modules.values():

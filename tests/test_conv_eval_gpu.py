@@ -118,3 +118,27 @@ def test_network_evaluation_matches_the_library_route(backbone, monkeypatch):
     # the fused layers round where the separate ones do
     for out in (fused, hooked):
         assert torch.equal(out, plain)
+
+
+@pytest.mark.parametrize("own", ["subclass", "instance"])
+def test_a_convolution_with_a_forward_of_its_own_is_called(own):
+    from autodist_b200.models import cnn
+
+    class Doubled(cnn.Conv2d):
+        def forward(self, x, stats=None, fork=None):
+            return 2 * super().forward(x, stats, fork)
+
+    torch.manual_seed(0)
+    layer = cnn.ConvBN(16, 24, 3, 1, 1).cuda().eval()
+    x = torch.randn(2, 16, 7, 7, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    with torch.no_grad():
+        y = layer(x)
+        if own == "subclass":
+            conv = Doubled(16, 24, 3, 1, 1).cuda().eval()
+            conv.load_state_dict(layer.conv.state_dict())
+            layer.conv = conv
+        else:
+            plain = layer.conv.forward
+            layer.conv.forward = lambda x, stats=None, fork=None: 2 * plain(x, stats, fork)
+        twice = layer(x)
+    assert y.any() and torch.allclose(twice.float(), 2 * y.float(), rtol=2.0 ** -7, atol=1e-3)
