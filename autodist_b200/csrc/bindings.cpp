@@ -649,7 +649,8 @@ void lstm_cell_bwd(const Tensor& gates, const Tensor& c_prev, const Tensor& c, c
 void sumsq(const Tensor& x, Tensor acc, double weight) { adb200::sumsq(x.data_ptr<float>(), x.numel(), acc.data_ptr<float>(), (float)weight, STREAM); }
 void clip_scale(Tensor x, const Tensor& acc, double max_norm) { adb200::clip_scale(x.data_ptr<float>(), x.numel(), acc.data_ptr<float>(), (float)max_norm, STREAM); }
 // Batch-norm over a channels-last matrix x [rows, C] (training mode statistics), optional residual addend and fused ReLU:
-// y = relu?(bn(x) + res). `keep` (uint8, one byte per 8 channels) receives which outputs a fused ReLU let through. `sums` (optional, fp32 [2, C]) holds sum x and sum x^2 already (from the convolution's epilogue).
+// y = relu?(bn(x) + res). `keep` (uint8, one byte per 8 channels) receives which outputs a fused ReLU let through. `sums`
+// (optional, fp32 [2, C]) holds sum x and sum x^2 already (from the convolution's epilogue).
 void bn_fwd(const Tensor& x, const Tensor& gamma, const Tensor& beta, const optional<Tensor>& res, Tensor y, Tensor mean, Tensor rstd,
             double eps, bool relu, const optional<Tensor>& sums_in, const optional<Tensor>& run_mean, const optional<Tensor>& run_var,
             const optional<Tensor>& batches, double momentum, const optional<Tensor>& keep) {

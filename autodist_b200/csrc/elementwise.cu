@@ -375,8 +375,7 @@ __global__ void scatter_add_rows_kernel(float* __restrict__ dst, const int64_t* 
   }
 }
 
-// out[k][c] = sum over rows r = k + j*stride (j < count) of x[r][c]: position-embedding gradient (k = position).
-// The same with fp32 source rows: one thread per four columns (vector atomics when the rows are 16-byte aligned). Replaces the
+// scatter_add_rows_kernel with fp32 source rows: one thread per four columns (vector atomics when the rows are 16-byte aligned). Replaces the
 // sort-based embedding gradient of the library: 16384 rows of 192 took 16 radix-sort passes and a dozen helpers, 0.3 ms.
 __global__ void scatter_add_rows_f32_kernel(float* __restrict__ dst, const int64_t* __restrict__ idx, const float* __restrict__ src,
                                             long long total, int h4, int H, int vec) {
@@ -394,6 +393,7 @@ __global__ void scatter_add_rows_f32_kernel(float* __restrict__ dst, const int64
   }
 }
 
+// out[k][c] = sum over rows r = k + j*stride (j < count) of x[r][c]: position-embedding gradient (k = position).
 __global__ void strided_rowsum_kernel(const bf16* __restrict__ x, float* __restrict__ out, int keys, int stride, int count, int H) {
   pdl_sync();
   const int k = blockIdx.y;
@@ -1886,9 +1886,6 @@ int bn_parts(int rows, int C) {
   if (parts > 512) parts = 512;
   return parts < 1 ? 1 : parts;
 }
-// part: [bn_parts, 2, C]; sums: [2, C]; coef (backward): [3, C]
-// sums_given: `sums` already holds the per-channel sum and sum of squares (the convolution's epilogue produced them); the
-// whole normalisation is then one launch.
 // One wave of resident blocks (`per_sm` per SM) unless that leaves a thread fewer than kBnUnroll rows.
 dim3 bn_grid(long long rows, int C, int per_sm) {
   const int c8 = C / 8, tpr = c8 < kBnThreads ? c8 : kBnThreads, rpb = kBnThreads / tpr, gy = (c8 + kBnThreads - 1) / kBnThreads;
@@ -1903,6 +1900,9 @@ void bn_sums(const bf16* x, float* part, float* sums, int rows, int C, cudaStrea
   launch_pdl(bn_stats_kernel, dim3(dim3(blocks_for(C, 64), parts)), dim3(256), 0, st, x, part, rows, C, rpb);
   launch_pdl(colsum_f32_kernel, dim3(blocks_for(2 * C, 32)), dim3(256), 0, st, part, sums, parts, 2 * C, 0);
 }
+// part: [bn_parts, 2, C]; sums: [2, C]
+// sums_given: `sums` already holds the per-channel sum and sum of squares (the convolution's epilogue produced them); the
+// whole normalisation is then one launch.
 // keep (optional, [rows, C / 8] bytes): which outputs are positive, for the backward pass of a fused ReLU
 void bn_fwd(const bf16* x, const float* gamma, const float* beta, const bf16* res, bf16* y, uint8_t* keep, float* mean, float* rstd, float* part,
             float* sums, int rows, int C, float eps, int relu, int sums_given, float* run_mean, float* run_var, long long* batches,
@@ -1916,6 +1916,7 @@ void bn_eval(const bf16* x, const bf16* res, bf16* y, const float* gamma, const 
              int rows, int C, int relu, cudaStream_t st) {
   launch_pdl(bn_eval_kernel, bn_grid(rows, C, 2), dim3(kBnThreads), 0, st, x, res, y, (long long)rows, C, relu, gamma, beta, mean, var, eps);
 }
+// part: [bn_bwd_part_floats], zero between calls; sums: [2, C]; coef: [3, C]
 void bn_bwd(const bf16* dy, const bf16* x, const uint8_t* keep, const float* mean, const float* rstd, const float* gamma, bf16* dx, bf16* dres,
             float* part, float* sums, float* coef, int rows, int C, int relu, float* dgamma_acc, float* dbeta_acc, const bf16* add, long long add_ld,
             cudaStream_t st) {
