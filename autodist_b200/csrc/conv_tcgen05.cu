@@ -128,12 +128,7 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// Evaluation mode, 32 rows x 32 columns of one warp: bias, batch-norm, residual, ReLU, rounded to bf16 wherever layers of their own would
-// round (see eval_norm.cuh). A thread that owns a row needs the four coefficients of every column, 128 floats per 32 outputs, and the
-// shared-memory reads of those bounded the drain; so the accumulator is read in the fragment layout: lane l holds columns
-// 8 k + 2 (l % 4), + 1 of the rows l / 4 + 8 i, and a column's coefficients serve four rows (one ResNet-50 evaluation pass of 32 images:
-// a row per thread 1285 us, this 1133).
-// `tab`: the columns' coefficients, BN floats between two of them; `rows`: shared address of the warp's 32 staged lines.
+// Pairs of fp32 values in one register pair: one instruction for two elements.
 __device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -157,6 +152,12 @@ __device__ __forceinline__ uint32_t round2(uint64_t v) {
 }
 __device__ __forceinline__ uint64_t widen2(uint32_t u) { return pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
 
+// Evaluation mode, 32 rows x 32 columns of one warp: bias, batch-norm, residual, ReLU, rounded to bf16 wherever layers of their own would
+// round (see eval_norm.cuh). A thread that owns a row needs the four coefficients of every column, 128 floats per 32 outputs, and the
+// shared-memory reads of those bounded the drain; so the accumulator is read in the fragment layout: lane l holds columns
+// 8 k + 2 (l % 4), + 1 of the rows l / 4 + 8 i, and a column's coefficients serve four rows (one ResNet-50 evaluation pass of 32 images:
+// a row per thread 1285 us, this 1133).
+// `tab`: the columns' coefficients, BN floats between two of them; `rows`: shared address of the warp's 32 staged lines.
 template <int BN>
 __device__ __forceinline__ void eval_piece(uint32_t taddr, int cols, const float* tab, bool bias, bool add, bool relu, uint32_t rows, int chunk, int lane) {
   uint32_t r[32];                              // [rows 0-15, 16-31][k][row l / 4 or + 8][column]
