@@ -134,7 +134,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 10; ++i) mbar_init(&bars[i], &bars[i] == p_full ? FWD_SOFT / 32 : 1);
     *abort_flag = 0;
@@ -157,7 +157,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
   const int H = p.heads * 64;
 
   if (warp == 8) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       int nk = 0, nv = 0;
       mbar_expect_tx(q_full, TILE);
@@ -185,7 +185,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
       }
     }
   } else if (warp == 9) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t id_s = make_idesc(128, false, false), id_o = make_idesc(64, false, true);
       const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV), aP = smem_u32(sP);
       bool ok = mbar_wait(q_full, 0, abort_flag) && mbar_wait(&k_full[0], 0, abort_flag);
@@ -316,7 +316,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
+      if (elect_one()) mbar_arrive(p_full);
     }
     soft_wait(o_full, (tiles - 1) & 1, abort_flag, ok);
     tc_fence_after();
@@ -387,7 +387,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 12; ++i) mbar_init(&bars[i], (&bars[i] == pd_full || &bars[i] == acc_free) ? BWD_SOFT / 32 : 1);
     *abort_flag = 0;
@@ -414,7 +414,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
   auto batch_of = [&](int item) { return (MODE == BWD_ALL ? item : item / tiles) / p.heads; };
 
   if (warp == 16) {
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       int n_own = 0, n_oth = 0;
       for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
@@ -446,7 +446,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
       }
     }
   } else if (warp == 17) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t id_s = make_idesc(128, false, false), id_t = make_idesc(64, true, true), id_q = make_idesc(64, false, true);
       const uint32_t aOwn = smem_u32(sOwn), aOth = smem_u32(sOth), aP = smem_u32(sP), aD = smem_u32(sD);
       const int my_items = items > (int)blockIdx.x ? (items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
@@ -573,7 +573,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
           if (c == 0) {
             if (t > 0) soft_wait(acc_done, (uint32_t)(t - 1) & 1u, abort_flag, ok);      // P and dS of the iteration before have been multiplied
             if (stored) {                                  // the last item's gradients have left the staging the next lines write over
-              if (lane == 0) bulk_wait_read<0>();
+              if (elect_one()) bulk_wait_read<0>();
               __syncwarp();
               named_sync(2 + q, 128);                      // the four warps of these rows
               stored = false;
@@ -589,7 +589,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(pd_full);
+        if (elect_one()) mbar_arrive(pd_full);
       }
       // The item's gradients. Direct stores would write 32-byte pieces of rows 3 * heads * 128 bytes apart; instead warp (q, a) stages 32
       // rows of accumulator a (dV, dK, dQ) in the idle P / dS buffers and hands the box to the TMA unit. Rows past S are clipped.
@@ -611,7 +611,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0 && ok) {
+        if (elect_one() && ok) {
           tma_store_4d(&grads.m[MODE == BWD_Q ? 0 : 2 - cb], box, 0, ot * 128 + q * 32, h, b);      // dqkv holds q, k, v
           bulk_commit();
         }
@@ -619,9 +619,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
       stored = true;
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(acc_free);
+      if (elect_one()) mbar_arrive(acc_free);
     }
-    if (lane == 0) bulk_wait_all();                        // this warp's copies have landed
+    if (elect_one()) bulk_wait_all();                        // this warp's copies have landed
     if (!ok && lane == 0 && p.error_flag) atomicExch(p.error_flag, 66);
   }
   tc_fence_before();

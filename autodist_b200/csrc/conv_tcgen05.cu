@@ -214,11 +214,11 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
   constexpr int CW = BN / 2;                           // columns of this warp
   constexpr int BOXES = BN == 256 ? 2 : 1;             // boxes it takes part in per tile
   constexpr int PARTY = BN == 64 ? 256 : 128;          // threads that fill a box together
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int q = warp & 3, hf = (warp - 2) >> 2;
   const int r = q * 32 + lane;
   const int rows = p.tw * p.th * p.tn;
-  const bool issuer = lane == 0 && (BN == 64 ? warp == 2 : (warp - 2) % 4 == 0);
+  const bool issuing = BN == 64 ? warp == 2 : (warp - 2) % 4 == 0;   // its elected lane issues the copies
   const int bar_id = BN == 64 ? 2 : 2 + hf;
   const uint32_t boxes = staging + (BN == 64 ? 0u : (uint32_t)hf * 2u * A_BYTES);       // two buffers
   uint64_t* abar = add_bars + (BN == 64 ? 0 : 2 * hf);
@@ -259,7 +259,7 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
     const int c_w = tc_.c0 + hf * CW;                  // first column of this warp
     const int c_box = BN == 64 ? tc_.c0 : c_w;         // first column of its first box
     const long long tw0 = trace != nullptr ? clock64() : 0;
-    if (issuer) {
+    if (issuing && elect_one()) {
       store_wait_read();                               // the copies of the tile before have left the buffers
       if (add) {
 #pragma unroll
@@ -372,7 +372,7 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       meet();
-      if (issuer && ok) store_box(&maps.out, box, c_box + 64 * g, tc_.w0, tc_.h0, tc_.n0);
+      if (issuing && elect_one() && ok) store_box(&maps.out, box, c_box + 64 * g, tc_.w0, tc_.h0, tc_.n0);
       if constexpr (MODE == CONV_FPROP) {
         if (do_stats) {
           // statistics of what the next layer reads: the staged bf16 values. 64-wide tiles: each half takes 16 of the quarter's rows.
@@ -397,7 +397,7 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
     if (++as == 2) { as = 0; aphase ^= 1; }
   }
   if (MODE == CONV_FPROP && do_stats) flush();
-  if (issuer) {
+  if (issuing && elect_one()) {
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");                            // this thread's copies have landed
     for (int b = 0; add && !ok && b < 2; ++b) {        // addends nobody waited for land before the CTA leaves
       const long long w0 = clock64();
@@ -430,7 +430,7 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
   uint64_t* add_bars = tempty + 3;                 // pixel modes: two per half of the epilogue warps (behind the slot and the flag)
   float* s_stat = reinterpret_cast<float*>(staging + C::STAGING + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const bool do_stats = (MODE == CONV_FPROP) && p.stats != nullptr;
 
@@ -553,12 +553,12 @@ conv_kernel(const __grid_constant__ ConvMaps maps, const __grid_constant__ ConvP
     }
   };
   if (warp == 0) {
-    if (lane == 0) produce(std::integral_constant<int, 0>{});
+    if (elect_one()) produce(std::integral_constant<int, 0>{});
   } else if (warp == 2 + C::EPI_WARPS) {
-    if (lane == 0) produce(std::integral_constant<int, 1>{});
+    if (elect_one()) produce(std::integral_constant<int, 1>{});
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc(BN, A_MN, B_MN);
       int stage = 0; uint32_t phase = 0; int as = 0; uint32_t aphase = 0; bool ok = true;
       for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {

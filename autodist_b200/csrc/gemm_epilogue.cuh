@@ -126,11 +126,11 @@ __device__ __forceinline__ void gemm_epilogue_prefetch(const GemmParams& p, EpiS
     if (col + 2 < p.N) st.bias.z = __ldg(p.bias + col + 2);
     if (col + 3 < p.N) st.bias.w = __ldg(p.bias + col + 3);
   } else if (p.epilogue == EPI_ADD || p.epilogue == EPI_MUL_GELU_GRAD) {
-    if (lane == 0) bulk_wait_read<0>();               // the previous tile's copies have left both buffers
+    if (elect_one()) bulk_wait_read<0>();               // the previous tile's copies have left both buffers
 #pragma unroll
     for (int g = 0; g < BNW / 64; ++g) {
       if (n0 + g * 64 >= p.N) break;
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_expect_tx(&st.aux_bar[g], 4096);
         asm volatile(
             "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
@@ -189,7 +189,7 @@ __device__ __forceinline__ bool gemm_epilogue_row_tma(const GemmParams& p, EpiSt
     for (int g = 0; g < BNW / 32; ++g) {
       const int gcol0 = n0 + g * 32;
       if (gcol0 >= p.N) break;                        // uniform over the CTA
-      if (lane == 0) bulk_wait_read<1>();             // the buffer about to be written is no longer being read
+      if (elect_one()) bulk_wait_read<1>();             // the buffer about to be written is no longer being read
       const uint32_t base = st.smem + (uint32_t)(st.units & 1) * 4096u;
       const uint32_t buf = base + (uint32_t)lane * 128u;
       float v[32];
@@ -202,7 +202,7 @@ __device__ __forceinline__ bool gemm_epilogue_row_tma(const GemmParams& p, EpiSt
                      __float_as_uint(v[4 * i + 3]));
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // the staged rows are visible to the TMA unit
       __syncwarp();
-      if (lane == 0) {
+      if (elect_one()) {
         if (p.beta != 0.0f) tma_reduce_add_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
         else tma_store_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
         bulk_commit();
@@ -222,7 +222,7 @@ __device__ __forceinline__ bool gemm_epilogue_row_tma(const GemmParams& p, EpiSt
       st.aux_phase ^= 1u << g;
       st.aux_pending &= ~(1u << g);
     } else {
-      if (lane == 0) bulk_wait_read<1>();             // the buffer about to be written is no longer being read
+      if (elect_one()) bulk_wait_read<1>();             // the buffer about to be written is no longer being read
       base = st.smem + (uint32_t)(st.units & 1) * 4096u;
     }
     const uint32_t buf = base + (uint32_t)lane * 128u;
@@ -256,14 +256,14 @@ __device__ __forceinline__ bool gemm_epilogue_row_tma(const GemmParams& p, EpiSt
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the staged rows are visible to the TMA unit
     __syncwarp();
-    if (lane == 0) {
+    if (elect_one()) {
       tma_store_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
       bulk_commit();
     }
     st.units += 1;
     if (two) {
       // second output from the values kept in registers, through the other buffer
-      if (lane == 0) bulk_wait_read<1>();
+      if (elect_one()) bulk_wait_read<1>();
       __syncwarp();
       const uint32_t base2 = st.smem + (uint32_t)(st.units & 1) * 4096u;
       const uint32_t buf2 = base2 + (uint32_t)lane * 128u;
@@ -272,7 +272,7 @@ __device__ __forceinline__ bool gemm_epilogue_row_tma(const GemmParams& p, EpiSt
         st_shared_v4(buf2 + (((uint32_t)j ^ swz) << 4), act[4 * j], act[4 * j + 1], act[4 * j + 2], act[4 * j + 3]);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) {
+      if (elect_one()) {
         tma_store_4d(st.tmC2, base2, gcol0, box_row, b_lo, b_hi);
         bulk_commit();
       }

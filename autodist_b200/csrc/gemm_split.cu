@@ -120,7 +120,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
 
@@ -152,7 +152,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int kb0 = (int)((long long)num_kb * rank / split), kb1 = (int)((long long)num_kb * (rank + 1) / split);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0; uint32_t phase = 0; bool ok = true; int issued = 0;
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
@@ -187,7 +187,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc(BN, A_MN, B_MN);
       int stage = 0; uint32_t phase = 0; bool ok = true;
       for (int kb = kb0; kb < kb1; ++kb) {

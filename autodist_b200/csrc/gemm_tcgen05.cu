@@ -66,7 +66,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
   constexpr int AUX_BARS = BN == 256 ? 2 * C::EPI_WARPS : 0;
   static_assert((2 * C::STAGES + 4 + 1 + AUX_BARS) * 8 <= 256, "barrier area");
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -95,7 +95,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0; uint32_t phase = 0; bool ok = true;
       for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
         const int b = (int)(t / per_batch), rem = (int)(t % per_batch);
@@ -145,7 +145,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc(BN, A_MN, B_MN);
       int stage = 0; uint32_t phase = 0; int as = 0; uint32_t aphase = 0; bool ok = true;
       for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
@@ -280,7 +280,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
       mbar_arrive(&tempty[as]);
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
-    if (BN == 256 && p.tma_store && lane == 0) bulk_wait_all();       // this warp's output copies have landed
+    if (BN == 256 && p.tma_store && elect_one()) bulk_wait_all();       // this warp's output copies have landed
     if (BN == 256) gemm_epilogue_drain(est);
     if (!ok && lane == 0) {
       *abort_flag = 1;

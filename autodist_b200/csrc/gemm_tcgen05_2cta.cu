@@ -68,7 +68,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   uint64_t* aux_bars = tempty + 3;                      // two per epilogue warp (behind the slot and the flag)
   static_assert((2 * STAGES2 + 4 + 1 + 2 * EPI_WARPS2) * 8 <= 256, "barrier area");
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   // trace (when given): 0 entry, 1 set-up done, 2 first stage full, 3 last MMA committed, 4 ns the MMA thread waited for
   // full stages, 5 ns it waited for a free accumulator, 6 ns the first epilogue warp spent draining, 7 end
@@ -106,7 +106,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (each CTA: its halves of A and B)
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0; uint32_t phase = 0; bool ok = true;
       for (long long t = pair; t < total && ok; t += pairs) {
         const int b = (int)(t / per_batch), rem = (int)(t % per_batch);
@@ -142,7 +142,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       const uint32_t idesc = make_idesc2(A_MN, B_MN);
       int stage = 0; uint32_t phase = 0; int as = 0; uint32_t aphase = 0; bool ok = true;
       for (long long t = pair; t < total && ok; t += pairs) {
@@ -208,11 +208,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       if (!ok) break;
       __syncwarp();
       tc_fence_before();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty[as]), 0));
+      if (elect_one()) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty[as]), 0));
       if (trace != nullptr && threadIdx.x == 64) trace[6] += now_ns() - e0;
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
-    if (p.tma_store && lane == 0) bulk_wait_all();       // this warp's output copies have landed
+    if (p.tma_store && elect_one()) bulk_wait_all();       // this warp's output copies have landed
     gemm_epilogue_drain(est);
     if (!ok && lane == 0) {
       *abort_flag = 1;
