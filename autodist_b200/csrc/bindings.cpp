@@ -971,7 +971,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_gathered_bt", &gemm_gathered_bt);
   m.def("ln_fwd", &ln_fwd);
   m.def("ln_bwd", &ln_bwd);
-  m.def("ln_bwd_blocks", &adb200::ln_bwd_blocks);
   m.def("ln_bwd_part_floats", &adb200::ln_bwd_part_floats);
   m.def("colsum_parts", &adb200::colsum_parts);
   m.def("embed_sum", &embed_sum);
