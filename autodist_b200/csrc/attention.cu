@@ -621,7 +621,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
       __syncwarp();
       if (elect_one()) mbar_arrive(acc_free);
     }
-    if (elect_one()) bulk_wait_all();                        // this warp's copies have landed
+    if (elect_one()) bulk_wait_read<0>();                    // this warp's copies have left their buffers (the end of the grid waits for them to land)
     if (!ok && lane == 0 && p.error_flag) atomicExch(p.error_flag, 66);
   }
   tc_fence_before();

@@ -117,41 +117,6 @@ __device__ __forceinline__ uint4 lds4(uint32_t addr) {
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
   return v;
 }
-__device__ __forceinline__ void sts1(uint32_t addr, uint32_t a) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(a) : "memory"); }
-__device__ __forceinline__ uint32_t lds1(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-  return v;
-}
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-
-// Pairs of fp32 values in one register pair: one instruction for two elements.
-__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint32_t round2(uint64_t v) {
-  const float2 f = unpack_f32x2(v);
-  return pack2(f.x, f.y);
-}
-__device__ __forceinline__ uint64_t widen2(uint32_t u) { return pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
-
 // Evaluation mode, 32 rows x 32 columns of one warp: bias, batch-norm, residual, ReLU, rounded to bf16 wherever layers of their own would
 // round (see eval_norm.cuh). A thread that owns a row needs the four coefficients of every column, 128 floats per 32 outputs, and the
 // shared-memory reads of those bounded the drain; so the accumulator is read in the fragment layout: lane l holds columns
@@ -160,16 +125,9 @@ __device__ __forceinline__ uint64_t widen2(uint32_t u) { return pack_f32x2(__uin
 // `tab`: the columns' coefficients, BN floats between two of them; `rows`: shared address of the warp's 32 staged lines.
 template <int BN>
 __device__ __forceinline__ void eval_piece(uint32_t taddr, int cols, const float* tab, bool bias, bool add, bool relu, uint32_t rows, int chunk, int lane) {
-  uint32_t r[32];                              // [rows 0-15, 16-31][k][row l / 4 or + 8][column]
+  uint32_t r[32];
   __syncwarp();
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr), "r"(taddr + (16u << 16)) : "memory");
+  tmem_ld_frag32(taddr, r);
   const uint32_t swz = (uint32_t)(lane >> 2);  // line % 8 of every row of this lane
   const uint32_t mine = rows + (uint32_t)(lane >> 2) * 128u + (uint32_t)(lane & 3) * 4u;
 #pragma unroll
@@ -398,7 +356,7 @@ __device__ __forceinline__ bool staged_epilogue(const ConvParams& p, const ConvM
   }
   if (MODE == CONV_FPROP && do_stats) flush();
   if (issuing && elect_one()) {
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");                            // this thread's copies have landed
+    store_wait_read();                                 // this thread's copies have left the buffers (the end of the grid waits for them to land)
     for (int b = 0; add && !ok && b < 2; ++b) {        // addends nobody waited for land before the CTA leaves
       const long long w0 = clock64();
       while (!mbar_try(&abar[b], use[b] & 1u) && clock64() - w0 < 2000000LL) {}

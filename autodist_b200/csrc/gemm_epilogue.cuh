@@ -66,18 +66,21 @@ __device__ __forceinline__ void gemm_epilogue_math16(const GemmParams& p, float*
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Output through shared memory and TMA. A thread owns one row, so direct stores leave a warp writing 32 different rows in
+// Output through shared memory and TMA, for the 256-wide tiles. Direct stores leave a warp writing 32 different rows in
 // 16-byte pieces - partial sectors that cost the L2 as much as full ones and compete with the operand loads. Here each
-// epilogue warp stages 32 rows x 128 bytes (64 bf16 or 32 fp32 columns) in the 128-byte-swizzled layout and one lane hands
-// the box to the TMA unit, which writes whole lines (or adds them into an fp32 output: beta = 1). Rows and columns
-// past the matrix are clipped by the copy itself. Two 4 KB buffers per warp alternate, so staging overlaps the copy.
+// epilogue warp owns 32 rows x 128 columns, stages 32 rows x 128 bytes (64 bf16 or 32 fp32 columns) in the 128-byte-swizzled layout
+// and one lane hands the box to the TMA unit, which writes whole lines (or adds them into an fp32 output: beta = 1). Rows and
+// columns past the matrix are clipped by the copy itself. Two 4 KB buffers per warp alternate, so staging overlaps the copy.
 //
-// With two warps per scheduler nothing hides a global load behind other work, so what the epilogue reads is requested while
-// the tile is still being multiplied: the auxiliary operand (addend or pre-activation) comes by TMA into the two staging
-// buffers and is replaced there by the result, each lane keeps four columns of the bias and hands them around by shuffles.
-// A tile's drain is exposed once per launch and, with a short contraction, once per tile: 4096 x 4096 x 1024 on SM pairs,
-// time of a 128 x 256 drain / whole product back to back: bias 5.5 -> 3.7 us / 35.6 -> 35, bias + GELU 8.5 -> 6.9 / 45 -> 39-43,
-// GELU derivative 47.9 -> 41, addend (4096 x 1024 x 4096) 35.3 -> 30.7.
+// What the epilogue reads is requested while the tile is still being multiplied: the auxiliary operand (addend or pre-activation)
+// comes by TMA into the two staging buffers and is replaced there by the result, the bias into registers. The accumulator of a bf16
+// output is read in the fragment layout (tmem_ld_frag32), where a lane needs 32 values of the bias for its 32 rows x 128 columns,
+// and the arithmetic is on pairs of values.
+// A tile's drain is exposed once per launch and, with a short contraction, once per tile: with GELU it took longer than the
+// multiplication of a 1024-deep tile. 4096 x 4096 x 1024 on SM pairs, back to back (a row per thread, the bias handed around by
+// shuffles -> now, us): bias + GELU 36.0 -> 32.9, GELU derivative 36.3 -> 31.5, plain 26.8 -> 25.7. Sixteen warps of 32 x 64 with one
+// buffer each: 34.3, 32.4, and 0.4 us more on every product.
+constexpr int kEpiCols = 128;    // columns of an epilogue warp, staged in two groups of 64
 struct EpiStage {
   const CUtensorMap* tmC;      // output map, box (128 bytes of columns, 32 rows, 1, 1), 128-byte swizzle
   const CUtensorMap* tmC2;     // EPI_BIAS_GELU: second output; EPI_ADD / EPI_MUL_GELU_GRAD: the auxiliary operand (same box)
@@ -86,7 +89,7 @@ struct EpiStage {
   int units;                   // copies issued so far by this warp (picks the buffer)
   uint32_t aux_phase;          // bit g: parity the next wait on aux_bar[g] expects
   uint32_t aux_pending;        // bit g: a load into buffer g has been requested and not yet waited for
-  float4 bias;                 // this lane's four of the 128 columns' biases (0 past the matrix or without a bias)
+  float2 bias[16];             // columns 8 k + 2 (lane % 4) and the next of this warp's 128 (0 past the matrix or without a bias)
 };
 
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
@@ -99,36 +102,33 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, uint32
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
+__device__ __forceinline__ void st_shared_v2(uint32_t addr, uint64_t v) { asm volatile("st.shared.b64 [%0], %1;" ::"r"(addr), "l"(v) : "memory"); }
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
+__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) { return pack2(a, b); }
+__device__ __forceinline__ bool epi_has_bias(const GemmParams& p) {
+  return p.epilogue == EPI_BIAS || p.epilogue == EPI_BIAS_GELU || p.epilogue == EPI_BIAS_TANH;
 }
 
-// Requests what the epilogue of the next tile reads (see EpiStage). BNW <= 128 columns starting at n0.
-template <int BNW>
+// Requests what the epilogue of the next tile reads (see EpiStage); n0: first of this warp's columns.
 __device__ __forceinline__ void gemm_epilogue_prefetch(const GemmParams& p, EpiStage& st, int box_row, int n0, int b_lo, int b_hi, int lane) {
   if (box_row >= p.M) return;
-  if (p.epilogue == EPI_BIAS || p.epilogue == EPI_BIAS_GELU || p.epilogue == EPI_BIAS_TANH) {
-    static_assert(BNW == 128, "one float4 of bias per lane");
-    const int col = n0 + lane * 4;
-    st.bias = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (col < p.N) st.bias.x = __ldg(p.bias + col);
-    if (col + 1 < p.N) st.bias.y = __ldg(p.bias + col + 1);
-    if (col + 2 < p.N) st.bias.z = __ldg(p.bias + col + 2);
-    if (col + 3 < p.N) st.bias.w = __ldg(p.bias + col + 3);
-  } else if (p.epilogue == EPI_ADD || p.epilogue == EPI_MUL_GELU_GRAD) {
-    if (elect_one()) bulk_wait_read<0>();               // the previous tile's copies have left both buffers
+  if (epi_has_bias(p)) {
 #pragma unroll
-    for (int g = 0; g < BNW / 64; ++g) {
+    for (int k = 0; k < 16; ++k) {
+      const int col = n0 + 8 * k + 2 * (lane & 3);
+      st.bias[k] = make_float2(col < p.N ? __ldg(p.bias + col) : 0.f, col + 1 < p.N ? __ldg(p.bias + col + 1) : 0.f);
+    }
+  } else if (p.epilogue == EPI_ADD || p.epilogue == EPI_MUL_GELU_GRAD) {
+    if (elect_one()) bulk_wait_read<0>();             // the previous tile's copies have left both buffers
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
       if (n0 + g * 64 >= p.N) break;
       if (elect_one()) {
         mbar_expect_tx(&st.aux_bar[g], 4096);
@@ -142,27 +142,6 @@ __device__ __forceinline__ void gemm_epilogue_prefetch(const GemmParams& p, EpiS
   }
 }
 
-// Scale, bias and tanh of NV values starting `col` columns into the 128 that `st.bias` covers.
-template <int NV>
-__device__ __forceinline__ void gemm_epilogue_bias(const GemmParams& p, const EpiStage& st, float* v, int col) {
-#pragma unroll
-  for (int j = 0; j < NV; ++j) v[j] *= p.alpha;
-  if (p.epilogue == EPI_BIAS || p.epilogue == EPI_BIAS_GELU || p.epilogue == EPI_BIAS_TANH) {
-#pragma unroll
-    for (int j = 0; j < NV; j += 4) {
-      const int src = (col + j) >> 2;
-      v[j] += __shfl_sync(0xffffffffu, st.bias.x, src);
-      v[j + 1] += __shfl_sync(0xffffffffu, st.bias.y, src);
-      v[j + 2] += __shfl_sync(0xffffffffu, st.bias.z, src);
-      v[j + 3] += __shfl_sync(0xffffffffu, st.bias.w, src);
-    }
-    if (p.epilogue == EPI_BIAS_TANH) {
-#pragma unroll
-      for (int j = 0; j < NV; ++j) v[j] = tanhf(v[j]);
-    }
-  }
-}
-
 // Before the warp leaves: auxiliary boxes that nobody waited for (another role gave up) land first.
 __device__ __forceinline__ void gemm_epilogue_drain(EpiStage& st) {
   for (int g = 0; g < 2; ++g)
@@ -172,114 +151,141 @@ __device__ __forceinline__ void gemm_epilogue_drain(EpiStage& st) {
     }
 }
 
-// box_row: first output row of this warp's 32 rows; lane = row inside the box. Other arguments as gemm_epilogue_row.
-// BNW: columns this warp drains (the tile's width, or half of it when two warps share a TMEM lane quarter). Returns false when
-// an auxiliary box did not arrive in time.
-template <int BNW>
-__device__ __forceinline__ bool gemm_epilogue_row_tma(const GemmParams& p, EpiStage& st, uint32_t t_row, int row, int box_row, int n0, int b_lo,
-                                                      int b_hi, int lane, volatile int* abort_flag) {
-  if (box_row >= p.M) return true;                    // none of this warp's rows exist
-  const bool f32 = p.c_is_fp32 != 0;
-  const bool two = p.epilogue == EPI_BIAS_GELU;      // two outputs (bf16): the pre-activation, then its GELU
-  const bool aux = p.epilogue == EPI_ADD || p.epilogue == EPI_MUL_GELU_GRAD;
-  const uint32_t swz = (uint32_t)(lane & 7);
-  if (f32) {
-    // fp32: boxes of 32 columns; bias is the only epilogue such outputs take
-#pragma unroll 1
-    for (int g = 0; g < BNW / 32; ++g) {
-      const int gcol0 = n0 + g * 32;
-      if (gcol0 >= p.N) break;                        // uniform over the CTA
-      if (elect_one()) bulk_wait_read<1>();             // the buffer about to be written is no longer being read
-      const uint32_t base = st.smem + (uint32_t)(st.units & 1) * 4096u;
-      const uint32_t buf = base + (uint32_t)lane * 128u;
-      float v[32];
-      __syncwarp();                                   // tcgen05.ld is warp-collective
-      tmem_ld32(t_row + g * 32, v);
-      gemm_epilogue_bias<32>(p, st, v, g * 32);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        st_shared_v4(buf + (((uint32_t)i ^ swz) << 4), __float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]), __float_as_uint(v[4 * i + 2]),
-                     __float_as_uint(v[4 * i + 3]));
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // the staged rows are visible to the TMA unit
-      __syncwarp();
-      if (elect_one()) {
-        if (p.beta != 0.0f) tma_reduce_add_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
-        else tma_store_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
-        bulk_commit();
-      }
-      st.units += 1;
-    }
-    return true;
+// The staged lines of a buffer -> the TMA unit.
+__device__ __forceinline__ void gemm_epilogue_hand_over(const CUtensorMap* map, uint32_t base, int col, int box_row, int b_lo, int b_hi, bool add) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (elect_one()) {
+    if (add) tma_reduce_add_4d(map, base, col, box_row, b_lo, b_hi);
+    else tma_store_4d(map, base, col, box_row, b_lo, b_hi);
+    bulk_commit();
   }
-#pragma unroll 1
-  for (int g = 0; g < BNW / 64; ++g) {
-    const int gcol0 = n0 + g * 64;
-    if (gcol0 >= p.N) break;                          // uniform over the CTA
+}
+// The buffer about to be written is no longer being read: all but the last copy have left theirs.
+__device__ __forceinline__ void gemm_epilogue_buffer_free() {
+  if (elect_one()) bulk_wait_read<1>();
+  __syncwarp();
+}
+
+// A warp's 32 x 128 accumulator elements, bf16 outputs. EPI is the product's epilogue: one copy of the code per kind, since a test
+// per element costs more than the arithmetic. Returns false when an auxiliary box did not arrive in time.
+template <int EPI, class Release>
+__device__ __forceinline__ bool gemm_epilogue_bf16(const GemmParams& p, EpiStage& st, uint32_t t_w, int box_row, int n0, int b_lo, int b_hi, int lane,
+                                                   volatile int* abort_flag, Release& release) {
+  constexpr bool BIAS = EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_TANH, AUX = EPI == EPI_ADD || EPI == EPI_MUL_GELU_GRAD;
+  const uint32_t swz = (uint32_t)(lane >> 2);         // line % 8 of every row of this lane
+  const uint32_t mine = (uint32_t)(lane >> 2) * 128u + (uint32_t)(lane & 3) * 4u;
+  const uint64_t alpha = both(p.alpha);
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    const int col0 = n0 + g * 64;
+    if (col0 >= p.N) {                                // uniform over the warp
+      if (g == 1) release();
+      break;
+    }
     uint32_t base;
-    if (aux) {
+    if (AUX) {
       base = st.smem + (uint32_t)g * 4096u;           // the auxiliary box is already there
       if (!mbar_wait(&st.aux_bar[g], (st.aux_phase >> g) & 1u, abort_flag)) return false;
       st.aux_phase ^= 1u << g;
       st.aux_pending &= ~(1u << g);
     } else {
-      if (elect_one()) bulk_wait_read<1>();             // the buffer about to be written is no longer being read
+      gemm_epilogue_buffer_free();
       base = st.smem + (uint32_t)(st.units & 1) * 4096u;
     }
-    const uint32_t buf = base + (uint32_t)lane * 128u;
-    uint32_t act[32];                                 // packed GELU values of the group (two outputs only)
+    uint32_t act[EPI == EPI_BIAS_GELU ? 32 : 1];      // GELU values (two outputs: the pre-activation, then its GELU)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      float v[32];
+      uint32_t r[32];
       __syncwarp();                                   // tcgen05.ld is warp-collective
-      tmem_ld32(t_row + g * 64 + h * 32, v);
-      if (aux) {
+      tmem_ld_frag32(t_w + g * 64 + h * 32, r);
+      if (g == 1 && h == 1) release();
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          float x[8];
-          unpack8_bf16(ld_shared_v4(buf + (((uint32_t)(h * 4 + i) ^ swz) << 4)), x);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[8 * i + j] *= p.alpha;
-          gemm_epilogue_aux<8>(p, v + 8 * i, x);
+          const uint32_t at = base + mine + (uint32_t)i * 1024u + (((uint32_t)(h * 4 + k) ^ swz) << 4);
+          const uint32_t* a = r + (i >> 1) * 16 + k * 4 + (i & 1) * 2;
+          uint64_t v = mul2(pack_f32x2(__uint_as_float(a[0]), __uint_as_float(a[1])), alpha);
+          if (BIAS) v = add2(v, pack_f32x2(st.bias[g * 8 + h * 4 + k].x, st.bias[g * 8 + h * 4 + k].y));
+          if (EPI == EPI_BIAS_TANH) {
+            const float2 f = unpack_f32x2(v);
+            v = pack_f32x2(tanhf(f.x), tanhf(f.y));
+          }
+          if (EPI == EPI_ADD) v = add2(v, widen2(lds1(at)));
+          if (EPI == EPI_MUL_GELU_GRAD) v = mul2(v, gelu_tanh_grad2(widen2(lds1(at))));
+          sts1(at, round2(v));
+          if (EPI == EPI_BIAS_GELU) act[h * 16 + k * 4 + i] = round2(gelu_tanh2(v));
         }
-      } else {
-        gemm_epilogue_bias<32>(p, st, v, g * 64 + h * 32);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        st_shared_v4(buf + (((uint32_t)(h * 4 + i) ^ swz) << 4), pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
-                     pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
-        if (two) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) act[h * 16 + i * 4 + j] = pack_bf16x2(gelu_tanh(v[8 * i + 2 * j]), gelu_tanh(v[8 * i + 2 * j + 1]));
-        }
-      }
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the staged rows are visible to the TMA unit
-    __syncwarp();
-    if (elect_one()) {
-      tma_store_4d(st.tmC, base, gcol0, box_row, b_lo, b_hi);
-      bulk_commit();
-    }
+    gemm_epilogue_hand_over(st.tmC, base, col0, box_row, b_lo, b_hi, false);
     st.units += 1;
-    if (two) {
-      // second output from the values kept in registers, through the other buffer
-      if (elect_one()) bulk_wait_read<1>();
-      __syncwarp();
-      const uint32_t base2 = st.smem + (uint32_t)(st.units & 1) * 4096u;
-      const uint32_t buf2 = base2 + (uint32_t)lane * 128u;
+    if (EPI == EPI_BIAS_GELU) {                       // the second output through the other buffer
+      gemm_epilogue_buffer_free();
+      base = st.smem + (uint32_t)(st.units & 1) * 4096u;
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        st_shared_v4(buf2 + (((uint32_t)j ^ swz) << 4), act[4 * j], act[4 * j + 1], act[4 * j + 2], act[4 * j + 3]);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (elect_one()) {
-        tma_store_4d(st.tmC2, base2, gcol0, box_row, b_lo, b_hi);
-        bulk_commit();
-      }
+      for (int j = 0; j < 32; ++j) sts1(base + mine + (uint32_t)(j & 3) * 1024u + (((uint32_t)(j >> 2) ^ swz) << 4), act[j]);
+      gemm_epilogue_hand_over(st.tmC2, base, col0, box_row, b_lo, b_hi, false);
       st.units += 1;
     }
   }
   return true;
+}
+
+// The same for fp32 outputs (boxes of 32 columns): a row per lane, whose staged lines are written in 16-byte pieces without bank
+// conflicts. Bias is the only epilogue such outputs take; it is read again here.
+template <class Release>
+__device__ __forceinline__ void gemm_epilogue_f32(const GemmParams& p, EpiStage& st, uint32_t t_w, int box_row, int n0, int b_lo, int b_hi, int lane,
+                                                  Release& release) {
+  const uint32_t swz = (uint32_t)(lane & 7);
+  const bool bias = epi_has_bias(p);
+#pragma unroll 1
+  for (int g = 0; g < kEpiCols / 32; ++g) {
+    const int col0 = n0 + g * 32;
+    if (col0 >= p.N) break;                           // uniform over the warp
+    gemm_epilogue_buffer_free();
+    const uint32_t base = st.smem + (uint32_t)(st.units & 1) * 4096u, buf = base + (uint32_t)lane * 128u;
+    float v[32];
+    __syncwarp();                                     // tcgen05.ld is warp-collective
+    tmem_ld32(t_w + g * 32, v);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] *= p.alpha;
+    if (bias) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        if (col0 + j < p.N) v[j] += __ldg(p.bias + col0 + j);
+        if (p.epilogue == EPI_BIAS_TANH) v[j] = tanhf(v[j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      st_shared_v4(buf + (((uint32_t)i ^ swz) << 4), __float_as_uint(v[4 * i]), __float_as_uint(v[4 * i + 1]), __float_as_uint(v[4 * i + 2]),
+                   __float_as_uint(v[4 * i + 3]));
+    gemm_epilogue_hand_over(st.tmC, base, col0, box_row, b_lo, b_hi, p.beta != 0.0f);
+    st.units += 1;
+  }
+  release();
+}
+
+// t_w: TMEM address of this warp's 32 lanes at the first of its columns; box_row: first of its output rows. `release` is called once,
+// when the accumulator has been read. Returns false when an auxiliary box did not arrive in time (`release` has not been called then).
+template <class Release>
+__device__ __forceinline__ bool gemm_epilogue_tma(const GemmParams& p, EpiStage& st, uint32_t t_w, int box_row, int n0, int b_lo, int b_hi, int lane,
+                                                  volatile int* abort_flag, Release&& release) {
+  if (box_row >= p.M || n0 >= p.N) {                  // none of this warp's elements exist
+    release();
+    return true;
+  }
+  if (p.c_is_fp32) {
+    gemm_epilogue_f32(p, st, t_w, box_row, n0, b_lo, b_hi, lane, release);
+    return true;
+  }
+  if (p.epilogue == EPI_ADD) return gemm_epilogue_bf16<EPI_ADD>(p, st, t_w, box_row, n0, b_lo, b_hi, lane, abort_flag, release);
+  if (p.epilogue == EPI_MUL_GELU_GRAD) return gemm_epilogue_bf16<EPI_MUL_GELU_GRAD>(p, st, t_w, box_row, n0, b_lo, b_hi, lane, abort_flag, release);
+  if (p.epilogue == EPI_BIAS) return gemm_epilogue_bf16<EPI_BIAS>(p, st, t_w, box_row, n0, b_lo, b_hi, lane, abort_flag, release);
+  if (p.epilogue == EPI_BIAS_GELU) return gemm_epilogue_bf16<EPI_BIAS_GELU>(p, st, t_w, box_row, n0, b_lo, b_hi, lane, abort_flag, release);
+  if (p.epilogue == EPI_BIAS_TANH) return gemm_epilogue_bf16<EPI_BIAS_TANH>(p, st, t_w, box_row, n0, b_lo, b_hi, lane, abort_flag, release);
+  return gemm_epilogue_bf16<EPI_NONE>(p, st, t_w, box_row, n0, b_lo, b_hi, lane, abort_flag, release);
 }
 
 // t_row: TMEM address of this thread's lane at the first column of the accumulator; row: output row (may be >= M);

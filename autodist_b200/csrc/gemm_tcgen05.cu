@@ -35,7 +35,7 @@ template <int BN> struct Cfg {
   static constexpr int STAGES = (BN == 256) ? 3 : (BN == 128 ? 6 : 8);
   // Epilogue warps: four cover the TMEM lane quarters; the widest tile has eight, two per quarter with half of the
   // columns each, because 128 threads cannot apply a bias or an activation to 32768 outputs in the time of one tile.
-  static constexpr int EPI_WARPS = (BN == 256) ? 8 : 4;
+  static constexpr int EPI_WARPS = (BN == 256) ? 4 * BN / kEpiCols : 4;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int CW = BN / (EPI_WARPS / 4);          // columns per epilogue warp
   static constexpr int TMEM_COLS = 2 * BN;              // double-buffered fp32 accumulator
@@ -62,7 +62,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint64_t* aux_bars = tempty + 3;                      // widest tile: two per epilogue warp (behind the slot and the flag)
+  uint64_t* aux_bars = tempty + 3;                      // widest tile: one per epilogue warp (behind the slot and the flag)
   constexpr int AUX_BARS = BN == 256 ? 2 * C::EPI_WARPS : 0;
   static_assert((2 * C::STAGES + 4 + 1 + AUX_BARS) * 8 <= 256, "barrier area");
 
@@ -180,24 +180,29 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..5 -> TMEM lane quarter warp % 4)
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;                  // 0, or 1 for the second warp of a lane quarter
+    const int part = (warp - 2) >> 2;                  // which CW of the tile's columns this warp drains
     int as = 0; uint32_t aphase = 0; bool ok = true;
     const bool vec_ok = p.vec_ok != 0;
-    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, make_float4(0.f, 0.f, 0.f, 0.f)};
+    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, {}};
     for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
       const int b = (int)(t / per_batch), rem = (int)(t % per_batch);
       const int tn = rem / tiles_m, tm = rem % tiles_m;
       const int b_lo = b % p.batch_lo, b_hi = b / p.batch_lo;
       const int row = tm * BM + q * 32 + lane;
-      const int n_w = tn * BN + half * C::CW;
+      const int n_w = tn * BN + part * C::CW;
       const int box_row = tm * BM + q * 32;
       if constexpr (BN == 256) {
-        if (p.tma_store) gemm_epilogue_prefetch<C::CW>(p, est, box_row, n_w, b_lo, b_hi, lane);
+        if (p.tma_store) gemm_epilogue_prefetch(p, est, box_row, n_w, b_lo, b_hi, lane);
       }
       if (!mbar_wait(&tfull[as], aphase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const long long coff = (long long)b_hi * p.strideC_hi + (long long)b_lo * p.strideC_lo + (long long)row * p.ldc;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN);
+      auto release = [&]() {                           // this warp has read its part of the accumulator
+        __syncwarp();
+        tc_fence_before();
+        mbar_arrive(&tempty[as]);
+      };
       bool handled = false;
       if constexpr (BN == 128) {
         if (p.epilogue == EPI_SOFTMAX || p.epilogue == EPI_SOFTMAX_GRAD) {
@@ -266,21 +271,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
         }
       }
       if (!handled) {
-        const uint32_t t_w = t_row + (uint32_t)(half * C::CW);
-        bool staged = false;
+        const uint32_t t_w = t_row + (uint32_t)(part * C::CW);
         if constexpr (BN == 256) {
-          staged = p.tma_store != 0;
-          if (staged) ok = gemm_epilogue_row_tma<C::CW>(p, est, t_w, row, box_row, n_w, b_lo, b_hi, lane, abort_flag);
+          handled = p.tma_store != 0;
+          if (handled) ok = gemm_epilogue_tma(p, est, t_w, box_row, n_w, b_lo, b_hi, lane, abort_flag, release);
         }
-        if (!staged) gemm_epilogue_row<C::CW>(p, t_w, row, n_w, coff, vec_ok);
+        if (!handled) {
+          gemm_epilogue_row<C::CW>(p, t_w, row, n_w, coff, vec_ok);
+          release();
+        }
+      } else {
+        release();
       }
       if (!ok) break;
-      __syncwarp();
-      tc_fence_before();
-      mbar_arrive(&tempty[as]);
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
-    if (BN == 256 && p.tma_store && elect_one()) bulk_wait_all();       // this warp's output copies have landed
+    if (BN == 256 && p.tma_store && elect_one()) bulk_wait_read<0>();   // this warp's copies have left its buffer (the end of the grid waits for them to land)
     if (BN == 256) gemm_epilogue_drain(est);
     if (!ok && lane == 0) {
       *abort_flag = 1;

@@ -12,7 +12,7 @@
 //   empty[s]   one per CTA: the leader's MMA thread commits to both (two tcgen05.commit, the second to the peer's
 //              address), releasing the stage in each CTA for that CTA's producer.
 //   tfull[a]   one per CTA, committed to in the same way when an accumulator is complete.
-//   tempty[a]  leader only: the eight epilogue warps of both CTAs arrive on it (remote mbarrier.arrive for the peer).
+//   tempty[a]  leader only: the epilogue warps of both CTAs arrive on it (remote mbarrier.arrive for the peer).
 // TMEM is allocated and freed by warp 1 of both CTAs with the cta_group::2 forms; a cluster barrier after the barrier
 // initialisation and another before the deallocation keep either CTA from touching the other too early or leaving
 // while the other still reads its shared memory. Every mbarrier wait is bounded as in the one-CTA kernel; both CTAs
@@ -37,7 +37,7 @@ constexpr int BN2 = 256;                 // tile width; each CTA stages BN2 / 2 
 constexpr int B2_BYTES = (BN2 / 2) * BK * 2;
 constexpr int STAGES2 = 5;              // 5 x 32 KB of operands + 64 KB of output staging: 226 of the SM's 227 KB
 constexpr int TMEM_COLS2 = 2 * BN2;
-constexpr int EPI_WARPS2 = 8;            // two per TMEM lane quarter, half of the tile's columns each
+constexpr int EPI_WARPS2 = 4 * BN2 / kEpiCols;    // two per TMEM lane quarter, half of the tile's columns each
 constexpr int kThreads2 = 64 + 32 * EPI_WARPS2;
 constexpr int STAGING2 = EPI_WARPS2 * 8192;   // TMA-store staging: two 4 KB buffers per epilogue warp
 constexpr int SMEM2 = STAGES2 * (A_BYTES + B2_BYTES) + STAGING2 + 1024 /*align*/ + 256 /*barriers*/;
@@ -185,34 +185,39 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..5 -> TMEM lane quarter warp % 4)
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;                  // which half of the tile's columns this warp drains
+    const int part = (warp - 2) >> 2;                  // which half of the tile's columns this warp drains
     int as = 0; uint32_t aphase = 0; bool ok = true;
     const bool vec_ok = p.vec_ok != 0;
-    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, make_float4(0.f, 0.f, 0.f, 0.f)};
+    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, {}};
     for (long long t = pair; t < total && ok; t += pairs) {
       const int b = (int)(t / per_batch), rem = (int)(t % per_batch);
       const int tn = rem / tiles_m, tm = rem % tiles_m;
       const int b_lo = b % p.batch_lo, b_hi = b / p.batch_lo;
       const int row = tm * 256 + (int)rank * 128 + q * 32 + lane;
-      const int n_w = tn * BN2 + half * (BN2 / 2);
+      const int n_w = tn * BN2 + part * kEpiCols;
       const int box_row = tm * 256 + (int)rank * 128 + q * 32;
-      if (p.tma_store) gemm_epilogue_prefetch<BN2 / 2>(p, est, box_row, n_w, b_lo, b_hi, lane);
+      if (p.tma_store) gemm_epilogue_prefetch(p, est, box_row, n_w, b_lo, b_hi, lane);
       if (!mbar_wait(&tfull[as], aphase, abort_flag)) { ok = false; break; }
       const long long e0 = trace != nullptr ? now_ns() : 0;
       tc_fence_after();
-      const long long coff = (long long)b_hi * p.strideC_hi + (long long)b_lo * p.strideC_lo + (long long)row * p.ldc;
-      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN2);
-      const uint32_t t_w = t_row + (uint32_t)(half * (BN2 / 2));
-      if (p.tma_store) ok = gemm_epilogue_row_tma<BN2 / 2>(p, est, t_w, row, box_row, n_w, b_lo, b_hi, lane, abort_flag);
-      else gemm_epilogue_row<BN2 / 2>(p, t_w, row, n_w, coff, vec_ok);
-      if (!ok) break;
-      __syncwarp();
-      tc_fence_before();
-      if (elect_one()) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty[as]), 0));
+      const uint32_t t_w = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN2 + part * kEpiCols);
+      auto release = [&]() {                           // this warp has read its part of the accumulator
+        __syncwarp();
+        tc_fence_before();
+        if (elect_one()) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty[as]), 0));
+      };
+      if (p.tma_store) {
+        ok = gemm_epilogue_tma(p, est, t_w, box_row, n_w, b_lo, b_hi, lane, abort_flag, release);
+        if (!ok) break;
+      } else {
+        const long long coff = (long long)b_hi * p.strideC_hi + (long long)b_lo * p.strideC_lo + (long long)row * p.ldc;
+        gemm_epilogue_row<kEpiCols>(p, t_w, row, n_w, coff, vec_ok);
+        release();
+      }
       if (trace != nullptr && threadIdx.x == 64) trace[6] += now_ns() - e0;
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
-    if (p.tma_store && elect_one()) bulk_wait_all();       // this warp's output copies have landed
+    if (p.tma_store && elect_one()) bulk_wait_read<0>();   // this warp's copies have left its buffer (the end of the grid waits for them to land)
     gemm_epilogue_drain(est);
     if (!ok && lane == 0) {
       *abort_flag = 1;

@@ -141,6 +141,54 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 32 rows x 32 columns in the fragment layout: lane l gets columns 8 k + 2 (l % 4) and the one beside it of the rows l / 4 + 8 i, so that
+// what belongs to a column (a bias, a coefficient) serves four rows of a lane. Element (i, k) is at r[(i / 2) * 16 + k * 4 + (i % 2) * 2].
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr), "r"(taddr + (16u << 16)) : "memory");
+}
+
+__device__ __forceinline__ void sts1(uint32_t addr, uint32_t a) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(a) : "memory"); }
+__device__ __forceinline__ uint32_t lds1(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+
+// Pairs of fp32 values in one register pair: one instruction for two elements.
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_f32x2(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint32_t round2(uint64_t v) {
+  const float2 f = unpack_f32x2(v);
+  return pack2(f.x, f.y);
+}
+__device__ __forceinline__ uint64_t widen2(uint32_t u) { return pack_f32x2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+
 // Dropout decisions: the same counter-based function as the layernorm / softmax kernels (elementwise.cu), so a mask
 // drawn in a fused epilogue is reproduced by any other kernel from (seed, element offset).
 __device__ __forceinline__ uint64_t mix64(uint64_t seed, uint64_t idx) {
@@ -197,6 +245,24 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
   const float x2 = x * x;
   const float t = tanh_fast(k * fmaf(0.044715f * x2, x, x));
   return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * k * fmaf(3.0f * 0.044715f, x2, 1.0f);
+}
+
+// The same two functions on two values at once, operation by operation.
+__device__ __forceinline__ uint64_t tanh_fast2(uint64_t x) {
+  const float2 f = unpack_f32x2(x);
+  return pack_f32x2(tanh_fast(f.x), tanh_fast(f.y));
+}
+__device__ __forceinline__ uint64_t both(float x) { return pack_f32x2(x, x); }
+__device__ __forceinline__ uint64_t gelu_tanh2(uint64_t x) {
+  const uint64_t t = tanh_fast2(mul2(both(0.7978845608028654f), fma2(mul2(mul2(both(0.044715f), x), x), x, x)));
+  return mul2(mul2(both(0.5f), x), add2(both(1.0f), t));
+}
+__device__ __forceinline__ uint64_t gelu_tanh_grad2(uint64_t x) {
+  const uint64_t k = both(0.7978845608028654f), one = both(1.0f), half = both(0.5f);
+  const uint64_t x2 = mul2(x, x);
+  const uint64_t t = tanh_fast2(mul2(k, fma2(mul2(both(0.044715f), x2), x, x)));
+  const uint64_t slope = mul2(mul2(mul2(half, x), fma2(mul2(both(-1.0f), t), t, one)), k);
+  return fma2(slope, fma2(both(3.0f * 0.044715f), x2, one), mul2(half, add2(one, t)));
 }
 
 }  // namespace tc
