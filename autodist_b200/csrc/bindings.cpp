@@ -16,6 +16,7 @@
 #include "comm.h"
 #include "elementwise.h"
 #include "gemm_tcgen05.h"
+#include "sampled_softmax.h"
 
 void register_conv(pybind11::module& m);
 
@@ -957,9 +958,57 @@ void relaxed_pull(const Tensor& p32_ptrs, Tensor master, Tensor p16, const Tenso
                               ll(seg_len), ll(seg_owner), ll(prefix), nseg, (int)rank, (int)blocks, STREAM);
 }
 
+adb200::SampledSoftmax sampled_of(const Tensor& raw, const Tensor& out, const Tensor& true_w, const Tensor& adj, const Tensor& ids, const Tensor& lse,
+                                 const Tensor& true_logit) {
+  for (const Tensor* t : {&raw, &out, &true_w}) {
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 2 && t->is_contiguous() && t->size(1) % 8 == 0 &&
+                    reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "contiguous bf16 matrices with rows of 16-byte multiples needed");
+  }
+  const int64_t N = raw.size(0), K = raw.size(1);
+  TORCH_CHECK(N > 0 && out.size(0) == N && true_w.sizes() == out.sizes() && N + K < (1LL << 30), "rows of the products, outputs and true weights differ");
+  TORCH_CHECK(adj.scalar_type() == at::kFloat && adj.numel() >= N + K && ids.scalar_type() == at::kInt && ids.numel() >= N + K &&
+                  lse.scalar_type() == at::kFloat && lse.numel() >= N && true_logit.scalar_type() == at::kFloat && true_logit.numel() >= N,
+              "scratch of the sampled softmax too small");
+  return {(int)N, (int)K, (int)out.size(1), CBF(out), CBF(true_w), adj.data_ptr<float>(), ids.data_ptr<int>(), lse.data_ptr<float>(),
+          true_logit.data_ptr<float>()};
+}
+// Losses of the rows; adj / ids [K + N], lse and true_logit [N] are what the backward pass needs.
+void sampled_softmax_fwd(const Tensor& raw, const Tensor& out, const Tensor& true_w, const Tensor& bias, const Tensor& neg, const Tensor& targets,
+                         double inv_log_v, double num_sampled, Tensor adj, Tensor ids, Tensor lse, Tensor true_logit, Tensor loss, Tensor error) {
+  const c10::cuda::CUDAGuard guard(raw.device());
+  const adb200::SampledSoftmax s = sampled_of(raw, out, true_w, adj, ids, lse, true_logit);
+  TORCH_CHECK(bias.scalar_type() == at::kFloat && bias.dim() == 1 && bias.is_contiguous(), "fp32 bias needed");
+  TORCH_CHECK(neg.scalar_type() == at::kLong && neg.is_contiguous() && neg.numel() == s.K && targets.scalar_type() == at::kLong &&
+                  targets.is_contiguous() && targets.numel() == s.N, "int64 ids of the sampled classes and of the targets needed");
+  TORCH_CHECK(loss.scalar_type() == at::kFloat && loss.numel() >= s.N, "a loss per row");
+  adb200::sampled_softmax_fwd(s, CBF(raw), bias.data_ptr<float>(), neg.data_ptr<int64_t>(), targets.data_ptr<int64_t>(), bias.numel(), (float)inv_log_v,
+                              (float)num_sampled, loss.data_ptr<float>(), error.data_ptr<int>(), STREAM);
+}
+void sampled_softmax_bwd(const Tensor& raw, const Tensor& out, const Tensor& true_w, const Tensor& adj, const Tensor& ids, const Tensor& lse,
+                         const Tensor& true_logit, const Tensor& grad, Tensor part, Tensor draw, Tensor d_out, Tensor d_true_w, Tensor dadj) {
+  const c10::cuda::CUDAGuard guard(raw.device());
+  const adb200::SampledSoftmax s = sampled_of(raw, out, true_w, adj, ids, lse, true_logit);
+  TORCH_CHECK(grad.scalar_type() == at::kFloat && grad.numel() == 1, "fp32 scalar gradient needed");
+  TORCH_CHECK(part.numel() >= (int64_t)adb200::sampled_softmax_chunks(s.N, s.K) * s.K && dadj.numel() >= s.N + s.K, "scratch too small");
+  for (auto p : {std::make_pair(&draw, &raw), std::make_pair(&d_out, &out), std::make_pair(&d_true_w, &true_w)})
+    TORCH_CHECK(p.first->scalar_type() == at::kBFloat16 && p.first->is_contiguous() && p.first->sizes() == p.second->sizes() &&
+                    reinterpret_cast<uintptr_t>(p.first->data_ptr()) % 16 == 0, "gradients must match what they belong to");
+  adb200::sampled_softmax_bwd(s, CBF(raw), grad.data_ptr<float>(), part.data_ptr<float>(), BF(draw), BF(d_out), BF(d_true_w), dadj.data_ptr<float>(), STREAM);
+}
+void sampled_softmax_bias_grad(const Tensor& ids, const Tensor& dadj, Tensor dbias) {
+  const c10::cuda::CUDAGuard guard(ids.device());
+  TORCH_CHECK(ids.scalar_type() == at::kInt && dadj.scalar_type() == at::kFloat && dadj.numel() >= ids.numel() && dbias.scalar_type() == at::kFloat &&
+                  dbias.is_contiguous(), "int32 ids and fp32 values");
+  adb200::sampled_softmax_bias_grad(ids.data_ptr<int>(), dadj.data_ptr<float>(), dbias.data_ptr<float>(), (int)ids.numel(), STREAM);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("sampled_softmax_fwd", &sampled_softmax_fwd);
+  m.def("sampled_softmax_bwd", &sampled_softmax_bwd);
+  m.def("sampled_softmax_bias_grad", &sampled_softmax_bias_grad);
+  m.def("sampled_softmax_chunks", &adb200::sampled_softmax_chunks);
   m.def("gemm_set_trace", &gemm_set_trace);
   m.def("gemm", &gemm);
   m.def("gemm_split", &gemm_split);

@@ -4,6 +4,7 @@
 produced in fp32). On CPU tensors the same functions fall back to the plain PyTorch expression, which is also the
 numerics reference of the tests.
 """
+import math
 import os
 import warnings
 
@@ -721,8 +722,7 @@ def dense_lookup(table, ids):
     """``F.embedding(ids, table)``. Where an engine keeps the table's gradient in a flat buffer, the gradient rows are added
     into it by atomics (the order of addition varies); deterministic runs and all other tables use the library."""
     direct = table.is_cuda and table.dtype == torch.float32 and table.dim() == 2 and ids.dtype == torch.int64 and _direct_grad(table) is not None
-    if direct and torch.is_grad_enabled() and os.environ.get("AUTODIST_DETERMINISTIC") != "1" and \
-            not torch.are_deterministic_algorithms_enabled():
+    if direct and torch.is_grad_enabled() and not _ordered():
         return _DenseLookupFn.apply(table, ids)
     return F.embedding(ids, table)
 
@@ -763,6 +763,63 @@ def sparse_lookup(table, ids):
     if table.is_cuda and table.dtype == torch.float32 and table.is_contiguous() and table.shape[1] % 8 == 0:
         return _SparseLookupFn.apply(table, ids)
     return F.embedding(ids, table, sparse=True)
+
+
+def _ordered():
+    """Whether gradients have to be added up in a fixed order (no atomics)."""
+    return os.environ.get("AUTODIST_DETERMINISTIC") == "1" or torch.are_deterministic_algorithms_enabled()
+
+
+class _SampledSoftmaxFn(torch.autograd.Function):
+    """Mean cross-entropy of the true class against shared sampled classes (csrc/sampled_softmax.cu)."""
+
+    @staticmethod
+    def forward(ctx, raw, out, true_w, bias, neg, targets, num_sampled):
+        E = ops.ext(required=True)
+        n, k = raw.shape
+        dev = raw.device
+        adj, ids = torch.empty(k + n, dtype=torch.float32, device=dev), torch.empty(k + n, dtype=torch.int32, device=dev)
+        lse, true_logit, loss = torch.empty(3, n, dtype=torch.float32, device=dev).unbind(0)
+        E.sampled_softmax_fwd(raw, out, true_w, bias.detach(), neg, targets, 1.0 / math.log(bias.numel() + 1.0), num_sampled, adj, ids, lse, true_logit,
+                              loss, _error_flag(dev))
+        ctx.save_for_backward(raw, out, true_w, adj, ids, lse, true_logit)
+        ctx.bias = bias
+        _count_use(ctx, bias, 3)
+        return loss.mean()
+
+    @staticmethod
+    def backward(ctx, grad):
+        E = ops.ext(required=True)
+        raw, out, true_w, adj, ids, lse, true_logit = ctx.saved_tensors
+        n, k = raw.shape
+        part = torch.empty(E.sampled_softmax_chunks(n, k), k, dtype=torch.float32, device=raw.device)
+        draw, d_out, d_true_w, dadj = torch.empty_like(raw), torch.empty_like(out), torch.empty_like(true_w), torch.empty_like(adj)
+        E.sampled_softmax_bwd(raw, out, true_w, adj, ids, lse, true_logit, grad.float().contiguous(), part, draw, d_out, d_true_w, dadj)
+        d_bias = None
+        if ctx.needs_input_grad[3]:
+            acc = _direct_grad(ctx.bias)
+            d_bias = torch.zeros(ctx.bias.shape, dtype=torch.float32, device=raw.device) if acc is None else acc
+            if _ordered():
+                d_bias.index_put_((ids.long().clamp_min_(0),), torch.where(ids >= 0, dadj, 0.0), accumulate=True)
+            else:
+                E.sampled_softmax_bias_grad(ids, dadj, d_bias)
+            if acc is not None:
+                d_bias = None
+                _grad_written(ctx.bias)
+        return draw, d_out, d_true_w, d_bias, None, None, None
+
+
+def sampled_softmax(neg_logits, out, true_w, bias, neg, targets, num_sampled):
+    """Mean over rows of ``-log softmax`` of the true class among itself and the sampled classes ``neg`` (log-uniform over ``bias.numel()``
+    classes). ``neg_logits``: ``out @ W[neg].T``; ``true_w``: ``W[targets]``; logits are corrected by ``bias`` and by the log of the
+    expected counts, negatives that hit the row's own class are masked. ``None`` where the kernels do not apply."""
+    mats = (neg_logits, out, true_w)
+    if not all(t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[0] and t.shape[1] and t.shape[1] % 8 == 0 for t in mats):
+        return None
+    if bias.dtype != torch.float32 or bias.dim() != 1 or not bias.is_contiguous() or neg.dtype != torch.int64 or targets.dtype != torch.int64:
+        return None
+    mats = [t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format) for t in mats]
+    return _SampledSoftmaxFn.apply(*mats, bias, neg.contiguous(), targets.contiguous(), float(num_sampled))
 
 
 _SPARSE_KINDS = {"sgd": 0, "lazy_adam": 1, "adagrad": 2}
