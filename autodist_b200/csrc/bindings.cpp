@@ -958,6 +958,48 @@ void relaxed_pull(const Tensor& p32_ptrs, Tensor master, Tensor p16, const Tenso
                               ll(seg_len), ll(seg_owner), ll(prefix), nseg, (int)rank, (int)blocks, STREAM);
 }
 
+void check_pair_tables(const Tensor& a, const Tensor& b, int64_t mf, const Tensor& users, const Tensor& items) {
+  for (const Tensor* t : {&a, &b})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->dim() == 2 && t->is_contiguous() && t->size(1) == a.size(1) &&
+                    reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "contiguous fp32 tables of one width needed");
+  TORCH_CHECK(mf % 4 == 0 && a.size(1) % 4 == 0 && mf > 0 && mf < a.size(1), "both parts of a row must be multiples of 4 columns");
+  TORCH_CHECK(users.scalar_type() == at::kLong && items.scalar_type() == at::kLong && users.is_contiguous() && items.is_contiguous() &&
+                  users.numel() == items.numel(), "int64 ids needed");
+}
+// gmf [n, mf] fp32, x [n, 2 h] bf16, kept (optional) [n, 2 mf] fp32; tables [.., mf + h]
+void pair_lookup(const Tensor& ut, const Tensor& it, const Tensor& users, const Tensor& items, int64_t mf, Tensor gmf, Tensor x,
+                 const optional<Tensor>& kept, Tensor error) {
+  check_pair_tables(ut, it, mf, users, items);
+  const int64_t n = users.numel(), h = ut.size(1) - mf;
+  TORCH_CHECK(gmf.numel() == n * mf && gmf.scalar_type() == at::kFloat && gmf.is_contiguous() && x.numel() == n * 2 * h &&
+                  x.scalar_type() == at::kBFloat16 && x.is_contiguous() && (!kept.has_value() || (kept->numel() == n * 2 * mf && kept->is_contiguous())),
+              "outputs must match the lookups");
+  adb200::pair_lookup(ut.data_ptr<float>(), it.data_ptr<float>(), users.data_ptr<int64_t>(), items.data_ptr<int64_t>(), gmf.data_ptr<float>(), BF(x), OPT_F(kept),
+                      n, (int)mf, (int)h, ut.size(0), it.size(0), error.data_ptr<int>(), STREAM);
+}
+// dgmf: fp32 [n, mf] with unit inner stride
+void pair_lookup_bwd(const Tensor& dgmf, const Tensor& dx, const Tensor& kept, const Tensor& users, const Tensor& items, Tensor gu, Tensor gi) {
+  const int64_t n = users.numel(), mf = dgmf.size(1);
+  check_pair_tables(gu, gi, mf, users, items);
+  const int64_t h = gu.size(1) - mf;
+  TORCH_CHECK(dgmf.scalar_type() == at::kFloat && dgmf.dim() == 2 && dgmf.size(0) == n && dgmf.stride(1) == 1 && dgmf.stride(0) % 4 == 0 &&
+                  reinterpret_cast<uintptr_t>(dgmf.data_ptr()) % 16 == 0, "rows of dgmf must start on 16-byte boundaries");
+  TORCH_CHECK(dx.scalar_type() == at::kBFloat16 && dx.is_contiguous() && dx.numel() == n * 2 * h && reinterpret_cast<uintptr_t>(dx.data_ptr()) % 8 == 0 &&
+                  kept.scalar_type() == at::kFloat && kept.is_contiguous() && kept.numel() == n * 2 * mf, "gradients must match the lookups");
+  adb200::pair_lookup_bwd(dgmf.data_ptr<float>(), dgmf.stride(0), CBF(dx), kept.data_ptr<float>(), users.data_ptr<int64_t>(), items.data_ptr<int64_t>(),
+                          gu.data_ptr<float>(), gi.data_ptr<float>(), n, (int)mf, (int)h, gu.size(0), gi.size(0), STREAM);
+}
+// part[i] = scale * the losses of elements 16384 i ...
+void bce_logits(const Tensor& x, const Tensor& y, Tensor part, double scale) {
+  TORCH_CHECK(x.scalar_type() == at::kFloat && y.scalar_type() == at::kFloat && x.is_contiguous() && y.is_contiguous() && y.numel() == x.numel() &&
+                  x.numel() > 0 && part.numel() >= adb200::bce_logits_parts(x.numel()), "contiguous fp32 logits and labels needed");
+  adb200::bce_logits(x.data_ptr<float>(), y.data_ptr<float>(), part.data_ptr<float>(), x.numel(), (float)scale, STREAM);
+}
+void bce_logits_bwd(const Tensor& x, const Tensor& y, const Tensor& grad, Tensor dx, double scale) {
+  TORCH_CHECK(x.is_contiguous() && y.is_contiguous() && dx.is_contiguous() && y.numel() == x.numel() && dx.numel() == x.numel() && grad.numel() == 1,
+              "gradients must match the logits");
+  adb200::bce_logits_bwd(x.data_ptr<float>(), y.data_ptr<float>(), grad.data_ptr<float>(), dx.data_ptr<float>(), x.numel(), (float)scale, STREAM);
+}
 adb200::SampledSoftmax sampled_of(const Tensor& raw, const Tensor& out, const Tensor& true_w, const Tensor& adj, const Tensor& ids, const Tensor& lse,
                                  const Tensor& true_logit) {
   for (const Tensor* t : {&raw, &out, &true_w}) {
@@ -1005,6 +1047,11 @@ void sampled_softmax_bias_grad(const Tensor& ids, const Tensor& dadj, Tensor dbi
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("pair_lookup", &pair_lookup);
+  m.def("pair_lookup_bwd", &pair_lookup_bwd);
+  m.def("bce_logits", &bce_logits);
+  m.def("bce_logits_bwd", &bce_logits_bwd);
+  m.def("bce_logits_parts", &adb200::bce_logits_parts);
   m.def("sampled_softmax_fwd", &sampled_softmax_fwd);
   m.def("sampled_softmax_bwd", &sampled_softmax_bwd);
   m.def("sampled_softmax_bias_grad", &sampled_softmax_bias_grad);

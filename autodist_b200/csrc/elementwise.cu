@@ -422,6 +422,98 @@ __global__ void scatter_add_rows_f32_kernel(float* __restrict__ dst, const int64
   }
 }
 
+// Lookups of (user, item) pairs in two fp32 tables of rows [mf | h columns]: gmf = product of the first mf columns (fp32), x = [user's
+// h, item's h] as bf16, what the first layer of the other branch reads. The first columns are kept for the backward pass. Four columns
+// per thread. An id outside its table reads zeros and is reported.
+__global__ void pair_lookup_kernel(const float* __restrict__ ut, const float* __restrict__ it, const int64_t* __restrict__ users, const int64_t* __restrict__ items,
+                                   float* __restrict__ gmf, bf16* __restrict__ x, float* __restrict__ kept, long long total, int mf4, int h4,
+                                   long long nu, long long ni, int* __restrict__ error) {
+  pdl_sync();
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  const int w4 = mf4 + h4;
+  const long long r = t / w4;
+  const int c = (int)(t % w4);
+  const long long u = users[r], i = items[r];
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+  if ((unsigned long long)u < (unsigned long long)nu) a = reinterpret_cast<const float4*>(ut)[u * w4 + c];
+  else atomicExch(error, 72);
+  if ((unsigned long long)i < (unsigned long long)ni) b = reinterpret_cast<const float4*>(it)[i * w4 + c];
+  else atomicExch(error, 72);
+  if (c < mf4) {
+    reinterpret_cast<float4*>(gmf)[r * mf4 + c] = make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
+    if (kept != nullptr) {
+      reinterpret_cast<float4*>(kept)[r * 2 * mf4 + c] = a;
+      reinterpret_cast<float4*>(kept)[(r * 2 + 1) * mf4 + c] = b;
+    }
+    return;
+  }
+  const int j = c - mf4;
+  auto put = [&](long long at, const float4& v) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    reinterpret_cast<uint2*>(x)[at] = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  };
+  put(r * 2 * h4 + j, a);
+  put((r * 2 + 1) * h4 + j, b);
+}
+
+// Its gradient: dgmf times the other row's columns, and dx, added into the tables' fp32 gradients (vector reductions, any order).
+__global__ void pair_lookup_bwd_kernel(const float* __restrict__ dgmf, long long ld, const bf16* __restrict__ dx, const float* __restrict__ kept,
+                                       const int64_t* __restrict__ users, const int64_t* __restrict__ items, float* __restrict__ gu,
+                                       float* __restrict__ gi, long long total, int mf4, int h4, long long nu, long long ni) {
+  pdl_sync();
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
+  const int w4 = mf4 + h4;
+  const long long r = t / w4;
+  const int c = (int)(t % w4);
+  const long long u = users[r], i = items[r];
+  float4 a, b;
+  if (c < mf4) {
+    const float4 d = *reinterpret_cast<const float4*>(dgmf + r * ld + 4 * c);
+    const float4 ku = reinterpret_cast<const float4*>(kept)[r * 2 * mf4 + c], ki = reinterpret_cast<const float4*>(kept)[(r * 2 + 1) * mf4 + c];
+    a = make_float4(d.x * ki.x, d.y * ki.y, d.z * ki.z, d.w * ki.w);
+    b = make_float4(d.x * ku.x, d.y * ku.y, d.z * ku.z, d.w * ku.w);
+  } else {
+    auto get = [&](long long at) {
+      const uint2 q = reinterpret_cast<const uint2*>(dx)[at];
+      return make_float4(__uint_as_float(q.x << 16), __uint_as_float(q.x & 0xffff0000u), __uint_as_float(q.y << 16), __uint_as_float(q.y & 0xffff0000u));
+    };
+    a = get(r * 2 * h4 + c - mf4);
+    b = get((r * 2 + 1) * h4 + c - mf4);
+  }
+  if ((unsigned long long)u < (unsigned long long)nu) atomicAdd(reinterpret_cast<float4*>(gu) + u * w4 + c, a);
+  if ((unsigned long long)i < (unsigned long long)ni) atomicAdd(reinterpret_cast<float4*>(gi) + i * w4 + c, b);
+}
+
+// Binary cross-entropy with logits: part[block] = sum over the block's elements of max(x, 0) - x y + log(1 + exp(-|x|)).
+constexpr int kBcePerBlock = 16384;
+__global__ void __launch_bounds__(1024) bce_logits_kernel(const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ part, long long n,
+                                                          float scale) {
+  pdl_sync();
+  __shared__ float sm[32];
+  const long long n0 = (long long)blockIdx.x * kBcePerBlock, n1 = n0 + kBcePerBlock < n ? n0 + kBcePerBlock : n;
+  float s = 0.f;
+#pragma unroll 4
+  for (long long i = n0 + threadIdx.x; i < n1; i += 1024) {
+    const float v = x[i];
+    s += (fmaxf(v, 0.f) - v * y[i]) + log1pf(expf(-fabsf(v)));
+  }
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = warp_sum(sm[threadIdx.x]);
+    if (threadIdx.x == 0) part[blockIdx.x] = s * scale;
+  }
+}
+__global__ void bce_logits_bwd_kernel(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ grad, float* __restrict__ dx,
+                                      long long n, float scale) {
+  pdl_sync();
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) dx[i] = (1.0f / (1.0f + expf(-x[i])) - y[i]) * (*grad * scale);
+}
+
 // out[k][c] = sum over rows r = k + j*stride (j < count) of x[r][c]: position-embedding gradient (k = position).
 __global__ void strided_rowsum_kernel(const bf16* __restrict__ x, float* __restrict__ out, int keys, int stride, int count, int H) {
   pdl_sync();
@@ -451,9 +543,22 @@ __global__ void keyed_colsum_kernel(const bf16* __restrict__ x, const int64_t* _
   const int r0 = blockIdx.y * rows_per_block, r1 = min(rows, r0 + rows_per_block);
   for (int k = 0; k < keys; ++k) {
     float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (c < H)
+    if (c < H && key == nullptr) {
+      for (int r = r0 + rl; r < r1; r += 128) {                // four rows in flight
+        uint4 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) q[u] = r + 32 * u < r1 ? *reinterpret_cast<const uint4*>(x + (long long)(r + 32 * u) * H + c) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float v[8];
+          unpack8(q[u], v);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) a[i] += v[i];
+        }
+      }
+    } else if (c < H)
       for (int r = r0 + rl; r < r1; r += 32) {
-        if (key && key[r] != k) continue;
+        if (key[r] != k) continue;
         float v[8];
         load8(x + (long long)r * H + c, v);
 #pragma unroll
@@ -1902,11 +2007,30 @@ void scatter_add_rows_f32(float* dst, const int64_t* idx, const float* src, long
   const int vec = H % 4 == 0 && ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0;
   if (rows > 0) launch_pdl(scatter_add_rows_f32_kernel, dim3(blocks_for(rows * h4, 256)), dim3(256), 0, st, dst, idx, src, rows * h4, h4, H, vec);
 }
+void pair_lookup(const float* ut, const float* it, const int64_t* users, const int64_t* items, float* gmf, bf16* x, float* kept, long long rows, int mf,
+                 int h, long long nu, long long ni, int* error, cudaStream_t st) {
+  const long long total = rows * ((mf + h) / 4);
+  if (total > 0) launch_pdl(pair_lookup_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, st, ut, it, users, items, gmf, x, kept, total, mf / 4, h / 4, nu, ni, error);
+}
+void pair_lookup_bwd(const float* dgmf, long long ld, const bf16* dx, const float* kept, const int64_t* users, const int64_t* items, float* gu, float* gi,
+                     long long rows, int mf, int h, long long nu, long long ni, cudaStream_t st) {
+  const long long total = rows * ((mf + h) / 4);
+  if (total > 0) launch_pdl(pair_lookup_bwd_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, st, dgmf, ld, dx, kept, users, items, gu, gi, total, mf / 4, h / 4, nu, ni);
+}
+int bce_logits_parts(long long n) { return blocks_for(n, kBcePerBlock); }
+void bce_logits(const float* x, const float* y, float* part, long long n, float scale, cudaStream_t st) {
+  launch_pdl(bce_logits_kernel, dim3(bce_logits_parts(n)), dim3(1024), 0, st, x, y, part, n, scale);
+}
+void bce_logits_bwd(const float* x, const float* y, const float* grad, float* dx, long long n, float scale, cudaStream_t st) {
+  launch_pdl(bce_logits_bwd_kernel, dim3(blocks_for(n, 256)), dim3(256), 0, st, x, y, grad, dx, n, scale);
+}
 void strided_rowsum(const bf16* x, float* out, int keys, int stride, int count, int H, cudaStream_t st) {
   dim3 grid(blocks_for(H / 8, 128), keys);
   launch_pdl(strided_rowsum_kernel, dim3(grid), dim3(128), 0, st, x, out, keys, stride, count, H);
 }
-int colsum_parts(int rows) { return rows >= 2048 ? 16 : (rows >= 256 ? 4 : 1); }
+// Chunks of rows: with 16 of them a narrow matrix of many rows (16384 x 64 to 256: bias gradients of a batch of pairs) ran in a few dozen
+// blocks, 7.6 us; a chunk per 256 rows takes 3.2.
+int colsum_parts(int rows) { return rows >= 4096 ? (rows / 256 < 64 ? rows / 256 : 64) : (rows >= 2048 ? 16 : (rows >= 256 ? 4 : 1)); }
 void keyed_colsum(const bf16* x, const int64_t* key, float* part, float* out, int rows, int H, int keys, int accumulate, cudaStream_t st) {
   const int parts = colsum_parts(rows);
   const int rpb = (rows + parts - 1) / parts;

@@ -19,6 +19,13 @@ void scatter_add_rows_f32(float* dst, const int64_t* idx, const float* src, long
 void lstm_seq_fwd(const bf16_t* gates, const float* c_prev, float* c, bf16_t* h, int B, int S, float fb, cudaStream_t st);
 void lstm_seq_bwd(const bf16_t* gates, const float* c_prev, const float* c, const bf16_t* dh, const float* dc_next, bf16_t* dgates, float* dc_prev,
                   int B, int S, float fb, cudaStream_t st);
+void pair_lookup(const float* ut, const float* it, const int64_t* users, const int64_t* items, float* gmf, bf16_t* x, float* kept, long long rows, int mf,
+                 int h, long long nu, long long ni, int* error, cudaStream_t st);
+void pair_lookup_bwd(const float* dgmf, long long ld, const bf16_t* dx, const float* kept, const int64_t* users, const int64_t* items, float* gu, float* gi,
+                     long long rows, int mf, int h, long long nu, long long ni, cudaStream_t st);
+int bce_logits_parts(long long n);
+void bce_logits(const float* x, const float* y, float* part, long long n, float scale, cudaStream_t st);
+void bce_logits_bwd(const float* x, const float* y, const float* grad, float* dx, long long n, float scale, cudaStream_t st);
 void strided_rowsum(const bf16_t* x, float* out, int keys, int stride, int count, int H, cudaStream_t st);
 int colsum_parts(int rows);
 void keyed_colsum(const bf16_t* x, const int64_t* key, float* part, float* out, int rows, int H, int keys, int accumulate, cudaStream_t st);

@@ -13,7 +13,8 @@ import torch
 from torch import nn
 import torch.nn.functional as F
 
-from autodist_b200.ops.functional import Linear, dense_lookup
+from autodist_b200.models.cnn import _as_built, _hooked
+from autodist_b200.ops.functional import Linear, bce_with_logits, dense_lookup, pair_lookup
 
 
 @dataclass
@@ -48,8 +49,18 @@ class NeuMF(nn.Module):
     def sparse_grad_parameters(self):
         return [] if self.config.dense_gradient else [self.user_emb, self.item_emb]
 
+    def _plain_layers(self):
+        """Whether the layers are the GEMM layers and nothing watches them: they may then be fed bf16 instead of the tables' dtype."""
+        return not _hooked(self.mlp, *self.mlp) and all(_as_built(m, Linear) and m.in_features % 8 == 0 and m.out_features % 8 == 0 for m in self.mlp)
+
     def logits(self, users, items):
         c = self.config
+        pair = pair_lookup(self.user_emb, self.item_emb, users, items, c.mf_dim) if c.dense_gradient and self._plain_layers() else None
+        if pair is not None:
+            gmf, x = pair
+            for layer in self.mlp:            # bf16 all the way: what the layers compute in
+                x = F.relu(layer(x))
+            return self.head(torch.cat([gmf, x.to(gmf.dtype)], 1)).squeeze(1)
         if c.dense_gradient:
             u, i = dense_lookup(self.user_emb, users), dense_lookup(self.item_emb, items)
         else:
@@ -65,9 +76,9 @@ class NeuMF(nn.Module):
     def forward(self, users, items, labels, weights=None):
         """Binary cross-entropy on (user, item) pairs; ``weights`` masks padded duplicates as the reference's
         ``valid_point_mask`` does."""
-        loss = F.binary_cross_entropy_with_logits(self.logits(users, items), labels.float(), reduction="none")
         if weights is None:
-            return loss.mean()
+            return bce_with_logits(self.logits(users, items), labels.float())
+        loss = F.binary_cross_entropy_with_logits(self.logits(users, items), labels.float(), reduction="none")
         w = weights.float()
         return (loss * w).sum() / w.sum().clamp_min(1.0)
 

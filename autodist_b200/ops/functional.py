@@ -727,6 +727,83 @@ def dense_lookup(table, ids):
     return F.embedding(ids, table)
 
 
+class _PairLookupFn(torch.autograd.Function):
+    """Both lookups of (user, item) pairs with the product of their first columns and the concatenation of the others; the
+    gradients go straight into the tables' flat gradient buffers."""
+
+    @staticmethod
+    def forward(ctx, users_table, items_table, users, items, mf):
+        E = ops.ext(required=True)
+        n, h, dev = users.numel(), users_table.shape[1] - mf, users_table.device
+        gmf, kept = (torch.empty(n, w, dtype=torch.float32, device=dev) for w in (mf, 2 * mf))
+        x = torch.empty(n, 2 * h, dtype=torch.bfloat16, device=dev)
+        E.pair_lookup(users_table.detach(), items_table.detach(), users, items, mf, gmf, x, kept, _error_flag(dev))
+        ctx.save_for_backward(kept, users, items)
+        ctx.tables = users_table, items_table
+        for k, table in enumerate(ctx.tables):
+            _count_use(ctx, table, k)
+        return gmf, x
+
+    @staticmethod
+    def backward(ctx, dgmf, dx):
+        E = ops.ext(required=True)
+        kept, users, items = ctx.saved_tensors
+        direct = [_direct_grad(t) for t in ctx.tables]
+        into = [torch.zeros(t.shape, dtype=torch.float32, device=dx.device) if g is None else g for t, g in zip(ctx.tables, direct)]
+        dgmf, dx = dgmf.float(), dx.to(torch.bfloat16).contiguous()
+        if dgmf.stride(1) != 1 or dgmf.stride(0) % 4 or dgmf.data_ptr() % 16:
+            dgmf = dgmf.clone(memory_format=torch.contiguous_format)
+        E.pair_lookup_bwd(dgmf, dx, kept, users, items, *into)
+        grads = []
+        for t, g, d in zip(ctx.tables, into, direct):
+            if d is not None:
+                _grad_written(t)
+            grads.append(g if d is None else None)
+        return grads[0], grads[1], None, None, None
+
+
+def pair_lookup(users_table, items_table, users, items, mf):
+    """``(u[:, :mf] * i[:, :mf], [u[:, mf:], i[:, mf:]] as bf16)`` for the rows ``u``, ``i`` of two fp32 tables whose gradients an engine
+    keeps in a flat buffer (the gradient rows are added by atomics); ``None`` where ``dense_lookup`` would use the library, or the
+    layout does not fit."""
+    tables = (users_table, items_table)
+    if not all(t.is_cuda and t.dtype == torch.float32 and t.dim() == 2 and t.is_contiguous() and t.shape[1] == users_table.shape[1] and
+               t.requires_grad and t.data_ptr() % 16 == 0 and t.shape[1] % 4 == 0 and _direct_grad(t) is not None for t in tables):
+        return None
+    if users_table is items_table or mf % 4 or not 0 < mf < users_table.shape[1] or any(i.dtype != torch.int64 or i.dim() != 1 for i in (users, items)) or \
+            users.numel() != items.numel() or not users.numel() or _ordered() or not torch.is_grad_enabled():
+        return None
+    if any(g.data_ptr() % 16 for g in (_direct_grad(t) for t in tables)):
+        return None
+    return _PairLookupFn.apply(users_table, items_table, users.contiguous(), items.contiguous(), int(mf))
+
+
+class _BCEFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, logits, labels):
+        E = ops.ext(required=True)
+        n = logits.numel()
+        part = torch.empty(E.bce_logits_parts(n), dtype=torch.float32, device=logits.device)
+        E.bce_logits(logits, labels, part, 1.0 / n)
+        ctx.save_for_backward(logits, labels)
+        return part.view(()) if part.numel() == 1 else part.sum()
+
+    @staticmethod
+    def backward(ctx, grad):
+        logits, labels = ctx.saved_tensors
+        dx = torch.empty_like(logits)
+        ops.ext(required=True).bce_logits_bwd(logits, labels, grad.float().contiguous(), dx, 1.0 / logits.numel())
+        return dx, None
+
+
+def bce_with_logits(logits, labels):
+    """``F.binary_cross_entropy_with_logits(logits, labels)`` (the mean), one kernel each way for fp32 CUDA logits."""
+    if logits.is_cuda and labels.is_cuda and logits.dtype == labels.dtype == torch.float32 and logits.shape == labels.shape and logits.numel() and \
+            not labels.requires_grad:
+        return _BCEFn.apply(logits.contiguous(), labels.contiguous())
+    return F.binary_cross_entropy_with_logits(logits, labels)
+
+
 class _ShardedLookupFn(torch.autograd.Function):
     """Lookup in a table that is kept as one row shard per rank (``parallel.fused_engine.ShardedRows``): rows are gathered
     from their owners inside the kernel; the backward pass adds the gradient rows straight into the owners' shards, so the
