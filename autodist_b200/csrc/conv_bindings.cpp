@@ -112,7 +112,53 @@ Patch choose_patch(int GW, int GH, int GN, int limit, bool exact, bool wsplit) {
   return p;
 }
 
-int pick_bn(int n) { return n >= 256 ? 256 : (n > 64 ? 128 : 64); }
+// Estimates behind the choice of a tile, in us, fitted to a sweep of 44 layers (13 to 64 images, 7 x 7 to 56 x 56, 1 x 1 and 3 x 3) with
+// every tile width; they name the fastest width in 112 of 114 rows.
+//
+// Pixel modes: a launch, its pipeline's start and last drain (fixed), then per wave of tiles the larger of its K blocks and a drain.
+// A K block is bounded by the fill of the operands, which slows down by a quarter or more when every SM takes part. Wide tiles read each
+// operand less often, narrow ones put small layers on more SMs: 256 -> 256 channels, 3 x 3, 13 images of 13 x 13 (18 patches) take
+// 16.7 us in tiles of 256, 11.0 of 128; 64 images of 14 x 14 18.8 and 20.4; 512 -> 512 at 7 x 7, 64 images 28.9 and 19.7.
+int pixel_bn(int mode, long long patches, int cols, int kbs) {
+  struct Cost { int bn; double fixed_fwd, fixed_grad, kb, drain_fwd, drain_grad; };
+  static const Cost costs[3] = {{256, 6.1, 4.5, 0.29, 3.3, 1.9}, {128, 4.9, 4.0, 0.17, 2.1, 1.1}, {64, 4.6, 3.7, 0.16, 1.8, 0.9}};
+  const bool grad = mode == adb200::CONV_DGRAD;
+  int best = 64;
+  double best_us = 1e30;
+  for (const Cost& c : costs) {
+    if (c.bn > 64 && cols <= c.bn / 2) continue;             // more than half of the tile would be padding
+    const long long tiles = patches * ((cols + c.bn - 1) / c.bn), sms = sm_count();
+    const double waves = (double)((tiles + sms - 1) / sms);
+    const double full = std::min(1.0, (double)tiles / sms);
+    const double mult = c.kb * kbs * (1.0 + (c.bn == 64 ? 0.4 * full * full * full : 0.25 * full));
+    const double us = (grad ? c.fixed_grad : c.fixed_fwd) + (waves - 1) * std::max(mult, grad ? c.drain_grad : c.drain_fwd) + mult;
+    if (us < best_us) { best_us = us; best = c.bn; }
+  }
+  return best;
+}
+
+// Weight gradient: tile width and CTAs per output tile (each takes a share of the 64-pixel patches and adds its fp32 tile to the
+// output, whose L2 traffic is what limits the split). Earlier rule: the widest tile and as many CTAs as one wave holds;
+// 256 -> 1024 channels 1 x 1, 64 images of 14 x 14: 13.8 us, with 128 columns 10.9; 1024 -> 128, 16 images of 7 x 7: 8.8 and 5.0.
+struct GradSplit { int bn, ksplit; };
+GradSplit grad_split(int m_tiles, int cols, int ntaps, long long patches, double out_mb, int only_bn = 0) {
+  struct Cost { int bn; double fixed, kb; };
+  static const Cost costs[3] = {{256, 6.4, 0.33}, {128, 4.6, 0.20}, {64, 3.4, 0.22}};
+  const long long sms = sm_count();
+  GradSplit best{64, 1};
+  double best_us = 1e30;
+  for (const Cost& c : costs) {
+    if (only_bn != 0 ? c.bn != only_bn : (c.bn > 64 && cols <= c.bn / 2)) continue;
+    const long long base = (long long)m_tiles * ((cols + c.bn - 1) / c.bn) * ntaps;
+    const long long most = std::max<long long>(1, std::min(std::max<long long>(1, sms / base), patches / 4));
+    for (long long ks = 1; ks <= most; ++ks) {
+      const double waves = (double)((base * ks + sms - 1) / sms);
+      const double us = c.fixed + waves * c.kb * (double)((patches + ks - 1) / ks) + 0.2 * out_mb * ks;
+      if (us < best_us) { best_us = us; best = {c.bn, (int)ks}; }
+    }
+  }
+  return best;
+}
 
 void check_act(const Tensor& t, const char* what) {
   TORCH_CHECK(t.is_cuda() && t.dim() == 4 && t.scalar_type() == at::kBFloat16 && t.is_contiguous(), what,
@@ -211,13 +257,6 @@ void launch(const adb200::ConvMaps& maps, const adb200::ConvParams& p_, int bn) 
   TORCH_CHECK(e == cudaSuccess, "convolution launch failed: ", cudaGetErrorString(e));
 }
 
-// CTAs per output tile of the weight gradient: as many as fit in one wave, each with at least four K blocks.
-int split_k(int base_tiles, long long patches) {
-  int ks = std::max(1, sm_count() / base_tiles);
-  ks = (int)std::min<long long>(ks, std::max<long long>(1, patches / 4));
-  return ks;
-}
-
 // Evaluation-mode batch-norm (and residual) fused behind a forward convolution.
 struct EvalNorm {
   const Tensor *gamma, *beta, *mean, *var;
@@ -255,7 +294,7 @@ void conv_fprop_impl(const Tensor& x, const Tensor& w, Tensor y, const optional<
   const Patch pt = choose_patch(GW, GH, GN, 128, false, false);
   set_grid(p, GW, GH, GN, pt);
   input_maps(maps, x, g, pt.tw, pt.th, pt.tn);
-  const int bn = pick_bn(g.Cout);
+  const int bn = pixel_bn(adb200::CONV_FPROP, (long long)p.tiles_w * p.tiles_h * p.tiles_n, g.Cout, g.KH * g.KW * ceil_div(g.Cin, 64));
   maps.w = map4(w.data_ptr(), g.Cin, g.KH * g.KW, g.Cout, 1, g.Cin, (int64_t)g.Cin * g.KH * g.KW, (int64_t)g.Cin * g.KH * g.KW * g.Cout, 64, 1,
                 bn, 1);
   maps.dy = maps.w;
@@ -339,7 +378,6 @@ void conv_dgrad(const Tensor& dy, const Tensor& w, Tensor dx, int64_t stride, in
     TORCH_CHECK(addend->sizes() == dx.sizes() && addend->data_ptr() != dx.data_ptr(), "addend must have dx's shape and its own storage");
   }
   const Geometry g = geometry(dx, w, dy, stride, pad);
-  const int bn = pick_bn(g.Cin);
   adb200::ConvMaps maps{};
   maps.w = map4(w.data_ptr(), g.Cin, g.KH * g.KW, g.Cout, 1, g.Cin, (int64_t)g.Cin * g.KH * g.KW, (int64_t)g.Cin * g.KH * g.KW * g.Cout, 64, 1,
                 64, 1);
@@ -400,7 +438,7 @@ void conv_dgrad(const Tensor& dy, const Tensor& w, Tensor dx, int64_t stride, in
       maps.out = grid_map(p.out, off, g.Cin, p, sw, sh, sn);
       maps.add = p.addend != nullptr ? grid_map(p.addend, off, g.Cin, p, sw, sh, sn) : maps.out;
       p.error_flag = error_flag.data_ptr<int>();
-      launch(maps, p, bn);
+      launch(maps, p, pixel_bn(adb200::CONV_DGRAD, (long long)p.tiles_w * p.tiles_h * p.tiles_n, g.Cin, n * ceil_div(g.Cout, 64)));
     }
 }
 
@@ -431,16 +469,14 @@ void conv_wgrad(const Tensor& dy, const Tensor& x, Tensor dw, int64_t stride, in
   else maps.dy = map4(dy.data_ptr(), C, g.OW, g.OH, g.N, C, (int64_t)g.OW * C, (int64_t)g.OH * g.OW * C, 64, pt.tw, pt.th, pt.tn);
   maps.w = maps.dy;
   p.ntaps = forward_taps(p.taps, g);
-  const int bn = pick_bn(g.Cin);
   p.Nc = g.Cin; p.Kc = 0; p.Mc = g.Cout;
-  const long long patches = (long long)p.tiles_w * p.tiles_h * p.tiles_n;
-  const int base_tiles = ceil_div(g.Cout, 128) * ceil_div(g.Cin, bn) * p.ntaps;
-  p.ksplit = split_k(base_tiles, patches);
+  const GradSplit gs = grad_split(ceil_div(g.Cout, 128), g.Cin, p.ntaps, (long long)p.tiles_w * p.tiles_h * p.tiles_n, dw.numel() * 4e-6);
+  p.ksplit = gs.ksplit;
   p.accumulate = (p.ksplit > 1 || accumulate) ? 1 : 0;
   if (p.accumulate && !accumulate) dw.zero_();
   p.out = dw.data_ptr(); p.ldc = (long long)g.KH * g.KW * g.Cin; p.wtap_stride = g.Cin;
   p.error_flag = error_flag.data_ptr<int>();
-  launch(maps, p, bn);
+  launch(maps, p, gs.bn);
 }
 
 // ---- first layer of an image network: 3 (<= 8) input channels ------------------------------------------------------------------
@@ -511,7 +547,7 @@ void conv_rowtap_fprop_impl(const Tensor& xp, const Tensor& wr, Tensor y, const 
     p.wsplit = 1; p.xstep = (int)stride * 8;
   }
   set_grid(p, OW, OH, N, pt);
-  const int bn = pick_bn(Cout);
+  const int bn = pixel_bn(adb200::CONV_FPROP, (long long)p.tiles_w * p.tiles_h * p.tiles_n, Cout, (int)KH);
   maps.w = map4(wr.data_ptr(), 64, KH, Cout, 1, 64, 64 * KH, (int64_t)64 * KH * Cout, 64, 1, bn, 1);
   maps.dy = maps.w;
   p.ntaps = rowtap_taps(p.taps, KH, stride);
@@ -574,8 +610,7 @@ void conv_rowtap_wgrad(const Tensor& dy, const Tensor& xp, Tensor dwr, int64_t s
   maps.w = maps.dy;
   p.ntaps = rowtap_taps(p.taps, KH, stride);
   p.Nc = 64; p.Mc = Cout;
-  const long long patches = (long long)p.tiles_w * p.tiles_h * p.tiles_n;
-  p.ksplit = split_k(ceil_div(Cout, 128) * KH, patches);
+  p.ksplit = grad_split(ceil_div(Cout, 128), 64, KH, (long long)p.tiles_w * p.tiles_h * p.tiles_n, dwr.numel() * 4e-6, 64).ksplit;
   p.accumulate = p.ksplit > 1 ? 1 : 0;
   if (p.accumulate) dwr.zero_();
   p.out = dwr.data_ptr(); p.ldc = (long long)KH * 64; p.wtap_stride = 64;
