@@ -958,6 +958,34 @@ void relaxed_pull(const Tensor& p32_ptrs, Tensor master, Tensor p16, const Tenso
                               ll(seg_len), ll(seg_owner), ll(prefix), nseg, (int)rank, (int)blocks, STREAM);
 }
 
+// dst[i] <- src[i] for contiguous tensors of one device, sizes and dtypes equal, in one launch per kMaxCopies of them. Returns false, and
+// copies nothing, when a pair does not qualify.
+bool copy_list(const std::vector<Tensor>& dst, const std::vector<Tensor>& src) {
+  if (dst.size() != src.size()) return false;
+  for (size_t i = 0; i < dst.size(); ++i) {
+    const Tensor &d = dst[i], &s = src[i];
+    if (!d.is_cuda() || !s.is_cuda() || d.device() != s.device() || d.device() != dst[0].device() || d.scalar_type() != s.scalar_type() ||
+        d.sizes() != s.sizes() || !d.is_contiguous() || !s.is_contiguous() || d.is_conj() != s.is_conj() || d.is_neg() != s.is_neg() ||
+        d.numel() * d.element_size() > (1LL << 40))
+      return false;
+  }
+  if (dst.empty()) return true;
+  const c10::cuda::CUDAGuard guard(dst[0].device());
+  for (size_t at = 0; at < dst.size(); at += adb200::kMaxCopies) {
+    adb200::CopyList c{};
+    long long blocks = 0;
+    for (size_t i = at; i < dst.size() && c.n < adb200::kMaxCopies; ++i) {
+      const long long bytes = (long long)dst[i].numel() * dst[i].element_size();
+      if (bytes == 0 || dst[i].data_ptr() == src[i].data_ptr()) continue;
+      c.src[c.n] = src[i].data_ptr(); c.dst[c.n] = dst[i].data_ptr(); c.bytes[c.n] = bytes;
+      c.first[c.n] = (int)blocks;
+      blocks += (bytes + adb200::kCopyBlockBytes - 1) / adb200::kCopyBlockBytes;
+      c.first[++c.n] = (int)blocks;
+    }
+    adb200::copy_list(c, STREAM);
+  }
+  return true;
+}
 void check_pair_tables(const Tensor& a, const Tensor& b, int64_t mf, const Tensor& users, const Tensor& items) {
   for (const Tensor* t : {&a, &b})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->dim() == 2 && t->is_contiguous() && t->size(1) == a.size(1) &&
@@ -1047,6 +1075,7 @@ void sampled_softmax_bias_grad(const Tensor& ids, const Tensor& dadj, Tensor dbi
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("copy_list", &copy_list);
   m.def("pair_lookup", &pair_lookup);
   m.def("pair_lookup_bwd", &pair_lookup_bwd);
   m.def("bce_logits", &bce_logits);

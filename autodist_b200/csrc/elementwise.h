@@ -26,6 +26,17 @@ void pair_lookup_bwd(const float* dgmf, long long ld, const bf16_t* dx, const fl
 int bce_logits_parts(long long n);
 void bce_logits(const float* x, const float* y, float* part, long long n, float scale, cudaStream_t st);
 void bce_logits_bwd(const float* x, const float* y, const float* grad, float* dx, long long n, float scale, cudaStream_t st);
+// dst[i][0 .. bytes[i]) = src[i]: up to kMaxCopies copies in one launch, the i-th by blocks first[i] .. first[i + 1] - 1.
+constexpr int kMaxCopies = 16;
+constexpr int kCopyBlockBytes = 16384;
+struct CopyList {
+  const void* src[kMaxCopies];
+  void* dst[kMaxCopies];
+  long long bytes[kMaxCopies];
+  int first[kMaxCopies + 1];
+  int n;
+};
+void copy_list(const CopyList& c, cudaStream_t st);
 void strided_rowsum(const bf16_t* x, float* out, int keys, int stride, int count, int H, cudaStream_t st);
 int colsum_parts(int rows);
 void keyed_colsum(const bf16_t* x, const int64_t* key, float* part, float* out, int rows, int H, int keys, int accumulate, cudaStream_t st);

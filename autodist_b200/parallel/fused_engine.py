@@ -955,8 +955,9 @@ class FusedStepEngine(StepEngine):
                 dist.barrier(group=self.backend.group)
             # the capture itself does not execute: fall through to a replay for this step
         _, graph, static, out = self._graph
-        for k, v in feeds.items():
-            static[k].copy_(v, non_blocking=True)
+        if not self.E.copy_list([static[k] for k in feeds], list(feeds.values())):
+            for k, v in feeds.items():
+                static[k].copy_(v, non_blocking=True)
         graph.replay()
         return out[:requested]
 
