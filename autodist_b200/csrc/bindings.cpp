@@ -131,28 +131,35 @@ void gemm_set_trace(const optional<Tensor>& t) {
 }
 
 // Which kernel runs a product: the tile width (512: the two-CTA kernel) and how many CTAs share the contraction of one tile.
-// The estimate in microseconds is launch + fill + drain of the kernel, plus, per wave of tiles, its K blocks of 64 (or the
-// epilogue of a tile, whichever is longer). The constants are measured over 60 products from 512 x 128 x 128 to
-// 32 x 4096 x 25088 (B200, replayed back to back on one set of operands and on rotating sets that do not fit the L2). A K
-// block is bound by shared-memory bandwidth: TMA writes it and the MMA reads it once, so 64 / 128 / 256 columns cost 48 / 64 /
-// 96 KB at 128 bytes per clock and narrow tiles only pay when they put more SMs to work. The two-CTA kernel moves the fewest
-// bytes per product and suffers least from operands that come from memory (4096 x 1024 x 3072 cold: 27.7 us against 31.5 of
-// the 256-wide one-CTA kernel; hot: 26.7 against 23.8), so it has the larger base and the smaller slope. Splitting adds the
-// exchange through distributed shared memory; it wins wherever the tiles leave SMs idle: 1024 x 1024 x 4096 29.2 -> 14.3 us
-// (256 wide, 4 CTAs), 768 x 768 x 1792 16.2 -> 9.0, 256 x 256 x 16384 94.7 -> 14.7, 640 x 1024 x 30522 172 -> 39,
-// 32 x 4096 x 25088 179 -> 38 (5.4 TB/s). Splits run one cluster per tile, so they are only considered while every cluster is
-// resident at once. The epilogue of a tile counts by kind (plain, bias, activation or auxiliary operand): narrow tiles store
-// directly and read what they need when they need it (8192 x 1024 x 128 fp32: 14.0 us with 64 columns, 9.2 with 256;
-// 1792 x 3072 x 768 with bias + GELU: 26.9 us with 128 columns, 18.2 with 256), and the last wave's is exposed.
+// The estimate in microseconds is launch + fill + first wave's K blocks of 64 + last drain, plus, per further wave of tiles, its K
+// blocks or the drain of a tile, whichever is longer. A K block costs more the more SMs take part (`load`): their fills share the L2.
+// The drain counts by kind (plain; bias or addend; activation; fp32 output): 64 and 128 columns store directly and read what they
+// need when they need it, wider tiles go through shared memory and TMA. Splitting the contraction adds the exchange through
+// distributed shared memory; it wins wherever the tiles leave SMs idle (256 x 256 x 16384 94.7 -> 14.7 us, 640 x 1024 x 30522
+// 172 -> 39). Splits run one cluster per tile, so they are only considered while every cluster is resident at once.
+// The constants are fitted to 170 products from 32 x 128 x 1000 to 8192 x 4096 x 1024 and 4096 x 25088 x 32 with every tile width and
+// split (B200, replayed back to back): the estimates' choices take 0.6 % more time in sum than the fastest kernel of each product.
+// Where the lines lie, in us:
+//   192 columns fill the SMs where 256 leave a third of them idle (128 x 192 tiles and 256 x 256 pairs):
+//     3072 x 1024 x 4096 20.0 (pairs 25.5), 4096 x 768 x 3072 16.2 (20.8), 1792 x 3072 x 768 with GELU 13.9 (15.7)
+//   pairs win once there are waves of them: 4096 x 4096 x 1024 with GELU 32.8 (192 columns 38.4), 8192 x 1024 x 4096 52.8 (68.9)
+//   256 columns on one CTA in between: 4096 x 1024 x 1024 10.1 (pairs 11.3, 192 columns 12.8)
 struct GemmChoice { int64_t bn, split; };
-GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split, int64_t epilogue, bool both_mn) {
-  struct Cost { int bn; double base, kb, epi[3], exchange; };
-  static const Cost costs[4] = {{64, 2.9, 0.30, {1.6, 2.0, 3.6}, 2.6},
-                                {128, 4.2, 0.33, {2.7, 3.4, 7.5}, 2.6},
-                                {256, 4.6, 0.48, {2.5, 3.7, 6.5}, 3.5},
-                                {512, 7.0, 0.41, {2.5, 3.7, 6.5}, 0.0}};
-  const int kind = epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2);
+GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split, int64_t epilogue, bool both_mn, bool fp32_out) {
+  struct Cost { int bn; double base, kb, load, mn, epi[4], wave, exchange; };      // exchange 0: no split of this width
+  static const Cost costs[5] = {{64, 2.87, 0.143, 0.17, 1.03, {1.3, 2.6, 3.5, 4.2}, 0.4, 2.0},
+                                {128, 3.35, 0.169, 0.31, 1.00, {2.8, 5.2, 6.8, 7.9}, 0.4, 2.0},
+                                {192, 3.16, 0.238, 0.18, 0.96, {3.4, 3.7, 5.7, 5.0}, 1.2, 0.0},
+                                {256, 3.29, 0.310, 0.31, 0.98, {4.0, 4.3, 6.4, 6.4}, 1.1, 5.0},
+                                {512, 4.24, 0.281, 0.22, 0.97, {4.0, 5.0, 6.7, 6.7}, 0.4, 0.0}};
+  const int kind = fp32_out ? 3 : (epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_ADD || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2));
   const int64_t kbs = (K + 63) / 64, sms = num_sms();
+  // Inside a step, where neighbours run beside a product, launching clusters costs more than back to back, and so do the many epilogue
+  // warps of a wide tile on a nearly empty GPU: a split has to be estimated that much faster, and 192 and 256 columns are
+  // considered where they fill close to half of the SMs (tiny BERT 377 -> 360 us, base tied 3757 -> 3660). In several waves of long
+  // contractions the widest tiles read the least from memory, which matters when the operands are not in the L2: narrower ones are
+  // left out there.
+  const double margin = 0.8;
   GemmChoice best{64, 1};
   double best_us = 1e30;
   for (const Cost& c : costs) {
@@ -162,16 +169,21 @@ GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allo
     const int64_t tm = pair ? 256 : 128, tn = pair ? 256 : c.bn;
     const int64_t tiles = ((M + tm - 1) / tm) * ((N + tn - 1) / tn) * batch;
     const int64_t slots = pair ? sms / 2 : sms;
+    const bool sparse = (c.bn == 192 || c.bn == 256) && 2 * tiles < sms - 20;
+    if (c.bn < 256 && N > 128 && tiles > sms && K > 1024) continue;
+    // long weight gradients stay on pairs, whose idle SMs run the optimizer beside them: 3072 x 1024 x 4096 alone 27 -> 21 us with 192
+    // columns, but the BERT-large step 12.26 -> 12.35 ms
+    if (c.bn == 192 && fp32_out && K > 2048) continue;
     const double waves = (double)((tiles + slots - 1) / slots);
-    const double kb = c.bn == 128 && both_mn ? 0.42 : c.kb;          // four copies per K block for one producer thread
     const double extra = c.epi[kind] - c.epi[0];                       // the last wave's drain (the plain one is part of the base)
-    const double us = c.base + (waves - 1) * std::max(kb * (double)kbs, c.epi[kind]) + kb * (double)kbs + extra;
-    if (us < best_us) { best_us = us; best = {c.bn, 1}; }
-    if (pair || !allow_split) continue;
+    auto blocks = [&](int64_t ctas, int64_t n) { return c.kb * (both_mn ? c.mn : 1.0) * (1.0 + c.load * std::min(1.0, (double)ctas / (double)slots)) * (double)n; };
+    const double us = c.base + (waves - 1) * std::max(blocks(tiles, kbs) + c.wave, c.epi[kind]) + blocks(tiles, kbs) + extra;
+    if (!sparse && us < best_us) { best_us = us; best = {c.bn, 1}; }
+    if (c.exchange == 0.0 || !allow_split) continue;
     for (int s = 2; s <= 8 && s <= kbs; ++s) {
       if (tiles * s > sms || tiles > adb200::gemm_split_max_clusters(s, (int)sms)) continue;
-      const double us_s = c.base + kb * (double)((kbs + s - 1) / s) + c.exchange + extra / s;
-      if (us_s < best_us) { best_us = us_s; best = {c.bn, s}; }
+      const double us_s = c.base + blocks(tiles * s, (kbs + s - 1) / s) + c.exchange + extra / s;
+      if (us_s < best_us - margin) { best_us = us_s; best = {c.bn, s}; }
     }
   }
   return best;
@@ -181,7 +193,7 @@ GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allo
 // for it in place of the estimate: products with a pair's tile in both extents whose tiles fill the SM pairs, or whose contraction
 // is at least that long.
 bool g_pair_unavailable = false;               // set when a cluster launch was refused once (see gemm_impl)
-GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn) {
+GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn, bool fp32_out) {
   static const bool pair_default = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR"); return e == nullptr || e[0] != '0'; }();
   static const int64_t pair_min_k = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR_MIN_K"); return e != nullptr ? std::atoll(e) : -1LL; }();
   const bool softmax_epi = epilogue == adb200::EPI_SOFTMAX || epilogue == adb200::EPI_SOFTMAX_GRAD;
@@ -191,11 +203,12 @@ GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t e
     if (M >= 256 && N >= 256 && (pair_tiles >= num_sms() / 2 || K >= pair_min_k)) return {512, 1};
     pair = false;
   }
-  return choose_gemm(M, N, K, batch, pair, !softmax_epi, epilogue, both_mn);
+  return choose_gemm(M, N, K, batch, pair, !softmax_epi, epilogue, both_mn, fp32_out);
 }
-// (tile width, contraction split) of gemm(..., bn = 0) for a product of these extents: 512 is the two-CTA kernel.
+// (tile width, contraction split) of gemm(..., bn = 0) for a product of these extents: 512 is the two-CTA kernel. Products of two
+// MN-major operands are weight gradients, whose output is fp32.
 std::tuple<int64_t, int64_t> gemm_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn) {
-  const GemmChoice g = auto_choice(M, N, K, batch, epilogue, both_mn);
+  const GemmChoice g = auto_choice(M, N, K, batch, epilogue, both_mn, both_mn);
   return {g.bn, g.split};
 }
 
@@ -212,16 +225,16 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
   TORCH_CHECK(a.size(0) == b.size(0) && a.size(1) == b.size(1), "batch dimensions of A and B differ");
   TORCH_CHECK(c.size(0) == a.size(0) && c.size(1) == a.size(1) && c.size(2) == M && c.size(3) == N, "output shape mismatch");
   TORCH_CHECK(c.stride(3) == 1, "output inner stride must be 1");
-  // bn: tile width 64 / 128 / 256 of the one-CTA kernel, or 512 = the 256 x 256 tile of the two-CTA kernel; 0 picks the kernel
+  // bn: tile width 64 / 128 / 192 / 256 of the one-CTA kernel, or 512 = the 256 x 256 tile of the two-CTA kernel; 0 picks the kernel
   // (see choose_gemm and auto_choice)
   const bool softmax_epi = epilogue == adb200::EPI_SOFTMAX || epilogue == adb200::EPI_SOFTMAX_GRAD;
   const bool auto_bn = bn <= 0;
   if (auto_bn) {
-    const GemmChoice g = auto_choice(M, N, K, a.size(0) * a.size(1), epilogue, a_mn && b_mn);
+    const GemmChoice g = auto_choice(M, N, K, a.size(0) * a.size(1), epilogue, a_mn && b_mn, c.scalar_type() == at::kFloat);
     bn = g.bn;
     split = g.split;
   }
-  TORCH_CHECK(bn == 64 || bn == 128 || bn == 256 || bn == 512, "bn must be 64, 128, 256 or 512 (two-CTA tile)");
+  TORCH_CHECK(bn == 64 || bn == 128 || bn == 192 || bn == 256 || bn == 512, "bn must be 64, 128, 192, 256 or 512 (two-CTA tile)");
   const bool pair = bn == 512;
   CUtensorMap tmA = make_map(a, a_mn ? 64 : 128);
   adb200::TmapArray tmB;
@@ -288,7 +301,7 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
   static const bool tma_store_default = [] { const char* e = std::getenv("AUTODIST_GEMM_TMA_STORE"); return e == nullptr || e[0] != '0'; }();
   CUtensorMap tmC, tmC2;
   p.tma_store = 0;
-  if (tma_store_default && !softmax_epi && bn >= 256 && (!p.c_is_fp32 || p.beta == 0.0f || p.beta == 1.0f) && make_store_map(c, &tmC)) {
+  if (tma_store_default && !softmax_epi && bn >= 192 && (!p.c_is_fp32 || p.beta == 0.0f || p.beta == 1.0f) && make_store_map(c, &tmC)) {
     p.tma_store = 1;
     tmC2 = tmC;
     if (epilogue == adb200::EPI_BIAS_GELU && !make_store_map(as4d(*c2), &tmC2)) p.tma_store = 0;

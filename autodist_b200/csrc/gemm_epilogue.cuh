@@ -66,30 +66,32 @@ __device__ __forceinline__ void gemm_epilogue_math16(const GemmParams& p, float*
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Output through shared memory and TMA, for the 256-wide tiles. Direct stores leave a warp writing 32 different rows in
+// Output through shared memory and TMA, for the tiles of 256 and 192 columns. Direct stores leave a warp writing 32 different rows in
 // 16-byte pieces - partial sectors that cost the L2 as much as full ones and compete with the operand loads. Here each
-// epilogue warp owns 32 rows x 128 columns, stages 32 rows x 128 bytes (64 bf16 or 32 fp32 columns) in the 128-byte-swizzled layout
+// epilogue warp owns 32 rows x 64 G columns (G = 2 for 256-wide tiles), stages 32 rows x 128 bytes (64 bf16 or 32 fp32 columns) in the 128-byte-swizzled layout
 // and one lane hands the box to the TMA unit, which writes whole lines (or adds them into an fp32 output: beta = 1). Rows and
-// columns past the matrix are clipped by the copy itself. Two 4 KB buffers per warp alternate, so staging overlaps the copy.
+// columns past the matrix are clipped by the copy itself. The 4 KB buffers of a warp take turns, so staging overlaps the copy.
 //
 // What the epilogue reads is requested while the tile is still being multiplied: the auxiliary operand (addend or pre-activation)
-// comes by TMA into the two staging buffers and is replaced there by the result, the bias into registers. The accumulator of a bf16
+// comes by TMA into the staging buffers and is replaced there by the result, the bias into registers. The accumulator of a bf16
 // output is read in the fragment layout (tmem_ld_frag32), where a lane needs 32 values of the bias for its 32 rows x 128 columns,
 // and the arithmetic is on pairs of values.
 // A tile's drain is exposed once per launch and, with a short contraction, once per tile: with GELU it took longer than the
 // multiplication of a 1024-deep tile. 4096 x 4096 x 1024 on SM pairs, back to back (a row per thread, the bias handed around by
 // shuffles -> now, us): bias + GELU 36.0 -> 32.9, GELU derivative 36.3 -> 31.5, plain 26.8 -> 25.7. Sixteen warps of 32 x 64 with one
 // buffer each: 34.3, 32.4, and 0.4 us more on every product.
-constexpr int kEpiCols = 128;    // columns of an epilogue warp, staged in two groups of 64
+//
+// G: groups of 64 columns per warp, and staging buffers: two for the 256-wide tiles, one for 192 (twelve warps, three per lane quarter).
+template <int G>
 struct EpiStage {
   const CUtensorMap* tmC;      // output map, box (128 bytes of columns, 32 rows, 1, 1), 128-byte swizzle
   const CUtensorMap* tmC2;     // EPI_BIAS_GELU: second output; EPI_ADD / EPI_MUL_GELU_GRAD: the auxiliary operand (same box)
-  uint32_t smem;               // shared address of this warp's two 4 KB staging buffers (1024-byte aligned)
-  uint64_t* aux_bar;           // two barriers of this warp: auxiliary box g has landed in buffer g
+  uint32_t smem;               // shared address of this warp's G staging buffers of 4 KB (1024-byte aligned)
+  uint64_t* aux_bar;           // G barriers of this warp: auxiliary box g has landed in buffer g
   int units;                   // copies issued so far by this warp (picks the buffer)
   uint32_t aux_phase;          // bit g: parity the next wait on aux_bar[g] expects
   uint32_t aux_pending;        // bit g: a load into buffer g has been requested and not yet waited for
-  float2 bias[16];             // columns 8 k + 2 (lane % 4) and the next of this warp's 128 (0 past the matrix or without a bias)
+  float2 bias[8 * G];          // columns 8 k + 2 (lane % 4) and the next of this warp's 64 G (0 past the matrix or without a bias)
 };
 
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
@@ -117,18 +119,19 @@ __device__ __forceinline__ bool epi_has_bias(const GemmParams& p) {
 }
 
 // Requests what the epilogue of the next tile reads (see EpiStage); n0: first of this warp's columns.
-__device__ __forceinline__ void gemm_epilogue_prefetch(const GemmParams& p, EpiStage& st, int box_row, int n0, int b_lo, int b_hi, int lane) {
+template <int G>
+__device__ __forceinline__ void gemm_epilogue_prefetch(const GemmParams& p, EpiStage<G>& st, int box_row, int n0, int b_lo, int b_hi, int lane) {
   if (box_row >= p.M) return;
   if (epi_has_bias(p)) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
+    for (int k = 0; k < 8 * G; ++k) {
       const int col = n0 + 8 * k + 2 * (lane & 3);
       st.bias[k] = make_float2(col < p.N ? __ldg(p.bias + col) : 0.f, col + 1 < p.N ? __ldg(p.bias + col + 1) : 0.f);
     }
   } else if (p.epilogue == EPI_ADD || p.epilogue == EPI_MUL_GELU_GRAD) {
-    if (elect_one()) bulk_wait_read<0>();             // the previous tile's copies have left both buffers
+    if (elect_one()) bulk_wait_read<0>();             // the previous tile's copies have left the buffers
 #pragma unroll
-    for (int g = 0; g < 2; ++g) {
+    for (int g = 0; g < G; ++g) {
       if (n0 + g * 64 >= p.N) break;
       if (elect_one()) {
         mbar_expect_tx(&st.aux_bar[g], 4096);
@@ -143,8 +146,9 @@ __device__ __forceinline__ void gemm_epilogue_prefetch(const GemmParams& p, EpiS
 }
 
 // Before the warp leaves: auxiliary boxes that nobody waited for (another role gave up) land first.
-__device__ __forceinline__ void gemm_epilogue_drain(EpiStage& st) {
-  for (int g = 0; g < 2; ++g)
+template <int G>
+__device__ __forceinline__ void gemm_epilogue_drain(EpiStage<G>& st) {
+  for (int g = 0; g < G; ++g)
     if (st.aux_pending & (1u << g)) {
       const long long t0 = clock64();
       while (!mbar_try(&st.aux_bar[g], (st.aux_phase >> g) & 1u) && clock64() - t0 < 20000000LL) {}
@@ -161,26 +165,27 @@ __device__ __forceinline__ void gemm_epilogue_hand_over(const CUtensorMap* map, 
     bulk_commit();
   }
 }
-// The buffer about to be written is no longer being read: all but the last copy have left theirs.
+// The buffer about to be written is no longer being read: all but the last G - 1 copies have left theirs.
+template <int G>
 __device__ __forceinline__ void gemm_epilogue_buffer_free() {
-  if (elect_one()) bulk_wait_read<1>();
+  if (elect_one()) bulk_wait_read<G - 1>();
   __syncwarp();
 }
 
-// A warp's 32 x 128 accumulator elements, bf16 outputs. EPI is the product's epilogue: one copy of the code per kind, since a test
+// A warp's 32 x 64 G accumulator elements, bf16 outputs. EPI is the product's epilogue: one copy of the code per kind, since a test
 // per element costs more than the arithmetic. Returns false when an auxiliary box did not arrive in time.
-template <int EPI, class Release>
-__device__ __forceinline__ bool gemm_epilogue_bf16(const GemmParams& p, EpiStage& st, uint32_t t_w, int box_row, int n0, int b_lo, int b_hi, int lane,
+template <int EPI, int G, class Release>
+__device__ __forceinline__ bool gemm_epilogue_bf16(const GemmParams& p, EpiStage<G>& st, uint32_t t_w, int box_row, int n0, int b_lo, int b_hi, int lane,
                                                    volatile int* abort_flag, Release& release) {
   constexpr bool BIAS = EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_TANH, AUX = EPI == EPI_ADD || EPI == EPI_MUL_GELU_GRAD;
   const uint32_t swz = (uint32_t)(lane >> 2);         // line % 8 of every row of this lane
   const uint32_t mine = (uint32_t)(lane >> 2) * 128u + (uint32_t)(lane & 3) * 4u;
   const uint64_t alpha = both(p.alpha);
 #pragma unroll
-  for (int g = 0; g < 2; ++g) {
+  for (int g = 0; g < G; ++g) {
     const int col0 = n0 + g * 64;
-    if (col0 >= p.N) {                                // uniform over the warp
-      if (g == 1) release();
+    if (col0 >= p.N) {                                // uniform over the warp; the first group exists
+      release();
       break;
     }
     uint32_t base;
@@ -190,8 +195,8 @@ __device__ __forceinline__ bool gemm_epilogue_bf16(const GemmParams& p, EpiStage
       st.aux_phase ^= 1u << g;
       st.aux_pending &= ~(1u << g);
     } else {
-      gemm_epilogue_buffer_free();
-      base = st.smem + (uint32_t)(st.units & 1) * 4096u;
+      gemm_epilogue_buffer_free<G>();
+      base = st.smem + (uint32_t)(st.units % G) * 4096u;
     }
     uint32_t act[EPI == EPI_BIAS_GELU ? 32 : 1];      // GELU values (two outputs: the pre-activation, then its GELU)
 #pragma unroll
@@ -199,7 +204,7 @@ __device__ __forceinline__ bool gemm_epilogue_bf16(const GemmParams& p, EpiStage
       uint32_t r[32];
       __syncwarp();                                   // tcgen05.ld is warp-collective
       tmem_ld_frag32(t_w + g * 64 + h * 32, r);
-      if (g == 1 && h == 1) release();
+      if (g == G - 1 && h == 1) release();
 #pragma unroll
       for (int k = 0; k < 4; ++k)
 #pragma unroll
@@ -221,8 +226,8 @@ __device__ __forceinline__ bool gemm_epilogue_bf16(const GemmParams& p, EpiStage
     gemm_epilogue_hand_over(st.tmC, base, col0, box_row, b_lo, b_hi, false);
     st.units += 1;
     if (EPI == EPI_BIAS_GELU) {                       // the second output through the other buffer
-      gemm_epilogue_buffer_free();
-      base = st.smem + (uint32_t)(st.units & 1) * 4096u;
+      gemm_epilogue_buffer_free<G>();
+      base = st.smem + (uint32_t)(st.units % G) * 4096u;
 #pragma unroll
       for (int j = 0; j < 32; ++j) sts1(base + mine + (uint32_t)(j & 3) * 1024u + (((uint32_t)(j >> 2) ^ swz) << 4), act[j]);
       gemm_epilogue_hand_over(st.tmC2, base, col0, box_row, b_lo, b_hi, false);
@@ -234,17 +239,17 @@ __device__ __forceinline__ bool gemm_epilogue_bf16(const GemmParams& p, EpiStage
 
 // The same for fp32 outputs (boxes of 32 columns): a row per lane, whose staged lines are written in 16-byte pieces without bank
 // conflicts. Bias is the only epilogue such outputs take; it is read again here.
-template <class Release>
-__device__ __forceinline__ void gemm_epilogue_f32(const GemmParams& p, EpiStage& st, uint32_t t_w, int box_row, int n0, int b_lo, int b_hi, int lane,
+template <int G, class Release>
+__device__ __forceinline__ void gemm_epilogue_f32(const GemmParams& p, EpiStage<G>& st, uint32_t t_w, int box_row, int n0, int b_lo, int b_hi, int lane,
                                                   Release& release) {
   const uint32_t swz = (uint32_t)(lane & 7);
   const bool bias = epi_has_bias(p);
 #pragma unroll 1
-  for (int g = 0; g < kEpiCols / 32; ++g) {
+  for (int g = 0; g < 2 * G; ++g) {
     const int col0 = n0 + g * 32;
     if (col0 >= p.N) break;                           // uniform over the warp
-    gemm_epilogue_buffer_free();
-    const uint32_t base = st.smem + (uint32_t)(st.units & 1) * 4096u, buf = base + (uint32_t)lane * 128u;
+    gemm_epilogue_buffer_free<G>();
+    const uint32_t base = st.smem + (uint32_t)(st.units % G) * 4096u, buf = base + (uint32_t)lane * 128u;
     float v[32];
     __syncwarp();                                     // tcgen05.ld is warp-collective
     tmem_ld32(t_w + g * 32, v);
@@ -269,8 +274,8 @@ __device__ __forceinline__ void gemm_epilogue_f32(const GemmParams& p, EpiStage&
 
 // t_w: TMEM address of this warp's 32 lanes at the first of its columns; box_row: first of its output rows. `release` is called once,
 // when the accumulator has been read. Returns false when an auxiliary box did not arrive in time (`release` has not been called then).
-template <class Release>
-__device__ __forceinline__ bool gemm_epilogue_tma(const GemmParams& p, EpiStage& st, uint32_t t_w, int box_row, int n0, int b_lo, int b_hi, int lane,
+template <int G, class Release>
+__device__ __forceinline__ bool gemm_epilogue_tma(const GemmParams& p, EpiStage<G>& st, uint32_t t_w, int box_row, int n0, int b_lo, int b_hi, int lane,
                                                   volatile int* abort_flag, Release&& release) {
   if (box_row >= p.M || n0 >= p.N) {                  // none of this warp's elements exist
     release();

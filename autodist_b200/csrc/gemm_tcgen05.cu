@@ -32,16 +32,19 @@ using namespace tc;
 
 template <int BN> struct Cfg {
   static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int STAGES = (BN == 256) ? 3 : (BN == 128 ? 6 : 8);
-  // Epilogue warps: four cover the TMEM lane quarters; the widest tile has eight, two per quarter with half of the
-  // columns each, because 128 threads cannot apply a bias or an activation to 32768 outputs in the time of one tile.
-  static constexpr int EPI_WARPS = (BN == 256) ? 4 * BN / kEpiCols : 4;
+  static constexpr int STAGES = BN == 256 ? 3 : (BN == 192 ? 4 : (BN == 128 ? 6 : 8));
+  // Epilogue warps: four cover the TMEM lane quarters; the widest tile has eight, two per quarter with half of the columns each, and 192
+  // columns twelve, three per quarter, because 128 threads cannot apply a bias or an activation to 32768 outputs in the time
+  // of one tile.
+  static constexpr bool WIDE = BN >= 192;
+  static constexpr int EPI_GROUPS = BN == 256 ? 2 : 1;     // groups of 64 columns per epilogue warp of a wide tile
+  static constexpr int EPI_WARPS = WIDE ? 4 * BN / (64 * EPI_GROUPS) : 4;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static constexpr int CW = BN / (EPI_WARPS / 4);          // columns per epilogue warp
-  static constexpr int TMEM_COLS = 2 * BN;              // double-buffered fp32 accumulator
-  // TMA-store staging (widest tile only): two 4 KB buffers per epilogue warp. The whole CTA stays near 210 KB so that the
+  static constexpr int TMEM_COLS = WIDE ? 512 : 2 * BN; // double-buffered fp32 accumulator; a power of two
+  // TMA-store staging (wide tiles only): 4 KB per epilogue warp and group. The whole CTA stays near 210 KB so that the
   // blocks of a small kernel launched behind it (programmatic dependent launch) still fit beside it on the SM.
-  static constexpr int STAGING = (BN == 256) ? EPI_WARPS * 8192 : 0;
+  static constexpr int STAGING = WIDE ? EPI_WARPS * EPI_GROUPS * 4096 : 0;
   static constexpr int SMEM = STAGES * (A_BYTES + B_BYTES) + STAGING + 1024 /*align*/ + 256 /*barriers*/;
 };
 
@@ -62,8 +65,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint64_t* aux_bars = tempty + 3;                      // widest tile: one per epilogue warp (behind the slot and the flag)
-  constexpr int AUX_BARS = BN == 256 ? 2 * C::EPI_WARPS : 0;
+  uint64_t* aux_bars = tempty + 3;                      // wide tiles: one per epilogue warp and group (behind the slot and the flag)
+  constexpr int AUX_BARS = C::WIDE ? C::EPI_GROUPS * C::EPI_WARPS : 0;
   static_assert((2 * C::STAGES + 4 + 1 + AUX_BARS) * 8 <= 256, "barrier area");
 
   const int warp = warp_index();
@@ -183,7 +186,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
     const int part = (warp - 2) >> 2;                  // which CW of the tile's columns this warp drains
     int as = 0; uint32_t aphase = 0; bool ok = true;
     const bool vec_ok = p.vec_ok != 0;
-    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, {}};
+    EpiStage<C::EPI_GROUPS> est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * (C::EPI_GROUPS * 4096u), aux_bars + C::EPI_GROUPS * (warp - 2),
+                                0, 0, 0, {}};
     for (long long t = blockIdx.x; t < total && ok; t += gridDim.x) {
       const int b = (int)(t / per_batch), rem = (int)(t % per_batch);
       const int tn = rem / tiles_m, tm = rem % tiles_m;
@@ -191,7 +195,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
       const int row = tm * BM + q * 32 + lane;
       const int n_w = tn * BN + part * C::CW;
       const int box_row = tm * BM + q * 32;
-      if constexpr (BN == 256) {
+      if constexpr (C::WIDE) {
         if (p.tma_store) gemm_epilogue_prefetch(p, est, box_row, n_w, b_lo, b_hi, lane);
       }
       if (!mbar_wait(&tfull[as], aphase, abort_flag)) { ok = false; break; }
@@ -272,7 +276,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
       }
       if (!handled) {
         const uint32_t t_w = t_row + (uint32_t)(part * C::CW);
-        if constexpr (BN == 256) {
+        if constexpr (C::WIDE) {
           handled = p.tma_store != 0;
           if (handled) ok = gemm_epilogue_tma(p, est, t_w, box_row, n_w, b_lo, b_hi, lane, abort_flag, release);
         }
@@ -286,8 +290,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ Tma
       if (!ok) break;
       if (++as == 2) { as = 0; aphase ^= 1; }
     }
-    if (BN == 256 && p.tma_store && elect_one()) bulk_wait_read<0>();   // this warp's copies have left its buffer (the end of the grid waits for them to land)
-    if (BN == 256) gemm_epilogue_drain(est);
+    if (C::WIDE && p.tma_store && elect_one()) bulk_wait_read<0>();   // this warp's copies have left its buffer (the end of the grid waits for them to land)
+    if (C::WIDE) gemm_epilogue_drain(est);
     if (!ok && lane == 0) {
       *abort_flag = 1;
       if (p.error_flag) atomicExch(p.error_flag, 3);
@@ -335,6 +339,7 @@ cudaError_t launch_gemm(const CUtensorMap& tmA, const TmapArray& tmB, const Gemm
     return launch_one<BN_, true, true>(tmA, tmB, p, num_sms, stream, tmC, tmC2);                          \
   }
   ADB_DISPATCH(256)
+  ADB_DISPATCH(192)
   ADB_DISPATCH(128)
   ADB_DISPATCH(64)
 #undef ADB_DISPATCH

@@ -41,7 +41,7 @@ struct TmapArray {
   CUtensorMap m[8];
 };
 
-// `bn` is the N extent of the tile (64, 128 or 256). The tensor maps must be 4-D bf16 maps with 128-byte swizzle:
+// `bn` is the N extent of the tile (64, 128, 192 or 256). The tensor maps must be 4-D bf16 maps with 128-byte swizzle:
 //   K-major operand : dims (K, rows, batch_lo, batch_hi), box (64, 128 for A / bn for B, 1, 1)
 //   MN-major operand: dims (rows, K, batch_lo, batch_hi), box (64, 64, 1, 1)
 // With p.tma_store, `tmC` (and `tmC2`: the second output of EPI_BIAS_GELU, the auxiliary operand of EPI_ADD and

@@ -37,7 +37,8 @@ constexpr int BN2 = 256;                 // tile width; each CTA stages BN2 / 2 
 constexpr int B2_BYTES = (BN2 / 2) * BK * 2;
 constexpr int STAGES2 = 5;              // 5 x 32 KB of operands + 64 KB of output staging: 226 of the SM's 227 KB
 constexpr int TMEM_COLS2 = 2 * BN2;
-constexpr int EPI_WARPS2 = 4 * BN2 / kEpiCols;    // two per TMEM lane quarter, half of the tile's columns each
+constexpr int EPI_COLS2 = 128;           // columns of an epilogue warp
+constexpr int EPI_WARPS2 = 4 * BN2 / EPI_COLS2;    // two per TMEM lane quarter, half of the tile's columns each
 constexpr int kThreads2 = 64 + 32 * EPI_WARPS2;
 constexpr int STAGING2 = EPI_WARPS2 * 8192;   // TMA-store staging: two 4 KB buffers per epilogue warp
 constexpr int SMEM2 = STAGES2 * (A_BYTES + B2_BYTES) + STAGING2 + 1024 /*align*/ + 256 /*barriers*/;
@@ -188,19 +189,19 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     const int part = (warp - 2) >> 2;                  // which half of the tile's columns this warp drains
     int as = 0; uint32_t aphase = 0; bool ok = true;
     const bool vec_ok = p.vec_ok != 0;
-    EpiStage est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, {}};
+    EpiStage<2> est{&tmC, &tmC2, smem_u32(staging) + (uint32_t)(warp - 2) * 8192u, aux_bars + 2 * (warp - 2), 0, 0, 0, {}};
     for (long long t = pair; t < total && ok; t += pairs) {
       const int b = (int)(t / per_batch), rem = (int)(t % per_batch);
       const int tn = rem / tiles_m, tm = rem % tiles_m;
       const int b_lo = b % p.batch_lo, b_hi = b / p.batch_lo;
       const int row = tm * 256 + (int)rank * 128 + q * 32 + lane;
-      const int n_w = tn * BN2 + part * kEpiCols;
+      const int n_w = tn * BN2 + part * EPI_COLS2;
       const int box_row = tm * 256 + (int)rank * 128 + q * 32;
       if (p.tma_store) gemm_epilogue_prefetch(p, est, box_row, n_w, b_lo, b_hi, lane);
       if (!mbar_wait(&tfull[as], aphase, abort_flag)) { ok = false; break; }
       const long long e0 = trace != nullptr ? now_ns() : 0;
       tc_fence_after();
-      const uint32_t t_w = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN2 + part * kEpiCols);
+      const uint32_t t_w = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN2 + part * EPI_COLS2);
       auto release = [&]() {                           // this warp has read its part of the accumulator
         __syncwarp();
         tc_fence_before();
@@ -211,7 +212,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         if (!ok) break;
       } else {
         const long long coff = (long long)b_hi * p.strideC_hi + (long long)b_lo * p.strideC_lo + (long long)row * p.ldc;
-        gemm_epilogue_row<kEpiCols>(p, t_w, row, n_w, coff, vec_ok);
+        gemm_epilogue_row<EPI_COLS2>(p, t_w, row, n_w, coff, vec_ok);
         release();
       }
       if (trace != nullptr && threadIdx.x == 64) trace[6] += now_ns() - e0;
