@@ -19,7 +19,8 @@
 // much as the rest of a pass, so the forward pass keeps the decisions as bits (1/16 of the scores' bf16 bytes).
 //
 // Per layer, 16 heads, dropout 0.1 (separate products and softmax kernels -> here): 32 x 128 tokens forward 37 -> 17 us, backward
-// 52 -> 21; 6 x 512 tokens forward about 85 -> 37, backward about 140 -> 64. The backward pass took 124 us while it hashed the
+// 52 -> 20; 6 x 512 tokens forward about 85 -> 36, backward about 140 -> 54 (60 with the next scores multiplied only once P and dS of
+// the current ones were in shared memory, and one value per instruction). The backward pass took 124 us while it hashed the
 // decisions again, read its row sums when it needed them and stored 32-byte pieces of the gradients directly.
 //
 // Every mbarrier wait is bounded: a role that gives up raises `abort`, which ends the waits of the others, and records a code.
@@ -61,6 +62,12 @@ constexpr float kLog2e = 1.4426950408889634f;
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
   return y;
 }
 
@@ -226,6 +233,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
     for (int c = threadIdx.x; c < tiles * 128; c += FWD_SOFT)
       s_mask[c] = c < p.S ? (p.mask != nullptr ? mask_base2(p.mask[(long long)b * p.S + c]) : 0.f) : -INFINITY;
     const float scale2 = p.scale * kLog2e;                 // scores, maxima and exponents are kept in base 2
+    const uint64_t scale2x = both(scale2);
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
     const uint32_t thresh = (uint32_t)(p.drop_p * 65536.0f);
     const uint32_t some = thresh > 0xffffu ? 0u : 0xffffffffu;      // probability 1: no 16-bit field reaches the threshold
@@ -256,7 +264,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
         tmem_ld16(tS + lane_base + hf * 64 + c * 16, v);
         if (plain) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) mx = fmaxf(mx, v[i]);
+          for (int i = 0; i < 16; i += 2) mx = max3(mx, v[i], v[i + 1]);
         } else {
 #pragma unroll
           for (int i = 0; i < 16; ++i) mx = fmaxf(mx, fmaf(v[i], scale2, mk[c * 16 + i]));
@@ -295,14 +303,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
           float v[16];
           tmem_ld16(tS + lane_base + hf * 64 + c * 32 + e * 16, v);
           if (plain) {
+            const uint64_t off = both(m0 - base);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = ex2(fmaf(v[i], scale2, m0 - base));
+            for (int i = 0; i < 16; i += 2) {
+              const float2 arg = unpack_f32x2(fma2(pack_f32x2(v[i], v[i + 1]), scale2x, off));
+              v[i] = ex2(arg.x);
+              v[i + 1] = ex2(arg.y);
+            }
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] = ex2(fmaf(v[i], scale2, mk[c * 32 + e * 16 + i] - base));
           }
+          uint64_t sum0 = 0, sum1 = 0;
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) l += (v[i] + v[i + 1]) + (v[i + 2] + v[i + 3]);
+          for (int i = 0; i < 16; i += 4) {
+            sum0 = add2(sum0, pack_f32x2(v[i], v[i + 1]));
+            sum1 = add2(sum1, pack_f32x2(v[i + 2], v[i + 3]));
+          }
+          const float2 sum = unpack_f32x2(add2(sum0, sum1));
+          l += sum.x + sum.y;
           if (p.drop_p > 0.f) {                            // 1 / keep probability is applied to the context at the end
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] = (bits >> (e * 16 + i)) & 1u ? v[i] : 0.f;
@@ -383,13 +402,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
   uint8_t* sD = sP + PTILE;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sD + PTILE);
   uint64_t *own_full = bars, *own_empty = bars + 2, *oth_full = bars + 4, *oth_empty = bars + 6, *s_full = bars + 8, *pd_full = bars + 9,
-           *acc_done = bars + 10, *acc_free = bars + 11;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+           *acc_done = bars + 10, *acc_free = bars + 11, *s_read = bars + 12;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 12; ++i) mbar_init(&bars[i], (&bars[i] == pd_full || &bars[i] == acc_free) ? BWD_SOFT / 32 : 1);
+    for (int i = 0; i < 13; ++i) mbar_init(&bars[i], (&bars[i] == pd_full || &bars[i] == acc_free || &bars[i] == s_read) ? BWD_SOFT / 32 : 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -485,14 +504,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
       };
       if (total > 0) ok = issue_scores(0);
       for (int t = 0; t < total && ok; ++t) {
-        ok = mbar_wait(pd_full, (uint32_t)t & 1u, abort_flag);        // P and dS are in shared memory, the scores have been read
+        // The next scores are multiplied while the second half of the current ones is worked on: their place is free once those have
+        // been read, which is before P and dS are in shared memory.
+        if (MODE != BWD_ALL && t + 1 < total) {
+          ok = mbar_wait(s_read, (uint32_t)t & 1u, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          ok = issue_scores(t + 1);
+          if (!ok) break;
+        }
+        ok = mbar_wait(pd_full, (uint32_t)t & 1u, abort_flag);        // P and dS are in shared memory
         if (!ok) break;
         tc_fence_after();
-        if (t % inner == inner - 1) {                                 // an item ends: its gradients are waited for
-          ok = issue_grads(t) && (t + 1 >= total || issue_scores(t + 1));
-        } else {
-          ok = issue_scores(t + 1) && issue_grads(t);
-        }
+        ok = issue_grads(t);
+        if (MODE == BWD_ALL && ok && t + 1 < total) ok = issue_scores(t + 1);      // an item ends here: its gradients are waited for next
       }
       if (!ok) {
         *abort_flag = 1;
@@ -542,6 +567,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
         const bool plain = __all_sync(0xffffffffu, mask2 == mask0);
         const float row_off = log2_keep - now.lse * kLog2e, nd = -now.delta * delta_scale;
         const float off0 = mask0 + row_off;
+        const uint64_t scale2x = both(scale2), scalex = both(p.scale), ndx = both(nd);
         soft_wait(s_full, (uint32_t)t & 1u, abort_flag, ok);
         tc_fence_after();
 #pragma unroll
@@ -550,9 +576,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
           __syncwarp();
           tmem_ld16(tS + lane_base + cb * 32 + c * 16, s);
           tmem_ld16(tDP + lane_base + cb * 32 + c * 16, d);
+          if (MODE != BWD_ALL && c == 1) {                 // this warp has read its scores
+            tc_fence_before();
+            __syncwarp();
+            if (elect_one()) mbar_arrive(s_read);
+          }
           if (plain) {
+            const uint64_t off = both(off0);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) s[e] = ex2(fmaf(s[e], scale2, off0));
+            for (int e = 0; e < 16; e += 2) {
+              const float2 arg = unpack_f32x2(fma2(pack_f32x2(s[e], s[e + 1]), scale2x, off));
+              s[e] = ex2(arg.x);
+              s[e + 1] = ex2(arg.y);
+            }
           } else {
 #pragma unroll
             for (int e = 0; e < 16; ++e) s[e] = ex2(fmaf(s[e], scale2, __shfl_sync(0xffffffffu, mask2, c * 16 + e) + row_off));
@@ -560,15 +596,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ 
           uint32_t pw[8], dw[8];
 #pragma unroll
           for (int e = 0; e < 16; e += 2) {
-            float x[2], y[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const bool kept = (now.keep >> (c * 16 + e + u)) & 1u;
-              x[u] = kept ? s[e + u] : 0.f;
-              y[u] = s[e + u] * (kept ? fmaf(d[e + u], p.scale, nd) : nd);
-            }
-            pw[e / 2] = pack_bf16x2(x[0], x[1]);
-            dw[e / 2] = pack_bf16x2(y[0], y[1]);
+            const float p0 = s[e], p1 = s[e + 1];
+            const float2 g = unpack_f32x2(fma2(pack_f32x2(d[e], d[e + 1]), scalex, ndx));
+            const bool k0 = (now.keep >> (c * 16 + e)) & 1u, k1 = (now.keep >> (c * 16 + e + 1)) & 1u;
+            pw[e / 2] = pack_bf16x2(k0 ? p0 : 0.f, k1 ? p1 : 0.f);
+            dw[e / 2] = round2(mul2(pack_f32x2(p0, p1), pack_f32x2(k0 ? g.x : nd, k1 ? g.y : nd)));
           }
           if (c == 0) {
             if (t > 0) soft_wait(acc_done, (uint32_t)(t - 1) & 1u, abort_flag, ok);      // P and dS of the iteration before have been multiplied
