@@ -220,8 +220,6 @@ def run_ours(model_name, args, n_gpus, world, rank):
             # started as soon as step i is launched (the session's `prefetch` argument), so it overlaps the step
             return sess.run([loss, train_op], feed(host_batches, i), prefetch=feed(host_batches, i + 1))[0]
 
-        # this extension's launches inside the device-timed region: eager launches are counted directly, a replayed CUDA graph
-        # by the launches of its capture
         counted = {"before": None, "after": None}
         ms, ms_e2e, last, clocks = _timed_with_count(step_dev, step_host, args, world, dev, rank, ops, counted)
         if hasattr(sess.engine, "check_errors"):
@@ -229,9 +227,7 @@ def run_ours(model_name, args, n_gpus, world, rank):
         engine_name = type(sess.engine).__name__
         if getattr(args, "flights", None) and hasattr(sess.engine, "flight_report"):
             _write_flights(args.flights, sess.engine, model_name, strategy, n_gpus, ms / args.steps, rank, world, dev)
-        graph_launches = getattr(sess.engine, "graph_kernels", 0)
-        eager = (counted["after"] or 0) - (counted["before"] or 0)
-        launches = eager if eager > 0 else graph_launches * args.steps
+        launches = _own_launches(counted, sess.engine, args.steps)
         sess.close()
     del sess, model, opt, dev_batches
     import gc
@@ -301,6 +297,14 @@ def _write_flights(path, engine, model_name, strategy, n_gpus, ms_step, rank, wo
     os.makedirs(os.path.dirname(os.path.abspath(path)), exist_ok=True)
     with open(path, "w") as f:
         f.write("\n".join(lines) + "\n")
+
+
+def _own_launches(counted, engine, steps):
+    """This extension's kernels inside the device-timed region: what was launched one by one (all of an eager step; of a graphed
+    one what runs beside the graph, such as the copy of the feed), and for every replay of a captured step the kernels of its capture."""
+    eager = (counted["after"] or 0) - (counted["before"] or 0)
+    replays = steps if getattr(engine, "_graph", None) is not None else 0
+    return eager + replays * getattr(engine, "graph_kernels", 0)
 
 
 def _timed_with_count(step_dev, step_host, args, world, dev, rank, ops, counted):

@@ -41,3 +41,18 @@ def test_flight_table_is_written_from_an_engines_report(tmp_path):
     # bus bandwidth of a 4-rank all-reduce: 2 * 3 / 4 * bytes / time
     assert rows[1].rstrip("|").split("|")[-1].strip() == str(round(1.5 * (2 << 20) * 4 / 0.5e-3 / 1e9))
     assert "busy 0.75 ms of the 12.50 ms step" in text and "ends 1.50 ms" in text
+
+
+def test_launch_count_adds_a_replays_kernels_to_those_beside_it():
+    sys.path.insert(0, ROOT)
+    import bench
+
+    class Engine:
+        _graph, graph_kernels = None, 0
+
+    eager, graphed = Engine(), Engine()
+    graphed._graph, graphed.graph_kernels = object(), 663
+    assert bench._own_launches({"before": 40, "after": 60}, graphed, 20) == 20 + 20 * 663        # one copy of the feed per replay
+    assert bench._own_launches({"before": 40, "after": 40}, graphed, 20) == 20 * 663
+    assert bench._own_launches({"before": 100, "after": 13400}, eager, 20) == 13300
+    assert bench._own_launches({"before": None, "after": None}, eager, 20) == 0
