@@ -131,60 +131,102 @@ void gemm_set_trace(const optional<Tensor>& t) {
 }
 
 // Which kernel runs a product: the tile width (512: the two-CTA kernel) and how many CTAs share the contraction of one tile.
-// The estimate in microseconds is launch + fill + first wave's K blocks of 64 + last drain, plus, per further wave of tiles, its K
-// blocks or the drain of a tile, whichever is longer. A K block costs more the more SMs take part (`load`): their fills share the L2.
-// The drain counts by kind (plain; bias or addend; activation; fp32 output): 64 and 128 columns store directly and read what they
-// need when they need it, wider tiles go through shared memory and TMA. Splitting the contraction adds the exchange through
-// distributed shared memory; it wins wherever the tiles leave SMs idle (256 x 256 x 16384 94.7 -> 14.7 us, 640 x 1024 x 30522
-// 172 -> 39). Splits run one cluster per tile, so they are only considered while every cluster is resident at once.
-// The constants are fitted to 170 products from 32 x 128 x 1000 to 8192 x 4096 x 1024 and 4096 x 25088 x 32 with every tile width and
-// split (B200, replayed back to back): the estimates' choices take 0.6 % more time in sum than the fastest kernel of each product.
-// Where the lines lie, in us:
+//
+// The two are chosen apart. A width changes no bit of the result: every kernel adds the products of an output in ascending order of
+// K. The number of shares does, since each share is summed by itself; what is rounded to bf16 behind the product then differs by an
+// ulp here and there, and a recurrence of such products carries that on (LM1B's gradients over 20 LSTM steps: 4e-4 of their norm
+// from one split to another). So the shares come from an estimate whose constants stay as they are, and only the width from
+// constants that follow the kernels.
+//
+// Both estimates are in microseconds: launch + fill + K blocks of 64 + drain, and per further wave of tiles its K blocks or the
+// drain of a tile, whichever is longer. Splitting adds the exchange through distributed shared memory; it wins wherever the tiles
+// leave SMs idle (256 x 256 x 16384 94.7 -> 14.7 us, 640 x 1024 x 30522 172 -> 39). Splits run one cluster per tile, so they are
+// only considered while every cluster is resident at once.
+//
+// Widths: a K block costs more the more SMs take part (`load`): their fills share the L2. The drain counts by kind (plain; bias or
+// addend; activation; fp32 output): 64 and 128 columns store directly and read what they need when they need it, wider tiles go
+// through shared memory and TMA. The constants are fitted to 170 products from 32 x 128 x 1000 to 8192 x 4096 x 1024 and 4096 x 25088 x 32
+// with every tile width (B200, replayed back to back). Where the lines lie, in us:
 //   192 columns fill the SMs where 256 leave a third of them idle (128 x 192 tiles and 256 x 256 pairs):
 //     3072 x 1024 x 4096 20.0 (pairs 25.5), 4096 x 768 x 3072 16.2 (20.8), 1792 x 3072 x 768 with GELU 13.9 (15.7)
 //   pairs win once there are waves of them: 4096 x 4096 x 1024 with GELU 32.8 (192 columns 38.4), 8192 x 1024 x 4096 52.8 (68.9)
 //   256 columns on one CTA in between: 4096 x 1024 x 1024 10.1 (pairs 11.3, 192 columns 12.8)
 struct GemmChoice { int64_t bn, split; };
-GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split, int64_t epilogue, bool both_mn, bool fp32_out) {
-  struct Cost { int bn; double base, kb, load, mn, epi[4], wave, exchange; };      // exchange 0: no split of this width
-  static const Cost costs[5] = {{64, 2.87, 0.143, 0.17, 1.03, {1.3, 2.6, 3.5, 4.2}, 0.4, 2.0},
-                                {128, 3.35, 0.169, 0.31, 1.00, {2.8, 5.2, 6.8, 7.9}, 0.4, 2.0},
-                                {192, 3.16, 0.238, 0.18, 0.96, {3.4, 3.7, 5.7, 5.0}, 1.2, 0.0},
-                                {256, 3.29, 0.310, 0.31, 0.98, {4.0, 4.3, 6.4, 6.4}, 1.1, 5.0},
-                                {512, 4.24, 0.281, 0.22, 0.97, {4.0, 5.0, 6.7, 6.7}, 0.4, 0.0}};
-  const int kind = fp32_out ? 3 : (epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_ADD || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2));
-  const int64_t kbs = (K + 63) / 64, sms = num_sms();
-  // Inside a step, where neighbours run beside a product, launching clusters costs more than back to back, and so do the many epilogue
-  // warps of a wide tile on a nearly empty GPU: a split has to be estimated that much faster, and 192 and 256 columns are
-  // considered where they fill close to half of the SMs (tiny BERT 377 -> 360 us, base tied 3757 -> 3660). In several waves of long
-  // contractions the widest tiles read the least from memory, which matters when the operands are not in the L2: narrower ones are
-  // left out there.
-  const double margin = 0.8;
-  GemmChoice best{64, 1};
+struct GemmTiles { int64_t tiles, slots; };              // output tiles of a width, and how many of them run at once
+// false: the width does not suit the product
+bool gemm_tiles(int bn, int64_t M, int64_t N, int64_t batch, bool allow_pair, GemmTiles* t) {
+  const bool pair = bn == 512;
+  if (pair && (!allow_pair || M < 256 || N < 256)) return false;
+  if (!pair && bn > 64 && N <= bn / 2) return false;                      // more than half of the tile would be padding
+  const int64_t tm = pair ? 256 : 128, tn = pair ? 256 : bn;
+  *t = {((M + tm - 1) / tm) * ((N + tn - 1) / tn) * batch, pair ? num_sms() / 2 : num_sms()};
+  return true;
+}
+bool gemm_split_fits(int64_t tiles, int s) { return tiles * s <= num_sms() && tiles <= adb200::gemm_split_max_clusters(s, (int)num_sms()); }
+
+// How many CTAs share the contraction: what the fastest kernel of the estimate would take, over 60 products from 512 x 128 x 128 to
+// 32 x 4096 x 25088.
+int choose_split(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, int64_t epilogue, bool both_mn) {
+  struct Cost { int bn; double base, kb, epi[3], exchange; };
+  static const Cost costs[4] = {{64, 2.9, 0.30, {1.6, 2.0, 3.6}, 2.6},
+                                {128, 4.2, 0.33, {2.7, 3.4, 7.5}, 2.6},
+                                {256, 4.6, 0.48, {2.5, 3.7, 6.5}, 3.5},
+                                {512, 7.0, 0.41, {2.5, 3.7, 6.5}, 0.0}};
+  const int kind = epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2);
+  const int64_t kbs = (K + 63) / 64;
+  int best = 1;
   double best_us = 1e30;
   for (const Cost& c : costs) {
-    const bool pair = c.bn == 512;
-    if (pair && (!allow_pair || M < 256 || N < 256)) continue;
-    if (c.bn < 512 && c.bn > 64 && N <= c.bn / 2) continue;              // more than half of the tile would be padding
-    const int64_t tm = pair ? 256 : 128, tn = pair ? 256 : c.bn;
-    const int64_t tiles = ((M + tm - 1) / tm) * ((N + tn - 1) / tn) * batch;
-    const int64_t slots = pair ? sms / 2 : sms;
-    const bool sparse = (c.bn == 192 || c.bn == 256) && 2 * tiles < sms - 20;
-    if (c.bn < 256 && N > 128 && tiles > sms && K > 1024) continue;
-    // long weight gradients stay on pairs, whose idle SMs run the optimizer beside them: 3072 x 1024 x 4096 alone 27 -> 21 us with 192
-    // columns, but the BERT-large step 12.26 -> 12.35 ms
-    if (c.bn == 192 && fp32_out && K > 2048) continue;
-    const double waves = (double)((tiles + slots - 1) / slots);
-    const double extra = c.epi[kind] - c.epi[0];                       // the last wave's drain (the plain one is part of the base)
-    auto blocks = [&](int64_t ctas, int64_t n) { return c.kb * (both_mn ? c.mn : 1.0) * (1.0 + c.load * std::min(1.0, (double)ctas / (double)slots)) * (double)n; };
-    const double us = c.base + (waves - 1) * std::max(blocks(tiles, kbs) + c.wave, c.epi[kind]) + blocks(tiles, kbs) + extra;
-    if (!sparse && us < best_us) { best_us = us; best = {c.bn, 1}; }
-    if (c.exchange == 0.0 || !allow_split) continue;
+    GemmTiles t;
+    if (!gemm_tiles(c.bn, M, N, batch, allow_pair, &t)) continue;
+    const double kb = c.bn == 128 && both_mn ? 0.42 : c.kb;
+    const double extra = c.epi[kind] - c.epi[0], waves = (double)((t.tiles + t.slots - 1) / t.slots);
+    const double us = c.base + (waves - 1) * std::max(kb * (double)kbs, c.epi[kind]) + kb * (double)kbs + extra;
+    if (us < best_us) { best_us = us; best = 1; }
+    if (c.exchange == 0.0) continue;
     for (int s = 2; s <= 8 && s <= kbs; ++s) {
-      if (tiles * s > sms || tiles > adb200::gemm_split_max_clusters(s, (int)sms)) continue;
-      const double us_s = c.base + blocks(tiles * s, (kbs + s - 1) / s) + c.exchange + extra / s;
-      if (us_s < best_us - margin) { best_us = us_s; best = {c.bn, s}; }
+      if (!gemm_split_fits(t.tiles, s)) continue;
+      const double us_s = c.base + kb * (double)((kbs + s - 1) / s) + c.exchange + extra / s;
+      if (us_s < best_us) { best_us = us_s; best = s; }
     }
+  }
+  return best;
+}
+
+GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split, int64_t epilogue, bool both_mn, bool fp32_out) {
+  struct Cost { int bn; double base, kb, load, mn, epi[4], wave; bool splits; };
+  static const Cost costs[5] = {{64, 2.87, 0.143, 0.17, 1.03, {1.3, 2.6, 3.5, 4.2}, 0.4, true},
+                                {128, 3.35, 0.169, 0.31, 1.00, {2.8, 5.2, 6.8, 7.9}, 0.4, true},
+                                {192, 3.16, 0.238, 0.18, 0.96, {3.4, 3.7, 5.7, 5.0}, 1.2, false},
+                                {256, 3.29, 0.310, 0.31, 0.98, {4.0, 4.3, 6.4, 6.4}, 1.1, true},
+                                {512, 4.24, 0.281, 0.22, 0.97, {4.0, 5.0, 6.7, 6.7}, 0.4, false}};
+  const int kind = fp32_out ? 3 : (epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_ADD || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2));
+  const int64_t kbs = (K + 63) / 64, sms = num_sms();
+  const int split = allow_split ? choose_split(M, N, K, batch, allow_pair, epilogue, both_mn) : 1;
+  GemmChoice best{64, split};
+  double best_us = 1e30;
+  for (const Cost& c : costs) {
+    GemmTiles t;
+    if (!gemm_tiles(c.bn, M, N, batch, allow_pair, &t)) continue;
+    const double extra = c.epi[kind] - c.epi[0];                       // the last wave's drain (the plain one is part of the base)
+    auto blocks = [&](int64_t ctas, int64_t n) { return c.kb * (both_mn ? c.mn : 1.0) * (1.0 + c.load * std::min(1.0, (double)ctas / (double)t.slots)) * (double)n; };
+    double us;
+    if (split > 1) {
+      if (!c.splits || !gemm_split_fits(t.tiles, split)) continue;
+      us = c.base + blocks(t.tiles * split, (kbs + split - 1) / split) + (c.bn == 256 ? 5.0 : 2.0) + extra / split;
+    } else {
+      // Inside a step, where neighbours run beside a product, the many epilogue warps of a wide tile cost more on a nearly empty GPU than
+      // back to back: 192 and 256 columns are considered where they fill close to half of the SMs. In several waves of long contractions
+      // the widest tiles read the least from memory, which matters when the operands are not in the L2.
+      if ((c.bn == 192 || c.bn == 256) && 2 * t.tiles < sms - 20) continue;
+      if (c.bn < 256 && N > 128 && t.tiles > sms && K > 1024) continue;
+      // long weight gradients stay on pairs, whose idle SMs run the optimizer beside them: 3072 x 1024 x 4096 alone 27 -> 21 us with 192
+      // columns, but the BERT-large step 12.26 -> 12.35 ms
+      if (c.bn == 192 && fp32_out && K > 2048) continue;
+      const double waves = (double)((t.tiles + t.slots - 1) / t.slots);
+      us = c.base + (waves - 1) * std::max(blocks(t.tiles, kbs) + c.wave, c.epi[kind]) + blocks(t.tiles, kbs) + extra;
+    }
+    if (us < best_us) { best_us = us; best.bn = c.bn; }
   }
   return best;
 }
