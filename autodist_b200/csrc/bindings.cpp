@@ -1083,48 +1083,51 @@ void bce_logits_bwd(const Tensor& x, const Tensor& y, const Tensor& grad, Tensor
               "gradients must match the logits");
   adb200::bce_logits_bwd(x.data_ptr<float>(), y.data_ptr<float>(), grad.data_ptr<float>(), dx.data_ptr<float>(), x.numel(), (float)scale, STREAM);
 }
-adb200::SampledSoftmax sampled_of(const Tensor& raw, const Tensor& out, const Tensor& true_w, const Tensor& adj, const Tensor& ids, const Tensor& lse,
-                                 const Tensor& true_logit) {
-  for (const Tensor* t : {&raw, &out, &true_w}) {
-    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 2 && t->is_contiguous() && t->size(1) % 8 == 0 &&
-                    reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "contiguous bf16 matrices with rows of 16-byte multiples needed");
-  }
+// logits [N, 1 + K] fp32 of the rows' own classes and the sampled ones; ids and corrections are scratch of [K + N] (and [K + N, 2]) that
+// the gradient passes read again. dot [N]: the own classes' products, bf16 or fp32.
+void sampled_logits(const Tensor& raw, const Tensor& dot, const Tensor& bias, const Tensor& neg, const Tensor& targets, double inv_log_v, double num_sampled,
+                    Tensor corrections, Tensor ids, Tensor logits, Tensor error) {
+  const c10::cuda::CUDAGuard guard(raw.device());
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&raw, &dot, &bias, &neg, &targets, &corrections, &ids, &logits})
+    TORCH_CHECK(t->is_cuda() && t->device() == raw.device() && t->is_contiguous(), "contiguous tensors on one GPU needed");
+  TORCH_CHECK(raw.scalar_type() == at::kBFloat16 && raw.dim() == 2 && raw.size(1) % 8 == 0, "bf16 products in rows of 16-byte multiples needed");
   const int64_t N = raw.size(0), K = raw.size(1);
-  TORCH_CHECK(N > 0 && out.size(0) == N && true_w.sizes() == out.sizes() && N + K < (1LL << 30), "rows of the products, outputs and true weights differ");
-  TORCH_CHECK(adj.scalar_type() == at::kFloat && adj.numel() >= N + K && ids.scalar_type() == at::kInt && ids.numel() >= N + K &&
-                  lse.scalar_type() == at::kFloat && lse.numel() >= N && true_logit.scalar_type() == at::kFloat && true_logit.numel() >= N,
-              "scratch of the sampled softmax too small");
-  return {(int)N, (int)K, (int)out.size(1), CBF(out), CBF(true_w), adj.data_ptr<float>(), ids.data_ptr<int>(), lse.data_ptr<float>(),
-          true_logit.data_ptr<float>()};
+  TORCH_CHECK(N > 0 && K > 0 && N + K < (1LL << 30) && dot.numel() == N && (dot.scalar_type() == at::kBFloat16 || dot.scalar_type() == at::kFloat),
+              "a product per row needed");
+  TORCH_CHECK(bias.scalar_type() == at::kFloat && bias.dim() == 1, "fp32 bias needed");
+  TORCH_CHECK(neg.scalar_type() == at::kLong && neg.numel() == K && targets.scalar_type() == at::kLong && targets.numel() == N,
+              "int64 ids of the sampled classes and of the targets needed");
+  TORCH_CHECK(corrections.scalar_type() == at::kFloat && corrections.numel() == 2 * (N + K) && ids.scalar_type() == at::kInt && ids.numel() == N + K &&
+                  logits.scalar_type() == at::kFloat && logits.numel() == N * (K + 1), "outputs must match the products");
+  adb200::sampled_logits(CBF(raw), dot.data_ptr(), dot.scalar_type() == at::kBFloat16, bias.data_ptr<float>(), neg.data_ptr<int64_t>(),
+                         targets.data_ptr<int64_t>(), (int)N, (int)K, bias.numel(), (float)inv_log_v, (float)num_sampled,
+                         reinterpret_cast<float2*>(corrections.data_ptr<float>()), ids.data_ptr<int>(), logits.data_ptr<float>(), error.data_ptr<int>(), STREAM);
 }
-// Losses of the rows; adj / ids [K + N], lse and true_logit [N] are what the backward pass needs.
-void sampled_softmax_fwd(const Tensor& raw, const Tensor& out, const Tensor& true_w, const Tensor& bias, const Tensor& neg, const Tensor& targets,
-                         double inv_log_v, double num_sampled, Tensor adj, Tensor ids, Tensor lse, Tensor true_logit, Tensor loss, Tensor error) {
-  const c10::cuda::CUDAGuard guard(raw.device());
-  const adb200::SampledSoftmax s = sampled_of(raw, out, true_w, adj, ids, lse, true_logit);
-  TORCH_CHECK(bias.scalar_type() == at::kFloat && bias.dim() == 1 && bias.is_contiguous(), "fp32 bias needed");
-  TORCH_CHECK(neg.scalar_type() == at::kLong && neg.is_contiguous() && neg.numel() == s.K && targets.scalar_type() == at::kLong &&
-                  targets.is_contiguous() && targets.numel() == s.N, "int64 ids of the sampled classes and of the targets needed");
-  TORCH_CHECK(loss.scalar_type() == at::kFloat && loss.numel() >= s.N, "a loss per row");
-  adb200::sampled_softmax_fwd(s, CBF(raw), bias.data_ptr<float>(), neg.data_ptr<int64_t>(), targets.data_ptr<int64_t>(), bias.numel(), (float)inv_log_v,
-                              (float)num_sampled, loss.data_ptr<float>(), error.data_ptr<int>(), STREAM);
-}
-void sampled_softmax_bwd(const Tensor& raw, const Tensor& out, const Tensor& true_w, const Tensor& adj, const Tensor& ids, const Tensor& lse,
-                         const Tensor& true_logit, const Tensor& grad, Tensor part, Tensor draw, Tensor d_out, Tensor d_true_w, Tensor dadj) {
-  const c10::cuda::CUDAGuard guard(raw.device());
-  const adb200::SampledSoftmax s = sampled_of(raw, out, true_w, adj, ids, lse, true_logit);
+// From the log-softmax of those logits: gradients of the products, of dot, and (dadj [K + N]) of every place's bias.
+void sampled_grad(const Tensor& logp, const Tensor& ids, const Tensor& grad, Tensor part, Tensor draw, Tensor ddot, Tensor dadj) {
+  const c10::cuda::CUDAGuard guard(logp.device());
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&logp, &ids, &grad, &part, &draw, &ddot, &dadj})
+    TORCH_CHECK(t->is_cuda() && t->device() == logp.device() && t->is_contiguous(), "contiguous tensors on one GPU needed");
+  TORCH_CHECK(draw.scalar_type() == at::kBFloat16 && draw.dim() == 2 && draw.size(1) % 8 == 0 && draw.numel() > 0, "bf16 gradient of the products needed");
+  const int64_t N = draw.size(0), K = draw.size(1);
+  TORCH_CHECK(logp.scalar_type() == at::kFloat && logp.numel() == N * (K + 1) && ids.scalar_type() == at::kInt && ids.numel() == N + K, "log-probabilities must match");
   TORCH_CHECK(grad.scalar_type() == at::kFloat && grad.numel() == 1, "fp32 scalar gradient needed");
-  TORCH_CHECK(part.numel() >= (int64_t)adb200::sampled_softmax_chunks(s.N, s.K) * s.K && dadj.numel() >= s.N + s.K, "scratch too small");
-  for (auto p : {std::make_pair(&draw, &raw), std::make_pair(&d_out, &out), std::make_pair(&d_true_w, &true_w)})
-    TORCH_CHECK(p.first->scalar_type() == at::kBFloat16 && p.first->is_contiguous() && p.first->sizes() == p.second->sizes() &&
-                    reinterpret_cast<uintptr_t>(p.first->data_ptr()) % 16 == 0, "gradients must match what they belong to");
-  adb200::sampled_softmax_bwd(s, CBF(raw), grad.data_ptr<float>(), part.data_ptr<float>(), BF(draw), BF(d_out), BF(d_true_w), dadj.data_ptr<float>(), STREAM);
+  TORCH_CHECK(ddot.numel() == N && (ddot.scalar_type() == at::kBFloat16 || ddot.scalar_type() == at::kFloat), "a gradient per row needed");
+  TORCH_CHECK(part.scalar_type() == at::kFloat && part.numel() >= (int64_t)adb200::sampled_grad_chunks((int)N, (int)K) * K && dadj.scalar_type() == at::kFloat &&
+                  dadj.numel() == N + K, "scratch too small");
+  adb200::sampled_grad(logp.data_ptr<float>(), ids.data_ptr<int>(), grad.data_ptr<float>(), (int)N, (int)K, part.data_ptr<float>(), BF(draw), ddot.data_ptr(),
+                       ddot.scalar_type() == at::kBFloat16, dadj.data_ptr<float>(), STREAM);
 }
-void sampled_softmax_bias_grad(const Tensor& ids, const Tensor& dadj, Tensor dbias) {
+// dbias[ids[i]] += dadj[i], in an order that the ids decide; at most SAMPLED_SCAN_MOST of them
+void sampled_bias_grad(const Tensor& ids, const Tensor& dadj, Tensor sums, Tensor firsts, Tensor dbias) {
   const c10::cuda::CUDAGuard guard(ids.device());
-  TORCH_CHECK(ids.scalar_type() == at::kInt && dadj.scalar_type() == at::kFloat && dadj.numel() >= ids.numel() && dbias.scalar_type() == at::kFloat &&
-                  dbias.is_contiguous(), "int32 ids and fp32 values");
-  adb200::sampled_softmax_bias_grad(ids.data_ptr<int>(), dadj.data_ptr<float>(), dbias.data_ptr<float>(), (int)ids.numel(), STREAM);
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&ids, &dadj, &sums, &firsts, &dbias})
+    TORCH_CHECK(t->is_cuda() && t->device() == ids.device() && t->is_contiguous(), "contiguous tensors on one GPU needed");
+  TORCH_CHECK(ids.scalar_type() == at::kInt && ids.numel() <= adb200::kSampledScanMost && dadj.scalar_type() == at::kFloat && dadj.numel() == ids.numel() &&
+                  dbias.scalar_type() == at::kFloat, "int32 ids and fp32 values");
+  const int64_t scratch = ids.numel() * adb200::sampled_bias_chunks((int)ids.numel());
+  TORCH_CHECK(sums.scalar_type() == at::kFloat && sums.numel() >= scratch && firsts.scalar_type() == at::kInt && firsts.numel() >= scratch, "scratch too small");
+  adb200::sampled_bias_grad(ids.data_ptr<int>(), dadj.data_ptr<float>(), sums.data_ptr<float>(), firsts.data_ptr<int>(), dbias.data_ptr<float>(), (int)ids.numel(), STREAM);
 }
 
 }  // namespace
@@ -1136,10 +1139,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bce_logits", &bce_logits);
   m.def("bce_logits_bwd", &bce_logits_bwd);
   m.def("bce_logits_parts", &adb200::bce_logits_parts);
-  m.def("sampled_softmax_fwd", &sampled_softmax_fwd);
-  m.def("sampled_softmax_bwd", &sampled_softmax_bwd);
-  m.def("sampled_softmax_bias_grad", &sampled_softmax_bias_grad);
-  m.def("sampled_softmax_chunks", &adb200::sampled_softmax_chunks);
+  m.def("sampled_logits", &sampled_logits);
+  m.def("sampled_grad", &sampled_grad);
+  m.def("sampled_bias_grad", &sampled_bias_grad);
+  m.def("sampled_grad_chunks", &adb200::sampled_grad_chunks);
+  m.def("sampled_bias_chunks", &adb200::sampled_bias_chunks);
+  m.attr("SAMPLED_SCAN_MOST") = adb200::kSampledScanMost;
   m.def("gemm_set_trace", &gemm_set_trace);
   m.def("gemm", &gemm);
   m.def("gemm_split", &gemm_split);

@@ -12,7 +12,7 @@ import torch
 from torch import nn
 import torch.nn.functional as F
 
-from autodist_b200.ops.functional import linear, lstm_layer, sampled_softmax, sparse_lookup
+from autodist_b200.ops.functional import linear, lstm_layer, sampled_softmax_of, sparse_lookup
 
 
 @dataclass
@@ -91,10 +91,11 @@ class LM1B(nn.Module):
         true_w = sparse_lookup(self.softmax_w, targets).to(dt)
         neg_w = sparse_lookup(self.softmax_w, neg).to(dt)
         products = linear(out, neg_w)                                          # [B*T, 512] x [8192, 512]^T on the tcgen05 GEMM
-        loss = sampled_softmax(products, out, true_w, self.softmax_b, neg, targets, c.num_sampled)
+        dot = (out * true_w).sum(1)
+        loss = sampled_softmax_of(products, dot, self.softmax_b, neg, targets, c.num_sampled)
         if loss is not None:
             return loss * c.num_steps
-        true_logit = (out * true_w).sum(1).float() + self.softmax_b[targets] - torch.log(
+        true_logit = dot.float() + self.softmax_b[targets] - torch.log(
             c.num_sampled * log_uniform_prob(targets, c.vocab_size))
         neg_logit = products.float() + self.softmax_b[neg]
         neg_logit = neg_logit - torch.log(c.num_sampled * log_uniform_prob(neg, c.vocab_size))

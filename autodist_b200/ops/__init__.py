@@ -26,13 +26,13 @@ def _dgrad_launches(dy, w, dx, stride, pad, *_):
 
 class _Counting:
     """Thin proxy over the extension module that counts kernel-launching calls."""
-    _NO_LAUNCH = {"ln_bwd_part_floats", "sampled_softmax_chunks", "bce_logits_parts", "colsum_parts", "gemm_choice", "gemm_set_trace", "conv_set_trace", "MAX_COMM_BLOCKS"}
+    _NO_LAUNCH = {"ln_bwd_part_floats", "sampled_grad_chunks", "sampled_bias_chunks", "bce_logits_parts", "colsum_parts", "gemm_choice", "gemm_set_trace", "conv_set_trace", "MAX_COMM_BLOCKS"}
     #: kernels per call where that is not one: a number, or a function of the call's arguments
     _MULTI = {"ln_bwd": 2, "keyed_colsum": 2, "relu_bwd_colsum": 2, "bn_sums": 2, "bn_bwd": 2,
               "bn_fwd": lambda *a: 1 if a[9] is not None else 3, "bn_fwd_nchw": lambda *a: 1 if a[6] is not None else 3,       # sums given or not
               "attn_bwd": lambda *a: 2 if a[8] <= 128 else 3,                                                                # tokens
               "xent": lambda *a: 2 if a[7] else 1,                                                                           # sums the weights
-              "sampled_softmax_fwd": 2, "sampled_softmax_bwd": 2, "conv_dgrad": _dgrad_launches}
+              "sampled_logits": 2, "sampled_grad": 2, "sampled_bias_grad": 2, "conv_dgrad": _dgrad_launches}
 
     def __init__(self, mod):
         self._mod = mod

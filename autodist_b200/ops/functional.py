@@ -847,56 +847,85 @@ def _ordered():
     return os.environ.get("AUTODIST_DETERMINISTIC") == "1" or torch.are_deterministic_algorithms_enabled()
 
 
+def _sampled_chain(neg_logits, dot, bias, neg, targets, num_sampled):
+    """What the sampled-softmax kernels compute, as PyTorch expressions (the log-softmax and the mean are theirs too)."""
+    def correction(ids):
+        f = ids.float()
+        return torch.log(num_sampled * (torch.log((f + 2.0) / (f + 1.0)) / math.log(bias.numel() + 1.0)))
+    own = dot.float() + bias[targets] - correction(targets)
+    others = neg_logits.float() + bias[neg] - correction(neg)
+    others = others.masked_fill(neg[None, :] == targets[:, None], -1e9)     # remove accidental hits
+    return F.cross_entropy(torch.cat([own[:, None], others], 1), torch.zeros_like(targets))
+
+
 class _SampledSoftmaxFn(torch.autograd.Function):
     """Mean cross-entropy of the true class against shared sampled classes (csrc/sampled_softmax.cu)."""
 
     @staticmethod
-    def forward(ctx, raw, out, true_w, bias, neg, targets, num_sampled):
+    def forward(ctx, raw, dot, bias, neg, targets, num_sampled):
         E = ops.ext(required=True)
         n, k = raw.shape
         dev = raw.device
-        adj, ids = torch.empty(k + n, dtype=torch.float32, device=dev), torch.empty(k + n, dtype=torch.int32, device=dev)
-        lse, true_logit, loss = torch.empty(3, n, dtype=torch.float32, device=dev).unbind(0)
-        E.sampled_softmax_fwd(raw, out, true_w, bias.detach(), neg, targets, 1.0 / math.log(bias.numel() + 1.0), num_sampled, adj, ids, lse, true_logit,
-                              loss, _error_flag(dev))
-        ctx.save_for_backward(raw, out, true_w, adj, ids, lse, true_logit)
-        ctx.bias = bias
-        _count_use(ctx, bias, 3)
-        return loss.mean()
+        corrections, ids = torch.empty(k + n, 2, dtype=torch.float32, device=dev), torch.empty(k + n, dtype=torch.int32, device=dev)
+        logits = torch.empty(n, k + 1, dtype=torch.float32, device=dev)
+        E.sampled_logits(raw, dot, bias.detach(), neg, targets, 1.0 / math.log(bias.numel() + 1.0), num_sampled, corrections, ids, logits, _error_flag(dev))
+        logp = torch.log_softmax(logits, 1)
+        ctx.save_for_backward(raw, dot, logp, ids, neg, targets)
+        ctx.bias, ctx.num_sampled = bias, num_sampled
+        _count_use(ctx, bias, 2)
+        return F.nll_loss(logp, torch.zeros_like(targets))
 
     @staticmethod
     def backward(ctx, grad):
         E = ops.ext(required=True)
-        raw, out, true_w, adj, ids, lse, true_logit = ctx.saved_tensors
-        n, k = raw.shape
-        part = torch.empty(E.sampled_softmax_chunks(n, k), k, dtype=torch.float32, device=raw.device)
-        draw, d_out, d_true_w, dadj = torch.empty_like(raw), torch.empty_like(out), torch.empty_like(true_w), torch.empty_like(adj)
-        E.sampled_softmax_bwd(raw, out, true_w, adj, ids, lse, true_logit, grad.float().contiguous(), part, draw, d_out, d_true_w, dadj)
-        d_bias = None
-        if ctx.needs_input_grad[3]:
-            acc = _direct_grad(ctx.bias)
-            d_bias = torch.zeros(ctx.bias.shape, dtype=torch.float32, device=raw.device) if acc is None else acc
-            if _ordered():
-                d_bias.index_put_((ids.long().clamp_min_(0),), torch.where(ids >= 0, dadj, 0.0), accumulate=True)
-            else:
-                E.sampled_softmax_bias_grad(ids, dadj, d_bias)
+        raw, dot, logp, ids, neg, targets = ctx.saved_tensors
+        acc = _direct_grad(ctx.bias) if ctx.needs_input_grad[2] else None
+        if torch.is_grad_enabled():                 # create_graph: a gradient that can itself be differentiated
+            wanted = [t for t, w in zip((raw, dot, ctx.bias), ctx.needs_input_grad) if w]
+            found = iter(torch.autograd.grad(_sampled_chain(raw, dot, ctx.bias, neg, targets, ctx.num_sampled), wanted, grad, create_graph=True))
+            draw, ddot, d_bias = (next(found) if w else None for w in ctx.needs_input_grad[:3])
             if acc is not None:
-                d_bias = None
-                _grad_written(ctx.bias)
-        return draw, d_out, d_true_w, d_bias, None, None, None
+                acc.add_(d_bias.detach())
+        else:
+            n, k = raw.shape
+            part = torch.empty(E.sampled_grad_chunks(n, k), k, dtype=torch.float32, device=raw.device)
+            draw, ddot, dadj = torch.empty_like(raw), torch.empty_like(dot), torch.empty(k + n, dtype=torch.float32, device=raw.device)
+            E.sampled_grad(logp, ids, grad.float().contiguous(), part, draw, ddot, dadj)
+            d_bias = None
+            if ctx.needs_input_grad[2]:
+                d_bias = torch.zeros(ctx.bias.shape, dtype=torch.float32, device=raw.device) if acc is None else acc
+                if k + n <= E.SAMPLED_SCAN_MOST:
+                    scratch = torch.empty(2, E.sampled_bias_chunks(k + n), k + n, dtype=torch.float32, device=raw.device)
+                    E.sampled_bias_grad(ids, dadj, scratch[0], scratch[1].view(torch.int32), d_bias)
+                else:
+                    d_bias.index_put_((ids.long().clamp_min_(0),), torch.where(ids >= 0, dadj, 0.0), accumulate=True)
+        if acc is not None:
+            d_bias = None
+            _grad_written(ctx.bias)
+        return draw, ddot, d_bias, None, None, None
 
 
-def sampled_softmax(neg_logits, out, true_w, bias, neg, targets, num_sampled):
+def sampled_softmax_of(neg_logits, dot, bias, neg, targets, num_sampled):
     """Mean over rows of ``-log softmax`` of the true class among itself and the sampled classes ``neg`` (log-uniform over ``bias.numel()``
-    classes). ``neg_logits``: ``out @ W[neg].T``; ``true_w``: ``W[targets]``; logits are corrected by ``bias`` and by the log of the
-    expected counts, negatives that hit the row's own class are masked. ``None`` where the kernels do not apply."""
-    mats = (neg_logits, out, true_w)
-    if not all(t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[0] and t.shape[1] and t.shape[1] % 8 == 0 for t in mats):
+    classes). ``neg_logits``: ``out @ W[neg].T``; ``dot``: the rows' products with their own classes, bf16 or fp32; logits are corrected by
+    ``bias`` and by the log of the expected counts, negatives that hit the row's own class are masked. ``None`` where the kernels do
+    not apply."""
+    raw = neg_logits
+    if not (raw.is_cuda and raw.dtype == torch.bfloat16 and raw.dim() == 2 and raw.shape[0] and raw.shape[1] and raw.shape[1] % 8 == 0):
+        return None
+    if dot.shape != raw.shape[:1] or dot.dtype not in (torch.bfloat16, torch.float32) or targets.shape != dot.shape or neg.shape != raw.shape[1:]:
         return None
     if bias.dtype != torch.float32 or bias.dim() != 1 or not bias.is_contiguous() or neg.dtype != torch.int64 or targets.dtype != torch.int64:
         return None
-    mats = [t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format) for t in mats]
-    return _SampledSoftmaxFn.apply(*mats, bias, neg.contiguous(), targets.contiguous(), float(num_sampled))
+    return _SampledSoftmaxFn.apply(raw.contiguous(), dot.contiguous(), bias, neg.contiguous(), targets.contiguous(), float(num_sampled))
+
+
+def sampled_softmax(neg_logits, out, true_w, bias, neg, targets, num_sampled):
+    """``sampled_softmax_of`` with the products of the rows ``out`` and their own classes' weights ``true_w`` (``W[targets]``) in fp32."""
+    if not all(t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[0] and t.shape[1] and t.shape[1] % 8 == 0
+               for t in (neg_logits, out, true_w)):
+        return None
+    return sampled_softmax_of(neg_logits, (out.float() * true_w.float()).sum(1), bias, neg, targets, num_sampled)
 
 
 _SPARSE_KINDS = {"sgd": 0, "lazy_adam": 1, "adagrad": 2}
