@@ -1041,6 +1041,10 @@ bool copy_list(const std::vector<Tensor>& dst, const std::vector<Tensor>& src) {
   }
   return true;
 }
+// A kernel gets the addresses of all of these.
+void check_one_gpu(std::initializer_list<const Tensor*> tensors) {
+  for (const Tensor* t : tensors) TORCH_CHECK(t->is_cuda() && t->device() == (*tensors.begin())->device(), "tensors on one GPU needed");
+}
 void check_pair_tables(const Tensor& a, const Tensor& b, int64_t mf, const Tensor& users, const Tensor& items) {
   for (const Tensor* t : {&a, &b})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->dim() == 2 && t->is_contiguous() && t->size(1) == a.size(1) &&
@@ -1052,6 +1056,7 @@ void check_pair_tables(const Tensor& a, const Tensor& b, int64_t mf, const Tenso
 // gmf [n, mf] fp32, x [n, 2 h] bf16, kept (optional) [n, 2 mf] fp32; tables [.., mf + h]
 void pair_lookup(const Tensor& ut, const Tensor& it, const Tensor& users, const Tensor& items, int64_t mf, Tensor gmf, Tensor x,
                  const optional<Tensor>& kept, Tensor error) {
+  check_one_gpu({&ut, &it, &users, &items, &gmf, &x, kept.has_value() ? &*kept : &x});
   check_pair_tables(ut, it, mf, users, items);
   const int64_t n = users.numel(), h = ut.size(1) - mf;
   TORCH_CHECK(gmf.numel() == n * mf && gmf.scalar_type() == at::kFloat && gmf.is_contiguous() && x.numel() == n * 2 * h &&
@@ -1062,6 +1067,7 @@ void pair_lookup(const Tensor& ut, const Tensor& it, const Tensor& users, const 
 }
 // dgmf: fp32 [n, mf] with unit inner stride
 void pair_lookup_bwd(const Tensor& dgmf, const Tensor& dx, const Tensor& kept, const Tensor& users, const Tensor& items, Tensor gu, Tensor gi) {
+  check_one_gpu({&dgmf, &dx, &kept, &users, &items, &gu, &gi});
   const int64_t n = users.numel(), mf = dgmf.size(1);
   check_pair_tables(gu, gi, mf, users, items);
   const int64_t h = gu.size(1) - mf;
@@ -1074,11 +1080,15 @@ void pair_lookup_bwd(const Tensor& dgmf, const Tensor& dx, const Tensor& kept, c
 }
 // part[i] = scale * the losses of elements 16384 i ...
 void bce_logits(const Tensor& x, const Tensor& y, Tensor part, double scale) {
+  check_one_gpu({&x, &y, &part});
   TORCH_CHECK(x.scalar_type() == at::kFloat && y.scalar_type() == at::kFloat && x.is_contiguous() && y.is_contiguous() && y.numel() == x.numel() &&
                   x.numel() > 0 && part.numel() >= adb200::bce_logits_parts(x.numel()), "contiguous fp32 logits and labels needed");
   adb200::bce_logits(x.data_ptr<float>(), y.data_ptr<float>(), part.data_ptr<float>(), x.numel(), (float)scale, STREAM);
 }
 void bce_logits_bwd(const Tensor& x, const Tensor& y, const Tensor& grad, Tensor dx, double scale) {
+  check_one_gpu({&x, &y, &grad, &dx});
+  TORCH_CHECK(x.scalar_type() == at::kFloat && y.scalar_type() == at::kFloat && dx.scalar_type() == at::kFloat && grad.scalar_type() == at::kFloat,
+              "fp32 tensors needed");
   TORCH_CHECK(x.is_contiguous() && y.is_contiguous() && dx.is_contiguous() && y.numel() == x.numel() && dx.numel() == x.numel() && grad.numel() == 1,
               "gradients must match the logits");
   adb200::bce_logits_bwd(x.data_ptr<float>(), y.data_ptr<float>(), grad.data_ptr<float>(), dx.data_ptr<float>(), x.numel(), (float)scale, STREAM);
@@ -1088,8 +1098,8 @@ void bce_logits_bwd(const Tensor& x, const Tensor& y, const Tensor& grad, Tensor
 void sampled_logits(const Tensor& raw, const Tensor& dot, const Tensor& bias, const Tensor& neg, const Tensor& targets, double inv_log_v, double num_sampled,
                     Tensor corrections, Tensor ids, Tensor logits, Tensor error) {
   const c10::cuda::CUDAGuard guard(raw.device());
-  for (const Tensor* t : std::initializer_list<const Tensor*>{&raw, &dot, &bias, &neg, &targets, &corrections, &ids, &logits})
-    TORCH_CHECK(t->is_cuda() && t->device() == raw.device() && t->is_contiguous(), "contiguous tensors on one GPU needed");
+  check_one_gpu({&raw, &dot, &bias, &neg, &targets, &corrections, &ids, &logits});
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&raw, &dot, &bias, &neg, &targets, &corrections, &ids, &logits}) TORCH_CHECK(t->is_contiguous(), "contiguous tensors needed");
   TORCH_CHECK(raw.scalar_type() == at::kBFloat16 && raw.dim() == 2 && raw.size(1) % 8 == 0, "bf16 products in rows of 16-byte multiples needed");
   const int64_t N = raw.size(0), K = raw.size(1);
   TORCH_CHECK(N > 0 && K > 0 && N + K < (1LL << 30) && dot.numel() == N && (dot.scalar_type() == at::kBFloat16 || dot.scalar_type() == at::kFloat),
@@ -1106,8 +1116,8 @@ void sampled_logits(const Tensor& raw, const Tensor& dot, const Tensor& bias, co
 // From the log-softmax of those logits: gradients of the products, of dot, and (dadj [K + N]) of every place's bias.
 void sampled_grad(const Tensor& logp, const Tensor& ids, const Tensor& grad, Tensor part, Tensor draw, Tensor ddot, Tensor dadj) {
   const c10::cuda::CUDAGuard guard(logp.device());
-  for (const Tensor* t : std::initializer_list<const Tensor*>{&logp, &ids, &grad, &part, &draw, &ddot, &dadj})
-    TORCH_CHECK(t->is_cuda() && t->device() == logp.device() && t->is_contiguous(), "contiguous tensors on one GPU needed");
+  check_one_gpu({&logp, &ids, &grad, &part, &draw, &ddot, &dadj});
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&logp, &ids, &grad, &part, &draw, &ddot, &dadj}) TORCH_CHECK(t->is_contiguous(), "contiguous tensors needed");
   TORCH_CHECK(draw.scalar_type() == at::kBFloat16 && draw.dim() == 2 && draw.size(1) % 8 == 0 && draw.numel() > 0, "bf16 gradient of the products needed");
   const int64_t N = draw.size(0), K = draw.size(1);
   TORCH_CHECK(logp.scalar_type() == at::kFloat && logp.numel() == N * (K + 1) && ids.scalar_type() == at::kInt && ids.numel() == N + K, "log-probabilities must match");
@@ -1121,8 +1131,8 @@ void sampled_grad(const Tensor& logp, const Tensor& ids, const Tensor& grad, Ten
 // dbias[ids[i]] += dadj[i], in an order that the ids decide; at most SAMPLED_SCAN_MOST of them
 void sampled_bias_grad(const Tensor& ids, const Tensor& dadj, Tensor sums, Tensor firsts, Tensor dbias) {
   const c10::cuda::CUDAGuard guard(ids.device());
-  for (const Tensor* t : std::initializer_list<const Tensor*>{&ids, &dadj, &sums, &firsts, &dbias})
-    TORCH_CHECK(t->is_cuda() && t->device() == ids.device() && t->is_contiguous(), "contiguous tensors on one GPU needed");
+  check_one_gpu({&ids, &dadj, &sums, &firsts, &dbias});
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&ids, &dadj, &sums, &firsts, &dbias}) TORCH_CHECK(t->is_contiguous(), "contiguous tensors needed");
   TORCH_CHECK(ids.scalar_type() == at::kInt && ids.numel() <= adb200::kSampledScanMost && dadj.scalar_type() == at::kFloat && dadj.numel() == ids.numel() &&
                   dbias.scalar_type() == at::kFloat, "int32 ids and fp32 values");
   const int64_t scratch = ids.numel() * adb200::sampled_bias_chunks((int)ids.numel());

@@ -727,6 +727,11 @@ def dense_lookup(table, ids):
     return F.embedding(ids, table)
 
 
+def _one_gpu(*tensors):
+    """Whether all of ``tensors`` lie on one GPU: a kernel is handed their addresses."""
+    return all(t.is_cuda and t.device == tensors[0].device for t in tensors)
+
+
 class _PairLookupFn(torch.autograd.Function):
     """Both lookups of (user, item) pairs with the product of their first columns and the concatenation of the others; the
     gradients go straight into the tables' flat gradient buffers."""
@@ -770,6 +775,8 @@ def pair_lookup(users_table, items_table, users, items, mf):
     if not all(t.is_cuda and t.dtype == torch.float32 and t.dim() == 2 and t.is_contiguous() and t.shape[1] == users_table.shape[1] and
                t.requires_grad and t.data_ptr() % 16 == 0 and t.shape[1] % 4 == 0 and _direct_grad(t) is not None for t in tables):
         return None
+    if not _one_gpu(users_table, items_table, users, items):
+        return None
     if users_table is items_table or mf % 4 or not 0 < mf < users_table.shape[1] or any(i.dtype != torch.int64 or i.dim() != 1 for i in (users, items)) or \
             users.numel() != items.numel() or not users.numel() or _ordered() or not torch.is_grad_enabled():
         return None
@@ -798,7 +805,7 @@ class _BCEFn(torch.autograd.Function):
 
 def bce_with_logits(logits, labels):
     """``F.binary_cross_entropy_with_logits(logits, labels)`` (the mean), one kernel each way for fp32 CUDA logits."""
-    if logits.is_cuda and labels.is_cuda and logits.dtype == labels.dtype == torch.float32 and logits.shape == labels.shape and logits.numel() and \
+    if _one_gpu(logits, labels) and logits.dtype == labels.dtype == torch.float32 and logits.shape == labels.shape and logits.numel() and \
             not labels.requires_grad:
         return _BCEFn.apply(logits.contiguous(), labels.contiguous())
     return F.binary_cross_entropy_with_logits(logits, labels)
@@ -911,7 +918,9 @@ def sampled_softmax_of(neg_logits, dot, bias, neg, targets, num_sampled):
     ``bias`` and by the log of the expected counts, negatives that hit the row's own class are masked. ``None`` where the kernels do
     not apply."""
     raw = neg_logits
-    if not (raw.is_cuda and raw.dtype == torch.bfloat16 and raw.dim() == 2 and raw.shape[0] and raw.shape[1] and raw.shape[1] % 8 == 0):
+    if not _one_gpu(raw, dot, bias, neg, targets):
+        return None
+    if not (raw.dtype == torch.bfloat16 and raw.dim() == 2 and raw.shape[0] and raw.shape[1] and raw.shape[1] % 8 == 0):
         return None
     if dot.shape != raw.shape[:1] or dot.dtype not in (torch.bfloat16, torch.float32) or targets.shape != dot.shape or neg.shape != raw.shape[1:]:
         return None
@@ -922,8 +931,8 @@ def sampled_softmax_of(neg_logits, dot, bias, neg, targets, num_sampled):
 
 def sampled_softmax(neg_logits, out, true_w, bias, neg, targets, num_sampled):
     """``sampled_softmax_of`` with the products of the rows ``out`` and their own classes' weights ``true_w`` (``W[targets]``) in fp32."""
-    if not all(t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[0] and t.shape[1] and t.shape[1] % 8 == 0
-               for t in (neg_logits, out, true_w)):
+    mats = (neg_logits, out, true_w)
+    if not _one_gpu(*mats) or not all(t.dtype == torch.bfloat16 and t.dim() == 2 and t.shape[0] and t.shape[1] and t.shape[1] % 8 == 0 for t in mats):
         return None
     return sampled_softmax_of(neg_logits, (out.float() * true_w.float()).sum(1), bias, neg, targets, num_sampled)
 
