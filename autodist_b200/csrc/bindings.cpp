@@ -1057,6 +1057,7 @@ void check_pair_tables(const Tensor& a, const Tensor& b, int64_t mf, const Tenso
 void pair_lookup(const Tensor& ut, const Tensor& it, const Tensor& users, const Tensor& items, int64_t mf, Tensor gmf, Tensor x,
                  const optional<Tensor>& kept, Tensor error) {
   check_one_gpu({&ut, &it, &users, &items, &gmf, &x, kept.has_value() ? &*kept : &x});
+  const c10::cuda::CUDAGuard guard(ut.device());
   check_pair_tables(ut, it, mf, users, items);
   const int64_t n = users.numel(), h = ut.size(1) - mf;
   TORCH_CHECK(gmf.numel() == n * mf && gmf.scalar_type() == at::kFloat && gmf.is_contiguous() && x.numel() == n * 2 * h &&
@@ -1068,6 +1069,7 @@ void pair_lookup(const Tensor& ut, const Tensor& it, const Tensor& users, const 
 // dgmf: fp32 [n, mf] with unit inner stride
 void pair_lookup_bwd(const Tensor& dgmf, const Tensor& dx, const Tensor& kept, const Tensor& users, const Tensor& items, Tensor gu, Tensor gi) {
   check_one_gpu({&dgmf, &dx, &kept, &users, &items, &gu, &gi});
+  const c10::cuda::CUDAGuard guard(dgmf.device());
   const int64_t n = users.numel(), mf = dgmf.size(1);
   check_pair_tables(gu, gi, mf, users, items);
   const int64_t h = gu.size(1) - mf;
@@ -1081,12 +1083,14 @@ void pair_lookup_bwd(const Tensor& dgmf, const Tensor& dx, const Tensor& kept, c
 // part[i] = scale * the losses of elements 16384 i ...
 void bce_logits(const Tensor& x, const Tensor& y, Tensor part, double scale) {
   check_one_gpu({&x, &y, &part});
+  const c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.scalar_type() == at::kFloat && y.scalar_type() == at::kFloat && x.is_contiguous() && y.is_contiguous() && y.numel() == x.numel() &&
                   x.numel() > 0 && part.numel() >= adb200::bce_logits_parts(x.numel()), "contiguous fp32 logits and labels needed");
   adb200::bce_logits(x.data_ptr<float>(), y.data_ptr<float>(), part.data_ptr<float>(), x.numel(), (float)scale, STREAM);
 }
 void bce_logits_bwd(const Tensor& x, const Tensor& y, const Tensor& grad, Tensor dx, double scale) {
   check_one_gpu({&x, &y, &grad, &dx});
+  const c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.scalar_type() == at::kFloat && y.scalar_type() == at::kFloat && dx.scalar_type() == at::kFloat && grad.scalar_type() == at::kFloat,
               "fp32 tensors needed");
   TORCH_CHECK(x.is_contiguous() && y.is_contiguous() && dx.is_contiguous() && y.numel() == x.numel() && dx.numel() == x.numel() && grad.numel() == 1,
