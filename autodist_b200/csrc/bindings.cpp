@@ -1045,6 +1045,11 @@ bool copy_list(const std::vector<Tensor>& dst, const std::vector<Tensor>& src) {
 void check_one_gpu(std::initializer_list<const Tensor*> tensors) {
   for (const Tensor* t : tensors) TORCH_CHECK(t->is_cuda() && t->device() == (*tensors.begin())->device(), "tensors on one GPU needed");
 }
+// Where a kernel reports an id outside its table: a word on the device, or in pinned host memory, which the host reads without waiting.
+int* report_word(const Tensor& t) {
+  TORCH_CHECK(t.scalar_type() == at::kInt && t.numel() >= 1 && (t.is_cuda() || t.is_pinned()), "an int32 word on the GPU or in pinned memory needed");
+  return t.data_ptr<int>();
+}
 void check_pair_tables(const Tensor& a, const Tensor& b, int64_t mf, const Tensor& users, const Tensor& items) {
   for (const Tensor* t : {&a, &b})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->dim() == 2 && t->is_contiguous() && t->size(1) == a.size(1) &&
@@ -1064,7 +1069,7 @@ void pair_lookup(const Tensor& ut, const Tensor& it, const Tensor& users, const 
                   x.scalar_type() == at::kBFloat16 && x.is_contiguous() && (!kept.has_value() || (kept->numel() == n * 2 * mf && kept->is_contiguous())),
               "outputs must match the lookups");
   adb200::pair_lookup(ut.data_ptr<float>(), it.data_ptr<float>(), users.data_ptr<int64_t>(), items.data_ptr<int64_t>(), gmf.data_ptr<float>(), BF(x), OPT_F(kept),
-                      n, (int)mf, (int)h, ut.size(0), it.size(0), error.data_ptr<int>(), STREAM);
+                      n, (int)mf, (int)h, ut.size(0), it.size(0), report_word(error), STREAM);
 }
 // dgmf: fp32 [n, mf] with unit inner stride
 void pair_lookup_bwd(const Tensor& dgmf, const Tensor& dx, const Tensor& kept, const Tensor& users, const Tensor& items, Tensor gu, Tensor gi) {
@@ -1115,7 +1120,7 @@ void sampled_logits(const Tensor& raw, const Tensor& dot, const Tensor& bias, co
                   logits.scalar_type() == at::kFloat && logits.numel() == N * (K + 1), "outputs must match the products");
   adb200::sampled_logits(CBF(raw), dot.data_ptr(), dot.scalar_type() == at::kBFloat16, bias.data_ptr<float>(), neg.data_ptr<int64_t>(),
                          targets.data_ptr<int64_t>(), (int)N, (int)K, bias.numel(), (float)inv_log_v, (float)num_sampled,
-                         reinterpret_cast<float2*>(corrections.data_ptr<float>()), ids.data_ptr<int>(), logits.data_ptr<float>(), error.data_ptr<int>(), STREAM);
+                         reinterpret_cast<float2*>(corrections.data_ptr<float>()), ids.data_ptr<int>(), logits.data_ptr<float>(), report_word(error), STREAM);
 }
 // From the log-softmax of those logits: gradients of the products, of dot, and (dadj [K + N]) of every place's bias.
 void sampled_grad(const Tensor& logp, const Tensor& ids, const Tensor& grad, Tensor part, Tensor draw, Tensor ddot, Tensor dadj) {

@@ -424,7 +424,7 @@ __global__ void scatter_add_rows_f32_kernel(float* __restrict__ dst, const int64
 
 // Lookups of (user, item) pairs in two fp32 tables of rows [mf | h columns]: gmf = product of the first mf columns (fp32), x = [user's
 // h, item's h] as bf16, what the first layer of the other branch reads. The first columns are kept for the backward pass. Four columns
-// per thread. An id outside its table reads zeros and is reported.
+// per thread. An id outside its table reads zeros and is reported by a plain store (the word may lie in host memory).
 __global__ void pair_lookup_kernel(const float* __restrict__ ut, const float* __restrict__ it, const int64_t* __restrict__ users, const int64_t* __restrict__ items,
                                    float* __restrict__ gmf, bf16* __restrict__ x, float* __restrict__ kept, long long total, int mf4, int h4,
                                    long long nu, long long ni, int* __restrict__ error) {
@@ -437,9 +437,9 @@ __global__ void pair_lookup_kernel(const float* __restrict__ ut, const float* __
   const long long u = users[r], i = items[r];
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
   if ((unsigned long long)u < (unsigned long long)nu) a = reinterpret_cast<const float4*>(ut)[u * w4 + c];
-  else atomicExch(error, 72);
+  else *const_cast<volatile int*>(error) = 72;
   if ((unsigned long long)i < (unsigned long long)ni) b = reinterpret_cast<const float4*>(it)[i * w4 + c];
-  else atomicExch(error, 72);
+  else *const_cast<volatile int*>(error) = 72;
   if (c < mf4) {
     reinterpret_cast<float4*>(gmf)[r * mf4 + c] = make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
     if (kept != nullptr) {

@@ -22,7 +22,32 @@ def _error_flag(device):
     return _err[device]
 
 
+#: Per device a word of pinned host memory that kernels write when an id lies outside its table (they read nothing there), and its numpy
+#: view: the host looks at it without waiting for the device.
+_id_flags = {}
+_ID_ERRORS = {71: "a sampled softmax met an id outside its vocabulary", 72: "a lookup of (user, item) pairs met an id outside its table"}
+
+
+def _id_flag(device):
+    if device not in _id_flags:
+        flag = torch.zeros(1, dtype=torch.int32).pin_memory()
+        _id_flags[device] = flag, flag.numpy()
+    return _id_flags[device][0]
+
+
+def raise_bad_ids():
+    """Raises for ids outside their tables that kernels have reported so far, once each. Costs no wait."""
+    for dev, (_, seen) in _id_flags.items():
+        code = int(seen[0])
+        if code:
+            seen[0] = 0
+            raise RuntimeError(f"{_ID_ERRORS.get(code, 'an id outside its table')} on {dev}: its row counted as zeros, the results are not valid")
+
+
 def check_errors():
+    for dev in _id_flags:
+        torch.cuda.synchronize(dev)
+    raise_bad_ids()
     for dev, flag in _err.items():
         code = int(flag.item())
         if code:
@@ -739,10 +764,11 @@ class _PairLookupFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, users_table, items_table, users, items, mf):
         E = ops.ext(required=True)
+        raise_bad_ids()
         n, h, dev = users.numel(), users_table.shape[1] - mf, users_table.device
         gmf, kept = (torch.empty(n, w, dtype=torch.float32, device=dev) for w in (mf, 2 * mf))
         x = torch.empty(n, 2 * h, dtype=torch.bfloat16, device=dev)
-        E.pair_lookup(users_table.detach(), items_table.detach(), users, items, mf, gmf, x, kept, _error_flag(dev))
+        E.pair_lookup(users_table.detach(), items_table.detach(), users, items, mf, gmf, x, kept, _id_flag(dev))
         ctx.save_for_backward(kept, users, items)
         ctx.tables = users_table, items_table
         for k, table in enumerate(ctx.tables):
@@ -871,11 +897,12 @@ class _SampledSoftmaxFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, raw, dot, bias, neg, targets, num_sampled):
         E = ops.ext(required=True)
+        raise_bad_ids()
         n, k = raw.shape
         dev = raw.device
         corrections, ids = torch.empty(k + n, 2, dtype=torch.float32, device=dev), torch.empty(k + n, dtype=torch.int32, device=dev)
         logits = torch.empty(n, k + 1, dtype=torch.float32, device=dev)
-        E.sampled_logits(raw, dot, bias.detach(), neg, targets, 1.0 / math.log(bias.numel() + 1.0), num_sampled, corrections, ids, logits, _error_flag(dev))
+        E.sampled_logits(raw, dot, bias.detach(), neg, targets, 1.0 / math.log(bias.numel() + 1.0), num_sampled, corrections, ids, logits, _id_flag(dev))
         logp = torch.log_softmax(logits, 1)
         ctx.save_for_backward(raw, dot, logp, ids, neg, targets)
         ctx.bias, ctx.num_sampled = bias, num_sampled

@@ -194,6 +194,12 @@ class StepEngine:
             self._publish_ps()
             self._pending_pull = False
 
+    def raise_reported(self):
+        """Raises for bad input that kernels have reported to the host by now; does not wait for the device."""
+        if self.device.type == "cuda":
+            from autodist_b200.ops.functional import raise_bad_ids
+            raise_bad_ids()
+
     def train_step(self, train_op, nodes, feeds):
         self.before_read()
         if self._async is not None:

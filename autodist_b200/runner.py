@@ -238,6 +238,7 @@ class WrappedSession:
 
     def _run(self, fetches, feed_dict, prefetch=None):
         rm, eng = self._remapper, self._engine
+        eng.raise_reported()                 # by a step whose results nobody fetched
         single = not isinstance(fetches, (list, tuple, dict))
         leaves, rebuild = rm.flatten_fetches([fetches] if single else fetches)
         kinds = [rm.classify(l) for l in leaves]
@@ -272,6 +273,7 @@ class WrappedSession:
                 if value.dtype == torch.bfloat16:
                     value = value.float()                       # numpy has no bfloat16
                 out[i] = np.array(value.cpu().numpy(), copy=True)   # a copy: never a view of live parameter memory
+        eng.raise_reported()                 # what was fetched is on the host, so this step has said what it had to say
         result = rebuild(out)
         return result[0] if single else result
 
@@ -288,8 +290,11 @@ class WrappedSession:
             self._engine._pending_pull = False
         try:
             self._engine.close()
+            if self._engine.device.type == "cuda":
+                torch.cuda.synchronize(self._engine.device)
         except Exception as e:  # shutting down: peers may already be gone
             logging.debug("engine close: %s", e)
+        self._engine.raise_reported()        # steps that nobody looked at
 
     def __enter__(self):
         return self
