@@ -757,6 +757,12 @@ def _one_gpu(*tensors):
     return all(t.is_cuda and t.device == tensors[0].device for t in tensors)
 
 
+def _reverse_mode_only():
+    """Whether nothing but reverse-mode differentiation can be going on: no ``torch.func`` transform, no forward-mode level. The kernels'
+    autograd functions know of nothing else."""
+    return not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+
+
 class _PairLookupFn(torch.autograd.Function):
     """Both lookups of (user, item) pairs with the product of their first columns and the concatenation of the others; the
     gradients go straight into the tables' flat gradient buffers."""
@@ -801,7 +807,7 @@ def pair_lookup(users_table, items_table, users, items, mf):
     if not all(t.is_cuda and t.dtype == torch.float32 and t.dim() == 2 and t.is_contiguous() and t.shape[1] == users_table.shape[1] and
                t.requires_grad and t.data_ptr() % 16 == 0 and t.shape[1] % 4 == 0 and _direct_grad(t) is not None for t in tables):
         return None
-    if not _one_gpu(users_table, items_table, users, items):
+    if not _one_gpu(users_table, items_table, users, items) or not _reverse_mode_only():
         return None
     if users_table is items_table or mf % 4 or not 0 < mf < users_table.shape[1] or any(i.dtype != torch.int64 or i.dim() != 1 for i in (users, items)) or \
             users.numel() != items.numel() or not users.numel() or _ordered() or not torch.is_grad_enabled():
@@ -824,6 +830,8 @@ class _BCEFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         logits, labels = ctx.saved_tensors
+        if torch.is_grad_enabled():                 # create_graph: a gradient that can itself be differentiated
+            return (torch.sigmoid(logits) - labels) * (grad / logits.numel()), None
         dx = torch.empty_like(logits)
         ops.ext(required=True).bce_logits_bwd(logits, labels, grad.float().contiguous(), dx, 1.0 / logits.numel())
         return dx, None
@@ -832,7 +840,7 @@ class _BCEFn(torch.autograd.Function):
 def bce_with_logits(logits, labels):
     """``F.binary_cross_entropy_with_logits(logits, labels)`` (the mean), one kernel each way for fp32 CUDA logits."""
     if _one_gpu(logits, labels) and logits.dtype == labels.dtype == torch.float32 and logits.shape == labels.shape and logits.numel() and \
-            not labels.requires_grad:
+            not labels.requires_grad and _reverse_mode_only():
         return _BCEFn.apply(logits.contiguous(), labels.contiguous())
     return F.binary_cross_entropy_with_logits(logits, labels)
 
@@ -945,7 +953,7 @@ def sampled_softmax_of(neg_logits, dot, bias, neg, targets, num_sampled):
     ``bias`` and by the log of the expected counts, negatives that hit the row's own class are masked. ``None`` where the kernels do
     not apply."""
     raw = neg_logits
-    if not _one_gpu(raw, dot, bias, neg, targets):
+    if not _one_gpu(raw, dot, bias, neg, targets) or not _reverse_mode_only():
         return None
     if not (raw.dtype == torch.bfloat16 and raw.dim() == 2 and raw.shape[0] and raw.shape[1] and raw.shape[1] % 8 == 0):
         return None
