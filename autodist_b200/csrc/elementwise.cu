@@ -486,7 +486,8 @@ __global__ void pair_lookup_bwd_kernel(const float* __restrict__ dgmf, long long
   if ((unsigned long long)i < (unsigned long long)ni) atomicAdd(reinterpret_cast<float4*>(gi) + i * w4 + c, b);
 }
 
-// Binary cross-entropy with logits: part[block] = sum over the block's elements of max(x, 0) - x y + log(1 + exp(-|x|)).
+// Binary cross-entropy with logits: part[block] = sum over the block's elements of max(x, 0) - x y + log(1 + exp(-|x|)). An infinite x gives
+// what the library's (1 - y) x - min(x, 0) + log(..) gives, which cancels for finite ones.
 constexpr int kBcePerBlock = 16384;
 __global__ void __launch_bounds__(1024) bce_logits_kernel(const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ part, long long n,
                                                           float scale) {
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(1024) bce_logits_kernel(const float* __restric
 #pragma unroll 4
   for (long long i = n0 + threadIdx.x; i < n1; i += 1024) {
     const float v = x[i];
-    s += (fmaxf(v, 0.f) - v * y[i]) + log1pf(expf(-fabsf(v)));
+    s += isinf(v) ? (1.0f - y[i]) * v - fminf(v, 0.f) : (fmaxf(v, 0.f) - v * y[i]) + log1pf(expf(-fabsf(v)));
   }
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
