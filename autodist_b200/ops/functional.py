@@ -790,6 +790,8 @@ class _PairLookupFn(torch.autograd.Function):
         dgmf, dx = dgmf.float(), dx.to(torch.bfloat16).contiguous()
         if dgmf.stride(1) != 1 or dgmf.stride(0) % 4 or dgmf.data_ptr() % 16:
             dgmf = dgmf.clone(memory_format=torch.contiguous_format)
+        if dx.data_ptr() % 8:                       # a slice: the kernel reads four values at once
+            dx = dx.clone()
         E.pair_lookup_bwd(dgmf, dx, kept, users, items, *into)
         grads = []
         for t, g, d in zip(ctx.tables, into, direct):
