@@ -1026,10 +1026,10 @@ bool copy_list(const std::vector<Tensor>& dst, const std::vector<Tensor>& src) {
   }
   if (dst.empty()) return true;
   const c10::cuda::CUDAGuard guard(dst[0].device());
-  for (size_t at = 0; at < dst.size(); at += adb200::kMaxCopies) {
+  for (size_t i = 0; i < dst.size();) {
     adb200::CopyList c{};
     long long blocks = 0;
-    for (size_t i = at; i < dst.size() && c.n < adb200::kMaxCopies; ++i) {
+    for (; i < dst.size() && c.n < adb200::kMaxCopies; ++i) {
       const long long bytes = (long long)dst[i].numel() * dst[i].element_size();
       if (bytes == 0 || dst[i].data_ptr() == src[i].data_ptr()) continue;
       c.src[c.n] = src[i].data_ptr(); c.dst[c.n] = dst[i].data_ptr(); c.bytes[c.n] = bytes;
