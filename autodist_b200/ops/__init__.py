@@ -24,6 +24,12 @@ def _dgrad_launches(dy, w, dx, stride, pad, *_):
                if any((ph + pad - r) % stride == 0 for r in range(kh)) and any((pw + pad - s) % stride == 0 for s in range(kw)))
 
 
+def _copy_list_launches(taken, dst, src):
+    """One launch per sixteen pairs that have something to copy; none when the list was refused."""
+    full = sum(1 for d, s in zip(dst, src) if d.numel() and d.data_ptr() != s.data_ptr()) if taken else 0
+    return (full + 15) // 16
+
+
 class _Counting:
     """Thin proxy over the extension module that counts kernel-launching calls."""
     _NO_LAUNCH = {"ln_bwd_part_floats", "sampled_grad_chunks", "sampled_bias_chunks", "bce_logits_parts", "colsum_parts", "gemm_choice", "gemm_set_trace", "conv_set_trace", "MAX_COMM_BLOCKS"}
@@ -34,6 +40,9 @@ class _Counting:
               "xent": lambda *a: 2 if a[7] else 1,                                                                           # sums the weights
               "sampled_logits": 2, "sampled_grad": 2, "sampled_bias_grad": 2, "conv_dgrad": _dgrad_launches}
 
+    #: kernels per call where that depends on what the call returned
+    _AFTER = {"copy_list": _copy_list_launches}
+
     def __init__(self, mod):
         self._mod = mod
         for name in dir(mod):
@@ -41,9 +50,18 @@ class _Counting:
                 continue
             attr = getattr(mod, name)
             if callable(attr) and name not in self._NO_LAUNCH:
-                setattr(self, name, self._wrap(attr, self._MULTI.get(name, 1)))
+                setattr(self, name, self._wrap_after(attr, self._AFTER[name]) if name in self._AFTER else self._wrap(attr, self._MULTI.get(name, 1)))
             else:
                 setattr(self, name, attr)
+
+    @staticmethod
+    def _wrap_after(fn, launches):
+        def call(*args):
+            global launch_count
+            result = fn(*args)
+            launch_count += launches(result, *args)
+            return result
+        return call
 
     @staticmethod
     def _wrap(fn, n):
