@@ -247,10 +247,10 @@ GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t e
   }
   return choose_gemm(M, N, K, batch, pair, !softmax_epi, epilogue, both_mn, fp32_out);
 }
-// (tile width, contraction split) of gemm(..., bn = 0) for a product of these extents: 512 is the two-CTA kernel. Products of two
-// MN-major operands are weight gradients, whose output is fp32.
-std::tuple<int64_t, int64_t> gemm_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn) {
-  const GemmChoice g = auto_choice(M, N, K, batch, epilogue, both_mn, both_mn);
+// (tile width, contraction split) of gemm(..., bn = 0) for a product of these extents: 512 is the two-CTA kernel. fp32_out: the type of
+// the output; where it is not given, that of a weight gradient (fp32) for two MN-major operands and bf16 for others.
+std::tuple<int64_t, int64_t> gemm_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn, const optional<bool>& fp32_out) {
+  const GemmChoice g = auto_choice(M, N, K, batch, epilogue, both_mn, fp32_out.value_or(both_mn));
   return {g.bn, g.split};
 }
 
@@ -1167,7 +1167,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_set_trace", &gemm_set_trace);
   m.def("gemm", &gemm);
   m.def("gemm_split", &gemm_split);
-  m.def("gemm_choice", &gemm_choice);
+  m.def("gemm_choice", &gemm_choice, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("batch"), py::arg("epilogue"), py::arg("both_mn"),
+        py::arg("fp32_out") = py::none());
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("gemm_softmax", &gemm_softmax);
