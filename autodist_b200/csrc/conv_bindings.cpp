@@ -137,6 +137,12 @@ int pixel_bn(int mode, long long patches, int cols, int kbs) {
   return best;
 }
 
+// A tile width asked for, or (0) the estimate's.
+int asked_bn(int64_t tile, int cols, int estimate) {
+  TORCH_CHECK(tile == 0 || tile == 64 || ((tile == 128 || tile == 256) && cols > tile / 2), "tile must be 64, 128 or 256 columns, at most half of them padding");
+  return tile == 0 ? estimate : (int)tile;
+}
+
 // Weight gradient: tile width and CTAs per output tile (each takes a share of the 64-pixel patches and adds its fp32 tile to the
 // output, whose L2 traffic is what limits the split). Earlier rule: the widest tile and as many CTAs as one wave holds;
 // 256 -> 1024 channels 1 x 1, 64 images of 14 x 14: 13.8 us, with 128 columns 10.9; 1024 -> 128, 16 images of 7 x 7: 8.8 and 5.0.
@@ -283,7 +289,7 @@ void set_eval_norm(adb200::ConvParams& p, const EvalNorm* n, const Tensor& y, in
 
 // y = conv(x, w) (+ bias) (ReLU); stats (optional, fp32 [2, Cout], zeroed by the caller) receives per-channel sum / sum of squares of y.
 void conv_fprop_impl(const Tensor& x, const Tensor& w, Tensor y, const optional<Tensor>& bias, bool relu, const optional<Tensor>& stats,
-                     int64_t stride, int64_t pad, Tensor error_flag, const EvalNorm* norm) {
+                     int64_t stride, int64_t pad, Tensor error_flag, const EvalNorm* norm, int64_t tile) {
   const c10::cuda::CUDAGuard guard(x.device());
   check_act(x, "x"); check_act(y, "y");
   const Geometry g = geometry(x, w, y, stride, pad);
@@ -294,7 +300,7 @@ void conv_fprop_impl(const Tensor& x, const Tensor& w, Tensor y, const optional<
   const Patch pt = choose_patch(GW, GH, GN, 128, false, false);
   set_grid(p, GW, GH, GN, pt);
   input_maps(maps, x, g, pt.tw, pt.th, pt.tn);
-  const int bn = pixel_bn(adb200::CONV_FPROP, (long long)p.tiles_w * p.tiles_h * p.tiles_n, g.Cout, g.KH * g.KW * ceil_div(g.Cin, 64));
+  const int bn = asked_bn(tile, g.Cout, pixel_bn(adb200::CONV_FPROP, (long long)p.tiles_w * p.tiles_h * p.tiles_n, g.Cout, g.KH * g.KW * ceil_div(g.Cin, 64)));
   maps.w = map4(w.data_ptr(), g.Cin, g.KH * g.KW, g.Cout, 1, g.Cin, (int64_t)g.Cin * g.KH * g.KW, (int64_t)g.Cin * g.KH * g.KW * g.Cout, 64, 1,
                 bn, 1);
   maps.dy = maps.w;
@@ -323,16 +329,16 @@ void conv_fprop_impl(const Tensor& x, const Tensor& w, Tensor y, const optional<
 }
 
 void conv_fprop(const Tensor& x, const Tensor& w, Tensor y, const optional<Tensor>& bias, bool relu, const optional<Tensor>& stats,
-                int64_t stride, int64_t pad, Tensor error_flag) {
-  conv_fprop_impl(x, w, y, bias, relu, stats, stride, pad, error_flag, nullptr);
+                int64_t stride, int64_t pad, Tensor error_flag, int64_t tile) {
+  conv_fprop_impl(x, w, y, bias, relu, stats, stride, pad, error_flag, nullptr, tile);
 }
 
 // y = relu?(batch_norm(conv(x, w) (+ bias)) (+ residual)) with running statistics (evaluation mode).
 void conv_fprop_bn_eval(const Tensor& x, const Tensor& w, Tensor y, const optional<Tensor>& bias, bool relu, const Tensor& gamma,
                         const Tensor& beta, const Tensor& mean, const Tensor& var, double eps, const optional<Tensor>& residual, int64_t stride,
-                        int64_t pad, Tensor error_flag) {
+                        int64_t pad, Tensor error_flag, int64_t tile) {
   const EvalNorm n{&gamma, &beta, &mean, &var, eps, &residual};
-  conv_fprop_impl(x, w, y, bias, relu, c10::nullopt, stride, pad, error_flag, &n);
+  conv_fprop_impl(x, w, y, bias, relu, c10::nullopt, stride, pad, error_flag, &n, tile);
 }
 
 // The same from and to logical [N, C, H, W] tensors (channels-last in memory, any float type in), with every check and allocation
@@ -364,13 +370,13 @@ optional<Tensor> conv_bn_eval_nchw(const Tensor& x, const Tensor& w, const optio
   const Tensor xh = x.permute({0, 2, 3, 1}).to(at::kBFloat16).contiguous();
   Tensor y = at::empty({x.size(0), oh, ow, cout}, xh.options());
   const EvalNorm n{&gamma, &beta, &mean, &var, eps, &res};
-  conv_fprop_impl(xh, w, y, bias, relu, c10::nullopt, stride, pad, error_flag, &n);
+  conv_fprop_impl(xh, w, y, bias, relu, c10::nullopt, stride, pad, error_flag, &n, 0);
   return y.permute({0, 3, 1, 2});
 }
 
 // dx = the input gradient of conv(x, w) given dy. Every element of dx is written.
 void conv_dgrad(const Tensor& dy, const Tensor& w, Tensor dx, int64_t stride, int64_t pad, Tensor error_flag,
-                const c10::optional<Tensor>& addend) {
+                const c10::optional<Tensor>& addend, int64_t tile) {
   const c10::cuda::CUDAGuard guard(dy.device());
   check_act(dy, "dy"); check_act(dx, "dx");
   if (addend.has_value()) {
@@ -438,13 +444,13 @@ void conv_dgrad(const Tensor& dy, const Tensor& w, Tensor dx, int64_t stride, in
       maps.out = grid_map(p.out, off, g.Cin, p, sw, sh, sn);
       maps.add = p.addend != nullptr ? grid_map(p.addend, off, g.Cin, p, sw, sh, sn) : maps.out;
       p.error_flag = error_flag.data_ptr<int>();
-      launch(maps, p, pixel_bn(adb200::CONV_DGRAD, (long long)p.tiles_w * p.tiles_h * p.tiles_n, g.Cin, n * ceil_div(g.Cout, 64)));
+      launch(maps, p, asked_bn(tile, g.Cin, pixel_bn(adb200::CONV_DGRAD, (long long)p.tiles_w * p.tiles_h * p.tiles_n, g.Cin, n * ceil_div(g.Cout, 64))));
     }
 }
 
 // dw (fp32 [Cout, KH, KW, Cin]) = the weight gradient of conv(x, w) given dy: overwritten, or added to with `accumulate`
 // (the parameter's gradient buffer, cleared once per step by its owner).
-void conv_wgrad(const Tensor& dy, const Tensor& x, Tensor dw, int64_t stride, int64_t pad, Tensor error_flag, bool accumulate) {
+void conv_wgrad(const Tensor& dy, const Tensor& x, Tensor dw, int64_t stride, int64_t pad, Tensor error_flag, bool accumulate, int64_t tile, int64_t ksplit) {
   const c10::cuda::CUDAGuard guard(dy.device());
   check_act(dy, "dy"); check_act(x, "x");
   TORCH_CHECK(dw.dim() == 4 && dw.scalar_type() == at::kFloat && dw.is_contiguous(), "dw must be contiguous fp32 [Cout, KH, KW, Cin]");
@@ -470,7 +476,10 @@ void conv_wgrad(const Tensor& dy, const Tensor& x, Tensor dw, int64_t stride, in
   maps.w = maps.dy;
   p.ntaps = forward_taps(p.taps, g);
   p.Nc = g.Cin; p.Kc = 0; p.Mc = g.Cout;
-  const GradSplit gs = grad_split(ceil_div(g.Cout, 128), g.Cin, p.ntaps, (long long)p.tiles_w * p.tiles_h * p.tiles_n, dw.numel() * 4e-6);
+  const long long patches = (long long)p.tiles_w * p.tiles_h * p.tiles_n;
+  GradSplit gs = grad_split(ceil_div(g.Cout, 128), g.Cin, p.ntaps, patches, dw.numel() * 4e-6, asked_bn(tile, g.Cin, 0));
+  TORCH_CHECK(ksplit >= 0 && ksplit <= patches, "at most one CTA per 64-pixel patch");
+  if (ksplit > 0) gs.ksplit = (int)ksplit;
   p.ksplit = gs.ksplit;
   p.accumulate = (p.ksplit > 1 || accumulate) ? 1 : 0;
   if (p.accumulate && !accumulate) dw.zero_();
@@ -621,15 +630,20 @@ void conv_rowtap_wgrad(const Tensor& dy, const Tensor& xp, Tensor dwr, int64_t s
 }  // namespace
 
 void register_conv(pybind11::module& m) {
+  namespace py = pybind11;
+  // tile: columns of a tile (64, 128, 256), 0: by estimate; ksplit: CTAs per output tile of the weight gradient, 0: by estimate
   m.def("conv_set_trace", &conv_set_trace);
-  m.def("conv_fprop", &conv_fprop);
-  m.def("conv_fprop_bn_eval", &conv_fprop_bn_eval);
+  m.def("conv_fprop", &conv_fprop, py::arg("x"), py::arg("w"), py::arg("y"), py::arg("bias"), py::arg("relu"), py::arg("stats"), py::arg("stride"),
+        py::arg("pad"), py::arg("error_flag"), py::arg("tile") = 0);
+  m.def("conv_fprop_bn_eval", &conv_fprop_bn_eval, py::arg("x"), py::arg("w"), py::arg("y"), py::arg("bias"), py::arg("relu"), py::arg("gamma"),
+        py::arg("beta"), py::arg("mean"), py::arg("var"), py::arg("eps"), py::arg("residual"), py::arg("stride"), py::arg("pad"), py::arg("error_flag"),
+        py::arg("tile") = 0);
   m.def("conv_bn_eval_nchw", &conv_bn_eval_nchw);
   m.def("conv_rowtap_fprop_bn_eval", &conv_rowtap_fprop_bn_eval);
-  namespace py = pybind11;
   m.def("conv_dgrad", &conv_dgrad, py::arg("dy"), py::arg("w"), py::arg("dx"), py::arg("stride"), py::arg("pad"), py::arg("error_flag"),
-        py::arg("addend") = py::none());
-  m.def("conv_wgrad", &conv_wgrad);
+        py::arg("addend") = py::none(), py::arg("tile") = 0);
+  m.def("conv_wgrad", &conv_wgrad, py::arg("dy"), py::arg("x"), py::arg("dw"), py::arg("stride"), py::arg("pad"), py::arg("error_flag"),
+        py::arg("accumulate"), py::arg("tile") = 0, py::arg("ksplit") = 0);
   m.def("conv_rowtap_fprop", &conv_rowtap_fprop);
   m.def("conv_rowtap_wgrad", &conv_rowtap_wgrad);
 }
