@@ -17,6 +17,7 @@
 #include "elementwise.h"
 #include "gemm_tcgen05.h"
 #include "sampled_softmax.h"
+#include "sm_count.h"
 
 void register_conv(pybind11::module& m);
 
@@ -42,15 +43,7 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-int num_sms() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return n;
-}
+int num_sms() { return adb200::sm_count(); }
 
 Tensor as4d(const Tensor& t) {
   TORCH_CHECK(t.dim() >= 2 && t.dim() <= 4, "operand must have 2 to 4 dimensions");

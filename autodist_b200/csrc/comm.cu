@@ -30,6 +30,7 @@
 #include <stdint.h>
 
 #include "comm.h"
+#include "sm_count.h"
 
 namespace adb200 {
 namespace {
@@ -554,7 +555,7 @@ void launch_reduce_scatter_update(const SymCtx& c, float* const* grads, __nv_bfl
 // 8192 rows of 512 in 32 blocks 25 us (gather) / 42 us (scatter-add), with a warp per row under 8 and 9.
 static int row_blocks(long long nrows) {
   const long long b = (nrows + 7) / 8;
-  return (int)(b < 1 ? 1 : (b < 148 * 32 ? b : 148 * 32));
+  return (int)(b < 1 ? 1 : (b < sm_count() * 32 ? b : sm_count() * 32));
 }
 
 void launch_sparse_scatter_add(const SymCtx& c, float* const* shard, uint8_t* const* touched, const int64_t* ids, const void* vals,

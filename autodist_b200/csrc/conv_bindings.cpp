@@ -12,6 +12,7 @@
 #include <mutex>
 
 #include "conv_tcgen05.h"
+#include "sm_count.h"
 
 namespace {
 
@@ -35,15 +36,7 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  }
-  return n;
-}
+using adb200::sm_count;
 
 // 4-D bf16 map, 128-byte swizzle, zero fill outside. dims / strides in elements, innermost stride 1.
 CUtensorMap map4(const void* base, int64_t d0, int64_t d1, int64_t d2, int64_t d3, int64_t s1, int64_t s2, int64_t s3, int b0, int b1,

@@ -15,6 +15,7 @@
 #include "elementwise.h"
 #include "eval_norm.cuh"
 #include "pdl.cuh"
+#include "sm_count.h"
 
 namespace adb200 {
 namespace {
@@ -2155,7 +2156,7 @@ inline int blocks_for(long long n, int per) { return (int)((n + per - 1) / per);
 void ln_fwd(const bf16* x, const bf16* res, const float* gamma, const float* beta, bf16* z, bf16* y, float* mean, float* rstd,
             int rows, int H, float eps, float p_drop, uint64_t seed, const long long* step, cudaStream_t st) {
   if (rows <= 0) return;
-  const int blocks = blocks_for(rows, kLnWarps) < 148 * 8 ? blocks_for(rows, kLnWarps) : 148 * 8;
+  const int blocks = blocks_for(rows, kLnWarps) < sm_count() * 8 ? blocks_for(rows, kLnWarps) : sm_count() * 8;
   auto kern = H <= 256 ? ln_fwd_kernel<1> : (H <= 512 ? ln_fwd_kernel<2> : (H <= 768 ? ln_fwd_kernel<3> : ln_fwd_kernel<4>));
   launch_pdl(kern, dim3(blocks), dim3(32 * kLnWarps), 0, st, x, res, gamma, beta, z, y, mean, rstd, rows, H, eps, p_drop, seed, step);
 }
@@ -2166,7 +2167,7 @@ void ln_bwd(const bf16* dy, const bf16* z, const float* mean, const float* rstd,
             bf16* dx, float* part, float* dgamma, float* dbeta, float* dsum, int rows, int H, float p_drop, uint64_t seed,
             const long long* step, int accumulate, cudaStream_t st) {
   // as many blocks as the SMs hold at once, so that a warp keeps several rows (a block's per-column sums are written once)
-  const int most = 148 * ln_bwd_resident((H + 255) / 256), want = blocks_for(rows, kLnWarps);
+  const int most = sm_count() * ln_bwd_resident((H + 255) / 256), want = blocks_for(rows, kLnWarps);
   const int blocks = want < 1 ? 1 : (want < most ? want : most);
   auto kern = H <= 256 ? ln_bwd_kernel<1> : (H <= 512 ? ln_bwd_kernel<2> : (H <= 768 ? ln_bwd_kernel<3> : ln_bwd_kernel<4>));
   launch_pdl(kern, dim3(blocks), dim3(32 * kLnWarps), 0, st, dy, z, mean, rstd, gamma, dz_add, dz, dx, part, rows, H, p_drop, seed, step, dsum != nullptr);
@@ -2272,7 +2273,7 @@ void add_bf16(const bf16* a, const bf16* b, bf16* out, long long n, cudaStream_t
 void adam_update(float* p, const float* g, float* m, float* v, bf16* p16, long long n, const float* lr, float b1, float b2,
                  float eps, float wd, int decoupled, const long long* step, float grad_scale, cudaStream_t st) {
   const long long groups = (n / 4 + 1) / 2 + 1;
-  const int blocks = (int)((groups + 255) / 256 < 148 * 16 ? (groups + 255) / 256 : 148 * 16);
+  const int blocks = (int)((groups + 255) / 256 < sm_count() * 16 ? (groups + 255) / 256 : sm_count() * 16);
   launch_pdl(adam_kernel, dim3(blocks < 1 ? 1 : blocks), dim3(256), 0, st, p, g, m, v, p16, n, lr, b1, b2, eps, wd, decoupled, step, grad_scale);
 }
 template <class Rule>
@@ -2281,7 +2282,7 @@ void flat_update(float* p, const float* g, float* state, bf16* p16, long long n,
   const int vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(state)) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(p16) & 7) == 0;
   const long long threads = vec ? (n / 4 + 1) / 2 + 1 : n;
-  const int blocks = (int)((threads + 255) / 256 < 148 * 16 ? (threads + 255) / 256 : 148 * 16);
+  const int blocks = (int)((threads + 255) / 256 < sm_count() * 16 ? (threads + 255) / 256 : sm_count() * 16);
   launch_pdl(flat_update_kernel<Rule>, dim3(blocks), dim3(256), 0, st, p, g, state, p16, n, lr, rule, vec);
 }
 void sgd_update(float* p, const float* g, float* mom, bf16* p16, long long n, const float* lr, float momentum, float dampening,
@@ -2304,7 +2305,7 @@ void flagged_rows_update(float* p, float* s1, float* s2, bf16* p16, float* g, ui
   const uintptr_t at = reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(s1) | reinterpret_cast<uintptr_t>(s2);
   const int vec = H % 4 == 0 && (at & 15) == 0 && (reinterpret_cast<uintptr_t>(p16) & 7) == 0;
   long long blocks = (rows + 31) / 32;           // one group of four flags per lane and a warp per 128 rows, up to eight blocks per SM
-  if (blocks > 148 * 8) blocks = 148 * 8;
+  if (blocks > sm_count() * 8) blocks = sm_count() * 8;
   auto kern = kind == 0 ? flagged_rows_update_kernel<0> : (kind == 1 ? flagged_rows_update_kernel<1> : flagged_rows_update_kernel<2>);
   launch_pdl(kern, dim3((int)blocks), dim3(256), 0, st, p, s1, s2, p16, g, flags, rows, H, lr, b1, b2, eps, step, vec);
 }
@@ -2343,7 +2344,7 @@ int bn_parts(int rows, int C) {
 dim3 bn_grid(long long rows, int C, int per_sm) {
   const int c8 = C / 8, tpr = c8 < kBnThreads ? c8 : kBnThreads, rpb = kBnThreads / tpr, gy = (c8 + kBnThreads - 1) / kBnThreads;
   long long blocks = (rows + (long long)rpb * kBnUnroll - 1) / ((long long)rpb * kBnUnroll);
-  const long long cap = (148 * per_sm + gy - 1) / gy;
+  const long long cap = (sm_count() * per_sm + gy - 1) / gy;
   if (blocks > cap) blocks = cap;
   return dim3((unsigned)(blocks < 1 ? 1 : blocks), (unsigned)gy);
 }
@@ -2363,7 +2364,7 @@ void bn_fwd(const bf16* x, const float* gamma, const float* beta, const bf16* re
   const float unbias = rows > 1 ? (float)rows / (float)(rows - 1) : 1.0f;
   if (!sums_given) bn_sums(x, part, sums, rows, C, st);
   dim3 grid = bn_grid(rows, C, 3);
-  if ((grid.x + 1) * grid.y <= 148 * 3 || grid.x == 1) grid.x += 1;      // the block of the statistics, within the same wave
+  if ((grid.x + 1) * grid.y <= sm_count() * 3 || grid.x == 1) grid.x += 1;      // the block of the statistics, within the same wave
   launch_pdl(bn_apply_kernel, grid, dim3(kBnThreads), 0, st, x, res, y, relu ? keep : nullptr, (long long)rows, C, relu, sums, gamma, beta,
              1.0f / rows, eps, mean, rstd, run_mean, run_var, batches, momentum, unbias);
 }
