@@ -41,7 +41,9 @@ __global__ void sampled_prep_kernel(const float* __restrict__ bias, const int64_
     return;
   }
   const float f = (float)id;
-  corrections[i] = make_float2(bias[id], logf(__fmul_rn(logf(__fdiv_rn(f + 2.0f, f + 1.0f)) * inv_log_v, num_sampled)));
+  // from 2^20 on the quotient's distance from 1 has few digits, from 2^24 on none; smaller ids keep it, and with it their results
+  const float step = f < 1048576.0f ? logf(__fdiv_rn(f + 2.0f, f + 1.0f)) : log1pf(__fdiv_rn(1.0f, f + 1.0f));
+  corrections[i] = make_float2(bias[id], logf(__fmul_rn(__fmul_rn(step, inv_log_v), num_sampled)));
   ids[i] = (int)id;
 }
 

@@ -12,7 +12,7 @@ import torch
 from torch import nn
 import torch.nn.functional as F
 
-from autodist_b200.ops.functional import linear, lstm_layer, sampled_softmax_of, sparse_lookup
+from autodist_b200.ops.functional import linear, log_uniform_steps, lstm_layer, sampled_softmax_of, sparse_lookup
 
 
 @dataclass
@@ -39,8 +39,7 @@ def log_uniform_sample(num_sampled, vocab, generator=None, device="cpu"):
 
 
 def log_uniform_prob(ids, vocab):
-    idf = ids.float()
-    return torch.log((idf + 2.0) / (idf + 1.0)) / math.log(vocab + 1.0)
+    return log_uniform_steps(ids) / math.log(vocab + 1.0)
 
 
 class LM1B(nn.Module):

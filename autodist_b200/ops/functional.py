@@ -890,11 +890,17 @@ def _ordered():
     return os.environ.get("AUTODIST_DETERMINISTIC") == "1" or torch.are_deterministic_algorithms_enabled()
 
 
+def log_uniform_steps(ids):
+    """``log((i + 2) / (i + 1))`` in fp32. Ids from 2^20 on take ``log1p(1 / (i + 1))``: the quotient's distance from 1 has few digits there and
+    none from 2^24 on, where its logarithm would be 0. Smaller ids keep the quotient, and with it the results of vocabularies that size."""
+    f = ids.float()
+    return torch.where(f < 2.0 ** 20, torch.log((f + 2.0) / (f + 1.0)), torch.log1p(1.0 / (f + 1.0)))
+
+
 def _sampled_chain(neg_logits, dot, bias, neg, targets, num_sampled):
     """What the sampled-softmax kernels compute, as PyTorch expressions (the log-softmax and the mean are theirs too)."""
     def correction(ids):
-        f = ids.float()
-        return torch.log(num_sampled * (torch.log((f + 2.0) / (f + 1.0)) / math.log(bias.numel() + 1.0)))
+        return torch.log(num_sampled * (log_uniform_steps(ids) / math.log(bias.numel() + 1.0)))
     own = dot.float() + bias[targets] - correction(targets)
     others = neg_logits.float() + bias[neg] - correction(neg)
     others = others.masked_fill(neg[None, :] == targets[:, None], -1e9)     # remove accidental hits
