@@ -124,26 +124,22 @@ void gemm_set_trace(const optional<Tensor>& t) {
 }
 
 // Which kernel runs a product: the tile width (512: the two-CTA kernel) and how many CTAs share the contraction of one tile.
-//
-// The two are chosen apart. A width changes no bit of the result: every kernel adds the products of an output in ascending order of
-// K. The number of shares does, since each share is summed by itself; what is rounded to bf16 behind the product then differs by an
-// ulp here and there, and a recurrence of such products carries that on (LM1B's gradients over 20 LSTM steps: 4e-4 of their norm
-// from one split to another). So the shares come from an estimate whose constants stay as they are, and only the width from
-// constants that follow the kernels.
-//
-// Both estimates are in microseconds: launch + fill + K blocks of 64 + drain, and per further wave of tiles its K blocks or the
-// drain of a tile, whichever is longer. Splitting adds the exchange through distributed shared memory; it wins wherever the tiles
-// leave SMs idle (256 x 256 x 16384 94.7 -> 14.7 us, 640 x 1024 x 30522 172 -> 39). Splits run one cluster per tile, so they are
-// only considered while every cluster is resident at once.
-//
-// Widths: a K block costs more the more SMs take part (`load`): their fills share the L2. The drain counts by kind (plain; bias or
-// addend; activation; fp32 output): 64 and 128 columns store directly and read what they need when they need it, wider tiles go
-// through shared memory and TMA. The constants are fitted to 170 products from 32 x 128 x 1000 to 8192 x 4096 x 1024 and 4096 x 25088 x 32
-// with every tile width (B200, replayed back to back). Where the lines lie, in us:
+// The estimate in microseconds is launch + fill + first wave's K blocks of 64 + last drain, plus, per further wave of tiles, its K
+// blocks or the drain of a tile, whichever is longer. A K block costs more the more SMs take part (`load`): their fills share the L2.
+// The drain counts by kind (plain; bias or addend; activation; fp32 output): 64 and 128 columns store directly and read what they
+// need when they need it, wider tiles go through shared memory and TMA. Splitting the contraction adds the exchange through
+// distributed shared memory; it wins wherever the tiles leave SMs idle (256 x 256 x 16384 94.7 -> 14.7 us, 640 x 1024 x 30522
+// 172 -> 39). Splits run one cluster per tile, so they are only considered while every cluster is resident at once.
+// The constants are fitted to 170 products from 32 x 128 x 1000 to 8192 x 4096 x 1024 and 4096 x 25088 x 32 with every tile width and
+// split (B200, replayed back to back): the estimates' choices take 0.6 % more time in sum than the fastest kernel of each product.
+// Where the lines lie, in us:
 //   192 columns fill the SMs where 256 leave a third of them idle (128 x 192 tiles and 256 x 256 pairs):
 //     3072 x 1024 x 4096 20.0 (pairs 25.5), 4096 x 768 x 3072 16.2 (20.8), 1792 x 3072 x 768 with GELU 13.9 (15.7)
 //   pairs win once there are waves of them: 4096 x 4096 x 1024 with GELU 32.8 (192 columns 38.4), 8192 x 1024 x 4096 52.8 (68.9)
 //   256 columns on one CTA in between: 4096 x 1024 x 1024 10.1 (pairs 11.3, 192 columns 12.8)
+//
+// A width changes no bit of the result: every kernel adds the products of an output in ascending order of K. The number of shares
+// does, since each share is summed by itself. See fixed_shares for products whose sums must not move with these constants.
 struct GemmChoice { int64_t bn, split; };
 struct GemmTiles { int64_t tiles, slots; };              // output tiles of a width, and how many of them run at once
 // false: the width does not suit the product
@@ -157,9 +153,55 @@ bool gemm_tiles(int bn, int64_t M, int64_t N, int64_t batch, bool allow_pair, Ge
 }
 bool gemm_split_fits(int64_t tiles, int s) { return tiles * s <= num_sms() && tiles <= adb200::gemm_split_max_clusters(s, (int)num_sms()); }
 
-// How many CTAs share the contraction: what the fastest kernel of the estimate would take, over 60 products from 512 x 128 x 128 to
-// 32 x 4096 x 25088.
-int choose_split(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, int64_t epilogue, bool both_mn) {
+// shares: how many CTAs have to share the contraction; 0: as many as the estimate says.
+GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split, int64_t epilogue, bool both_mn, bool fp32_out,
+                       int shares) {
+  struct Cost { int bn; double base, kb, load, mn, epi[4], wave, exchange; };      // exchange 0: no split of this width
+  static const Cost costs[5] = {{64, 2.87, 0.143, 0.17, 1.03, {1.3, 2.6, 3.5, 4.2}, 0.4, 2.0},
+                                {128, 3.35, 0.169, 0.31, 1.00, {2.8, 5.2, 6.8, 7.9}, 0.4, 2.0},
+                                {192, 3.16, 0.238, 0.18, 0.96, {3.4, 3.7, 5.7, 5.0}, 1.2, 0.0},
+                                {256, 3.29, 0.310, 0.31, 0.98, {4.0, 4.3, 6.4, 6.4}, 1.1, 5.0},
+                                {512, 4.24, 0.281, 0.22, 0.97, {4.0, 5.0, 6.7, 6.7}, 0.4, 0.0}};
+  const int kind = fp32_out ? 3 : (epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_ADD || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2));
+  const int64_t kbs = (K + 63) / 64, sms = num_sms();
+  // Inside a step, where neighbours run beside a product, launching clusters costs more than back to back, and so do the many epilogue
+  // warps of a wide tile on a nearly empty GPU: a split has to be estimated that much faster, and 192 and 256 columns are
+  // considered where they fill close to half of the SMs (tiny BERT 377 -> 360 us, base tied 3757 -> 3660). In several waves of long
+  // contractions the widest tiles read the least from memory, which matters when the operands are not in the L2: narrower ones are
+  // left out there.
+  const double margin = shares > 0 ? 0.0 : 0.8;
+  GemmChoice best{64, shares > 0 ? shares : 1};
+  double best_us = 1e30;
+  for (const Cost& c : costs) {
+    GemmTiles t;
+    if (!gemm_tiles(c.bn, M, N, batch, allow_pair, &t)) continue;
+    const double extra = c.epi[kind] - c.epi[0];                       // the last wave's drain (the plain one is part of the base)
+    auto blocks = [&](int64_t ctas, int64_t n) { return c.kb * (both_mn ? c.mn : 1.0) * (1.0 + c.load * std::min(1.0, (double)ctas / (double)t.slots)) * (double)n; };
+    const bool sparse = (c.bn == 192 || c.bn == 256) && 2 * t.tiles < sms - 20;
+    const bool narrow = c.bn < 256 && N > 128 && t.tiles > sms && K > 1024;
+    // long weight gradients stay on pairs, whose idle SMs run the optimizer beside them: 3072 x 1024 x 4096 alone 27 -> 21 us with 192
+    // columns, but the BERT-large step 12.26 -> 12.35 ms
+    const bool beside = c.bn == 192 && fp32_out && K > 2048;
+    if (shares <= 1 && !sparse && !narrow && !beside) {
+      const double waves = (double)((t.tiles + t.slots - 1) / t.slots);
+      const double us = c.base + (waves - 1) * std::max(blocks(t.tiles, kbs) + c.wave, c.epi[kind]) + blocks(t.tiles, kbs) + extra;
+      if (us < best_us) { best_us = us; best = {c.bn, 1}; }
+    }
+    if (c.exchange == 0.0 || !allow_split || shares == 1) continue;
+    for (int s = shares > 1 ? shares : 2; s <= (shares > 1 ? shares : 8) && s <= kbs; ++s) {
+      if (!gemm_split_fits(t.tiles, s)) continue;
+      const double us = c.base + blocks(t.tiles * s, (kbs + s - 1) / s) + c.exchange + extra / s;
+      if (us < best_us - margin) { best_us = us; best = {c.bn, s}; }
+    }
+  }
+  return best;
+}
+
+// Shares of a contraction for products that ask for them with bn = -1: an estimate over 60 products from 512 x 128 x 128 to
+// 32 x 4096 x 25088 whose constants stay as they are, whatever the kernels and the estimate above become. What is rounded to bf16 behind a
+// product changes by an ulp here and there with the order of its sums; a recurrence carries that on (LM1B's gradients over 20 LSTM steps:
+// 4e-4 of their norm from one number of shares to another), so the LSTM layer and what its gradient comes from ask for these.
+int fixed_shares(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, int64_t epilogue, bool both_mn) {
   struct Cost { int bn; double base, kb, epi[3], exchange; };
   static const Cost costs[4] = {{64, 2.9, 0.30, {1.6, 2.0, 3.6}, 2.6},
                                 {128, 4.2, 0.33, {2.7, 3.4, 7.5}, 2.6},
@@ -186,49 +228,11 @@ int choose_split(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair
   return best;
 }
 
-GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, bool allow_split, int64_t epilogue, bool both_mn, bool fp32_out) {
-  struct Cost { int bn; double base, kb, load, mn, epi[4], wave; bool splits; };
-  static const Cost costs[5] = {{64, 2.87, 0.143, 0.17, 1.03, {1.3, 2.6, 3.5, 4.2}, 0.4, true},
-                                {128, 3.35, 0.169, 0.31, 1.00, {2.8, 5.2, 6.8, 7.9}, 0.4, true},
-                                {192, 3.16, 0.238, 0.18, 0.96, {3.4, 3.7, 5.7, 5.0}, 1.2, false},
-                                {256, 3.29, 0.310, 0.31, 0.98, {4.0, 4.3, 6.4, 6.4}, 1.1, true},
-                                {512, 4.24, 0.281, 0.22, 0.97, {4.0, 5.0, 6.7, 6.7}, 0.4, false}};
-  const int kind = fp32_out ? 3 : (epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_ADD || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2));
-  const int64_t kbs = (K + 63) / 64, sms = num_sms();
-  const int split = allow_split ? choose_split(M, N, K, batch, allow_pair, epilogue, both_mn) : 1;
-  GemmChoice best{64, split};
-  double best_us = 1e30;
-  for (const Cost& c : costs) {
-    GemmTiles t;
-    if (!gemm_tiles(c.bn, M, N, batch, allow_pair, &t)) continue;
-    const double extra = c.epi[kind] - c.epi[0];                       // the last wave's drain (the plain one is part of the base)
-    auto blocks = [&](int64_t ctas, int64_t n) { return c.kb * (both_mn ? c.mn : 1.0) * (1.0 + c.load * std::min(1.0, (double)ctas / (double)t.slots)) * (double)n; };
-    double us;
-    if (split > 1) {
-      if (!c.splits || !gemm_split_fits(t.tiles, split)) continue;
-      us = c.base + blocks(t.tiles * split, (kbs + split - 1) / split) + (c.bn == 256 ? 5.0 : 2.0) + extra / split;
-    } else {
-      // Inside a step, where neighbours run beside a product, the many epilogue warps of a wide tile cost more on a nearly empty GPU than
-      // back to back: 192 and 256 columns are considered where they fill close to half of the SMs. In several waves of long contractions
-      // the widest tiles read the least from memory, which matters when the operands are not in the L2.
-      if ((c.bn == 192 || c.bn == 256) && 2 * t.tiles < sms - 20) continue;
-      if (c.bn < 256 && N > 128 && t.tiles > sms && K > 1024) continue;
-      // long weight gradients stay on pairs, whose idle SMs run the optimizer beside them: 3072 x 1024 x 4096 alone 27 -> 21 us with 192
-      // columns, but the BERT-large step 12.26 -> 12.35 ms
-      if (c.bn == 192 && fp32_out && K > 2048) continue;
-      const double waves = (double)((t.tiles + t.slots - 1) / t.slots);
-      us = c.base + (waves - 1) * std::max(blocks(t.tiles, kbs) + c.wave, c.epi[kind]) + blocks(t.tiles, kbs) + extra;
-    }
-    if (us < best_us) { best_us = us; best.bn = c.bn; }
-  }
-  return best;
-}
-
 // The kernel that bn = 0 asks for. AUTODIST_GEMM_PAIR=0 rules the two-CTA kernel out. AUTODIST_GEMM_PAIR_MIN_K sets a fixed rule
 // for it in place of the estimate: products with a pair's tile in both extents whose tiles fill the SM pairs, or whose contraction
 // is at least that long.
 bool g_pair_unavailable = false;               // set when a cluster launch was refused once (see gemm_impl)
-GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn, bool fp32_out) {
+GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn, bool fp32_out, bool fixed) {
   static const bool pair_default = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR"); return e == nullptr || e[0] != '0'; }();
   static const int64_t pair_min_k = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR_MIN_K"); return e != nullptr ? std::atoll(e) : -1LL; }();
   const bool softmax_epi = epilogue == adb200::EPI_SOFTMAX || epilogue == adb200::EPI_SOFTMAX_GRAD;
@@ -238,12 +242,14 @@ GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t e
     if (M >= 256 && N >= 256 && (pair_tiles >= num_sms() / 2 || K >= pair_min_k)) return {512, 1};
     pair = false;
   }
-  return choose_gemm(M, N, K, batch, pair, !softmax_epi, epilogue, both_mn, fp32_out);
+  const int shares = fixed && !softmax_epi ? fixed_shares(M, N, K, batch, pair, epilogue, both_mn) : 0;
+  return choose_gemm(M, N, K, batch, pair, !softmax_epi, epilogue, both_mn, fp32_out, shares);
 }
 // (tile width, contraction split) of gemm(..., bn = 0) for a product of these extents: 512 is the two-CTA kernel. fp32_out: the type of
-// the output; where it is not given, that of a weight gradient (fp32) for two MN-major operands and bf16 for others.
-std::tuple<int64_t, int64_t> gemm_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn, const optional<bool>& fp32_out) {
-  const GemmChoice g = auto_choice(M, N, K, batch, epilogue, both_mn, fp32_out.value_or(both_mn));
+// the output; where it is not given, that of a weight gradient (fp32) for two MN-major operands and bf16 for others. fixed: of bn = -1.
+std::tuple<int64_t, int64_t> gemm_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn, const optional<bool>& fp32_out,
+                                         bool fixed) {
+  const GemmChoice g = auto_choice(M, N, K, batch, epilogue, both_mn, fp32_out.value_or(both_mn), fixed);
   return {g.bn, g.split};
 }
 
@@ -261,11 +267,11 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
   TORCH_CHECK(c.size(0) == a.size(0) && c.size(1) == a.size(1) && c.size(2) == M && c.size(3) == N, "output shape mismatch");
   TORCH_CHECK(c.stride(3) == 1, "output inner stride must be 1");
   // bn: tile width 64 / 128 / 192 / 256 of the one-CTA kernel, or 512 = the 256 x 256 tile of the two-CTA kernel; 0 picks the kernel
-  // (see choose_gemm and auto_choice)
+  // (see choose_gemm and auto_choice), -1 only its tile, with the contraction shared as fixed_shares says
   const bool softmax_epi = epilogue == adb200::EPI_SOFTMAX || epilogue == adb200::EPI_SOFTMAX_GRAD;
   const bool auto_bn = bn <= 0;
   if (auto_bn) {
-    const GemmChoice g = auto_choice(M, N, K, a.size(0) * a.size(1), epilogue, a_mn && b_mn, c.scalar_type() == at::kFloat);
+    const GemmChoice g = auto_choice(M, N, K, a.size(0) * a.size(1), epilogue, a_mn && b_mn, c.scalar_type() == at::kFloat, bn == -1);
     bn = g.bn;
     split = g.split;
   }
@@ -1161,7 +1167,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm);
   m.def("gemm_split", &gemm_split);
   m.def("gemm_choice", &gemm_choice, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("batch"), py::arg("epilogue"), py::arg("both_mn"),
-        py::arg("fp32_out") = py::none());
+        py::arg("fp32_out") = py::none(), py::arg("fixed") = false);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("gemm_softmax", &gemm_softmax);

@@ -89,7 +89,7 @@ class LM1B(nn.Module):
         neg = log_uniform_sample(c.num_sampled, c.vocab_size, gen, x.device)
         true_w = sparse_lookup(self.softmax_w, targets).to(dt)
         neg_w = sparse_lookup(self.softmax_w, neg).to(dt)
-        products = linear(out, neg_w)                                          # [B*T, 512] x [8192, 512]^T on the tcgen05 GEMM
+        products = linear(out, neg_w, fixed_shares=True)      # [B*T, 512] x [8192, 512]^T on the tcgen05 GEMM
         dot = (out * true_w).sum(1)
         loss = sampled_softmax_of(products, dot, self.softmax_b, neg, targets, c.num_sampled)
         if loss is not None:

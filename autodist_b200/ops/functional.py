@@ -54,9 +54,13 @@ def check_errors():
             raise RuntimeError(f"a GEMM kernel on {dev} gave up waiting (code {code})")
 
 
+#: ``bn`` of a product whose sums must not depend on which kernel is the fastest: a recurrence carries an ulp on (see csrc/bindings.cpp)
+_FIXED_SHARES = -1
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, weight, bias, activation):
+    def forward(ctx, x, weight, bias, activation, bn):
         E = ops.ext(required=True)
         shape = x.shape
         x2 = x.reshape(-1, shape[-1]).to(torch.bfloat16).contiguous()
@@ -73,16 +77,16 @@ class _LinearFn(torch.autograd.Function):
         elif activation == "gelu":
             pre = torch.empty_like(y)
             E.gemm(x2, w16, pre, False, False, 2, b32 if b32 is not None else torch.zeros(weight.shape[0], device=x.device),
-                   y, None, 1.0, 0.0, err, 0)
+                   y, None, 1.0, 0.0, err, bn)
         elif b32 is not None:
-            E.gemm(x2, w16, y, False, False, 1, b32, None, None, 1.0, 0.0, err, 0)
+            E.gemm(x2, w16, y, False, False, 1, b32, None, None, 1.0, 0.0, err, bn)
         else:
-            E.gemm(x2, w16, y, False, False, 0, None, None, None, 1.0, 0.0, err, 0)
+            E.gemm(x2, w16, y, False, False, 0, None, None, None, 1.0, 0.0, err, bn)
         ctx.save_for_backward(x2, w16, pre)
         ctx.weight = weight
         _count_use(ctx, weight, 1)
         ctx.has_bias = bias is not None
-        ctx.shape = shape
+        ctx.shape, ctx.bn = shape, bn
         ctx.w_dtype = weight.dtype
         return y.view(*shape[:-1], weight.shape[0])
 
@@ -90,6 +94,7 @@ class _LinearFn(torch.autograd.Function):
     def backward(ctx, dy):
         E = ops.ext(required=True)
         x2, w16, pre = ctx.saved_tensors
+        bn = ctx.bn
         err = _error_flag(dy.device)
         dy2 = dy.reshape(-1, dy.shape[-1]).to(torch.bfloat16).contiguous()
         if pre is not None:
@@ -100,14 +105,14 @@ class _LinearFn(torch.autograd.Function):
         if ctx.gathered is not None:
             E.gemm_gathered_bt(dy2, ctx.gathered["ptrs"], ctx.gathered["rows"], w16.shape[1], dx, err)   # dX = dY . W, W from its owners
         else:
-            E.gemm(dy2, w16, dx, False, True, 0, None, None, None, 1.0, 0.0, err, 0)      # dX = dY . W
+            E.gemm(dy2, w16, dx, False, True, 0, None, None, None, 1.0, 0.0, err, bn)      # dX = dY . W
         acc = _direct_grad(ctx.weight)
         if acc is not None:
-            E.gemm(dy2, x2, acc, True, True, 0, None, None, None, 1.0, 1.0, err, 0)       # dW += dY^T . X, in the gradient buffer
+            E.gemm(dy2, x2, acc, True, True, 0, None, None, None, 1.0, 1.0, err, bn)       # dW += dY^T . X, in the gradient buffer
             dw = None
         else:
             dw = torch.empty(w16.shape, dtype=torch.float32, device=dy.device)
-            E.gemm(dy2, x2, dw, True, True, 0, None, None, None, 1.0, 0.0, err, 0)        # dW = dY^T . X
+            E.gemm(dy2, x2, dw, True, True, 0, None, None, None, 1.0, 0.0, err, bn)        # dW = dY^T . X
         db = None
         if ctx.has_bias:
             n = dy2.shape[1]
@@ -119,13 +124,14 @@ class _LinearFn(torch.autograd.Function):
                 db = dy2.float().sum(0)
         if dw is None:
             _grad_written(ctx.weight)
-        return dx.view(ctx.shape).to(dy.dtype), None if dw is None else dw.to(ctx.w_dtype), db, None
+        return dx.view(ctx.shape).to(dy.dtype), None if dw is None else dw.to(ctx.w_dtype), db, None, None
 
 
-def linear(x, weight, bias=None, activation=None):
-    """``activation(x @ weight.T + bias)`` with ``activation`` in ``{None, "gelu"}`` (tanh form)."""
+def linear(x, weight, bias=None, activation=None, fixed_shares=False):
+    """``activation(x @ weight.T + bias)`` with ``activation`` in ``{None, "gelu"}`` (tanh form). ``fixed_shares``: how many CTAs share a
+    contraction, and with it the order of its sums, does not follow the kernels' timings."""
     if x.is_cuda and x.shape[-1] % 8 == 0 and (weight.shape[0] % 8 == 0):
-        return _LinearFn.apply(x, weight, bias, activation)
+        return _LinearFn.apply(x, weight, bias, activation, _FIXED_SHARES if fixed_shares else 0)
     y = F.linear(x, weight.to(x.dtype), None if bias is None else bias.to(x.dtype))
     return F.gelu(y, approximate="tanh") if activation == "gelu" else y
 
@@ -191,9 +197,9 @@ class _LSTMLayerFn(torch.autograd.Function):
         c[0].zero_()
         hid = torch.empty(T, B, S, dtype=torch.bfloat16, device=dev)
         for t in range(T):
-            E.gemm(xh[t], w16, gates[t], False, False, 1, b32, None, None, 1.0, 0.0, err, 0)
+            E.gemm(xh[t], w16, gates[t], False, False, 1, b32, None, None, 1.0, 0.0, err, _FIXED_SHARES)
             E.lstm_seq_fwd(gates[t], c[t], c[t + 1], hid[t], forget_bias)
-            E.gemm(hid[t], p16, xh[t + 1, :, D:], False, False, 0, None, None, None, 1.0, 0.0, err, 0)
+            E.gemm(hid[t], p16, xh[t + 1, :, D:], False, False, 0, None, None, None, 1.0, 0.0, err, _FIXED_SHARES)
         ctx.save_for_backward(xh, gates, c, hid, w16, p16)
         ctx.params, ctx.fb, ctx.dims, ctx.x_dtype = (weight, bias, proj), forget_bias, (B, T, D, P, S), inputs.dtype
         for k, p in ((1, weight), (2, bias), (3, proj)):
@@ -216,9 +222,9 @@ class _LSTMLayerFn(torch.autograd.Function):
         dhid = torch.empty(B, S, dtype=torch.bfloat16, device=dev)
         dc = torch.empty(B, S, dtype=torch.float32, device=dev)
         for t in range(T - 1, -1, -1):
-            E.gemm(dxh[t + 1, :, D:], p16, dhid, False, True, 0, None, None, None, 1.0, 0.0, err, 0)
+            E.gemm(dxh[t + 1, :, D:], p16, dhid, False, True, 0, None, None, None, 1.0, 0.0, err, _FIXED_SHARES)
             E.lstm_seq_bwd(gates[t], c[t], c[t + 1], dhid, dc if t + 1 < T else None, dgates[t], dc, ctx.fb)
-            E.gemm(dgates[t], w16, dxh[t], False, True, 4, None, None, dxh[t], 1.0, 0.0, err, 0)
+            E.gemm(dgates[t], w16, dxh[t], False, True, 4, None, None, dxh[t], 1.0, 0.0, err, _FIXED_SHARES)
         rows = T * B
         dg2, x2, h2 = dgates.view(rows, 4 * S), xh[:T].view(rows, D + P), hid.view(rows, S)
         dh2 = dxh[1:].view(rows, D + P)[:, D:]
@@ -226,7 +232,7 @@ class _LSTMLayerFn(torch.autograd.Function):
         for p, a, b in ((weight, dg2, x2), (proj, dh2, h2)):
             acc = _direct_grad(p)
             g = acc if acc is not None else torch.empty(p.shape, dtype=torch.float32, device=dev)
-            E.gemm(a, b, g, True, True, 0, None, None, None, 1.0, 1.0 if acc is not None else 0.0, err, 0)
+            E.gemm(a, b, g, True, True, 0, None, None, None, 1.0, 1.0 if acc is not None else 0.0, err, _FIXED_SHARES)
             if acc is not None:
                 _grad_written(p)
             grads.append(None if acc is not None else g.to(p.dtype))

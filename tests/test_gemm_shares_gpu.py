@@ -1,5 +1,5 @@
-"""The sums of a product do not depend on the tile the chooser takes: every width adds in the same order, and the number of shares a
-contraction is cut into, which does decide that order, is a fixed function of the extents."""
+"""The sums of a product do not depend on the tile the chooser takes: every width adds in the same order. The number of shares a contraction is
+cut into does decide that order; products that ask for it (an LSTM's) get a fixed function of the extents."""
 import pytest
 import torch
 
@@ -29,7 +29,7 @@ def test_every_width_gives_the_same_bits(M, N, K, a_mn, b_mn):
         assert all(torch.equal(outs[0], c) for c in outs[1:])
 
 
-# the recurrence of an LSTM of 2048 cells, its weight gradients, an output projection, BERT layers and bias-like products
+# the recurrence of an LSTM of 2048 cells, its weight gradients, the products with sampled classes, and a long contraction
 @pytest.mark.parametrize("M,N,K,mn,shares", [(128, 8192, 1024, False, 1), (128, 512, 2048, False, 8), (128, 2048, 512, False, 1),
                                              (128, 1024, 8192, False, 8), (512, 2048, 2560, True, 4), (2560, 512, 8192, False, 3),
                                              (8192, 512, 2560, True, 1), (256, 256, 16384, False, 8)])
@@ -38,13 +38,13 @@ def test_shares_of_a_contraction(M, N, K, mn, shares):
     E = ops.ext(required=True)
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
         pytest.skip("the counts below are for 148 SMs")
-    bn, split = E.gemm_choice(M, N, K, 1, 0, mn)
+    bn, split = E.gemm_choice(M, N, K, 1, 0, mn, True, True)
     assert split == shares
     torch.manual_seed(K)
     a = torch.randn((K, M) if mn else (M, K), device="cuda").bfloat16()
     b = torch.randn((K, N) if mn else (N, K), device="cuda").bfloat16()
     got, want = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
-    E.gemm(a, b, got, mn, mn, 0, None, None, None, 1.0, 0.0, _err(), 0)
+    E.gemm(a, b, got, mn, mn, 0, None, None, None, 1.0, 0.0, _err(), -1)
     if shares > 1:
         E.gemm_split(a, b, want, mn, mn, 0, None, None, None, 1.0, 0.0, _err(), bn, shares)
     else:
