@@ -26,8 +26,10 @@ def _dgrad_launches(dy, w, dx, stride, pad, *_):
 
 def _copy_list_launches(taken, dst, src):
     """One launch per sixteen pairs that have something to copy; none when the list was refused."""
-    full = sum(1 for d, s in zip(dst, src) if d.numel() and d.data_ptr() != s.data_ptr()) if taken else 0
-    return (full + 15) // 16
+    if not taken:
+        return 0
+    full = (1 for d, s in zip(dst, src) if d.numel() and d.data_ptr() != s.data_ptr())
+    return next(full, 0) if len(dst) <= 16 else (sum(full) + 15) // 16        # (a step's time: the first pair settles a short list)
 
 
 class _Counting:

@@ -27,6 +27,7 @@ from torch import nn
 
 from autodist_b200.kernel.common import op_info
 from autodist_b200.kernel.synchronization.compressor import Compressor
+from autodist_b200.ops import functional
 from autodist_b200.utils import logging
 
 warnings.filterwarnings("ignore", message="Sparse invariant checks")
@@ -197,8 +198,7 @@ class StepEngine:
     def raise_reported(self):
         """Raises for bad input that kernels have reported to the host by now; does not wait for the device."""
         if self.device.type == "cuda":
-            from autodist_b200.ops.functional import raise_bad_ids
-            raise_bad_ids()
+            functional.raise_bad_ids()
 
     def train_step(self, train_op, nodes, feeds):
         self.before_read()
