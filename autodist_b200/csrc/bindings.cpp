@@ -139,7 +139,7 @@ void gemm_set_trace(const optional<Tensor>& t) {
 //   256 columns on one CTA in between: 4096 x 1024 x 1024 10.1 (pairs 11.3, 192 columns 12.8)
 //
 // A width changes no bit of the result: every kernel adds the products of an output in ascending order of K. The number of shares
-// does, since each share is summed by itself. See fixed_shares for products whose sums must not move with these constants.
+// does, since each share is summed by itself. See broad_choice for products whose sums must not move with these constants.
 struct GemmChoice { int64_t bn, split; };
 struct GemmTiles { int64_t tiles, slots; };              // output tiles of a width, and how many of them run at once
 // false: the width does not suit the product
@@ -197,11 +197,17 @@ GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allo
   return best;
 }
 
-// Shares of a contraction for products that ask for them with bn = -1: an estimate over 60 products from 512 x 128 x 128 to
-// 32 x 4096 x 25088 whose constants stay as they are, whatever the kernels and the estimate above become. What is rounded to bf16 behind a
-// product changes by an ulp here and there with the order of its sums; a recurrence carries that on (LM1B's gradients over 20 LSTM steps:
-// 4e-4 of their norm from one number of shares to another), so the LSTM layer and what its gradient comes from ask for these.
-int fixed_shares(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, int64_t epilogue, bool both_mn) {
+// An older and broader estimate, over 60 products from 512 x 128 x 128 to 32 x 4096 x 25088, hot and cold. Its constants stay as they are,
+// whatever the kernels and the estimate above become, for the sake of the first of the two things it decides:
+// 1. Shares of a contraction for products that ask for them with bn = -1. What is rounded to bf16 behind a product changes by an ulp here and
+//    there with the order of its sums; a recurrence carries that on (LM1B's gradients over 20 LSTM steps: 4e-4 of their norm from one number
+//    of shares to another), so the LSTM layer and what its gradient comes from ask for these.
+// 2. Everything for long contractions over operands whose rows do not start on 128-byte lines. Every box of such an operand lies on two lines
+//    per row, so fills cost more than the estimate above knows (a K block of 192 columns 0.48 us instead of 0.25), and it takes
+//    tiles that are too narrow and shares that are too few. Sums over random products, us, estimate above / this one / the fastest:
+//    K >= 4096 10587 / 10405 / 10366 (217 products; 33 of them more than 10 % slower than with this one), 2048 to 4096 1614 / 1588 / 1574 (84, 15),
+//    1024 to 2048 950 / 981 / 919, below 2105 / 2108 / 2026. Rows on lines: 10476 / 10607 / 10286 (594, K from 64 to 32000).
+GemmChoice broad_choice(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair, int64_t epilogue, bool both_mn) {
   struct Cost { int bn; double base, kb, epi[3], exchange; };
   static const Cost costs[4] = {{64, 2.9, 0.30, {1.6, 2.0, 3.6}, 2.6},
                                 {128, 4.2, 0.33, {2.7, 3.4, 7.5}, 2.6},
@@ -209,7 +215,7 @@ int fixed_shares(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair
                                 {512, 7.0, 0.41, {2.5, 3.7, 6.5}, 0.0}};
   const int kind = epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2);
   const int64_t kbs = (K + 63) / 64;
-  int best = 1;
+  GemmChoice best{64, 1};
   double best_us = 1e30;
   for (const Cost& c : costs) {
     GemmTiles t;
@@ -217,22 +223,24 @@ int fixed_shares(int64_t M, int64_t N, int64_t K, int64_t batch, bool allow_pair
     const double kb = c.bn == 128 && both_mn ? 0.42 : c.kb;
     const double extra = c.epi[kind] - c.epi[0], waves = (double)((t.tiles + t.slots - 1) / t.slots);
     const double us = c.base + (waves - 1) * std::max(kb * (double)kbs, c.epi[kind]) + kb * (double)kbs + extra;
-    if (us < best_us) { best_us = us; best = 1; }
+    if (us < best_us) { best_us = us; best = {c.bn, 1}; }
     if (c.exchange == 0.0) continue;
     for (int s = 2; s <= 8 && s <= kbs; ++s) {
       if (!gemm_split_fits(t.tiles, s)) continue;
       const double us_s = c.base + kb * (double)((kbs + s - 1) / s) + c.exchange + extra / s;
-      if (us_s < best_us) { best_us = us_s; best = s; }
+      if (us_s < best_us) { best_us = us_s; best = {c.bn, s}; }
     }
   }
   return best;
 }
+constexpr int64_t kLongContraction = 2048;
 
 // The kernel that bn = 0 asks for. AUTODIST_GEMM_PAIR=0 rules the two-CTA kernel out. AUTODIST_GEMM_PAIR_MIN_K sets a fixed rule
 // for it in place of the estimate: products with a pair's tile in both extents whose tiles fill the SM pairs, or whose contraction
 // is at least that long.
 bool g_pair_unavailable = false;               // set when a cluster launch was refused once (see gemm_impl)
-GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn, bool fp32_out, bool fixed) {
+GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn, bool fp32_out, bool fixed,
+                       bool off_lines) {
   static const bool pair_default = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR"); return e == nullptr || e[0] != '0'; }();
   static const int64_t pair_min_k = [] { const char* e = std::getenv("AUTODIST_GEMM_PAIR_MIN_K"); return e != nullptr ? std::atoll(e) : -1LL; }();
   const bool softmax_epi = epilogue == adb200::EPI_SOFTMAX || epilogue == adb200::EPI_SOFTMAX_GRAD;
@@ -242,14 +250,20 @@ GemmChoice auto_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t e
     if (M >= 256 && N >= 256 && (pair_tiles >= num_sms() / 2 || K >= pair_min_k)) return {512, 1};
     pair = false;
   }
-  const int shares = fixed && !softmax_epi ? fixed_shares(M, N, K, batch, pair, epilogue, both_mn) : 0;
-  return choose_gemm(M, N, K, batch, pair, !softmax_epi, epilogue, both_mn, fp32_out, shares);
+  if (!softmax_epi && (fixed || (off_lines && K >= kLongContraction))) {
+    const GemmChoice broad = broad_choice(M, N, K, batch, pair, epilogue, both_mn);
+    if (off_lines && K >= kLongContraction) return broad;
+    return choose_gemm(M, N, K, batch, pair, true, epilogue, both_mn, fp32_out, (int)broad.split);
+  }
+  return choose_gemm(M, N, K, batch, pair, !softmax_epi, epilogue, both_mn, fp32_out, 0);
 }
 // (tile width, contraction split) of gemm(..., bn = 0) for a product of these extents: 512 is the two-CTA kernel. fp32_out: the type of
-// the output; where it is not given, that of a weight gradient (fp32) for two MN-major operands and bf16 for others. fixed: of bn = -1.
+// the output; where it is not given, that of a weight gradient (fp32) for two MN-major operands and bf16 for others. fixed: of bn = -1. The operands'
+// rows follow one another.
 std::tuple<int64_t, int64_t> gemm_choice(int64_t M, int64_t N, int64_t K, int64_t batch, int64_t epilogue, bool both_mn, const optional<bool>& fp32_out,
                                          bool fixed) {
-  const GemmChoice g = auto_choice(M, N, K, batch, epilogue, both_mn, fp32_out.value_or(both_mn), fixed);
+  const bool off_lines = both_mn ? M % 64 != 0 && N % 64 != 0 : K % 64 != 0;
+  const GemmChoice g = auto_choice(M, N, K, batch, epilogue, both_mn, fp32_out.value_or(both_mn), fixed, off_lines);
   return {g.bn, g.split};
 }
 
@@ -267,11 +281,13 @@ void gemm_impl(const Tensor& a_, const Tensor& b_, Tensor c_, bool a_mn, bool b_
   TORCH_CHECK(c.size(0) == a.size(0) && c.size(1) == a.size(1) && c.size(2) == M && c.size(3) == N, "output shape mismatch");
   TORCH_CHECK(c.stride(3) == 1, "output inner stride must be 1");
   // bn: tile width 64 / 128 / 192 / 256 of the one-CTA kernel, or 512 = the 256 x 256 tile of the two-CTA kernel; 0 picks the kernel
-  // (see choose_gemm and auto_choice), -1 only its tile, with the contraction shared as fixed_shares says
+  // (see choose_gemm and auto_choice), -1 only its tile, with the contraction shared as broad_choice says
   const bool softmax_epi = epilogue == adb200::EPI_SOFTMAX || epilogue == adb200::EPI_SOFTMAX_GRAD;
   const bool auto_bn = bn <= 0;
   if (auto_bn) {
-    const GemmChoice g = auto_choice(M, N, K, a.size(0) * a.size(1), epilogue, a_mn && b_mn, c.scalar_type() == at::kFloat, bn == -1);
+    auto off_lines = [](const Tensor& t) { return t.stride(2) % 64 != 0 || reinterpret_cast<uintptr_t>(t.data_ptr()) % 128 != 0; };
+    const GemmChoice g = auto_choice(M, N, K, a.size(0) * a.size(1), epilogue, a_mn && b_mn, c.scalar_type() == at::kFloat, bn == -1,
+                                     off_lines(a) && off_lines(b));
     bn = g.bn;
     split = g.split;
   }

@@ -50,3 +50,26 @@ def test_shares_of_a_contraction(M, N, K, mn, shares):
     else:
         E.gemm(a, b, want, mn, mn, 0, None, None, None, 1.0, 0.0, _err(), 64)
     assert torch.equal(got, want)
+
+
+def test_long_contractions_over_rows_off_their_lines():
+    """Operands whose rows do not start on 128-byte lines cost more to fetch: wide tiles and many shares."""
+    from autodist_b200 import ops
+    E = ops.ext(required=True)
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the counts below are for 148 SMs")
+    assert E.gemm_choice(88, 3512, 31296, 1, 0, True) == (256, 8)
+    assert E.gemm_choice(2144, 176, 17480, 1, 2, False) == (256, 6)
+    assert E.gemm_choice(2376, 968, 5520, 1, 1, False) == (512, 1)
+    assert E.gemm_choice(1592, 1640, 12072, 1, 0, False) == (512, 1)
+    for M, N, K in ((176, 5456, 3912), (3072, 1024, 4096), (232, 232, 5512)):
+        torch.manual_seed(M)
+        a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+        bn, split = E.gemm_choice(M, N, K, 1, 0, False, True)
+        got, want = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+        E.gemm(a, b, got, False, False, 0, None, None, None, 1.0, 0.0, _err(), 0)
+        if split > 1:
+            E.gemm_split(a, b, want, False, False, 0, None, None, None, 1.0, 0.0, _err(), bn, split)
+        else:
+            E.gemm(a, b, want, False, False, 0, None, None, None, 1.0, 0.0, _err(), bn)
+        assert torch.equal(got, want)
