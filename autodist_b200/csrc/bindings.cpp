@@ -164,11 +164,16 @@ GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allo
                                 {512, 4.24, 0.281, 0.22, 0.97, {4.0, 5.0, 6.7, 6.7}, 0.4, 0.0}};
   const int kind = fp32_out ? 3 : (epilogue == adb200::EPI_NONE ? 0 : (epilogue == adb200::EPI_BIAS || epilogue == adb200::EPI_ADD || epilogue == adb200::EPI_BIAS_TANH ? 1 : 2));
   const int64_t kbs = (K + 63) / 64, sms = num_sms();
-  // Inside a step, where neighbours run beside a product, launching clusters costs more than back to back, and so do the many epilogue
-  // warps of a wide tile on a nearly empty GPU: a split has to be estimated that much faster, and 192 and 256 columns are
-  // considered where they fill close to half of the SMs (tiny BERT 377 -> 360 us, base tied 3757 -> 3660). In several waves of long
-  // contractions the widest tiles read the least from memory, which matters when the operands are not in the L2: narrower ones are
-  // left out there.
+  // Terms that the fit does not hold, with the sums over random products whose choice they decide, in us, with the term / without it,
+  // replayed on one set of operands; and on sets that do not fit the L2:
+  //   margin  a split has to be estimated that much faster: launching clusters costs more beside neighbours than back to back
+  //           24 products 158.7 / 163.3; 161.5 / 164.9
+  //   sparse  192 and 256 columns, whose epilogue has many warps, only where they fill close to half of the SMs
+  //           22 products 124.6 / 135.1; 127.3 / 141.9   (tiny BERT 377 -> 360 us, base tied 3757 -> 3660, with the margin)
+  //   narrow  in several waves of long contractions the widest tiles read the least from memory
+  //           22 products 939 / 919; 966 / 1015
+  //   beside  long weight gradients stay on pairs, whose idle SMs run the optimizer beside them; without one they pay for it
+  //           22 products 694 / 615; 704 / 695           (BERT-large step 12.26 ms / 12.35)
   const double margin = shares > 0 ? 0.0 : 0.8;
   GemmChoice best{64, shares > 0 ? shares : 1};
   double best_us = 1e30;
@@ -179,8 +184,6 @@ GemmChoice choose_gemm(int64_t M, int64_t N, int64_t K, int64_t batch, bool allo
     auto blocks = [&](int64_t ctas, int64_t n) { return c.kb * (both_mn ? c.mn : 1.0) * (1.0 + c.load * std::min(1.0, (double)ctas / (double)t.slots)) * (double)n; };
     const bool sparse = (c.bn == 192 || c.bn == 256) && 2 * t.tiles < sms - 20;
     const bool narrow = c.bn < 256 && N > 128 && t.tiles > sms && K > 1024;
-    // long weight gradients stay on pairs, whose idle SMs run the optimizer beside them: 3072 x 1024 x 4096 alone 27 -> 21 us with 192
-    // columns, but the BERT-large step 12.26 -> 12.35 ms
     const bool beside = c.bn == 192 && fp32_out && K > 2048;
     if (shares <= 1 && !sparse && !narrow && !beside) {
       const double waves = (double)((t.tiles + t.slots - 1) / t.slots);
