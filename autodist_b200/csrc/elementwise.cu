@@ -920,7 +920,8 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
   }
 }
 
-// One element of the updates with at most one state per weight: `p` and the state `s` in place.
+// One element of the updates with at most one state per weight: `p` and the state `s` in place. The roundings are spelled out, so that every
+// kernel gives a weight the same bits.
 struct SgdRule {
   float momentum, dampening, wd, grad_scale;
   int nesterov;
@@ -928,12 +929,12 @@ struct SgdRule {
   __device__ __forceinline__ bool state() const { return momentum != 0.f; }
   __device__ __forceinline__ bool first() const { return state() && *step_ptr <= 1; }       // the state starts as the first gradient
   __device__ __forceinline__ void operator()(float& p, float g, float& s, float lr, bool first_step) const {
-    float gr = g * grad_scale + wd * p;
+    float gr = fmaf(g, grad_scale, wd * p);
     if (momentum != 0.f) {
-      s = first_step ? gr : momentum * s + (1.0f - dampening) * gr;
-      gr = nesterov ? gr + momentum * s : s;
+      s = first_step ? gr : fmaf(1.0f - dampening, gr, momentum * s);
+      gr = nesterov ? fmaf(momentum, s, gr) : s;
     }
-    p = p - lr * gr;
+    p = fmaf(-lr, gr, p);
   }
 };
 struct AdagradRule {
@@ -941,27 +942,47 @@ struct AdagradRule {
   __device__ __forceinline__ bool state() const { return true; }
   __device__ __forceinline__ bool first() const { return false; }
   __device__ __forceinline__ void operator()(float& p, float g, float& s, float lr, bool) const {
-    const float gr = g * grad_scale + wd * p;
-    s = s + gr * gr;
+    const float gr = fmaf(g, grad_scale, wd * p);
+    s = fmaf(gr, gr, s);
     p = p - lr * gr / (sqrtf(s) + eps);
   }
 };
 
-// HBM-bound: 22 bytes per weight (with a state). `vec`: every buffer starts on a 16-byte boundary (8 for the bf16 copy); then a thread
-// has two 16-byte groups of each buffer in flight, as in adam_kernel. One weight per thread, the form for other bases, ran at
-// 0.57 of the copy rate (138 M weights of VGG-16 with momentum: 820 us in four launches, in groups 502, 0.92 of it).
+// HBM-bound: 22 bytes per weight (with a state). In groups (every buffer on a 16-byte boundary, 8 for the bf16 copy) a thread has two 16-byte
+// groups of each buffer in flight, as in adam_kernel: 138 M weights of VGG-16 with momentum 820 us -> 502 in four launches, 0.92 of
+// the copy rate. One weight per thread for other bases, and for few weights, where a thread's chain of eight roots and divisions
+// counts. us, momentum and Adagrad, one per thread / in groups: 4096 1.7, 1.8 / 2.0, 3.5; 524288 2.9, 3.7 / 3.3, 4.9; 1048576 5.1, 5.8 / 3.6, 5.4;
+// 4194304 17.8, 18.5 / 9.1, 15.2.
+constexpr long long kFlatGroupsLeast = 1 << 20;
+template <class Rule>
+__device__ __forceinline__ void flat_one(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ s, bf16* __restrict__ p16, long long i,
+                                         float lr, const Rule& rule, bool state, bool first) {
+  float pp = p[i], ss = state && !first ? s[i] : 0.f;
+  rule(pp, g[i], ss, lr, first);
+  p[i] = pp;
+  if (state) s[i] = ss;
+  if (p16) p16[i] = __float2bfloat16(pp);
+}
 template <class Rule>
 __global__ void flat_update_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ s, bf16* __restrict__ p16,
-                                   long long n, const float* __restrict__ lr_ptr, const Rule rule, int vec) {
+                                   long long n, const float* __restrict__ lr_ptr, const Rule rule) {
+  pdl_sync();
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) flat_one(p, g, s, p16, i, *lr_ptr, rule, rule.state(), rule.first());
+}
+template <class Rule>
+__global__ void __launch_bounds__(256, 4) flat_update_groups_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ s, bf16* __restrict__ p16,
+                                          long long n, const float* __restrict__ lr_ptr, const Rule rule) {
   pdl_sync();
   const float lr = *lr_ptr;
   const bool state = rule.state(), first = rule.first();
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
-  const long long nvec = vec ? n / 4 : 0;
-  for (long long q = tid; q < nvec; q += 2 * stride) {
-    float4 P[2], G[2], S[2];
+  const long long nvec = n / 4;
+  constexpr int U = 2;
+  for (long long q = tid; q < nvec; q += U * stride) {
+    float4 P[U], G[U], S[U];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < U; ++u) {
       const long long k = q + u * stride;
       S[u] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (k < nvec) {
@@ -971,7 +992,7 @@ __global__ void flat_update_kernel(float* __restrict__ p, const float* __restric
       }
     }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < U; ++u) {
       const long long k = q + u * stride;
       if (k >= nvec) continue;
       rule(P[u].x, G[u].x, S[u].x, lr, first);
@@ -986,13 +1007,7 @@ __global__ void flat_update_kernel(float* __restrict__ p, const float* __restric
       }
     }
   }
-  for (long long i = nvec * 4 + tid; i < n; i += stride) {
-    float pp = p[i], ss = state && !first ? s[i] : 0.f;
-    rule(pp, g[i], ss, lr, first);
-    p[i] = pp;
-    if (state) s[i] = ss;
-    if (p16) p16[i] = __float2bfloat16(pp);
-  }
+  if (tid < n - nvec * 4) flat_one(p, g, s, p16, nvec * 4 + tid, lr, rule, state, first);
 }
 
 // Row-sparse updates: only the rows that received a gradient are touched (rows must be unique, i.e. a coalesced
@@ -2279,11 +2294,14 @@ void adam_update(float* p, const float* g, float* m, float* v, bf16* p16, long l
 template <class Rule>
 void flat_update(float* p, const float* g, float* state, bf16* p16, long long n, const float* lr, const Rule& rule, cudaStream_t st) {
   if (n <= 0) return;
-  const int vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(state)) & 15) == 0 &&
-                  (reinterpret_cast<uintptr_t>(p16) & 7) == 0;
-  const long long threads = vec ? (n / 4 + 1) / 2 + 1 : n;
-  const int blocks = (int)((threads + 255) / 256 < sm_count() * 16 ? (threads + 255) / 256 : sm_count() * 16);
-  launch_pdl(flat_update_kernel<Rule>, dim3(blocks), dim3(256), 0, st, p, g, state, p16, n, lr, rule, vec);
+  const bool groups = n >= kFlatGroupsLeast && ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(state)) & 15) == 0 &&
+                      (reinterpret_cast<uintptr_t>(p16) & 7) == 0;
+  if (groups) {
+    const long long blocks = (n / 8 + 1 + 255) / 256, most = sm_count() * 16LL;
+    launch_pdl(flat_update_groups_kernel<Rule>, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, st, p, g, state, p16, n, lr, rule);
+  } else {
+    launch_pdl(flat_update_kernel<Rule>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, p, g, state, p16, n, lr, rule);
+  }
 }
 void sgd_update(float* p, const float* g, float* mom, bf16* p16, long long n, const float* lr, float momentum, float dampening,
                 float wd, int nesterov, const long long* step, float grad_scale, cudaStream_t st) {
