@@ -11,6 +11,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "elementwise.h"
 #include "eval_norm.cuh"
@@ -116,7 +117,10 @@ struct LnDrop {
 constexpr int kLnWarps = 4;              // warps (rows) per block
 
 // z = dropout(x) + residual is written back (it is what the backward pass needs), y = LN(z) * gamma + beta.
-template <int NV>
+// EARLY: gamma and beta are requested with the row, in 16 NV registers more, instead of behind the reductions. For few rows, where one
+// more latency counts and the registers do not: us, a block per row / late / early: 4 x 608 2.2 / 2.6 / 2.3,
+// 302 x 816 with dropout 2.9 / 3.5 / 2.9, 512 x 128 with dropout 2.3 / 2.3 / 2.1, 1184 x 1024 3.6 / 3.7 / 3.5; beyond two blocks per SM late ones.
+template <int NV, bool EARLY>
 __global__ void __launch_bounds__(32 * kLnWarps) ln_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, const float* __restrict__ gamma,
                               const float* __restrict__ beta, bf16* __restrict__ z, bf16* __restrict__ y,
                               float* __restrict__ mean, float* __restrict__ rstd, int rows, int H, float eps,
@@ -136,6 +140,16 @@ __global__ void __launch_bounds__(32 * kLnWarps) ln_fwd_kernel(const bf16* __res
         xq[k] = *reinterpret_cast<const uint4*>(x + off + 256 * k);
         if (res) rq[k] = *reinterpret_cast<const uint4*>(res + off + 256 * k);
       }
+    }
+    float4 gq[EARLY ? NV : 1][2], bq[EARLY ? NV : 1][2];
+    if (EARLY) {
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (lane * 8 + 256 * k < H) {
+          const float4* gp = reinterpret_cast<const float4*>(gamma + lane * 8 + 256 * k);
+          const float4* bp = reinterpret_cast<const float4*>(beta + lane * 8 + 256 * k);
+          gq[k][0] = gp[0]; gq[k][1] = gp[1]; bq[k][0] = bp[0]; bq[k][1] = bp[1];
+        }
     }
     const uint64_t counter = sd + (uint64_t)(off >> 2) * kGolden;
     float v[NV][8];
@@ -165,7 +179,9 @@ __global__ void __launch_bounds__(32 * kLnWarps) ln_fwd_kernel(const bf16* __res
         if (z) store8(z + off + 256 * k, v[k]);
         const float4* gp = reinterpret_cast<const float4*>(gamma + lane * 8 + 256 * k);
         const float4* bp = reinterpret_cast<const float4*>(beta + lane * 8 + 256 * k);
-        const float4 g0 = gp[0], g1 = gp[1], b0 = bp[0], b1 = bp[1];
+        constexpr int have = EARLY ? 1 : 0;
+        const float4 g0 = EARLY ? gq[k * have][0] : gp[0], g1 = EARLY ? gq[k * have][1] : gp[1];
+        const float4 b0 = EARLY ? bq[k * have][0] : bp[0], b1 = EARLY ? bq[k * have][1] : bp[1];
         const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
         float o[8];
 #pragma unroll
@@ -2172,7 +2188,11 @@ void ln_fwd(const bf16* x, const bf16* res, const float* gamma, const float* bet
             int rows, int H, float eps, float p_drop, uint64_t seed, const long long* step, cudaStream_t st) {
   if (rows <= 0) return;
   const int blocks = blocks_for(rows, kLnWarps) < sm_count() * 8 ? blocks_for(rows, kLnWarps) : sm_count() * 8;
-  auto kern = H <= 256 ? ln_fwd_kernel<1> : (H <= 512 ? ln_fwd_kernel<2> : (H <= 768 ? ln_fwd_kernel<3> : ln_fwd_kernel<4>));
+  auto pick = [&](auto early) {
+    constexpr bool E = decltype(early)::value;
+    return H <= 256 ? ln_fwd_kernel<1, E> : (H <= 512 ? ln_fwd_kernel<2, E> : (H <= 768 ? ln_fwd_kernel<3, E> : ln_fwd_kernel<4, E>));
+  };
+  auto kern = rows <= sm_count() * 2 * kLnWarps ? pick(std::true_type{}) : pick(std::false_type{});
   launch_pdl(kern, dim3(blocks), dim3(32 * kLnWarps), 0, st, x, res, gamma, beta, z, y, mean, rstd, rows, H, eps, p_drop, seed, step);
 }
 int ln_bwd_part_floats(int H) { return 3 * kLnSlots * H; }
