@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(32 * kLnWarps) ln_fwd_kernel(const bf16* __res
 // (sum of the output), slot = block % kLnSlots. `part` must be zero on entry; the reduction kernel that follows clears what it
 // reads, so the buffer is zero again afterwards.
 constexpr int kLnSlots = 16;
-constexpr int ln_bwd_resident(int nv) { return nv <= 2 ? 4 : (nv == 3 ? 3 : 2); }     // blocks per SM that hold 24 * nv sums per thread without spills
+constexpr int ln_bwd_resident(int nv) { return nv <= 2 ? 4 : (nv == 3 ? 3 : 2); }     // blocks per SM whose registers hold 24 * nv sums per thread (four bytes of 1024 columns are spilled)
 
 template <int NV>
 __global__ void __launch_bounds__(32 * kLnWarps, ln_bwd_resident(NV))
@@ -1612,7 +1612,7 @@ __global__ void __launch_bounds__(kBnThreads, 2) bn_eval_kernel(const bf16* __re
 //   dx = gamma * rstd * (dy' - dbeta / M - xhat * dgamma / M) = A * dy' + B * x + K per channel; coef = [A (C), B (C), K (C)]
 // together with sums = [dbeta (C), dgamma (C)], which are also added into dbeta_acc / dgamma_acc (the parameters'
 // gradient buffers) when those are given. `counters` ([C / 64]) and `part` ([kBnSlots, 2, C]) must be zero on entry and
-// are zero again on exit.
+// are zero again on exit. Four blocks per SM leave 64 registers a thread, of which 8 bytes are spilled.
 constexpr int kBnSlots = 16;
 constexpr int kBnCounterFloats = 256;          // ticket counters in front of the slots: one per 64 channels, C <= 16384
 
@@ -2342,7 +2342,7 @@ void flagged_rows_update(float* p, float* s1, float* s2, bf16* p16, float* g, ui
   if (rows <= 0) return;
   const uintptr_t at = reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(s1) | reinterpret_cast<uintptr_t>(s2);
   const int vec = H % 4 == 0 && (at & 15) == 0 && (reinterpret_cast<uintptr_t>(p16) & 7) == 0;
-  long long blocks = (rows + 31) / 32;           // one group of four flags per lane and a warp per 128 rows, up to eight blocks per SM
+  long long blocks = (rows + 31) / 32;           // a lane per group of four rows: spread over as many warps as there are groups, up to eight blocks per SM, then up to 32 groups a warp
   if (blocks > sm_count() * 8) blocks = sm_count() * 8;
   auto kern = kind == 0 ? flagged_rows_update_kernel<0> : (kind == 1 ? flagged_rows_update_kernel<1> : flagged_rows_update_kernel<2>);
   launch_pdl(kern, dim3((int)blocks), dim3(256), 0, st, p, s1, s2, p16, g, flags, rows, H, lr, b1, b2, eps, step, vec);

@@ -3,8 +3,10 @@
 // One persistent CTA per SM, warp-specialised:
 //   warp 0    TMA producer   cp.async.bulk.tensor (4-D tiled maps, 128-byte swizzle) into a ring of smem stages
 //   warp 1    MMA issuer     one lane issues tcgen05.mma (cta_group::1, kind::f16, 128 x BN x 16), accumulators in TMEM
-//   warps 2-5 epilogue       tcgen05.ld of the accumulator (two TMEM buffers, so tile i+1 is multiplied while tile i
-//                            is written), fused bias / GELU / GELU-derivative / scale, direct 32-byte row stores
+//   warps 2.. epilogue       tcgen05.ld of the accumulator (two TMEM buffers, so tile i+1 is multiplied while tile i
+//                            is written), fused bias / GELU / GELU-derivative / scale. Tiles of 64 and 128 columns have four
+//                            such warps, a row per thread and direct 32-byte row stores; 192 columns have twelve and 256 eight, which
+//                            stage the tile in shared memory for TMA stores (gemm_epilogue.cuh)
 //
 // Either operand may be K-major (contraction dimension contiguous in memory) or MN-major (the M or N dimension
 // contiguous): the backward GEMMs of a linear layer (dX = dY W, dW = dY^T X) and of attention read the same
@@ -35,7 +37,7 @@ template <int BN> struct Cfg {
   static constexpr int STAGES = BN == 256 ? 3 : (BN == 192 ? 4 : (BN == 128 ? 6 : 8));
   // Epilogue warps: four cover the TMEM lane quarters; the widest tile has eight, two per quarter with half of the columns each, and 192
   // columns twelve, three per quarter, because 128 threads cannot apply a bias or an activation to 32768 outputs in the time
-  // of one tile.
+  // of one tile. With 448 threads there are 128 registers for each: 192 columns spill 32 bytes (60 are read back).
   static constexpr bool WIDE = BN >= 192;
   static constexpr int EPI_GROUPS = BN == 256 ? 2 : 1;     // groups of 64 columns per epilogue warp of a wide tile
   static constexpr int EPI_WARPS = WIDE ? 4 * BN / (64 * EPI_GROUPS) : 4;
