@@ -1,22 +1,17 @@
-// Number of SMs of the current device, asked once per device.
+// Number of SMs of a GPU of this node, whose GPUs are alike: asked once, since an eager pass asks several times per layer and even the
+// question which device is current shows in its time (ResNet-50 evaluation, 9 images, bound by the host: 13 us of 930).
 #pragma once
 #include <cuda_runtime.h>
-
-#include <atomic>
 
 namespace adb200 {
 
 inline int sm_count() {
-  constexpr int kDevices = 64;
-  static std::atomic<int> known[kDevices];                 // 0: not asked yet
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return 148;
-  int n = known[dev].load(std::memory_order_relaxed);
-  if (n == 0) {
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
-    known[dev].store(n, std::memory_order_relaxed);
-  }
-  return n;
+  static const int known = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    return n;
+  }();
+  return known;
 }
 
 }  // namespace adb200
