@@ -270,18 +270,20 @@ class AutoDist:
         return self._create_distributed_session()
 
     def _shutdown(self):
-        if self._session is not None:
-            self._session.close()
-        if dist.is_initialized():
-            try:
-                dist.destroy_process_group()
-            except Exception as e:  # peers may already be gone
-                logging.debug("destroy_process_group: %s", e)
-        if self._coordinator is not None:
-            try:
-                self._coordinator.join(timeout=30)
-            except Exception as e:
-                logging.error("%s", e)
+        try:
+            if self._session is not None:
+                self._session.close()            # may raise for what the last steps reported; the rest is still wound up
+        finally:
+            if dist.is_initialized():
+                try:
+                    dist.destroy_process_group()
+                except Exception as e:  # peers may already be gone
+                    logging.debug("destroy_process_group: %s", e)
+            if self._coordinator is not None:
+                try:
+                    self._coordinator.join(timeout=30)
+                except Exception as e:
+                    logging.error("%s", e)
 
     # ------------------------------------------------------------------ function-style entry
     def _args_to_placeholders(self, args, kwargs):
