@@ -28,8 +28,13 @@ def _copy_list_launches(taken, dst, src):
     """One launch per sixteen pairs that have something to copy; none when the list was refused."""
     if not taken:
         return 0
-    full = (1 for d, s in zip(dst, src) if d.numel() and d.data_ptr() != s.data_ptr())
-    return next(full, 0) if len(dst) <= 16 else (sum(full) + 15) // 16        # (a step's time: the first pair settles a short list)
+    full = 0
+    for d, s in zip(dst, src):
+        if d.numel() and d.data_ptr() != s.data_ptr():
+            if len(dst) <= 16:
+                return 1                        # (a step's time: the first pair settles a short list)
+            full += 1
+    return (full + 15) // 16
 
 
 class _Counting:

@@ -38,8 +38,8 @@ def _id_flag(device):
 def raise_bad_ids():
     """Raises for ids outside their tables that kernels have reported so far, once each. Costs no wait."""
     for dev, (_, seen) in _id_flags.items():
-        code = int(seen[0])
-        if code:
+        if seen[0]:
+            code = int(seen[0])
             seen[0] = 0
             raise RuntimeError(f"{_ID_ERRORS.get(code, 'an id outside its table')} on {dev}: its row counted as zeros, the results are not valid")
 

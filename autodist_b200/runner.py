@@ -238,7 +238,6 @@ class WrappedSession:
 
     def _run(self, fetches, feed_dict, prefetch=None):
         rm, eng = self._remapper, self._engine
-        eng.raise_reported()                 # by a step whose results nobody fetched
         single = not isinstance(fetches, (list, tuple, dict))
         leaves, rebuild = rm.flatten_fetches([fetches] if single else fetches)
         kinds = [rm.classify(l) for l in leaves]
@@ -273,7 +272,7 @@ class WrappedSession:
                 if value.dtype == torch.bfloat16:
                     value = value.float()                       # numpy has no bfloat16
                 out[i] = np.array(value.cpu().numpy(), copy=True)   # a copy: never a view of live parameter memory
-        eng.raise_reported()                 # what was fetched is on the host, so this step has said what it had to say
+        eng.raise_reported()                 # what was fetched is on the host, so this step has said what it had to say; earlier ones too
         result = rebuild(out)
         return result[0] if single else result
 
